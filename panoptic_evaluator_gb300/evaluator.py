@@ -318,33 +318,48 @@ def panoptic_quality(prediction: PanopticBatch, target: PanopticBatch, num_class
     pred, pc, _ = _prepare(prediction, num_classes, ignore_crowd=True)
     if gt.shape != pred.shape or gt.device != pred.device:
         raise ValueError("prediction and target must share shape and device")
-    stats = reward_statistics(gt, pred, gc, pc, crowd, num_classes, _tables(target), _tables(prediction), validate)
+    statistics = reward_statistics(gt, pred, gc, pc, crowd, num_classes, _tables(target), _tables(prediction), validate)
     if return_stats:
-        return stats
-    return reward_scores(stats)
+        sums, tp, fp, fn = statistics
+        return torch.stack((sums, tp.double(), fp.double(), fn.double()), -1)
+    return reward_scores(*statistics)
 
 
 def reward_statistics(gt, pred, gc, pc, crowd, num_classes, gt_tables=(None, None), pred_tables=(None, None),
                       validate=True):
-    """[B, C, 4] (iou_sum, tp, fp, fn) per image, computed by one pe_update in reward mode."""
-    B, G, P = gt.shape[0], gc.shape[1], pc.shape[1]
+    """Per image [B, C]: IoU sums (float64) and tp, fp, fn (int64), computed by one pe_update in reward mode."""
+    B, G, P, C = gt.shape[0], gc.shape[1], pc.shape[1], num_classes
     device = gt.device
-    longs = torch.zeros((3, B, num_classes), dtype=torch.int64, device=device)
-    sums = torch.zeros((B, num_classes), dtype=torch.float64, device=device)
-    code = native.update(gt, pred, gc, pc, crowd,
-                         torch.empty((B, G, P), dtype=torch.int64, device=device),
-                         torch.empty((B, G + P), dtype=torch.int64, device=device),
-                         torch.empty((B, G), dtype=torch.int32, device=device),
-                         longs[0], longs[1], longs[2], sums, torch.empty(0, dtype=torch.int64, device=device),
-                         *gt_tables, *pred_tables, torch.zeros(1, dtype=torch.int32, device=device), validate,
-                         True)
+    rows = torch.zeros((4, B, C), dtype=torch.int64, device=device)  # 0.0 is the all-zero bit pattern
+    tp, fp, fn, sums = rows.unbind(0)
+    sums = sums.view(torch.float64)
+    # Scratch of the call in one allocation: pairs [B, G, P], areas [B, G + P], then int32 matched [B, G], error.
+    longs = B * (G * P + G + P)
+    work = torch.empty(longs + (B * G) // 2 + 1, dtype=torch.int64, device=device)
+    if gt_tables[0] is None and pred_tables[0] is None:
+        # Compact maps: checked by _prepare, so the C ABI is called without the extension shim's checks.
+        base, row = work.data_ptr(), rows.data_ptr()
+        matched = base + 8 * longs
+        with N.on_device(device):
+            code = N.call("pe_update", gt.data_ptr(), 0, pred.data_ptr(), 0, B, gt.shape[1] * gt.shape[2],
+                          gc.data_ptr(), pc.data_ptr(), crowd.data_ptr(), G, P, C, base, base + 8 * B * G * P, matched,
+                          row, row + 8 * B * C, row + 16 * B * C, row + 24 * B * C, None, None, None, None, None,
+                          matched + 4 * B * G, int(bool(validate)), 1, N.stream_handle(device))
+    else:
+        ints = work[longs:].view(torch.int32)
+        code = native.update(gt, pred, gc, pc, crowd, work[:B * G * P].view(B, G, P),
+                             work[B * G * P:longs].view(B, G + P), ints[:B * G].view(B, G), tp, fp, fn, sums,
+                             torch.empty(0, dtype=torch.int64, device=device), *gt_tables, *pred_tables,
+                             ints[B * G:B * G + 1], validate, True)
     raise_validation(code)
-    return torch.stack((sums, longs[0].double(), longs[1].double(), longs[2].double()), -1)
+    return sums, tp, fp, fn
 
 
-def reward_scores(stats):
-    """Mean over active classes of PQ per image (evaluator.py:539-544)."""
-    sums, tp, fp, fn = stats.unbind(-1)
-    denominator = tp + 0.5 * (fp + fn)
-    active = denominator > 0
-    return (sums / denominator.clamp_min(1)).sum(1) / active.sum(1).clamp_min(1)
+def reward_scores(sums, tp, fp, fn):
+    """Mean over active classes of PQ per image (evaluator.py:539-544), one kernel over the [B, C] statistics."""
+    B, C = tp.shape
+    scores = torch.empty(B, dtype=torch.float64, device=tp.device)
+    with N.on_device(tp.device):
+        N.call("pe_reward_pq", tp.data_ptr(), fp.data_ptr(), fn.data_ptr(), sums.data_ptr(), B, C, scores.data_ptr(),
+               None, None, None, None, N.stream_handle(tp.device))
+    return scores
