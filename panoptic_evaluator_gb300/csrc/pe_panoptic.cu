@@ -18,6 +18,7 @@
 #include "pe_common.cuh"
 #include "pe_score.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <map>
@@ -26,11 +27,13 @@
 namespace pe {
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int kHistThreads = 512;
 constexpr int kPixelsPerThread = 8;
 constexpr int kTilePixels = kHistThreads * kPixelsPerThread;
-constexpr int kScoreThreads = 256;
-constexpr int kComputeThreads = 1024;
+constexpr int kScoreThreads = 1024;
+constexpr size_t kScoreSmem = 200 * 1024;  // scoring tables and entry list of one image, at most
 constexpr int kMaxSmemBins = 50 * 1024;  // 200 KB of uint32 bins
 
 template <typename T>
@@ -162,7 +165,168 @@ pair_histogram(const GT* __restrict__ gt, const PR* __restrict__ pred, int64_t p
   if (bad && error) atomicOr(error, 1);
 }
 
-// flags: 1 = areas, 2 = validate (needs areas), 4 = accumulate, 8 = gate on *error.
+// Compact int32 maps (no lookup tables), 16 images of 640 x 640 with 101 x 121
+// bins: 28.7 -> 15.8 us (52 MB of maps, 7.8 us at the copy rate). Reading the maps is the floor; a CTA
+// reaches it only with loads in flight while it bins, so each thread holds the
+// next tile's pixels in registers (two CTAs per SM hold 64 KB of loads). Tiles start at the 16-byte word
+// holding the image's first pixel, so images of any pixel count keep 16-byte
+// loads as long as both maps have the same offset mod 16; threads reaching over
+// either end of the image, and maps of different offsets, load pixel by pixel.
+// Binning run by run cost 505 instructions per warp and tile and bounded the
+// kernel; counting the pixels equal to a lane's first or last key takes a fifth.
+template <bool SMEM>
+__global__ void __launch_bounds__(kHistThreads, 2)
+slot_histogram(const int* __restrict__ gt, const int* __restrict__ pred, int64_t pixels, int64_t B, int G, int P,
+               int64_t tiles_per_image, int64_t tiles_per_cta, u64* __restrict__ pairs, int* __restrict__ error) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  u32* bins = reinterpret_cast<u32*>(smem_raw);
+  const int bins_count = G * P;
+  const int64_t t_begin = (int64_t)blockIdx.x * tiles_per_cta;
+  const int64_t t_end = min(t_begin + tiles_per_cta, B * tiles_per_image);
+  const bool together = ((reinterpret_cast<uintptr_t>(gt) ^ reinterpret_cast<uintptr_t>(pred)) & 15) == 0;
+  bool bad = false;
+  int64_t current = -1;
+
+  auto flush = [&](int64_t image) {
+    __syncthreads();
+    u64* out = pairs + image * (int64_t)bins_count;
+    for (int k = threadIdx.x; k < bins_count; k += blockDim.x) {
+      const u32 v = bins[k];
+      if (v) atomicAdd(out + k, (u64)v);
+    }
+  };
+  struct Pixels {
+    int g[kPixelsPerThread], p[kPixelsPerThread];
+    u32 valid;  // bit j: pixel j lies inside the image
+  };
+  auto load = [&](int64_t t, Pixels& v) {
+    v.valid = 0;
+    if (t >= t_end) return;
+    const int64_t b = t / tiles_per_image;
+    const int* g = gt + b * pixels;
+    const int* p = pred + b * pixels;
+    const int shift = (int)((reinterpret_cast<uintptr_t>(g) >> 2) & 3);
+    const int64_t x = (t % tiles_per_image) * kTilePixels - shift + (int64_t)threadIdx.x * kPixelsPerThread;
+    if (together && x >= 0 && x + kPixelsPerThread <= pixels) {
+      v.valid = (1u << kPixelsPerThread) - 1;
+#pragma unroll
+      for (int k = 0; k < kPixelsPerThread / 4; ++k) {
+        const int4 a = __ldg(reinterpret_cast<const int4*>(g + x) + k);
+        const int4 c = __ldg(reinterpret_cast<const int4*>(p + x) + k);
+        v.g[4 * k] = a.x; v.g[4 * k + 1] = a.y; v.g[4 * k + 2] = a.z; v.g[4 * k + 3] = a.w;
+        v.p[4 * k] = c.x; v.p[4 * k + 1] = c.y; v.p[4 * k + 2] = c.z; v.p[4 * k + 3] = c.w;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < kPixelsPerThread; ++j) {
+        v.g[j] = v.p[j] = 0;
+        if (x + j >= 0 && x + j < pixels) {
+          v.valid |= 1u << j;
+          v.g[j] = __ldg(g + x + j);
+          v.p[j] = __ldg(p + x + j);
+        }
+      }
+    }
+  };
+  auto count = [&](int64_t t, const Pixels& v) {
+    const int64_t b = t / tiles_per_image;
+    if (SMEM && b != current) {
+      if (current >= 0) flush(current);
+      __syncthreads();
+      const uint4 zero = make_uint4(0, 0, 0, 0);
+      for (int k = threadIdx.x * 4; k < bins_count; k += blockDim.x * 4) *reinterpret_cast<uint4*>(bins + k) = zero;
+      __syncthreads();
+    }
+    current = b;
+    u64* out = pairs + b * (int64_t)bins_count;
+    auto add = [&](u32 key, u32 n) {
+      if (SMEM) atomicAdd(bins + key, n);
+      else atomicAdd(out + key, (u64)n);
+    };
+    constexpr u32 kFull = (1u << kPixelsPerThread) - 1;
+    u32 first = ~0u, n_first = 0;  // the lane's first key, combined over the warp
+    u32 g_max = 0, p_max = 0;
+#pragma unroll
+    for (int j = 0; j < kPixelsPerThread; ++j) {
+      g_max = max(g_max, (u32)v.g[j]);
+      p_max = max(p_max, (u32)v.p[j]);
+    }
+    if (v.valid == kFull && g_max < (u32)G && p_max < (u32)P) {
+      // Eight neighbouring pixels usually lie in one or two segment pairs: those equal to the first or
+      // the last pixel's key are counted, the others are added one by one (predicated, no branches).
+      u32 key[kPixelsPerThread];
+#pragma unroll
+      for (int j = 0; j < kPixelsPerThread; ++j) key[j] = (u32)(v.g[j] * P + v.p[j]);
+      const u32 last = key[kPixelsPerThread - 1];
+      first = key[0];
+      n_first = 1;
+      u32 n_last = 0;
+#pragma unroll
+      for (int j = 1; j < kPixelsPerThread; ++j) {
+        const bool a = key[j] == first, c = key[j] == last;
+        n_first += a;
+        n_last += !a && c;
+        if (!a && !c) add(key[j], 1);
+      }
+      if (n_last) add(last, n_last);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kPixelsPerThread; ++j) {
+        if (!((v.valid >> j) & 1u)) continue;
+        if ((u32)v.g[j] < (u32)G && (u32)v.p[j] < (u32)P) add((u32)(v.g[j] * P + v.p[j]), 1);
+        else bad = true;
+      }
+    }
+    const u32 peers = __match_any_sync(0xffffffffu, first);
+    const u32 total = __reduce_add_sync(peers, n_first);
+    if ((threadIdx.x & 31) == (u32)(__ffs(peers) - 1) && total) add(first, total);
+  };
+
+  Pixels ahead;
+  load(t_begin, ahead);
+  for (int64_t t = t_begin; t < t_end; ++t) {
+    const Pixels now = ahead;
+    load(t + 1, ahead);
+    count(t, now);
+  }
+  if (SMEM && current >= 0) flush(current);
+  if (bad && error) atomicOr(error, 1);
+}
+
+// flags: 1 = areas, 2 = validate (needs areas), 4 = accumulate, 8 = gate on *error. One CTA per image,
+// scored in one pass (pe_score.cuh); smem: dynamic shared memory of the launch.
+template <bool REWARD>
+__global__ void __launch_bounds__(1024)
+score_blocks(const u64* __restrict__ pairs, const int* __restrict__ gc, const int* __restrict__ pc,
+             const uint8_t* __restrict__ crowd, u64* __restrict__ areas, int* __restrict__ matched,
+             u64* __restrict__ tp, u64* __restrict__ fp, u64* __restrict__ fn, double* __restrict__ iou_sum,
+             u64* __restrict__ confusion, int G, int P, int C, int flags, int smem, int* __restrict__ error) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int64_t b = blockIdx.x;
+  if ((flags & 8) && *reinterpret_cast<volatile int*>(error)) return;
+  pairs += b * (int64_t)G * P;
+  gc += b * G;
+  pc += b * P;
+  crowd += b * G;
+  const int64_t o = REWARD ? b * C : 0;
+  const ScoreTables t = ScoreTables::at(smem_raw, G, P, C, smem);
+  score_totals(pairs, t, gc, crowd, G, P, C);
+  if (flags & 1) {
+    areas += b * (int64_t)(G + P);
+    for (int k = threadIdx.x; k < G; k += blockDim.x) areas[k] = t.row[k];
+    for (int k = threadIdx.x; k < P; k += blockDim.x) areas[G + k] = t.col[k];
+    if (flags & 2) {
+      const int err = score_checks<REWARD>(t, gc, pc, crowd, G, P, C);
+      if (err) atomicOr(error, err);
+    }
+  }
+  if (!(flags & 4)) return;
+  score_matches<u64, REWARD>(pairs, t, pc, G, P, C,
+                             ScoreOut{tp + o, fp + o, fn + o, iou_sum + o, REWARD ? nullptr : confusion});
+  for (int g = threadIdx.x; g < G; g += blockDim.x) matched[b * G + g] = t.matched[g];
+}
+
+// The same for images of 2^32 pixels and more (64-bit counts) or more slots than the tables above hold.
 template <bool REWARD>
 __global__ void __launch_bounds__(1024)
 score(const u64* __restrict__ pairs, const int* __restrict__ gc, const int* __restrict__ pc,
@@ -285,22 +449,30 @@ rgb_slots_kernel(const uint8_t* __restrict__ rgb, int64_t pixels, const int64_t*
 
 // Per-class PQ/SQ/RQ and semantic IoU, group means and mIoU for K rows of
 // statistics, plus independent copies of the inputs (compute_kernel.cu:9-63).
-// One CTA per row. The confusion matrix is read once, row-major and coalesced:
-// warp w takes rows w, w + 32, ..., reduces each row with shuffles and keeps
-// column partials in registers, added into shared column sums at the end of a
-// 256-column tile. FP64 runs only where a value is produced: one class per
-// thread for the per-class ratios, then one warp per summed quantity (fixed
-// order: lane-strided classes, then a butterfly), so no warp issues FP64 adds
-// of zeros (GB300's FP64 pipe runs at 1/64 of the FP32 rate).
+// One cluster of CL CTAs per row. Latency bounds it (one SM pulls 143 KB of
+// 64-bit confusion at 133 classes), so the CTAs of a cluster share the matrix's
+// rows, each read once, summed and copied from the same registers: a warp
+// reduces its rows with shuffles and keeps column partials in registers, which
+// meet in a shared [warp][column] buffer and then across the cluster through
+// distributed shared memory. FP64 runs only where a value is produced: one
+// class per thread for the per-class ratios (each CTA its share of classes),
+// then, in the first CTA, one warp per summed quantity (fixed order:
+// lane-strided classes, then a butterfly), so no warp issues FP64 adds of zeros
+// (GB300's FP64 pipe runs at 1/64 of the FP32 rate).
+constexpr int kComputeThreads = 512;
 constexpr int kComputeTile = 256;  // confusion columns per register tile (8 per lane)
+constexpr int kComputeCluster = 8;
+constexpr int kComputeClusterClasses = 64;
 
+template <int CL>
 __global__ void __launch_bounds__(kComputeThreads)
 compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, const int64_t* __restrict__ fn,
                const double* __restrict__ sums, const int64_t* __restrict__ confusion,
                const bool* __restrict__ things, double* per_class, double* summaries, int64_t* counts,
                double* miou, int64_t* out_tp, int64_t* out_fp, int64_t* out_fn, double* out_sums,
                int64_t* out_confusion, int C) {
-  const int64_t k = blockIdx.x;
+  const int64_t k = blockIdx.x / CL;
+  const int rank = blockIdx.x % CL;
   tp += k * C; fp += k * C; fn += k * C; sums += k * C;
   confusion += k * C * (int64_t)(C + 1);
   per_class += k * 4 * C;
@@ -311,112 +483,118 @@ compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, c
     out_confusion += k * C * (int64_t)(C + 1);
   }
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  int64_t* row_sum = reinterpret_cast<int64_t*>(smem_raw);  // C confusion row sums
-  int64_t* col_sum = row_sum + C;                            // C column sums
+  int64_t* row_sum = reinterpret_cast<int64_t*>(smem_raw);  // C confusion row sums (this CTA's rows)
+  int64_t* col_sum = row_sum + C;                            // C column sums over this CTA's rows
+  int64_t* partial = col_sum + C;                            // [warps][kComputeTile], before `value` is written
   double* value = reinterpret_cast<double*>(col_sum + C);    // [4][C]: pq, sq, rq, iou (NaN: no pixels)
   int* group = reinterpret_cast<int*>(value + 4 * C);        // C: 0 inactive, 1 thing, 2 stuff (active)
-  __shared__ double total[10];
-  __shared__ int n_group[3], n_iou;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, warps = blockDim.x >> 5;
-  for (int c = t; c < C; c += blockDim.x) row_sum[c] = col_sum[c] = 0;
-  if (t < 3) n_group[t] = 0;
-  if (t == 0) n_iou = 0;
-  // Snapshot copies (independent of everything below): 16-byte words when aligned.
-  if (out_tp) {
-    for (int c = t; c < C; c += blockDim.x) {
-      out_tp[c] = tp[c]; out_fp[c] = fp[c]; out_fn[c] = fn[c]; out_sums[c] = sums[c];
-    }
-    const int64_t n = (int64_t)C * (C + 1);
-    if (((reinterpret_cast<uintptr_t>(confusion) | reinterpret_cast<uintptr_t>(out_confusion)) & 15) == 0) {
-      const int4* src = reinterpret_cast<const int4*>(confusion);
-      int4* dst = reinterpret_cast<int4*>(out_confusion);
-      for (int64_t i = t; i < n / 2; i += blockDim.x) dst[i] = src[i];
-      if (t == 0 && (n & 1)) out_confusion[n - 1] = confusion[n - 1];
-    } else {
-      for (int64_t i = t; i < n; i += blockDim.x) out_confusion[i] = confusion[i];
-    }
-  }
+  const int r_begin = (int)((int64_t)C * rank / CL), r_end = (int)((int64_t)C * (rank + 1) / CL);
+  // This thread's (first) class: its counts are in flight while the matrix is read.
+  struct Class {
+    int64_t tp, fp, fn, diag;
+    double sum;
+  } cls = {};
+  auto load_class = [&](int c) {
+    if (c < r_end) cls = {tp[c], fp[c], fn[c], confusion[(int64_t)c * (C + 1) + c], sums[c]};
+  };
+  load_class(r_begin + t);
+  for (int c = r_begin + t; c < r_end; c += blockDim.x) row_sum[c] = 0;
   __syncthreads();
-  // Row and column sums in one coalesced pass over the confusion rows.
+  // Row and column sums, and the snapshot, in one coalesced pass over the confusion rows.
   for (int t0 = 0; t0 <= C; t0 += kComputeTile) {
+    const int width = min(kComputeTile, C + 1 - t0);
     int64_t acc[kComputeTile / 32];
 #pragma unroll
     for (int i = 0; i < kComputeTile / 32; ++i) acc[i] = 0;
-    for (int r = warp; r < C; r += warps) {
-      const int64_t* row = confusion + (int64_t)r * (C + 1);
-      int64_t part = 0;
+    for (int r = r_begin + warp; r < r_end; r += warps) {
+      const int64_t* src = confusion + (int64_t)r * (C + 1) + t0 + lane;
+      int64_t* dst = out_tp ? out_confusion + (int64_t)r * (C + 1) + t0 + lane : nullptr;
+      int64_t v[kComputeTile / 32], part = 0;
+#pragma unroll
+      for (int i = 0; i < kComputeTile / 32; ++i) v[i] = lane + 32 * i < width ? src[32 * i] : 0;
 #pragma unroll
       for (int i = 0; i < kComputeTile / 32; ++i) {
-        const int j = t0 + lane + 32 * i;
-        if (j <= C) {
-          const int64_t v = row[j];
-          part += v;
-          if (j < C) acc[i] += v;
-        }
+        part += v[i];
+        acc[i] += v[i];
+        if (dst && lane + 32 * i < width) dst[32 * i] = v[i];
       }
 #pragma unroll
       for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
       if (lane == 0) row_sum[r] += part;  // row r belongs to this warp alone
     }
 #pragma unroll
-    for (int i = 0; i < kComputeTile / 32; ++i) {
-      const int j = t0 + lane + 32 * i;
-      if (j < C && acc[i]) atomicAdd(reinterpret_cast<unsigned long long*>(col_sum + j), (unsigned long long)acc[i]);
+    for (int i = 0; i < kComputeTile / 32; ++i) partial[warp * kComputeTile + lane + 32 * i] = acc[i];
+    __syncthreads();
+    for (int j = t; j < width && t0 + j < C; j += blockDim.x) {
+      int64_t sum = 0;
+#pragma unroll 8
+      for (int w = 0; w < warps; ++w) sum += partial[w * kComputeTile + j];
+      col_sum[t0 + j] = sum;
     }
+    __syncthreads();
   }
-  __syncthreads();
+  cg::cluster_group cluster = cg::this_cluster();
+  if (CL > 1) cluster.sync();
+  double* value0 = CL > 1 ? cluster.map_shared_rank(value, 0) : value;
+  int* group0 = CL > 1 ? cluster.map_shared_rank(group, 0) : group;
   // Per-class ratios, one class per thread.
-  for (int c = t; c < C; c += blockDim.x) {
-    const int64_t a = tp[c], f = fp[c], n = fn[c];
-    const double s = sums[c];
+  for (int c = r_begin + t; c < r_end; c += blockDim.x) {
+    const int64_t a = cls.tp, f = cls.fp, n = cls.fn, diag = cls.diag;
+    const double s = cls.sum;
+    if (out_tp) { out_tp[c] = a; out_fp[c] = f; out_fn[c] = n; out_sums[c] = s; }
+    load_class(c + blockDim.x);
+    int64_t column = 0;
+#pragma unroll
+    for (int q = 0; q < CL; ++q) column += CL > 1 ? cluster.map_shared_rank(col_sum, q)[c] : col_sum[c];
     const double denom = (double)a + 0.5 * ((double)f + (double)n);
     const double pq = denom > 0 ? s / denom : 0.0;
     const double sq = a ? s / (double)a : 0.0;
     const double rq = denom > 0 ? (double)a / denom : 0.0;
-    const int64_t diag = confusion[(int64_t)c * (C + 1) + c];
-    const int64_t uni = row_sum[c] + col_sum[c] - diag;
+    const int64_t uni = row_sum[c] + column - diag;
     const double iou = uni ? (double)diag / (double)uni : __longlong_as_double(0x7ff8000000000000ll);
     per_class[c] = pq;
     per_class[C + c] = sq;
     per_class[2 * C + c] = rq;
     per_class[3 * C + c] = iou;
-    value[c] = pq;
-    value[C + c] = sq;
-    value[2 * C + c] = rq;
-    value[3 * C + c] = iou;
-    const int g = denom > 0 ? (things[c] ? 1 : 2) : 0;
-    group[c] = g;
-    if (g) { atomicAdd(&n_group[0], 1); atomicAdd(&n_group[g], 1); }
-    if (uni) atomicAdd(&n_iou, 1);
+    value0[c] = pq;
+    value0[C + c] = sq;
+    value0[2 * C + c] = rq;
+    value0[3 * C + c] = iou;
+    group0[c] = denom > 0 ? (things[c] ? 1 : 2) : 0;
   }
-  __syncthreads();
+  if (CL > 1) cluster.sync();
+  else __syncthreads();
+  if (rank) return;
   // Ten sums, one warp each: quantity q = 3 * scope + metric (scope 0 all, 1 things, 2 stuff), q = 9 IoU.
-  for (int q = warp; q < 10; q += warps) {
-    const int metric = q < 9 ? q % 3 : 3, scope = q < 9 ? q / 3 : 0;
+  if (warp < 10) {
+    const int q = warp, metric = q < 9 ? q % 3 : 3, scope = q < 9 ? q / 3 : 0;
     double part = 0.0;
+    int members = 0;
     for (int c = lane; c < C; c += 32) {
       const bool in = q < 9 ? (group[c] != 0 && (scope == 0 || group[c] == scope)) : !isnan(value[3 * C + c]);
       if (in) part += value[metric * C + c];
+      members += in;
     }
+    members = __reduce_add_sync(0xffffffffu, members);
 #pragma unroll
     for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) total[q] = part;
+    if (lane == 0) {
+      const double mean = members ? part / (double)members : 0.0;
+      if (q < 9) summaries[q] = mean;
+      else miou[k] = mean;
+      if (q < 9 && metric == 0) counts[scope] = members;
+    }
   }
-  __syncthreads();
-  if (t < 9) {
-    const int scope = t / 3;
-    const int n = n_group[scope];
-    summaries[t] = n ? total[t] / (double)n : 0.0;
-  }
-  if (t < 3) counts[t] = n_group[t];
-  if (t == 0) miou[k] = n_iou ? total[9] / (double)n_iou : 0.0;
 }
 
 // Launch choices of the per-call update, set by the host's tuner per bucket of
 // (floor(log2(G * P)), floor(log2(pixels per image))): histogram bins in shared memory or in
 // global memory, histogram CTAs per SM, and threads of each image's scoring CTA. Without an entry
-// the built-in rule applies: shared bins whenever they fit, up to 4 CTAs per SM as their shared
-// memory allows, 256 scoring threads.
+// the built-in rule applies: shared bins whenever they fit, up to 2 CTAs per SM as their shared
+// memory allows (more CTAs clear and flush more bins for the same pixels: 16 images of 640 x 640 with
+// 101 x 121 bins 15.8 us at 2, 19.9 at 3, 18.3 at 4; global bins 19.3-21.5), 1024 scoring threads (the
+// same images 10.7 us; 512 threads 12.3, 256 16.3).
 struct UpdateChoice {
   int smem;           // 1: shared-memory bins, 0: global bins
   int per_sm;         // histogram CTAs per SM
@@ -437,7 +615,7 @@ int max_per_sm(bool smem, int64_t bins) {
 
 UpdateChoice update_choice(int64_t bins, int64_t pixels) {
   const bool fits = bins <= kMaxSmemBins;
-  UpdateChoice choice{fits ? 1 : 0, std::min(4, max_per_sm(fits, bins)), kScoreThreads};
+  UpdateChoice choice{fits ? 1 : 0, std::min(2, max_per_sm(fits, bins)), kScoreThreads};
   {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     const auto it = g_update_tuning.find({log2_bucket(bins), log2_bucket(pixels)});
@@ -445,8 +623,37 @@ UpdateChoice update_choice(int64_t bins, int64_t pixels) {
   }
   choice.smem = choice.smem && fits;  // a tuned choice never exceeds what this launch can hold
   choice.per_sm = std::max(1, std::min(choice.per_sm, max_per_sm(choice.smem, bins)));
-  if (choice.score_threads != 512 && choice.score_threads != 1024) choice.score_threads = kScoreThreads;
+  if (choice.score_threads != 256 && choice.score_threads != 512) choice.score_threads = kScoreThreads;
   return choice;
+}
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// CTAs and tiles per CTA of a histogram over `tiles` tiles.
+struct HistogramGrid {
+  int64_t ctas, per_cta;
+  HistogramGrid(int64_t tiles, int per_sm) {
+    per_cta = ceil_div(tiles, std::min<int64_t>(tiles, (int64_t)sm_count() * per_sm));
+    ctas = ceil_div(tiles, per_cta);
+  }
+};
+
+int launch_slot_histogram(const int* gt, const int* pred, int64_t B, int64_t pixels, int G, int P, u64* pairs,
+                          int* error, cudaStream_t stream) {
+  const int64_t bins = (int64_t)G * P;
+  const UpdateChoice choice = update_choice(bins, pixels);
+  const size_t smem_bytes = choice.smem ? (size_t)round_up(bins, 4) * sizeof(u32) : 0;
+  const int64_t lead = pixels % 4 == 0 && aligned16(gt) ? 0 : 3;  // pixels a first tile may start early
+  const int64_t tiles_per_image = ceil_div(pixels + lead, kTilePixels);
+  const HistogramGrid grid(B * tiles_per_image, choice.per_sm);
+  auto kernel = choice.smem ? slot_histogram<true> : slot_histogram<false>;
+  if (smem_bytes > 48 * 1024)
+    PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
+  kernel<<<(unsigned)grid.ctas, kHistThreads, smem_bytes, stream>>>(gt, pred, pixels, B, G, P, tiles_per_image,
+                                                                    grid.per_cta, pairs, error);
+  PE_LAUNCHED("slot_histogram");
+  count_launch();
+  return kOk;
 }
 
 template <typename GT, typename PR>
@@ -458,11 +665,7 @@ int launch_histogram(const void* gt, const void* pred, int64_t B, int64_t pixels
   const bool smem = choice.smem;
   const size_t smem_bytes = smem ? (size_t)round_up(bins, 4) * sizeof(u32) : 0;
   const int64_t tiles_per_image = ceil_div(pixels, kTilePixels);
-  const int64_t total_tiles = B * tiles_per_image;
-  const int per_sm = choice.per_sm;
-  const int64_t max_ctas = (int64_t)sm_count() * per_sm;
-  const int64_t tiles_per_cta = ceil_div(total_tiles, std::min<int64_t>(total_tiles, max_ctas));
-  const int64_t grid = ceil_div(total_tiles, tiles_per_cta);
+  const HistogramGrid grid(B * tiles_per_image, choice.per_sm);
   auto* g = static_cast<const GT*>(gt);
   auto* p = static_cast<const PR*>(pred);
 #define PE_HIST(SM, VC)                                                                                \
@@ -470,8 +673,8 @@ int launch_histogram(const void* gt, const void* pred, int64_t B, int64_t pixels
     auto kernel = pair_histogram<GT, PR, SM, VC>;                                                      \
     if (smem_bytes > 48 * 1024)                                                                        \
       PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes)); \
-    kernel<<<(unsigned)grid, kHistThreads, smem_bytes, stream>>>(g, p, pixels, B, G, P, tiles_per_image, \
-                                                                 tiles_per_cta, gi, gs, pi, ps, pairs, error); \
+    kernel<<<(unsigned)grid.ctas, kHistThreads, smem_bytes, stream>>>(g, p, pixels, B, G, P, tiles_per_image, \
+                                                                      grid.per_cta, gi, gs, pi, ps, pairs, error); \
   } while (0)
   if (smem) {
     if (vec) PE_HIST(true, true); else PE_HIST(true, false);
@@ -483,8 +686,6 @@ int launch_histogram(const void* gt, const void* pred, int64_t B, int64_t pixels
   count_launch();
   return kOk;
 }
-
-bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace
 }  // namespace pe
@@ -516,10 +717,12 @@ PE_API int pe_update(const void* gt, int gt_is_int64, const void* pred, int pred
     PE_REQUIRE(gt && pred, "null map pointer");
     const bool no_lookup = gt_ids == nullptr && pred_ids == nullptr;
     int status;
-    if (!gt_is_int64 && !pred_is_int64) {
-      const bool vec = no_lookup && pixels % 4 == 0 && aligned16(gt) && aligned16(pred);
+    if (!gt_is_int64 && !pred_is_int64 && no_lookup) {
+      status = launch_slot_histogram(static_cast<const int*>(gt), static_cast<const int*>(pred), B, pixels, (int)G,
+                                     (int)P, upairs, err, stream);
+    } else if (!gt_is_int64 && !pred_is_int64) {
       status = launch_histogram<int, int>(gt, pred, B, pixels, (int)G, (int)P, gt_ids, gt_slots, pred_ids,
-                                          pred_slots, upairs, err, vec, stream);
+                                          pred_slots, upairs, err, false, stream);
     } else if (gt_is_int64 && pred_is_int64) {
       const bool vec = pixels % 2 == 0 && aligned16(gt) && aligned16(pred);
       status = launch_histogram<int64_t, int64_t>(gt, pred, B, pixels, (int)G, (int)P, gt_ids, gt_slots,
@@ -533,35 +736,43 @@ PE_API int pe_update(const void* gt, int gt_is_int64, const void* pred, int pred
     }
     if (status != kOk) return status;
   }
-  const size_t smem = score_staging_bytes(P);
-  PE_REQUIRE(smem <= 200 * 1024, "too many prediction slots for the scoring kernel (P=%lld)", (long long)P);
-  auto kernel = reward ? score<true> : score<false>;
   const int score_threads = update_choice(G * P, pixels).score_threads;
-  if (smem > 48 * 1024)
-    PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   auto* ua = reinterpret_cast<u64*>(areas);
   auto* utp = reinterpret_cast<u64*>(tp);
   auto* ufp = reinterpret_cast<u64*>(fp);
   auto* ufn = reinterpret_cast<u64*>(fn);
   auto* uconf = reinterpret_cast<u64*>(confusion);
-  auto* cr = crowd;
+  const bool blocks = ScoreTables::base_bytes(G, P, C) <= kScoreSmem && pixels < (int64_t(1) << 32);
+  const size_t smem = blocks ? std::min(score_bytes(G, P, C, G * P), kScoreSmem) : score_staging_bytes(P);
+  PE_REQUIRE(smem <= 200 * 1024, "too many prediction slots for the scoring kernel (P=%lld)", (long long)P);
+  auto by_blocks = reward ? score_blocks<true> : score_blocks<false>;
+  auto in_place = reward ? score<true> : score<false>;
+  if (smem > 48 * 1024)
+    PE_CUDA(cudaFuncSetAttribute(blocks ? reinterpret_cast<const void*>(by_blocks)
+                                        : reinterpret_cast<const void*>(in_place),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto launch = [&](int flags, int* word) {
+    if (blocks)
+      by_blocks<<<(unsigned)B, score_threads, smem, stream>>>(upairs, gc, pc, crowd, ua, matched, utp, ufp, ufn,
+                                                              iou_sum, uconf, (int)G, (int)P, (int)C, flags,
+                                                              (int)smem, word);
+    else
+      in_place<<<(unsigned)B, score_threads, smem, stream>>>(upairs, gc, pc, crowd, ua, matched, utp, ufp, ufn,
+                                                             iou_sum, uconf, (int)G, (int)P, (int)C, flags, word);
+    count_launch();
+  };
   if (validate) {
-    kernel<<<(unsigned)B, score_threads, smem, stream>>>(upairs, gc, pc, cr, ua, matched, utp, ufp, ufn, iou_sum,
-                                                         uconf, (int)G, (int)P, (int)C, 1 | 2, error);
+    launch(1 | 2, error);
     PE_LAUNCHED("score(areas)");
-    kernel<<<(unsigned)B, score_threads, smem, stream>>>(upairs, gc, pc, cr, ua, matched, utp, ufp, ufn, iou_sum,
-                                                         uconf, (int)G, (int)P, (int)C, 4 | 8, error);
+    launch(4 | 8, error);
     PE_LAUNCHED("score(accumulate)");
-    count_launch(2);
     int code = 0;
     PE_CUDA(cudaMemcpyAsync(&code, error, sizeof(int), cudaMemcpyDeviceToHost, stream));
     PE_CUDA(cudaStreamSynchronize(stream));
     return code;
   }
-  kernel<<<(unsigned)B, score_threads, smem, stream>>>(upairs, gc, pc, cr, ua, matched, utp, ufp, ufn, iou_sum,
-                                                       uconf, (int)G, (int)P, (int)C, 1 | 4, nullptr);
+  launch(1 | 4, nullptr);
   PE_LAUNCHED("score");
-  count_launch();
   return kOk;
 }
 
@@ -609,13 +820,32 @@ PE_API int pe_compute(const int64_t* tp, const int64_t* fp, const int64_t* fn, c
                       int64_t* out_fn, double* out_sums, int64_t* out_confusion, cudaStream_t stream) {
   PE_REQUIRE(C > 0 && C < INT_MAX && K >= 0 && K < INT_MAX, "invalid category or row count");
   if (K == 0) return kOk;
-  const size_t smem = (sizeof(int64_t) * 2 + sizeof(double) * 4 + sizeof(int)) * (size_t)C;
-  PE_REQUIRE(smem <= 200 * 1024, "too many categories for the compute kernel (C=%lld)", (long long)C);
+  const size_t partial = sizeof(int64_t) * (kComputeThreads / 32) * kComputeTile;
+  const size_t values = (sizeof(double) * 4 + sizeof(int)) * (size_t)C;
+  PE_REQUIRE(values + sizeof(int64_t) * 2 * (size_t)C <= 200 * 1024,
+             "too many categories for the compute kernel (C=%lld)", (long long)C);
+  const size_t smem = sizeof(int64_t) * 2 * (size_t)C + std::max(partial, values);
+  // A cluster per row while the rows leave SMs idle and a row has work for several CTAs: at 133 classes
+  // one CTA took 14.2 us and eight take 10.9; at 20 classes one takes 6.4, little more than its launch
+  // and two load latencies.
+  const bool shared_rows = C >= kComputeClusterClasses && K * kComputeCluster <= 2 * (int64_t)sm_count();
+  auto kernel = shared_rows ? compute_kernel<kComputeCluster> : compute_kernel<1>;
   if (smem > 48 * 1024)
-    PE_CUDA(cudaFuncSetAttribute(compute_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  compute_kernel<<<(unsigned)K, kComputeThreads, smem, stream>>>(tp, fp, fn, sums, confusion, reinterpret_cast<const bool*>(things),
-                                                  per_class, summaries, counts, miou, out_tp, out_fp, out_fn,
-                                                  out_sums, out_confusion, (int)C);
+    PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)(K * (shared_rows ? kComputeCluster : 1)));
+  config.blockDim = dim3(kComputeThreads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = kComputeCluster;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  config.attrs = &cluster;
+  config.numAttrs = shared_rows ? 1 : 0;
+  PE_CUDA(cudaLaunchKernelEx(&config, kernel, tp, fp, fn, sums, confusion, reinterpret_cast<const bool*>(things),
+                             per_class, summaries, counts, miou, out_tp, out_fp, out_fn, out_sums, out_confusion,
+                             (int)C));
   PE_LAUNCHED("compute");
   count_launch();
   return kOk;

@@ -594,14 +594,16 @@ __global__ void prefix_scan_kernel(const int64_t* __restrict__ descs, const u32*
   }
 }
 
-// Canvas PQ of one (image, checkpoint) row. With stage_pairs > 0 the row's G x (N+1) histogram is
-// copied to shared memory first (it fits when G x (N+1) <= stage_pairs) and scored one warp per mask.
+__host__ __device__ inline size_t label_bytes(int64_t P) { return ((size_t)P * sizeof(int) + 15) & ~size_t{15}; }
+
+// Canvas PQ of one (image, checkpoint) row, scored in one pass (pe_score.cuh). smem: dynamic shared memory of
+// the launch (labels, then tables and entry list); rows whose tables do not fit it are scored in place.
 constexpr int kPrefixScoreThreads = 512;
 __global__ void __launch_bounds__(kPrefixScoreThreads)
 prefix_score_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __restrict__ pairs,
                     const int* __restrict__ classes, const int* __restrict__ gc, const uint8_t* __restrict__ crowd,
                     int C, int64_t* __restrict__ tp, int64_t* __restrict__ fp, int64_t* __restrict__ fn,
-                    double* __restrict__ sums, int64_t* __restrict__ confusion, int stage_pairs, int hist_off) {
+                    double* __restrict__ sums, int64_t* __restrict__ confusion, int smem) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t row = blockIdx.x;
   const int64_t b = find_image(descs, B, kPQBegin, row);
@@ -612,28 +614,29 @@ prefix_score_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __r
   gc += d[kPSlotBegin];
   crowd += d[kPSlotBegin];
   classes += d[kPDetBegin];
-  u64* areas = reinterpret_cast<u64*>(smem_raw);
-  int* matched = reinterpret_cast<int*>(areas + G + P);
-  int* labels = matched + G;
-  unsigned char* staging = reinterpret_cast<unsigned char*>(labels + P);
-  staging += (16 - reinterpret_cast<uintptr_t>(staging) % 16) % 16;
-  const bool staged = (int64_t)G * P <= stage_pairs;
-  if (staged) {
-    u32* hs = reinterpret_cast<u32*>(smem_raw + hist_off);
-    stage_counts(hs, pq, G * P);
-    __syncthreads();
-    pq = hs;
-  }
-  score_areas<u32, false>(pq, gc, labels, crowd, areas, G, P, C, false);
-  __syncthreads();
-  // Active labels: a mask's class while it has visible pixels (prefix.py:82).
-  for (int p = threadIdx.x; p < P; p += blockDim.x) labels[p] = (p > 0 && areas[G + p] > 0) ? classes[p - 1] : -1;
-  __syncthreads();
   ScoreOut out{reinterpret_cast<u64*>(tp + row * C), reinterpret_cast<u64*>(fp + row * C),
                reinterpret_cast<u64*>(fn + row * C), sums + row * C,
                reinterpret_cast<u64*>(confusion + row * C * (int64_t)(C + 1))};
-  if (staged) score_accumulate_warps<false>(pq, gc, labels, crowd, areas, matched, G, P, C, out, staging);
-  else score_accumulate<u32, false>(pq, gc, labels, crowd, areas, matched, G, P, C, out, staging);
+  int* labels = reinterpret_cast<int*>(smem_raw);
+  const size_t tables_at = label_bytes(P);
+  // Active labels: a mask's class while it has visible pixels (prefix.py:82).
+  if (tables_at + ScoreTables::base_bytes(G, P, C) <= (size_t)smem) {
+    const ScoreTables t = ScoreTables::at(smem_raw + tables_at, G, P, C, smem - tables_at);
+    score_totals(pq, t, gc, crowd, G, P, C);
+    for (int p = threadIdx.x; p < P; p += blockDim.x) labels[p] = (p > 0 && t.col[p] > 0) ? classes[p - 1] : -1;
+    __syncthreads();
+    score_matches<u32, false>(pq, t, labels, G, P, C, out);
+    return;
+  }
+  u64* areas = reinterpret_cast<u64*>(smem_raw + tables_at);
+  int* matched = reinterpret_cast<int*>(areas + G + P);
+  unsigned char* staging = reinterpret_cast<unsigned char*>(matched + G);
+  staging += (16 - reinterpret_cast<uintptr_t>(staging) % 16) % 16;
+  score_areas<u32, false>(pq, gc, labels, crowd, areas, G, P, C, false);
+  __syncthreads();
+  for (int p = threadIdx.x; p < P; p += blockDim.x) labels[p] = (p > 0 && areas[G + p] > 0) ? classes[p - 1] : -1;
+  __syncthreads();
+  score_accumulate<u32, false>(pq, gc, labels, crowd, areas, matched, G, P, C, out, staging);
 }
 
 // Greedy generation-order matching (prefix.py:106-118) and the validation of one image's metadata: one
@@ -954,19 +957,17 @@ PE_API int pe_prefix(const int64_t* descs, int64_t B, int64_t total_chunks, int6
     count_launch();
   }
   if (total_rows) {
-    const size_t base =
-        (sizeof(u64) * (max_g + max_p) + sizeof(int) * (max_g + max_p) + score_staging_bytes(max_p) + 32 + 15) &
-        ~size_t{15};
-    PE_REQUIRE(base <= 200 * 1024, "prefix histogram too large for scoring (G=%lld, N+1=%lld)", (long long)max_g,
+    const size_t in_place = label_bytes(max_p) + sizeof(u64) * (max_g + max_p) + sizeof(int) * max_g +
+                            score_staging_bytes(max_p) + 32;
+    PE_REQUIRE(in_place <= 200 * 1024, "prefix histogram too large for scoring (G=%lld, N+1=%lld)", (long long)max_g,
                (long long)max_p);
-    // Stage each row's histogram when the largest fits 100 KB (two CTAs per SM); else read in place.
-    const int64_t cells = std::max<int64_t>(max_g, 1) * std::max<int64_t>(max_p, 1);
-    const int stage = cells * 4 <= 100 * 1024 ? (int)cells : 0;
-    const size_t smem = base + 4 * (size_t)stage;
+    // Two CTAs per SM.
+    const size_t want = label_bytes(max_p) + score_bytes(max_g, max_p, C, max_g * max_p);
+    const size_t smem = std::max(in_place, std::min<size_t>(want, 110 * 1024));
     if (smem > 48 * 1024)
       PE_CUDA(cudaFuncSetAttribute(prefix_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     prefix_score_kernel<<<(unsigned)total_rows, kPrefixScoreThreads, smem, stream>>>(
-        descs, B, pairs, classes, gc, crowd, (int)C, tp, fp, fn, sums, confusion, stage, (int)base);
+        descs, B, pairs, classes, gc, crowd, (int)C, tp, fp, fn, sums, confusion, (int)smem);
     PE_LAUNCHED("prefix_score");
     count_launch();
   }

@@ -41,8 +41,8 @@ constexpr int kPassThreads = 512;
 constexpr int kPassPixels = 16;
 constexpr int kChunk = kPassThreads * kPassPixels;  // 8192 pixels
 constexpr int kSortCap = 4096;
-constexpr int kScoreThreads = 512;  // 16 warps per image (0.062 ms for 256 images; 0.082 with 8 warps, 0.066 with 32)
-constexpr size_t kScoreStageBytes = 100 * 1024;  // largest G x P histogram staged in shared memory
+constexpr int kScoreThreads = 1024;  // half of them when images outnumber the SMs
+constexpr size_t kScoreSmemAlone = 200 * 1024, kScoreSmemShared = 110 * 1024;
 
 __device__ __forceinline__ bool score_before(double sa, int ia, double sb, int ib) {
   return sa > sb || (sa == sb && ia < ib);
@@ -470,7 +470,8 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
 }
 
 // 3. Per-image scoring. mode bit 1: areas + validation, bit 2: accumulate
-// (gated by *error when bit 4 is set).
+// (gated by *error when bit 4 is set). smem: dynamic shared memory of the launch;
+// an image whose tables do not fit it is scored in place.
 __global__ void __launch_bounds__(kScoreThreads)
 seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pairs, const u32* __restrict__ dpairs,
                  const int* __restrict__ gc, const int* __restrict__ pc, const uint8_t* __restrict__ crowd,
@@ -478,7 +479,7 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
                  const uint8_t* __restrict__ isthing, const int* __restrict__ det_classes,
                  const double* __restrict__ det_scores, double* __restrict__ det_pa, double* __restrict__ slot_ga,
                  int* __restrict__ slot_class, const double* __restrict__ ann_in, double* __restrict__ ann_out,
-                 int mode, int validate, int reward, int stage_pairs, int hist_off, u32* __restrict__ class_bits,
+                 int mode, int validate, int reward, int smem, u32* __restrict__ class_bits,
                  int* __restrict__ error) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if ((mode & 4) && *reinterpret_cast<volatile int*>(error)) return;
@@ -486,24 +487,24 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
   const int G = (int)d[kG], P = (int)d[kP], D = (int)d[kD];
   const int64_t sb = d[kSlotBegin], pb = d[kPSlotBegin], db = d[kDetBegin];
   const u32* pan = pairs + d[kPairBegin];
-  // The image's G x P histogram in shared memory when it fits (coalesced once; every later pass reads it
-  // there), else read in place.
-  const bool staged = P > 0 && (int64_t)G * P <= stage_pairs;
-  if (staged) {
-    u32* hs = reinterpret_cast<u32*>(smem_raw + hist_off);
-    stage_counts(hs, pan, G * P);
-    __syncthreads();
-    pan = hs;
-  }
+  const bool blocks = P > 0 && ScoreTables::base_bytes(G, P, C) <= (size_t)smem;
+  const ScoreTables t = ScoreTables::at(smem_raw, G, P, C, blocks ? smem : ScoreTables::base_bytes(G, P, C));
   const u32* det = dpairs + d[kDPairBegin];
   gc += sb; crowd += sb; matched += sb;
   pc += pb;
   u64* ar = areas + sb + pb;  // per image G + P entries at offset (slot_begin + pslot_begin)
+  if (blocks) score_totals(pan, t, gc, crowd, G, P, C);
   if (mode & 1) {
     int err = 0;
-    if (P > 0)
+    if (blocks) {
+      for (int k = threadIdx.x; k < G; k += blockDim.x) ar[k] = t.row[k];
+      for (int k = threadIdx.x; k < P; k += blockDim.x) ar[G + k] = t.col[k];
+      if (validate)
+        err = reward ? score_checks<true>(t, gc, pc, crowd, G, P, C) : score_checks<false>(t, gc, pc, crowd, G, P, C);
+    } else if (P > 0) {
       err = reward ? score_areas<u32, true>(pan, gc, pc, crowd, ar, G, P, C, validate)
                    : score_areas<u32, false>(pan, gc, pc, crowd, ar, G, P, C, validate);
+    }
     // Detection areas (full mask area: every slot, including void and stuff): a warp sums the rows
     // of kAreaRows detections at once with coalesced loads, so their L2 round trips overlap.
     constexpr int kAreaRows = 4;
@@ -550,11 +551,11 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
   if (reward) {  // per-image rows [B][C], no confusion (evaluator.py:497-538)
     const int64_t o = (int64_t)blockIdx.x * C;
     ScoreOut row{out.tp + o, out.fp + o, out.fn + o, out.iou_sum + o, nullptr};
-    if (staged) score_accumulate_warps<true>(pan, gc, pc, crowd, ar, matched, G, P, C, row, smem_raw);
+    if (blocks) score_matches<u32, true>(pan, t, pc, G, P, C, row);
     else if (P > 0) score_accumulate<u32, true>(pan, gc, pc, crowd, ar, matched, G, P, C, row, smem_raw);
     return;
   }
-  if (staged) score_accumulate_warps<false>(pan, gc, pc, crowd, ar, matched, G, P, C, out, smem_raw);
+  if (blocks) score_matches<u32, false>(pan, t, pc, G, P, C, out);
   else if (P > 0) score_accumulate<u32, false>(pan, gc, pc, crowd, ar, matched, G, P, C, out, smem_raw);
   // Classes present in the image for the matching (per-image bits): thing targets, and detections
   // (a class outside [0, C) marks class 0, whose matching warp handles such detections).
@@ -862,34 +863,39 @@ PE_API int pe_seg_score(const int64_t* descs, int64_t B, int64_t max_p, int64_t 
   PE_REQUIRE(B >= 0 && C > 0 && C < INT_MAX, "invalid batch");
   u32* bits = reward ? nullptr : reinterpret_cast<u32*>(class_bits);
   if (B == 0) return kOk;
-  const size_t base = (score_staging_bytes(std::max<int64_t>(max_p, 1)) + 15) & ~size_t{15};
-  PE_REQUIRE(base <= 200 * 1024, "too many prediction slots (P=%lld)", (long long)max_p);
-  // Stage histograms up to kScoreStageBytes (two CTAs still fit an SM); larger images read theirs in place.
-  const int stage = max_pairs > 0 && (size_t)max_pairs * 4 <= kScoreStageBytes ? (int)max_pairs : 0;
-  const size_t smem = base + 4 * (size_t)stage;
+  const size_t in_place = score_staging_bytes(std::max<int64_t>(max_p, 1));
+  PE_REQUIRE(in_place <= 200 * 1024, "too many prediction slots (P=%lld)", (long long)max_p);
+  // Tables and entry list of the largest image, the target tables counted as for kScoreSlots slots (an
+  // image with more takes the list's room, or the in-place form). One CTA per SM may take 200 KB; more
+  // images than SMs share them, two CTAs each.
+  constexpr int64_t kScoreSlots = 1024;
+  const bool alone = B <= sm_count();
+  const size_t want = score_bytes(kScoreSlots, max_p, C, max_pairs);
+  const size_t smem = std::max(in_place, std::min(want, alone ? kScoreSmemAlone : kScoreSmemShared));
+  const int threads = alone ? kScoreThreads : kScoreThreads / 2;
   if (smem > 48 * 1024)
     PE_CUDA(cudaFuncSetAttribute(seg_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   ScoreOut out{reinterpret_cast<u64*>(tp), reinterpret_cast<u64*>(fp), reinterpret_cast<u64*>(fn), iou_sum,
                reinterpret_cast<u64*>(confusion)};
   auto* ua = reinterpret_cast<u64*>(areas);
   if (validate) {
-    seg_score_kernel<<<(unsigned)B, kScoreThreads, smem, stream>>>(descs, pairs, dpairs, gc, pc, crowd, ua, matched,
+    seg_score_kernel<<<(unsigned)B, threads, smem, stream>>>(descs, pairs, dpairs, gc, pc, crowd, ua, matched,
                                                                    out, (int)C, isthing, det_classes, det_scores,
                                                                    det_pa, slot_ga, slot_class, ann_in, ann_out, 1, 1,
-                                                                   reward, stage, (int)base, nullptr, error);
+                                                                   reward, (int)smem, nullptr, error);
     PE_LAUNCHED("seg_score(areas)");
-    seg_score_kernel<<<(unsigned)B, kScoreThreads, smem, stream>>>(descs, pairs, dpairs, gc, pc, crowd, ua, matched,
+    seg_score_kernel<<<(unsigned)B, threads, smem, stream>>>(descs, pairs, dpairs, gc, pc, crowd, ua, matched,
                                                                    out, (int)C, isthing, det_classes, det_scores,
                                                                    det_pa, slot_ga, slot_class, ann_in, ann_out, 2 | 4,
-                                                                   1, reward, stage, (int)base, bits, error);
+                                                                   1, reward, (int)smem, bits, error);
     PE_LAUNCHED("seg_score(accumulate)");
     count_launch(2);
     return kOk;
   }
-  seg_score_kernel<<<(unsigned)B, kScoreThreads, smem, stream>>>(descs, pairs, dpairs, gc, pc, crowd, ua, matched, out,
+  seg_score_kernel<<<(unsigned)B, threads, smem, stream>>>(descs, pairs, dpairs, gc, pc, crowd, ua, matched, out,
                                                                  (int)C, isthing, det_classes, det_scores, det_pa,
                                                                  slot_ga, slot_class, ann_in, ann_out, 1 | 2, 0,
-                                                                 reward, stage, (int)base, bits, error);
+                                                                 reward, (int)smem, bits, error);
   PE_LAUNCHED("seg_score");
   count_launch();
   return kOk;
