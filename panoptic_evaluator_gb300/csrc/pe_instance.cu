@@ -1,22 +1,19 @@
 // COCO mask AP/AR: detection x target-slot histograms, mask overlaps, greedy
 // matching and 101-point precision/recall accumulation.
 //
-// Matching runs one warp per (image, class): the warp compacts the class's
-// detections (score order, top 100 ranked) and ground truths (metadata
-// order) with ballots, then each lane owns one of the 40 (area range x IoU
-// threshold) chains and runs COCO's greedy scan for it. Per detection the warp
-// first ballots, for each of the 10 thresholds, the targets whose IoU reaches
-// it; a chain then visits only those candidates (bit masks of crowd and
-// area-ignored targets remove the rest), in metadata order as the reference's
-// scan does.
+// Matching runs one CTA per (image, class): the class's detections (score
+// order, top 100 ranked) and ground truths (metadata order) are compacted with
+// ballots, every detection's candidate targets (IoU at least 0.5) are listed by
+// falling IoU, one warp per detection, and then each of 40 threads owns one
+// (area range x IoU threshold) chain and walks the detections through their
+// candidate lists.
 //
-// Accumulation runs one CTA per class: it gathers the class's records in
-// order (sorting them by descending score when they are not presorted), then
-// each of 120 threads owns one (threshold, area, maxDets) chain. A chain puts
-// the precision of every record into the bucket of its recall grid position
-// and the interpolated curve is the suffix maximum of the buckets, which is
-// the reference's searchsorted-on-envelope rule evaluated in one pass.
+// Accumulation runs kAccParts CTAs per class, each with two of the ten IoU
+// thresholds: it gathers the class's records, sorts them by descending score,
+// and one warp at a time builds a (threshold, area, maxDets) chain's precision
+// envelope with integer comparisons only.
 #include "pe_common.cuh"
+#include "pe_sort.cuh"
 
 #include <cfloat>
 
@@ -25,7 +22,7 @@ namespace {
 
 constexpr int kChains = 40;
 constexpr int kMaxDets = 100;
-constexpr int kMatchWarps = 8;
+constexpr int kMatchThreads = 128;
 
 __device__ __forceinline__ void area_range(int a, double& lo, double& hi) {
   lo = a == 2 ? 1024.0 : (a == 3 ? 9216.0 : 0.0);
@@ -38,18 +35,16 @@ __device__ __forceinline__ double iou_threshold(int t) {
   return table[t];
 }
 
-constexpr int kIouCap = 512;  // (detection, target) IoUs of one class staged up front when they fit
+// Candidate entries of one class held at a time; a class with more lists one detection's at a time.
+constexpr int kMatchList = 512;
+__host__ __device__ inline int match_entries(int g_max) { return g_max > kMatchList ? g_max : kMatchList; }
 
-__host__ __device__ inline int iou_entries(int g_max) { return g_max > kIouCap ? g_max : kIouCap; }
-
-// Shared memory of one matching warp for up to g_max targets per image: the class's IoU table (or
-// one detection's row), its detections and targets, 40 chains' taken bits, target bit masks (crowd,
-// ignored per area range, reaching each IoU threshold), per-target and per-detection flags.
-__host__ __device__ inline size_t match_warp_bytes(int g_max) {
+// Shared memory of one matching CTA for up to g_max targets per image: candidate IoUs and targets, the
+// detections' list ranges, 40 chains' taken bits, the class's detections and targets.
+__host__ __device__ inline size_t match_bytes(int g_max) {
   const int words = (g_max + 31) / 32;
-  const size_t bytes = sizeof(long long) * (size_t)iou_entries(g_max) + sizeof(int) * ((size_t)100 + g_max) +
-                       sizeof(uint32_t) * (size_t)(40 + 15) * words + 2 * (size_t)g_max + 100;
-  return (bytes + 15) / 16 * 16;
+  return (sizeof(long long) + sizeof(uint32_t)) * (size_t)match_entries(g_max) + sizeof(int) * 3 * kMaxDets +
+         sizeof(uint32_t) * kChains * (size_t)words + sizeof(uint16_t) * (size_t)g_max + (size_t)g_max + kMaxDets + 16;
 }
 
 struct FlagLayout {
@@ -86,30 +81,34 @@ __device__ __forceinline__ int nth_present_class(const u32* __restrict__ row, in
   return -1;
 }
 
+// What bounds a class is the chain over its detections, so everything that does
+// not depend on earlier matches is done before it and in parallel: IoUs (FP64
+// division runs at 1/64 of the FP32 rate, and only pairs that can reach 0.5 are
+// divided), candidates sorted by falling IoU, later targets first on ties, each
+// with its crowd and area-ignored bits. A chain's step is then a walk to the
+// first usable entry, usually one or two shared reads. 32 COCO-like images of
+// 100 detections: 21.8 us against 50.7 with one warp per class that divided and
+// balloted inside the chain; 8 images of 256 detections 27.4 against 153.
 template <typename Count>
-__global__ void __launch_bounds__(kMatchWarps * 32, 4)  // four CTAs per SM, as shared memory allows at g_max 150
+__global__ void __launch_bounds__(kMatchThreads)
 match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_off,
              const int64_t* __restrict__ d_off, const int64_t* __restrict__ g_off, int single_d, int single_g,
              const int* __restrict__ pc, const double* __restrict__ pa,
              const int* __restrict__ gc, const double* __restrict__ ga, const uint8_t* __restrict__ crowd,
              const double* __restrict__ areas, int C, int g_max, FlagLayout flags, int* __restrict__ ranks,
-             int64_t* __restrict__ counts, const int* __restrict__ gate, int per_warp,
-             const u32* __restrict__ class_bits, int batch) {
+             int64_t* __restrict__ counts, const int* __restrict__ gate,
+             const u32* __restrict__ class_bits) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (gate && *reinterpret_cast<const volatile int*>(gate)) return;  // validation failed upstream
   // Image b covers detections [d_off[b], d_off[b+1]) and targets [g_off[b], g_off[b+1]);
-  // its D x G intersections start at pair_off[b]. Without offsets: one image.
-  // One warp per (image, class) at a time: CTA k of an image covers warps x per_warp classes, warp w
-  // taking entries c_base + w, c_base + w + warps, ... of the image's class list. Without per-image
-  // class bits the list is every class and the CTAs go image by image. With them it is the classes
-  // present in the image (about a third of them in COCO-like batches), so the busy warps fill CTAs
-  // instead of sharing them with warps that have nothing to do, and the CTAs go class block by class
-  // block (block 0 of every image first) so that the CTAs left without classes come last.
-  const int warps = blockDim.x >> 5;
-  const int class_blocks = (C + warps * per_warp - 1) / (warps * per_warp);
-  const int b = class_bits ? (int)(blockIdx.x % (unsigned)batch) : (int)(blockIdx.x / class_blocks);
-  const int block = class_bits ? (int)(blockIdx.x / (unsigned)batch) : (int)(blockIdx.x % class_blocks);
-  const int c_base = block * warps * per_warp + (threadIdx.x >> 5);
+  // its D x G intersections start at pair_off[b]. Without offsets: one image. CTA (b, k) takes the k-th
+  // class of image b: of all classes, or with per-image class bits of those present in it (about a third
+  // in COCO-like batches), so that the CTAs left without a class come last.
+  const int b = (int)blockIdx.x, entry = (int)(blockIdx.y + gridDim.y * blockIdx.z);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = kMatchThreads / 32;
+  const int bit_words = (C + 31) / 32;
+  const int c = class_bits ? nth_present_class(class_bits + (int64_t)b * bit_words, bit_words, entry, lane) : entry;
+  if (c < 0 || c >= C) return;
   const int64_t d0 = d_off ? d_off[b] : 0, g0 = g_off ? g_off[b] : 0;
   const int D = d_off ? (int)(d_off[b + 1] - d0) : single_d;
   const int G = g_off ? (int)(g_off[b + 1] - g0) : single_g;
@@ -117,33 +116,24 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
   pc += d0; pa += d0; ranks += d0;
   gc += g0; ga += g0; crowd += g0; areas += g0;
   int8_t* fbase = flags.base + d0 * flags.det_stride;
-  const int bit_words = (C + 31) / 32;
-  auto one_class = [&](const int c) {
-  // Classes with neither detections nor targets in this image (per-image bits, when given) have no work.
-  if (class_bits && !((class_bits[(int64_t)b * bit_words + (c >> 5)] >> (c & 31)) & 1u)) return;
-  const int words = (g_max + 31) / 32;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char* mine = smem_raw + (size_t)warp * match_warp_bytes(g_max);
+  const int words = (g_max + 31) / 32, capacity = match_entries(g_max);
   // IoUs as IEEE bit patterns: for non-negative doubles the int64 order is the
-  // numeric order, so the chains compare integers only.
-  long long* iou_s = reinterpret_cast<long long*>(mine);      // IoU table of the class, or the current row
-  int* dets = reinterpret_cast<int*>(iou_s + iou_entries(g_max));
-  int* gts = dets + kMaxDets;
-  u32* used = reinterpret_cast<u32*>(gts + g_max);
-  u32* crowd_m = used + kChains * words;  // bit j of word w: target 32 w + j is a crowd
-  u32* ignore_m = crowd_m + words;        // [4][words]: ignored in area range a
-  u32* reach_m = ignore_m + 4 * words;    // [10][words]: IoU with the current detection reaches threshold t
-  unsigned char* crowd_s = reinterpret_cast<unsigned char*>(reach_m + 10 * words);
-  unsigned char* ignore_s = crowd_s + g_max;                   // bit a: target ignored in area range a
-  unsigned char* range_s = ignore_s + g_max;                   // bit a: detection area inside range a
+  // numeric order, so lists and chains compare integers only.
+  long long* iou_s = reinterpret_cast<long long*>(smem_raw);
+  u32* cand = reinterpret_cast<u32*>(iou_s + capacity);  // target j | ignored-in-range bits << 16 | crowd << 20
+  int* dets = reinterpret_cast<int*>(cand + capacity);
+  int* first = dets + kMaxDets;                          // a detection's entries: [first, first + length)
+  int* length = first + kMaxDets;
+  u32* used = reinterpret_cast<u32*>(length + kMaxDets);
+  uint16_t* gts = reinterpret_cast<uint16_t*>(used + kChains * words);
+  uint8_t* target_bits = reinterpret_cast<uint8_t*>(gts + g_max);  // bits 0-3: ignored in range a, bit 4: crowd
+  uint8_t* range_s = target_bits + g_max;                          // bit a: detection area inside range a
+  __shared__ int s_nd, s_ng, s_total;
   const u32 below = (1u << lane) - 1;
-  {
-    // Every detection's rank and flags are written by exactly one warp: the
-    // warp of its class (beyond the 100-detection cap: rank 0, all flags -1),
-    // or warp 0 of class block 0 for classes outside [0, C).
-    // The class lists are read kScanBlocks blocks of 32 at a time, every lane's loads issued before the
-    // ballots use them (one L2 round trip per group instead of one per block).
-    constexpr int kScanBlocks = 4;
+  constexpr int kScanBlocks = 4;  // blocks of 32 whose loads a lane issues before the ballots use them
+  if (warp == 0) {
+    // Every detection's rank and flags are written by exactly one CTA: that of its class (beyond the
+    // 100-detection cap: rank 0, all flags -1), or that of class 0 for classes outside [0, C).
     int nd = 0;
     for (int group = 0; group < D; group += 32 * kScanBlocks) {
       int dcs[kScanBlocks];
@@ -154,14 +144,10 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
       }
 #pragma unroll
       for (int u = 0; u < kScanBlocks; ++u) {
-        const int base = group + 32 * u;
-        if (base >= D) break;  // whole warp
-        const int d = base + lane;
-        const int dc = dcs[u];
-        const bool sel = d < D && dc == c;
+        const int d = group + 32 * u + lane;
+        const bool sel = d < D && dcs[u] == c;
         const u32 ballot = __ballot_sync(0xffffffffu, sel);
-        const bool stray = c == 0 && d < D && (dc < 0 || dc >= C);
-        bool unranked = stray;
+        bool unranked = c == 0 && d < D && (dcs[u] < 0 || dcs[u] >= C);
         if (sel) {
           const int rank = nd + __popc(ballot & below);
           if (rank < kMaxDets) {
@@ -178,178 +164,170 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
         nd += __popc(ballot);
       }
     }
-    nd = min(nd, kMaxDets);
+    if (lane == 0) s_nd = min(nd, kMaxDets);
+  } else if (warp == 1) {
     int ng = 0;
     int positive[4] = {0, 0, 0, 0};
-    int gcs[kScanBlocks];
-    for (int base = 0; base < G; base += 32) {
-      const int u = (base >> 5) % kScanBlocks;
-      if (u == 0) {
+    for (int group = 0; group < G; group += 32 * kScanBlocks) {
+      int gcs[kScanBlocks];
 #pragma unroll
-        for (int v = 0; v < kScanBlocks; ++v) {
-          const int g = base + 32 * v + lane;
-          gcs[v] = g < G ? gc[g] : -1;
+      for (int u = 0; u < kScanBlocks; ++u) {
+        const int g = group + 32 * u + lane;
+        gcs[u] = g < G ? gc[g] : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < kScanBlocks; ++u) {
+        const int g = group + 32 * u + lane;
+        const bool sel = g < G && gcs[u] == c;
+        const u32 ballot = __ballot_sync(0xffffffffu, sel);
+        if (!ballot) continue;  // whole warp
+        u32 bits = 0;
+        if (sel) {
+          const bool cr = crowd[g] != 0;
+          const double area = areas[g];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            double lo, hi;
+            area_range(a, lo, hi);
+            const bool out = area < lo || area > hi;
+            bits |= (u32)(cr || out) << a;
+            positive[a] += !cr && area >= lo && area <= hi;
+          }
+          const int j = ng + __popc(ballot & below);
+          gts[j] = (uint16_t)g;
+          target_bits[j] = (uint8_t)(bits | (u32)cr << 4);
         }
-      }
-      const int g = base + lane;
-      int gcu = gcs[0];
-#pragma unroll
-      for (int v = 1; v < kScanBlocks; ++v) gcu = u == v ? gcs[v] : gcu;
-      const bool sel = g < G && gcu == c;
-      const u32 ballot = __ballot_sync(0xffffffffu, sel);
-      if (sel) gts[ng + __popc(ballot & below)] = g;
-      ng += __popc(ballot);
-      const bool eligible = sel && !crowd[g];
-      const double area = eligible ? areas[g] : 0.0;
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        double lo, hi;
-        area_range(a, lo, hi);
-        positive[a] += __popc(__ballot_sync(0xffffffffu, eligible && area >= lo && area <= hi));
+        ng += __popc(ballot);
       }
     }
-    if (lane == 0 && ng)
-      for (int a = 0; a < 4; ++a)
-        if (positive[a]) atomicAdd(reinterpret_cast<u64*>(counts) + c * 4 + a, (u64)positive[a]);
-    if (nd == 0) return;
-    for (int k = lane; k < kChains * words; k += 32) used[k] = 0;
-    // Per-target and per-detection range tests and every (detection, target)
-    // IoU are evaluated once, lane-parallel (FP64 is slow on this part).
-    // Targets' crowd / ignore bits and detections' area-range bits in one pass (their loads overlap).
-    __syncwarp();  // gts / dets entries written by other lanes
-    for (int j = lane; j < max(ng, nd); j += 32) {
-      const int g = j < ng ? gts[j] : 0;
-      const bool cr = j < ng && crowd[g] != 0;
-      const double area = j < ng ? areas[g] : 0.0;
-      const double dpa = j < nd ? pa[dets[j]] : 0.0;
-      unsigned char ignore_bits = 0, range_bits = 0;
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        double lo, hi;
-        area_range(a, lo, hi);
-        ignore_bits |= (unsigned char)((cr || area < lo || area > hi) << a);
-        range_bits |= (unsigned char)((lo <= dpa && dpa <= hi) << a);
-      }
-      if (j < ng) {
-        crowd_s[j] = cr;
-        ignore_s[j] = ignore_bits;
-      }
-      if (j < nd) range_s[j] = range_bits;
+    for (int a = 0; a < 4; ++a) {
+      const int n = __reduce_add_sync(0xffffffffu, positive[a]);
+      if (lane == 0 && n) atomicAdd(reinterpret_cast<u64*>(counts) + c * 4 + a, (u64)n);
     }
-    // Every (detection, target) IoU is computed once, lane-parallel, and read by all 40 chains
-    // (FP64 division runs at 1/64 of the FP32 rate here): the whole table up front when it fits
-    // kIouCap entries, else one detection's row at a time in score order.
-    const bool staged = nd * ng <= kIouCap;
-    // Entries e0 .. e0 + count of the row-major nd x ng table; each lane issues the loads of kFillLoads
-    // entries before using them.
-    constexpr int kFillLoads = 4;
-    auto fill = [&](int e0, int count) {
-      const int end = e0 + count;
-      for (int e = e0 + lane; e < end; e += 32 * kFillLoads) {
-        double inter[kFillLoads], pa_d[kFillLoads], ga_g[kFillLoads];
+    if (lane == 0) s_ng = ng;
+  } else {
+    for (int k = threadIdx.x - 64; k < kChains * words; k += kMatchThreads - 64) used[k] = 0;
+    if (threadIdx.x == 64) s_total = 0;
+  }
+  __syncthreads();
+  const int nd = s_nd, ng = s_ng;
+  if (nd == 0) return;
+  for (int i = threadIdx.x; i < nd; i += kMatchThreads) {
+    const double dpa = pa[dets[i]];
+    u32 bits = 0;
 #pragma unroll
-        for (int u = 0; u < kFillLoads; ++u) {
-          const int eu = e + 32 * u;
-          inter[u] = pa_d[u] = ga_g[u] = 0.0;
-          if (eu < end) {
-            const int i = eu / ng, j = eu - i * ng;
-            const int d = dets[i], g = gts[j];
-            inter[u] = (double)P[(int64_t)d * G + g];
-            pa_d[u] = pa[d];
-            ga_g[u] = ga[g];
+    for (int a = 0; a < 4; ++a) {
+      double lo, hi;
+      area_range(a, lo, hi);
+      bits |= (u32)(lo <= dpa && dpa <= hi) << a;
+    }
+    range_s[i] = (uint8_t)bits;
+  }
+  // Candidates of detection i into entries [at, at + n), sorted; `at` from the shared counter, or 0 for
+  // one detection at a time. Entries past the capacity are counted, not stored. One warp.
+  auto list_candidates = [&](int i, bool alone) {
+    const int d = dets[i];
+    const double pa_d = pa[d];
+    const Count* row = P + (int64_t)d * G;
+    auto iou_of = [&](int j) -> long long {
+      if (j >= ng) return -1;
+      const int g = gts[j];
+      const double inter = (double)row[g];
+      if (!(inter > 0.0)) return -1;
+      const double uni = fmax((target_bits[j] & 16) ? pa_d : (pa_d + ga[g]) - inter, 1.0);
+      if (inter * 2.001 < uni) return -1;  // clearly under the lowest threshold: no division
+      return __double_as_longlong(inter / uni);
+    };
+    const long long lowest = __double_as_longlong(0.5);
+    const long long own = iou_of(lane);  // up to 32 targets: one evaluation serves both passes
+    int n = __popc(__ballot_sync(0xffffffffu, own >= lowest)), at = 0;
+    for (int j0 = 32; j0 < ng; j0 += 32) n += __popc(__ballot_sync(0xffffffffu, iou_of(j0 + lane) >= lowest));
+    if (n && !alone) {
+      if (lane == 0) at = atomicAdd(&s_total, n);
+      at = __shfl_sync(0xffffffffu, at, 0);
+    }
+    for (int j0 = 0, k = at; k < at + n; j0 += 32) {
+      const long long iou = j0 ? iou_of(j0 + lane) : own;
+      const u32 ballot = __ballot_sync(0xffffffffu, iou >= lowest);
+      const int e = k + __popc(ballot & below);
+      if (iou >= lowest && e < capacity) {
+        iou_s[e] = iou;
+        cand[e] = (u32)(j0 + lane) | (u32)target_bits[j0 + lane] << 16;
+      }
+      k += __popc(ballot);
+    }
+    if (lane == 0) {
+      first[i] = at;
+      length[i] = n;
+    }
+    __syncwarp();
+    if (n < 2 || at + n > capacity) return;
+    // Falling IoU, later targets first on ties (entries were stored by rising target).
+    if (n <= 32) {
+      const long long v = lane < n ? iou_s[at + lane] : -1;
+      const u32 w = lane < n ? cand[at + lane] : 0;
+      int rank = 0;
+      for (int k = 0; k < n; ++k) {
+        const long long o = __shfl_sync(0xffffffffu, v, k);
+        rank += o > v || (o == v && k > lane);
+      }
+      __syncwarp();
+      if (lane < n) {
+        iou_s[at + rank] = v;
+        cand[at + rank] = w;
+      }
+    } else {  // odd-even transposition: many near-identical masks
+      for (int phase = 0; phase < n; ++phase) {
+        for (int k = (phase & 1) + 2 * lane; k + 1 < n; k += 64) {
+          const long long x = iou_s[at + k], y = iou_s[at + k + 1];
+          const u32 jx = cand[at + k], jy = cand[at + k + 1];
+          if (x < y || (x == y && (jx & 0xffffu) < (jy & 0xffffu))) {
+            iou_s[at + k] = y; iou_s[at + k + 1] = x;
+            cand[at + k] = jy; cand[at + k + 1] = jx;
           }
         }
-#pragma unroll
-        for (int u = 0; u < kFillLoads; ++u) {
-          const int eu = e + 32 * u;
-          if (eu >= end) break;
-          const int j = eu - (eu / ng) * ng;
-          const double uni = crowd_s[j] ? pa_d[u] : (pa_d[u] + ga_g[u]) - inter[u];
-          iou_s[staged ? eu : j] = __double_as_longlong(inter[u] / fmax(uni, 1.0));
-        }
-      }
-    };
-    __syncwarp();  // crowd_s entries written by other lanes
-    if (staged) fill(0, nd * ng);
-    // Target masks of the class, one bit per target in metadata order.
-    const int wc = (ng + 31) / 32;
-    for (int w = 0; w < wc; ++w) {
-      const int j = 32 * w + lane;
-      const bool in = j < ng;
-      const u32 crowd_bits = __ballot_sync(0xffffffffu, in && crowd_s[j]);
-      if (lane == 0) crowd_m[w] = crowd_bits;
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const u32 bits = __ballot_sync(0xffffffffu, in && ((ignore_s[j] >> a) & 1));
-        if (lane == 0) ignore_m[a * words + w] = bits;
+        __syncwarp();
       }
     }
     __syncwarp();
-    for (int i = 0; i < nd; ++i) {
-      const int d = dets[i];
-      if (!staged) {
-        fill(i * ng, ng);
-        __syncwarp();
-      }
-      const long long* row = staged ? iou_s + i * ng : iou_s;
-      // Targets whose IoU with this detection reaches each threshold: a chain then visits only its
-      // candidates (usually one or two) instead of every target of the class.
-      for (int w = 0; w < wc; ++w) {
-        const int j = 32 * w + lane;
-        const long long iou = j < ng ? row[j] : -1ll;
-#pragma unroll
-        for (int t = 0; t < 10; ++t) {
-          const u32 bits = __ballot_sync(0xffffffffu, iou >= __double_as_longlong(iou_threshold(t)));
-          if (lane == 0) reach_m[t * words + w] = bits;
-        }
-      }
-      __syncwarp();
-      for (int chain = lane; chain < kChains; chain += 32) {
-        const int a = chain / 10, t = chain % 10;
-        const long long thr = __double_as_longlong(iou_threshold(t));
-        u32* taken = used + chain * words;
-        int best = -1;
-        bool best_ignored = false;
-        long long best_iou = thr;
-        // Eligible ground truth first, then ignored, each in metadata order (a taken target is skipped
-        // unless it is a crowd); a later entry with an equal IoU replaces the earlier one.
-        for (int pass = 0; pass < 2 && best < 0; ++pass) {
-          for (int w = 0; w < wc; ++w) {
-            const u32 ig = ignore_m[a * words + w];
-            u32 m = reach_m[t * words + w] & ~(taken[w] & ~crowd_m[w]) & (pass ? ig : ~ig);
-            while (m) {
-              const int j = 32 * w + __ffs(m) - 1;
-              m &= m - 1;
-              const long long iou = row[j];
-              if (iou >= best_iou) {
-                best = j;
-                best_iou = iou;
-                best_ignored = pass == 1;
-              }
-            }
-          }
-        }
-        int8_t flag = -1;
-        if (best >= 0) {
-          taken[best >> 5] |= 1u << (best & 31);
-          flag = best_ignored ? -1 : 1;
-        } else if ((range_s[i] >> a) & 1) {
-          flag = 0;
-        }
-        fbase[chain * flags.chain_stride + (int64_t)d * flags.det_stride] = flag;
-      }
-      __syncwarp();  // the threshold masks (and an unstaged row) are rewritten for the next detection
-    }
-  }
   };
-  for (int k = 0; k < per_warp; ++k) {
-    const int entry = c_base + k * warps;
-    const int c = class_bits ? nth_present_class(class_bits + (int64_t)b * bit_words, bit_words, entry,
-                                                 threadIdx.x & 31)
-                             : entry;
-    if (c < 0 || c >= C) break;  // whole warp: the list is exhausted
-    one_class(c);
-    __syncwarp();  // the warp's shared scratch is reused by its next class
+  // One detection of one chain: eligible targets before ignored ones, the largest IoU, the later target
+  // on ties (a taken target is skipped unless it is a crowd).
+  const int chain = threadIdx.x, a = chain / 10;
+  const long long thr = chain < kChains ? __double_as_longlong(iou_threshold(chain % 10)) : 0;
+  u32* taken = used + chain * words;
+  auto step = [&](int i) {
+    int best = -1, ignored = -1;
+    for (int e = first[i], end = e + length[i]; e < end; ++e) {
+      if (iou_s[e] < thr) break;
+      const u32 w = cand[e];
+      const int j = (int)(w & 0xffffu);
+      if (!((w >> 20) & 1u) && ((taken[j >> 5] >> (j & 31)) & 1u)) continue;
+      if (!((w >> (16 + a)) & 1u)) {
+        best = j;
+        break;
+      }
+      if (ignored < 0) ignored = j;
+    }
+    int8_t flag = best >= 0 ? 1 : -1;
+    if (best < 0) best = ignored;
+    if (best >= 0) taken[best >> 5] |= 1u << (best & 31);
+    else if ((range_s[i] >> a) & 1) flag = 0;
+    fbase[chain * flags.chain_stride + (int64_t)dets[i] * flags.det_stride] = flag;
+  };
+  for (int i = warp; i < nd; i += warps) list_candidates(i, false);
+  __syncthreads();
+  if (s_total <= capacity) {
+    if (chain < kChains)
+      for (int i = 0; i < nd; ++i) step(i);
+    return;
+  }
+  for (int i = 0; i < nd; ++i) {  // more candidates than the list holds: one detection at a time
+    if (warp == 0) list_candidates(i, true);
+    __syncthreads();
+    if (chain < kChains) step(i);
+    __syncthreads();
   }
 }
 
@@ -357,9 +335,14 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
 
 constexpr int kAccThreads = 256;
 constexpr int kSortCap = 1024;  // records of one class sorted and staged in shared memory, at most
-constexpr int kAccParts = 2;    // CTAs sharing a class's chains at that cap (two fit on an SM)
-constexpr int kSmallCap = 512;  // classes up to this many records: a smaller stage, more CTAs per class
-constexpr int kSmallParts = 4;  // (256 records per class, 256 images: 0.096 ms against 0.114 at one cap)
+constexpr int kSmallCap = 512;  // classes up to this many records: a smaller stage, more CTAs per SM
+constexpr int kAccT = 2;        // IoU thresholds of one CTA
+constexpr int kAccParts = 10 / kAccT;
+constexpr int kAccChains = 12 * kAccT;  // (threshold, area, maxDets) chains of one CTA
+constexpr int kRankSort = 192;  // records of a class sorted by counting rather than by a bitonic network
+// Records up to which every CTA scans the class array itself; above, three kernels group the records by
+// class first (at 3200 records and 80 classes they and their memset took 8 us of the stream).
+constexpr int64_t kScanRecords = 8192;
 
 __global__ void class_histogram_kernel(const int* __restrict__ classes, int64_t n, int C, int* __restrict__ hist) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -412,163 +395,151 @@ __global__ void class_scatter_kernel(const int* __restrict__ classes, int64_t n,
   }
 }
 
-// Sort key of a score: an unsigned integer that orders like the score descending (-0.0 taken as 0.0, so
-// equal scores give equal keys), compared with integers instead of FP64 (GB300's FP64 pipe runs at 1/64
-// of the FP32 rate). Ties sort by record index, which makes the sort stable.
-__device__ __forceinline__ unsigned long long score_key(double score) {
-  unsigned long long b = (unsigned long long)__double_as_longlong(score == 0.0 ? 0.0 : score);
-  b = (b >> 63) ? ~b : (b | 0x8000000000000000ull);  // ascending in the score
-  return ~b;                                           // descending
+// Recall thresholds r at which the quotient r / 100 reaches the threshold fl(r * 0.01) (the product can
+// round above it), as bits.
+struct RecallBits {
+  u64 lo, hi;
+};
+constexpr RecallBits recall_bits() {
+  RecallBits b{0, 0};
+  for (int r = 0; r <= 100; ++r)
+    if ((double)r / 100.0 >= (double)r * 0.01) (r < 64 ? b.lo : b.hi) |= 1ull << (r & 63);
+  return b;
 }
 
-__device__ __forceinline__ bool before(unsigned long long ka, int ia, unsigned long long kb, int ib) {
-  return ka < kb || (ka == kb && ia < ib);
+// The smallest true-positive count t whose recall fl(t / np) reaches fl(r * 0.01). t / np and r / 100
+// are equal or at least 1 / (100 np) apart, far more than the rounding of either side, so the exact
+// integer comparison decides except where they are equal, and there the bit of r does.
+__device__ __forceinline__ int64_t recall_reached_at(int64_t np, int r) {
+  constexpr RecallBits bits = recall_bits();
+  const int64_t scaled = np * r, t = (scaled + 99) / 100;
+  const bool exact_ok = ((r < 64 ? bits.lo : bits.hi) >> (r & 63)) & 1ull;
+  return t + (t * 100 == scaled && !exact_ok ? 1 : 0);
 }
 
-// Bitonic sort of n <= cap (key, index) pairs, n padded to a power of two with
-// sentinels that sort last. `global` arrays need a fence before each barrier.
-template <bool kGlobal>
-__device__ void bitonic_sort(unsigned long long* key, int* idx, int n, int padded) {
-  for (int i = n + threadIdx.x; i < padded; i += blockDim.x) {
-    key[i] = ~0ull;
-    idx[i] = INT_MAX;
-  }
-  __syncthreads();
-  for (int size = 2; size <= padded; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < padded; i += blockDim.x) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool ascending = (i & size) == 0;
-          const unsigned long long ki = key[i], kj = key[j];
-          const int ii = idx[i], ij = idx[j];
-          const bool swap = ascending ? before(kj, ij, ki, ii) : before(ki, ii, kj, ij);
-          if (swap) { key[i] = kj; key[j] = ki; idx[i] = ij; idx[j] = ii; }
-        }
-      }
-      if constexpr (kGlobal) __threadfence_block();
-      __syncthreads();
-    }
-  }
-}
-
-// One CTA per class. `scores` == nullptr means the records are already in
+// kAccParts CTAs per class. `scores` == nullptr means the records are already in
 // global descending-score order. Records: classes[n], ranks[n] and flags at
-// flags[chain * chain_stride + record * det_stride]. Classes with more than
-// kSortCap records use per-class workspace regions instead of shared memory.
+// flags[chain * chain_stride + record * det_stride]; list / cursor / hist: the
+// records grouped by class, or list == nullptr and every CTA scans `classes`.
+// Classes with more than kSortCap records use per-class workspace regions (and
+// one CTA, since the sort works in place there) instead of shared memory.
 //
-// Each of the 120 chains (threshold, area, maxDets) is handled by one warp at a
-// time. Prefix counts of true and false positives over the score-ordered
-// records come from ballots; the j-th true positive's cumulative false positives
-// are kept per j. The precision envelope of the reference (the running maximum
-// of precision from the end, instance.py:321) is a suffix maximum over j, taken
-// with a warp scan; recall threshold r is first reached at the true positive
-// j = tp_min[r], so precision[r] is the envelope at that j (instance.py:322-329).
-// Runs of thresholds with the same envelope pair become segments, converted to
-// FP64 once each with every lane converting a different segment. chain_stats
-// [c][chain] receives the sum of the chain's 101 precision values and its recall
-// (-1 when the class has no positives) for the summaries.
-template <int kCap, int kParts>
+// A chain is handled by one warp at a time. Prefix counts of true and false
+// positives over the score-ordered records come from ballots; the j-th true
+// positive's cumulative false positives are kept per j. The precision envelope
+// of the reference (the running maximum of precision from the end,
+// instance.py:321) is a suffix maximum over j, taken with a warp scan; recall
+// threshold r is first reached at the true positive j = tp_min[r], so
+// precision[r] is the envelope at that j (instance.py:322-329). Runs of
+// thresholds with the same envelope pair become segments. FP64 (1/64 of the FP32
+// rate here) is spent only with full warps: every lane divides a different
+// segment, then one warp sums all chains, a lane per chain. A CTA holds all
+// twelve (area, maxDets) chains of its thresholds, so the precision array is
+// written in 96-byte runs (one chain at a time wrote single 8-byte words, four
+// times the sectors). chain_stats [c][chain] receives the sum of the chain's 101
+// precision values and its recall (-1 when the class has no positives) for the
+// summaries. 3200 records of 80 classes: 17.9 us (43.2, after 8 us of grouping
+// kernels, with all 120 chains walked by four CTAs and FP64 recall thresholds);
+// 100 records 10.5 (26.9).
+template <int kCap>
+struct AccShared {
+  unsigned long long key[kCap];
+  int idx[kCap];
+  int rank[kCap];
+  int8_t flags[kCap][4 * kAccT];  // the staged records' flags of this CTA's thresholds, [t][area]
+  long long seg[kAccChains][101];   // packed (tp, fp) of a segment, then its value
+  unsigned char seg_lo[kAccChains][101 + 3];
+  unsigned short env[kAccThreads / 32][2][kCap + 1];
+  int tp_min[4][101];
+  int nseg[kAccChains], hi[kAccChains], tp[kAccChains], off[kAccChains + 1];
+  int64_t npos[4];
+  int count, before;
+};
+
+template <int kCap>
 __global__ void __launch_bounds__(kAccThreads)
-accumulate_kernel(const int* __restrict__ list, const int* __restrict__ cursor, const int* __restrict__ ranks,
+accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restrict__ list,
+                  const int* __restrict__ cursor, const int* __restrict__ hist, const int* __restrict__ ranks,
                   const int8_t* __restrict__ flags, int64_t chain_stride, int64_t det_stride,
                   const double* __restrict__ scores, const int64_t* __restrict__ positives,
-                  const int* __restrict__ hist, unsigned long long* __restrict__ ws_key, int* __restrict__ ws_idx,
-                  int C, long long* __restrict__ seg_ws, int* __restrict__ env_ws, double* __restrict__ precision,
+                  unsigned long long* __restrict__ ws_key, int* __restrict__ ws_idx,
+                  int C, int* __restrict__ env_ws, double* __restrict__ precision,
                   double* __restrict__ recall, double* __restrict__ chain_stats, int above) {
   // The bitonic sort pads a class's records to the next power of two inside the kCap-entry stage.
   static_assert(kCap > 0 && (kCap & (kCap - 1)) == 0, "a stage cap must be a power of two");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int c = blockIdx.x / kParts, part = blockIdx.x % kParts;
-  int64_t offset = 0;
-  for (int k = 0; k < c; ++k) {
-    const int h = hist[k];
-    offset += h > kSortCap ? (int64_t)1 << (32 - __clz(h - 1)) : 0;
+  AccShared<kCap>& sm = *reinterpret_cast<AccShared<kCap>*>(smem_raw);
+  const int c = blockIdx.x / kAccParts, part = blockIdx.x % kAccParts;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = kAccThreads / 32;
+  const unsigned below = (1u << lane) - 1u;
+  if (threadIdx.x < 4) sm.npos[threadIdx.x] = positives[c * 4 + threadIdx.x];
+  // Records of this class, and of the classes before it (where its workspace regions start).
+  int count, before;
+  if (list) {
+    count = hist[c];
+    before = cursor[c] - count;  // cursor[c] ends one past the class's segment after the scatter
+  } else {
+    if (threadIdx.x == 0) sm.count = sm.before = 0;
+    __syncthreads();
+    int lower = 0;
+    constexpr int kLoads = 4;
+    for (int64_t i0 = threadIdx.x; i0 < n; i0 += kLoads * kAccThreads) {
+      int v[kLoads];
+#pragma unroll
+      for (int j = 0; j < kLoads; ++j) v[j] = i0 + j * kAccThreads < n ? classes[i0 + j * kAccThreads] : -1;
+#pragma unroll
+      for (int j = 0; j < kLoads; ++j) {
+        lower += v[j] >= 0 && v[j] < c;
+        if (v[j] != c) continue;
+        const int at = atomicAdd(&sm.count, 1);
+        if (at < kCap) sm.idx[at] = (int)(i0 + j * kAccThreads);
+      }
+    }
+    if (lower) atomicAdd(&sm.before, lower);
+    __syncthreads();
+    count = sm.count;
+    before = sm.before;
   }
-  const int count = hist[c];
   // Classes of up to kCap records (more than `above`) are this launch's: the other launch takes the rest.
   if (count <= above || (kCap < kSortCap && count > kCap)) return;
   const bool staged = count <= kCap;
-  // A staged class's chains are shared by kParts CTAs (each sorts and stages the class itself); a class
-  // sorted in the workspace has one CTA, since the sort works in place there.
-  const int parts = staged ? kParts : 1;
+  const int parts = staged ? kAccParts : 1;
   if (part >= parts) return;
   int padded = 1;
   while (padded < max(count, 1)) padded <<= 1;
-  unsigned long long* key = staged ? reinterpret_cast<unsigned long long*>(smem_raw) : ws_key + offset;
-  int* idx = staged ? reinterpret_cast<int*>(smem_raw + sizeof(unsigned long long) * kCap) : ws_idx + offset;
-  int* st_rank = reinterpret_cast<int*>(smem_raw + (sizeof(unsigned long long) + sizeof(int)) * kCap);
-  int8_t* st_flags = reinterpret_cast<int8_t*>(st_rank + kCap);
-  unsigned char* seg_lo = reinterpret_cast<unsigned char*>(st_flags + kChains * kCap);  // [120][101]
-  // Per warp: cumulative false positives at the j-th true positive, then the envelope pair at j.
-  unsigned short* env_s = reinterpret_cast<unsigned short*>(seg_lo + 120 * 101);  // [warps][2][kCap + 1]
-  __shared__ int s_nseg[120], s_seg_off[121], s_hi[120];
-  __shared__ double s_recall[120];
-  for (int ch = threadIdx.x; ch < 120; ch += blockDim.x) s_nseg[ch] = 0;  // chains of the other parts stay empty
-  // This class's record indices (from the per-class list), then sorted by (score desc, index asc); without
-  // scores every key is equal and the sort restores record order.
-  const int begin = cursor[c] - count;  // cursor[c] ends one past the class's segment after the scatter
-  for (int k = threadIdx.x; k < count; k += blockDim.x) {
-    const int i = list[begin + k];
+  unsigned long long* key = staged ? sm.key : ws_key + 2 * (int64_t)before;
+  int* idx = staged ? sm.idx : ws_idx + 2 * (int64_t)before;
+  if (!list && !staged) {  // more records than the stage: the scan again, into the workspace
+    __syncthreads();
+    if (threadIdx.x == 0) sm.count = 0;
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < n; i += kAccThreads)
+      if (classes[i] == c) idx[atomicAdd(&sm.count, 1)] = (int)i;
+    __syncthreads();
+  }
+  // Sorted by (score desc, index asc); without scores every key is equal and the sort restores record order.
+  for (int k = threadIdx.x; k < count; k += kAccThreads) {
+    const int i = list ? list[before + k] : idx[k];
     idx[k] = i;
     key[k] = score_key(scores ? scores[i] : 0.0);
   }
+  for (int e = threadIdx.x; e < 4 * 101; e += kAccThreads) {
+    const int a = e / 101, r = e % 101;
+    sm.tp_min[a][r] = (int)recall_reached_at(positives[c * 4 + a], r);
+  }
   __syncthreads();
-  if (count > 1) {
+  if (staged && count <= kRankSort) {
+    rank_sort(key, idx, count);
+  } else if (count > 1) {
     if (staged) bitonic_sort<false>(key, idx, count, padded);
     else bitonic_sort<true>(key, idx, count, padded);
   }
   __syncthreads();
-  // Recall thresholds per area: tp_min[a][r] = the smallest true-positive count whose recall
-  // fl(tp / npos) reaches fl(r * 0.01), found with a few exact FP64 checks around the estimate, so the
-  // walk below compares integers (recall is monotone in tp).
-  __shared__ int s_tpmin[4][101];
-  for (int e = threadIdx.x; e < 4 * 101; e += blockDim.x) {
-    const int a = e / 101, r = e % 101;
-    const int64_t np = positives[c * 4 + a];
-    int64_t t = 0;
-    if (np > 0) {
-      const double thr = (double)r * 0.01, den = (double)np;
-      t = (int64_t)ceil(thr * den);
-      t = t < 0 ? 0 : (t > np ? np : t);
-      while (t > 0 && (double)(t - 1) / den >= thr) --t;
-      while (t <= np && (double)t / den < thr) ++t;
-    }
-    s_tpmin[a][r] = (int)t;
-  }
-  if (staged) {  // ranks and the 40 flags of every record, in walk order
-    for (int k = threadIdx.x; k < count; k += blockDim.x) st_rank[k] = ranks[idx[k]];
-    if (chain_stride == 1 && det_stride == kChains && reinterpret_cast<uintptr_t>(flags) % 8 == 0) {
-      // Record-major flags (the record store): one thread copies a record's 40 bytes as five 8-byte words.
-      for (int k = threadIdx.x; k < count; k += blockDim.x) {
-        const uint2* src = reinterpret_cast<const uint2*>(flags + (int64_t)idx[k] * kChains);
-        uint2* dst = reinterpret_cast<uint2*>(st_flags + k * kChains);
-        uint2 w[kChains / 8];
-#pragma unroll
-        for (int j = 0; j < kChains / 8; ++j) w[j] = src[j];
-#pragma unroll
-        for (int j = 0; j < kChains / 8; ++j) dst[j] = w[j];
-      }
-    } else {
-      for (int e = threadIdx.x; e < count * kChains; e += blockDim.x) {
-        const int k = e / kChains, ch = e % kChains;
-        st_flags[e] = flags[ch * chain_stride + (int64_t)idx[k] * det_stride];
-      }
-    }
-  }
-  __syncthreads();
-  // Phase A (integers only): one warp per chain builds the chain's envelope segments. Phase B: every
-  // segment's FP64 value, the segments spread over all threads. Phase C: one warp per chain writes the
-  // 101 precision values and sums them.
-  long long* segs = seg_ws + (int64_t)c * 120 * 101;  // [chain][segment]: packed (tp, fp), then its value
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const unsigned below = (1u << lane) - 1u;
-  const int64_t prec_step = (int64_t)C * 12;  // distance between consecutive recall thresholds r
   // Envelope arrays of this warp: 16-bit in shared memory when the class is staged, else 32-bit in the
   // workspace (each class owns 2 * warps * (count + 1) ints there).
-  unsigned short* fp16 = env_s + (int64_t)warp * 2 * (kCap + 1);
-  unsigned short* t16 = fp16 + (kCap + 1);
-  int* fp32 = env_ws + 2 * (int64_t)warps * ((int64_t)begin + c) + (int64_t)warp * 2 * (count + 1);
+  unsigned short* fp16 = sm.env[warp][0];
+  unsigned short* t16 = sm.env[warp][1];
+  int* fp32 = env_ws + 2 * (int64_t)warps * ((int64_t)before + c) + (int64_t)warp * 2 * (count + 1);
   int* t32 = fp32 + (count + 1);
   auto load_fp = [&](int j) -> unsigned { return staged ? fp16[j] : (unsigned)fp32[j]; };
   auto store_fp = [&](int j, unsigned v) { if (staged) fp16[j] = (unsigned short)v; else fp32[j] = (int)v; };
@@ -582,167 +553,161 @@ accumulate_kernel(const int* __restrict__ list, const int* __restrict__ cursor, 
     const int64_t lhs = (int64_t)ct * ((int64_t)bt + bf), rhs = (int64_t)bt * ((int64_t)ct + cf);
     return lhs > rhs || (lhs == rhs && bt + bf == 1 && ct + cf >= 2);
   };
-  for (int ch = part + parts * warp; ch < 120; ch += parts * warps) {
-    const int m = ch % 3, a = (ch / 3) % 4, t = ch / 12;
-    const int64_t out_r = ((int64_t)t * C + c) * 4 + a;
-    const int64_t npos = positives[c * 4 + a];
-    double* prec = precision + ((((int64_t)t * 101) * C + c) * 4 + a) * 3 + m;
-    double* stats = chain_stats ? chain_stats + ((int64_t)c * 120 + ch) * 2 : nullptr;
-    int nseg = 0, hi = 0;
-    if (!npos) {
-      for (int r = lane; r <= 100; r += 32) prec[r * prec_step] = -1.0;
+  for (int group = part; group < kAccParts; group += parts) {
+    const int t_base = group * kAccT;
+    if (staged) {  // ranks and this group's flags of every record, in walk order
+      for (int k = threadIdx.x; k < count; k += kAccThreads) sm.rank[k] = ranks[idx[k]];
+      for (int e = threadIdx.x; e < count * 4 * kAccT; e += kAccThreads) {
+        const int k = e / (4 * kAccT), f = e % (4 * kAccT), a = f % 4, t = f / 4;
+        sm.flags[k][f] = flags[(a * 10 + t_base + t) * chain_stride + (int64_t)idx[k] * det_stride];
+      }
+      __syncthreads();
+    }
+    // Phase A (integers only): one warp per chain builds the chain's envelope segments.
+    for (int ch = warp; ch < kAccChains; ch += warps) {
+      const int m = ch % 3, a = (ch / 3) % 4, t = ch / 12;
+      int nseg = 0, hi = 0;
+      unsigned tp = 0;
+      if (sm.npos[a]) {
+        const int limit = m == 0 ? 1 : (m == 1 ? 10 : 100);
+        const int64_t chain = (int64_t)(a * 10 + t_base + t) * chain_stride;
+        // Prefix counts over the records within maxDets: the j-th true positive's cumulative false
+        // positives (those before it) go to fp[j].
+        unsigned fp = 0, selected = 0;
+        for (int base = 0; base < count; base += 32) {
+          const int k = base + lane;
+          int f = -1;
+          bool sel = false;
+          if (k < count) {
+            const int rank = staged ? sm.rank[k] : ranks[idx[k]];
+            sel = rank >= 1 && rank <= limit;
+            if (sel) f = staged ? sm.flags[k][t * 4 + a] : flags[chain + (int64_t)idx[k] * det_stride];
+          }
+          const unsigned bt = __ballot_sync(0xffffffffu, f == 1), bf = __ballot_sync(0xffffffffu, f == 0);
+          selected |= __ballot_sync(0xffffffffu, sel);
+          if (f == 1) store_fp(tp + __popc(bt & below) + 1, fp + __popc(bf & below));
+          tp += __popc(bt);
+          fp += __popc(bf);
+        }
+        if (selected) {  // without a detection within maxDets: a zero curve (instance.py:315-318)
+          const int* tp_min = sm.tp_min[a];
+          int reached = 0;  // thresholds reached at the final recall (tp_min is nondecreasing in r)
+          for (int r = lane; r <= 100; r += 32) reached += tp_min[r] <= (int)tp;
+          hi = __reduce_add_sync(0xffffffffu, reached);
+          __syncwarp();
+          // Suffix maximum of the envelope over j = tp, tp - 1, ..., 1 (lane 0 holds the largest j of a
+          // chunk); the pair at j replaces fp[j] (its own entry, read first) and goes to t[j].
+          unsigned ct = 0, cf = 0;  // the best pair of the chunks already scanned
+          for (int top = (int)tp; top >= 1; top -= 32) {
+            const int j = top - lane;
+            unsigned vt = 0, vf = 0;
+            if (j >= 1) { vt = (unsigned)j; vf = load_fp(j); }
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+              const unsigned ot = __shfl_up_sync(0xffffffffu, vt, off), of = __shfl_up_sync(0xffffffffu, vf, off);
+              if (lane >= off && beats(ot, of, vt, vf)) { vt = ot; vf = of; }
+            }
+            if (beats(ct, cf, vt, vf)) { vt = ct; vf = cf; }
+            if (j >= 1) { store_t(j, vt); store_fp(j, vf); }
+            ct = __shfl_sync(0xffffffffu, vt, 31);
+            cf = __shfl_sync(0xffffffffu, vf, 31);
+          }
+          __syncwarp();
+          // Threshold r < hi takes the envelope at j = tp_min[r] (thresholds reached with no true positive
+          // take the envelope over all of them); runs of equal pairs are the chain's segments.
+          int prev_t = -1, prev_f = -1;
+          for (int r0 = 0; r0 < hi; r0 += 32) {
+            const int r = r0 + lane;
+            unsigned pt = 0, pf = 0;
+            if (r < hi && tp > 0) {
+              const int j = max(tp_min[r], 1);
+              pt = load_t(j);
+              pf = load_fp(j);
+            }
+            int lt = __shfl_up_sync(0xffffffffu, (int)pt, 1), lf = __shfl_up_sync(0xffffffffu, (int)pf, 1);
+            if (lane == 0) { lt = prev_t; lf = prev_f; }
+            const bool start = r < hi && ((int)pt != lt || (int)pf != lf);
+            const unsigned starts = __ballot_sync(0xffffffffu, start);
+            if (start) {
+              const int at = nseg + __popc(starts & below);
+              sm.seg_lo[ch][at] = (unsigned char)r;
+              sm.seg[ch][at] = (long long)(((unsigned long long)pt << 32) | pf);
+            }
+            nseg += __popc(starts);
+            prev_t = __shfl_sync(0xffffffffu, (int)pt, 31);
+            prev_f = __shfl_sync(0xffffffffu, (int)pf, 31);
+          }
+        }
+      }
       if (lane == 0) {
-        recall[out_r * 3 + m] = -1.0;
-        if (stats) { stats[0] = -1.0; stats[1] = -1.0; }
-      }
-    } else {
-      const int limit = m == 0 ? 1 : (m == 1 ? 10 : 100);
-      const int chain = a * 10 + t;
-      // Prefix counts over the records within maxDets: the j-th true positive's cumulative false
-      // positives (those before it) go to fp[j].
-      unsigned tp = 0, fp = 0, selected = 0;
-      for (int base = 0; base < count; base += 32) {
-        const int k = base + lane;
-        int f = -1;
-        bool sel = false;
-        if (k < count) {
-          const int rank = staged ? st_rank[k] : ranks[idx[k]];
-          sel = rank >= 1 && rank <= limit;
-          if (sel) f = staged ? st_flags[k * kChains + chain] : flags[chain * chain_stride + (int64_t)idx[k] * det_stride];
-        }
-        const unsigned bt = __ballot_sync(0xffffffffu, f == 1), bf = __ballot_sync(0xffffffffu, f == 0);
-        const unsigned bs = __ballot_sync(0xffffffffu, sel);
-        if (f == 1) store_fp(tp + __popc(bt & below) + 1, fp + __popc(bf & below));
-        tp += __popc(bt);
-        fp += __popc(bf);
-        selected += __popc(bs);
-      }
-      if (!selected) {  // no detection within maxDets: zero curve (instance.py:315-318)
-        for (int r = lane; r <= 100; r += 32) prec[r * prec_step] = 0.0;
-        if (lane == 0) {
-          recall[out_r * 3 + m] = 0.0;
-          if (stats) { stats[0] = 0.0; stats[1] = 0.0; }
-        }
-      } else {
-        if (lane == 0) s_recall[ch] = recall[out_r * 3 + m] = (double)tp / (double)npos;
-        const int* tp_min = s_tpmin[a];
-        int reached = 0;  // thresholds reached at the final recall (tp_min is nondecreasing in r)
-        for (int r = lane; r <= 100; r += 32) reached += tp_min[r] <= (int)tp;
-#pragma unroll
-        for (int off = 16; off; off >>= 1) reached += __shfl_xor_sync(0xffffffffu, reached, off);
-        hi = reached;
-        for (int r = hi + lane; r <= 100; r += 32) prec[r * prec_step] = 0.0;  // thresholds never reached
-        __syncwarp();
-        // Suffix maximum of the envelope over j = tp, tp - 1, ..., 1 (lane 0 holds the largest j of a
-        // chunk); the pair at j replaces fp[j] (its own entry, read first) and goes to t[j].
-        unsigned ct = 0, cf = 0;  // the best pair of the chunks already scanned
-        for (int top = (int)tp; top >= 1; top -= 32) {
-          const int j = top - lane;
-          unsigned vt = 0, vf = 0;
-          if (j >= 1) { vt = (unsigned)j; vf = load_fp(j); }
-#pragma unroll
-          for (int off = 1; off < 32; off <<= 1) {
-            const unsigned ot = __shfl_up_sync(0xffffffffu, vt, off), of = __shfl_up_sync(0xffffffffu, vf, off);
-            if (lane >= off && beats(ot, of, vt, vf)) { vt = ot; vf = of; }
-          }
-          if (beats(ct, cf, vt, vf)) { vt = ct; vf = cf; }
-          if (j >= 1) { store_t(j, vt); store_fp(j, vf); }
-          ct = __shfl_sync(0xffffffffu, vt, 31);
-          cf = __shfl_sync(0xffffffffu, vf, 31);
-        }
-        __syncwarp();
-        // Threshold r < hi takes the envelope at j = tp_min[r] (thresholds reached with no true positive
-        // take the envelope over all of them); runs of equal pairs are the chain's segments.
-        unsigned char* lo_of = seg_lo + ch * 101;
-        long long* pair_of = segs + ch * 101;
-        int prev_t = -1, prev_f = -1;
-        for (int r0 = 0; r0 < hi; r0 += 32) {
-          const int r = r0 + lane;
-          unsigned pt = 0, pf = 0;
-          if (r < hi && tp > 0) {
-            const int j = max(tp_min[r], 1);
-            pt = load_t(j);
-            pf = load_fp(j);
-          }
-          int lt = __shfl_up_sync(0xffffffffu, (int)pt, 1), lf = __shfl_up_sync(0xffffffffu, (int)pf, 1);
-          if (lane == 0) { lt = prev_t; lf = prev_f; }
-          const bool start = r < hi && ((int)pt != lt || (int)pf != lf);
-          const unsigned starts = __ballot_sync(0xffffffffu, start);
-          if (start) {
-            const int sidx = nseg + __popc(starts & below);
-            lo_of[sidx] = (unsigned char)r;
-            pair_of[sidx] = (long long)(((unsigned long long)pt << 32) | pf);
-          }
-          nseg += __popc(starts);
-          prev_t = __shfl_sync(0xffffffffu, (int)pt, 31);
-          prev_f = __shfl_sync(0xffffffffu, (int)pf, 31);
-        }
+        sm.nseg[ch] = nseg;
+        sm.hi[ch] = hi;
+        sm.tp[ch] = (int)tp;
       }
     }
-    if (lane == 0) {
-      s_nseg[ch] = nseg;
-      s_hi[ch] = hi;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {  // segment offsets (exclusive scan over the 120 chains)
-    int carry = 0;
-    for (int base = 0; base < 120; base += 32) {
-      const int ch = base + (int)threadIdx.x;
-      const int v0 = ch < 120 ? s_nseg[ch] : 0;
+    __syncthreads();
+    if (warp == 0) {  // segment offsets (exclusive scan over the chains)
+      static_assert(kAccChains <= 32, "one lane per chain");
+      const int v0 = lane < kAccChains ? sm.nseg[lane] : 0;
       int v = v0;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
         const int u = __shfl_up_sync(0xffffffffu, v, off);
-        if ((int)threadIdx.x >= off) v += u;
+        if (lane >= off) v += u;
       }
-      if (ch < 120) s_seg_off[ch] = carry + v - v0;
-      carry += __shfl_sync(0xffffffffu, v, 31);
+      if (lane < kAccChains) sm.off[lane] = v - v0;
+      if (lane == 31) sm.off[kAccChains] = v;
     }
-    if (threadIdx.x == 0) s_seg_off[120] = carry;
-  }
-  __syncthreads();
-  // Phase B: every segment's value, fl(tp / ((tp + fp) + eps)), the segments spread over all threads.
-  const int total_segs = s_seg_off[120];
-  for (int e = threadIdx.x; e < total_segs; e += blockDim.x) {
-    int lo = 0, hi = 119;  // chain holding flat segment e
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (s_seg_off[mid] <= e) lo = mid; else hi = mid - 1;
-    }
-    long long* slot = segs + lo * 101 + (e - s_seg_off[lo]);
-    const unsigned long long pair = (unsigned long long)*slot;
-    const double bt = (double)(int64_t)(pair >> 32), bf = (double)(int64_t)(pair & 0xffffffffull);
-    *slot = __double_as_longlong(bt / ((bt + bf) + DBL_EPSILON));
-  }
-  __syncthreads();
-  // Phase C: each chain's precision values from its segments (segment s covers [lo_s, lo_{s+1}), the
-  // last up to hi), and their sum for the summaries.
-  for (int ch = part + parts * warp; ch < 120; ch += parts * warps) {
-    const int nseg = s_nseg[ch];
-    if (nseg == 0) continue;
-    const int m = ch % 3, a = (ch / 3) % 4, t = ch / 12;
-    double* prec = precision + ((((int64_t)t * 101) * C + c) * 4 + a) * 3 + m;
-    const unsigned char* lo_of = seg_lo + ch * 101;
-    const long long* val_of = segs + ch * 101;
-    double psum = 0.0;
-    for (int r = lane; r < s_hi[ch]; r += 32) {
-      int lo = 0, hi = nseg - 1;  // the last segment starting at or before r
+    __syncthreads();
+    // Phase B: every segment's value, fl(tp / ((tp + fp) + eps)), the segments spread over all threads.
+    for (int e = threadIdx.x; e < sm.off[kAccChains]; e += kAccThreads) {
+      int lo = 0, hi = kAccChains - 1;  // chain holding flat segment e
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (lo_of[mid] <= r) lo = mid; else hi = mid - 1;
+        if (sm.off[mid] <= e) lo = mid; else hi = mid - 1;
       }
-      const double v = __longlong_as_double(val_of[lo]);
-      prec[r * prec_step] = v;
-      psum += v;
+      long long& slot = sm.seg[lo][e - sm.off[lo]];
+      const unsigned long long pair = (unsigned long long)slot;
+      const double bt = (double)(int)(pair >> 32), bf = (double)(int)(pair & 0xffffffffull);
+      slot = __double_as_longlong(bt / ((bt + bf) + DBL_EPSILON));
     }
-#pragma unroll
-    for (int off = 16; off; off >>= 1) psum += __shfl_xor_sync(0xffffffffu, psum, off);
-    if (lane == 0 && chain_stats) {
-      double* stats = chain_stats + ((int64_t)c * 120 + ch) * 2;
-      stats[0] = psum;
-      stats[1] = s_recall[ch];
+    __syncthreads();
+    // Phase C: precision values (segment s covers [lo_s, lo_{s+1}), the last up to hi), twelve chains of a
+    // (threshold, recall) next to one another; the last warp writes recalls and the chains' sums.
+    if (warp == warps - 1) {
+      if (lane < kAccChains) {
+        const int a = (lane / 3) % 4, t = t_base + lane / 12;
+        const int64_t np = sm.npos[a];
+        const double rc = np ? (double)sm.tp[lane] / (double)np : -1.0;
+        recall[((int64_t)t * C + c) * 12 + lane % 12] = rc;
+        if (chain_stats) {
+          double sum = np ? 0.0 : -1.0;
+          const int nseg = sm.nseg[lane], hi = sm.hi[lane];
+          for (int k = 0; k < nseg; ++k) {
+            const int end = k + 1 < nseg ? sm.seg_lo[lane][k + 1] : hi;
+            sum += __longlong_as_double(sm.seg[lane][k]) * (double)(end - sm.seg_lo[lane][k]);
+          }
+          double* stats = chain_stats + ((int64_t)c * 120 + t * 12 + lane % 12) * 2;
+          stats[0] = sum;
+          stats[1] = rc;
+        }
+      }
+    } else {
+      for (int e = threadIdx.x; e < kAccChains * 101; e += kAccThreads - 32) {
+        const int k = e % 12, r = (e / 12) % 101, t = e / (12 * 101), ch = t * 12 + k;
+        double v = sm.npos[k / 3] ? 0.0 : -1.0;
+        if (r < sm.hi[ch]) {
+          int lo = 0, hi = sm.nseg[ch] - 1;  // the last segment starting at or before r
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (sm.seg_lo[ch][mid] <= r) lo = mid; else hi = mid - 1;
+          }
+          v = __longlong_as_double(sm.seg[ch][lo]);
+        }
+        precision[(((int64_t)(t_base + t) * 101 + r) * C + c) * 12 + k] = v;
+      }
     }
+    if (group + parts < kAccParts) __syncthreads();  // the next group rewrites the tables
   }
 }
 
@@ -1017,33 +982,27 @@ int launch_match(const void* pairs, bool pairs_u32, const int64_t* pair_off, con
                  int8_t* flags, int64_t chain_stride, int64_t det_stride, int* ranks, int64_t* counts,
                  cudaStream_t stream, const int* gate = nullptr, const uint32_t* class_bits = nullptr) {
   if (B == 0) return kOk;
-  const size_t per_warp = match_warp_bytes(g_max);
-  int warps = kMatchWarps;
-  while (warps > 1 && per_warp * warps > 200 * 1024) warps >>= 1;
-  if (per_warp * warps > 200 * 1024) {
+  const size_t smem = match_bytes(g_max);
+  if (smem > 200 * 1024 || g_max > 65536) {
     set_error("too many ground-truth slots per image for matching (G=%d)", g_max);
     return kUnsupported;
   }
-  const size_t smem = per_warp * warps;
-  const int classes_per_warp = 1;  // 2 or 4 measured the same on 256 images; one CTA per image 35 % slower
-  const int64_t grid = B * ceil_div(C, warps * classes_per_warp);
-  if (grid > INT_MAX) {
-    set_error("too many (image, class) pairs for one matching launch (B=%lld, C=%d)", (long long)B, C);
-    return kUnsupported;
-  }
+  PE_REQUIRE(B <= INT_MAX, "too many images for one matching launch (B=%lld)", (long long)B);
+  const unsigned rows = (unsigned)std::min(C, 65535);
+  const dim3 grid((unsigned)B, rows, (unsigned)ceil_div(C, rows));
   FlagLayout layout{flags, chain_stride, det_stride};
   if (pairs_u32) {
     auto kernel = match_kernel<u32>;
     if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<(unsigned)grid, warps * 32, smem, stream>>>(static_cast<const u32*>(pairs), pair_off, d_off, g_off, single_d,
+    kernel<<<grid, kMatchThreads, smem, stream>>>(static_cast<const u32*>(pairs), pair_off, d_off, g_off, single_d,
                                                       single_g, pc, pa, gc, ga, crowd, areas, C, g_max, layout, ranks,
-                                                      counts, gate, classes_per_warp, class_bits, (int)B);
+                                                      counts, gate, class_bits);
   } else {
     auto kernel = match_kernel<int64_t>;
     if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<(unsigned)grid, warps * 32, smem, stream>>>(static_cast<const int64_t*>(pairs), pair_off, d_off, g_off,
+    kernel<<<grid, kMatchThreads, smem, stream>>>(static_cast<const int64_t*>(pairs), pair_off, d_off, g_off,
                                                       single_d, single_g, pc, pa, gc, ga, crowd, areas, C, g_max,
-                                                      layout, ranks, counts, gate, classes_per_warp, class_bits, (int)B);
+                                                      layout, ranks, counts, gate, class_bits);
   }
   PE_LAUNCHED("match");
   count_launch();
@@ -1060,11 +1019,28 @@ int launch_match_gated(const void* pairs, bool pairs_u32, const int64_t* pair_of
 }
 
 int64_t accumulate_workspace_bytes(int64_t n, int64_t C) {
-  // Per-class overflow regions padded to powers of two (at most 2n entries), the per-class list (n), then
-  // every class's envelope segments (120 chains x 101 of 8 bytes).
+  // Per-class overflow regions (each class's padded to a power of two, at most twice its records: 2n
+  // entries), the per-class list (n), then the envelope arrays of classes sorted there.
   return (int64_t)round_up(2 * n + 1, 64) * (int64_t)(sizeof(double) + sizeof(int)) +
-         (int64_t)round_up(n + 1, 64) * (int64_t)sizeof(int) + C * 120 * 101 * (int64_t)sizeof(long long) +
+         (int64_t)round_up(n + 1, 64) * (int64_t)sizeof(int) +
          2 * (kAccThreads / 32) * (n + C) * (int64_t)sizeof(int);
+}
+
+template <int kCap>
+int launch_accumulate_cap(const int* classes, int64_t n, const int* list, const int* cursor, const int* hist,
+                          const int* ranks, const int8_t* flags, int64_t chain_stride, int64_t det_stride,
+                          const double* scores, const int64_t* positives, unsigned long long* ws_key, int* ws_idx,
+                          int C, int* env_ws, double* precision, double* recall, double* chain_stats, int above,
+                          cudaStream_t stream) {
+  auto kernel = accumulate_kernel<kCap>;
+  const size_t smem = sizeof(AccShared<kCap>);
+  PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<(unsigned)(C * kAccParts), kAccThreads, smem, stream>>>(
+      classes, n, list, cursor, hist, ranks, flags, chain_stride, det_stride, scores, positives, ws_key, ws_idx, C,
+      env_ws, precision, recall, chain_stats, above);
+  PE_LAUNCHED("accumulate");
+  count_launch();
+  return kOk;
 }
 
 int launch_accumulate(const int* classes, const int* ranks, const int8_t* flags, int64_t chain_stride,
@@ -1076,16 +1052,15 @@ int launch_accumulate(const int* classes, const int* ranks, const int8_t* flags,
     set_error("accumulate workspace too small: %lld < %lld bytes", (long long)workspace_bytes, (long long)need);
     return kWorkspaceTooSmall;
   }
-  PE_CUDA(cudaMemsetAsync(hist, 0, sizeof(int) * C, stream));
   const int64_t entries = round_up(2 * n + 1, 64);
   auto* ws_key = static_cast<unsigned long long*>(workspace);
   int* ws_idx = reinterpret_cast<int*>(ws_key + entries);
   int* list = ws_idx + entries;
-  long long* seg_ws = reinterpret_cast<long long*>(
-      static_cast<char*>(workspace) + round_up(2 * n + 1, 64) * (int64_t)(sizeof(double) + sizeof(int)) +
-      round_up(n + 1, 64) * (int64_t)sizeof(int));
-  int* env_ws = reinterpret_cast<int*>(seg_ws + (int64_t)C * 120 * 101);
-  if (n > 0) {
+  int* env_ws = list + round_up(n + 1, 64);
+  if (n <= kScanRecords) {
+    list = nullptr;
+  } else {
+    PE_CUDA(cudaMemsetAsync(hist, 0, sizeof(int) * C, stream));
     const int64_t blocks = std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 4);
     class_histogram_kernel<<<(unsigned)blocks, 256, 0, stream>>>(classes, n, C, hist);
     PE_LAUNCHED("class_histogram");
@@ -1095,28 +1070,16 @@ int launch_accumulate(const int* classes, const int* ranks, const int8_t* flags,
     PE_LAUNCHED("class_scatter");
     count_launch(3);
   }
-  // Classes of up to kSmallCap records in a smaller stage with kSmallParts CTAs each; when some class
-  // can be larger, a second launch takes those (staged up to kSortCap, else in the workspace).
-  auto smem_for = [](int cap) {
-    return (sizeof(unsigned long long) + 2 * sizeof(int) + kChains) * cap + 120 * 101 +
-           sizeof(unsigned short) * 2 * (kAccThreads / 32) * (cap + 1);
-  };
-  auto small = accumulate_kernel<kSmallCap, kSmallParts>;
-  PE_CUDA(cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_for(kSmallCap)));
-  small<<<(unsigned)(C * kSmallParts), kAccThreads, smem_for(kSmallCap), stream>>>(
-      list, cursor, ranks, flags, chain_stride, det_stride, scores, positives, hist, ws_key, ws_idx, C, seg_ws,
-      env_ws, precision, recall, chain_stats, -1);
-  PE_LAUNCHED("accumulate");
-  count_launch();
-  if (n > kSmallCap) {
-    auto large = accumulate_kernel<kSortCap, kAccParts>;
-    PE_CUDA(cudaFuncSetAttribute(large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_for(kSortCap)));
-    large<<<(unsigned)(C * kAccParts), kAccThreads, smem_for(kSortCap), stream>>>(
-        list, cursor, ranks, flags, chain_stride, det_stride, scores, positives, hist, ws_key, ws_idx, C, seg_ws,
-        env_ws, precision, recall, chain_stats, kSmallCap);
-    PE_LAUNCHED("accumulate(large classes)");
-    count_launch();
-  }
+  // Classes of up to kSmallCap records in a smaller stage; when some class can be larger, a second launch
+  // takes those (staged up to kSortCap, else in the workspace).
+  int status = launch_accumulate_cap<kSmallCap>(classes, n, list, cursor, hist, ranks, flags, chain_stride, det_stride,
+                                                scores, positives, ws_key, ws_idx, C, env_ws, precision, recall,
+                                                chain_stats, -1, stream);
+  if (status == kOk && n > kSmallCap)
+    status = launch_accumulate_cap<kSortCap>(classes, n, list, cursor, hist, ranks, flags, chain_stride, det_stride,
+                                             scores, positives, ws_key, ws_idx, C, env_ws, precision, recall,
+                                             chain_stats, kSmallCap, stream);
+  if (status != kOk) return status;
   if (summary) {
     summarize_chains_kernel<<<12, kSummarizeThreads, 0, stream>>>(chain_stats, C, summary);
     PE_LAUNCHED("summarize_chains");
