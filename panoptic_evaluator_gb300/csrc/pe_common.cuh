@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <climits>
 #include <algorithm>
+#include <initializer_list>
 
 #include "pe_gb300.h"
 
@@ -58,6 +59,13 @@ void set_error(const char* fmt, ...);
 
 int sm_count();            // SMs of the current device (cached per device)
 int current_device();
+// Zeroes buffers on the stream, those that follow one another in memory with one memset (a memset costs
+// about 2 us of host time and 1.4 us of the stream). A Status.
+struct ZeroSpan {
+  void* ptr;
+  int64_t bytes;
+};
+int zero_spans(std::initializer_list<ZeroSpan> spans, cudaStream_t stream);
 void count_launch(int n = 1);  // launch counter exposed through pe_launch_count()
 
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }

@@ -876,9 +876,8 @@ PE_API int pe_inst_contract(const int64_t* descs, const int64_t* blocks, int64_t
   PE_REQUIRE(n_blocks >= 0 && total_chunks >= 0 && inter_len >= 0 && pa_len >= 0 && ga_len >= 0, "invalid batch");
   PE_REQUIRE(n_blocks > 0 || total_chunks == 0, "chunks without blocks");
   PE_REQUIRE((reinterpret_cast<uintptr_t>(maps) & 63) == 0, "tensor maps must be 64-byte aligned");
-  if (inter_len) PE_CUDA(cudaMemsetAsync(inter, 0, sizeof(uint32_t) * inter_len, stream));
-  if (pa_len) PE_CUDA(cudaMemsetAsync(pa, 0, sizeof(uint64_t) * pa_len, stream));
-  if (ga_len) PE_CUDA(cudaMemsetAsync(ga, 0, sizeof(uint64_t) * ga_len, stream));
+  const int zeroed = zero_spans({{inter, 4 * inter_len}, {pa, 8 * pa_len}, {ga, 8 * ga_len}}, stream);
+  if (zeroed != kOk) return zeroed;
   if (total_chunks == 0) return kOk;
   PE_REQUIRE(!cta_bounds || (ctas > 0 && ctas <= INT_MAX), "invalid CTA count");
   const int64_t even = std::min<int64_t>(total_chunks, sm_count());

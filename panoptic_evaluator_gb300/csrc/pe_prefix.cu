@@ -21,44 +21,24 @@
 //                    them into precision / recall over the whole grid.
 //   5. pe_compute    per-checkpoint PQ/SQ/RQ/IoU summaries.
 #include "pe_common.cuh"
+#include "pe_fields.h"
 #include "pe_score.cuh"
 #include "pe_bins.cuh"
 
 namespace pe {
 namespace {
 
-// Descriptor fields (int64 each).
-enum : int {
-  kPTarget = 0,   // int32 target slot map
-  kPMasks,        // uint8 0/1 masks in generation order, rows kPStride bytes apart
-  kPPixels,
-  kPStride,
-  kPChunkBegin,   // first 4096-pixel chunk of this image
-  kPN,            // masks
-  kPG,            // target slots
-  kPDetBegin,     // offset into flat per-mask arrays (classes) and raw rows / N
-  kPSlotBegin,    // offset into flat per-slot arrays (gc, crowd, ga)
-  kPQBegin,       // first output row (checkpoint) of this image
-  kPQ,            // checkpoints of this image
-  kPPairBegin,    // offset of this image's [Q][G][N+1] histograms
-  kPRawBegin,     // offset of this image's [N][G] raw intersections
-  kPFlags,        // bit 0: target map 16-byte vectorisable, bit 1: mask rows 16-byte vectorisable
-  kPStepBegin,    // offset of this image's step table (N+1 entries: checkpoint index or -1)
-  kPCountBegin,   // offset of this image's [T][C][2] matching counters
-  kPFields
-};
-
 constexpr int kPxThreads = 256;
 constexpr int kPxChunk = kPxThreads * 16;
 constexpr int kPxWindow = 4;  // masks whose 16-byte words each lane loads before processing them
 
-__device__ __forceinline__ const int64_t* pdesc(const int64_t* descs, int64_t b) { return descs + b * kPFields; }
+__device__ __forceinline__ const int64_t* pdesc(const int64_t* descs, int64_t b) { return descs + b * kPrefixFields; }
 
 __device__ __forceinline__ int64_t find_image(const int64_t* descs, int64_t B, int field, int64_t value) {
   int64_t lo = 0, hi = B - 1;
   while (lo < hi) {
     const int64_t mid = (lo + hi + 1) >> 1;
-    if (descs[mid * kPFields + field] <= value) lo = mid; else hi = mid - 1;
+    if (descs[mid * kPrefixFields + field] <= value) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
@@ -322,24 +302,24 @@ template <bool kBytes>
 __global__ void __launch_bounds__(kPxThreads, 2)
 prefix_pass_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __restrict__ step_q, u32* __restrict__ ga,
                    u32* __restrict__ raw, int* __restrict__ delta, int* __restrict__ error) {
-  const int64_t b = find_image(descs, B, kPChunkBegin, blockIdx.x);
+  const int64_t b = find_image(descs, B, kPrefixChunkBegin, blockIdx.x);
   const int64_t* d = pdesc(descs, b);
-  const int64_t pixels = d[kPPixels];
-  const int64_t x = (blockIdx.x - d[kPChunkBegin]) * (int64_t)kPxChunk + (int64_t)threadIdx.x * 16;
-  const int N = (int)d[kPN], G = (int)d[kPG];
-  const int* target = reinterpret_cast<const int*>(d[kPTarget]);
-  const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kPMasks]);
-  const int64_t stride = d[kPStride];
-  const bool vec_map = d[kPFlags] & 1, vec_masks = d[kPFlags] & 2;
-  const int* steps = step_q + d[kPStepBegin];
-  int* delta_img = delta + d[kPPairBegin];
-  u32* raw_img = raw + d[kPRawBegin];
+  const int64_t pixels = d[kPrefixPixels];
+  const int64_t x = (blockIdx.x - d[kPrefixChunkBegin]) * (int64_t)kPxChunk + (int64_t)threadIdx.x * 16;
+  const int N = (int)d[kPrefixN], G = (int)d[kPrefixG];
+  const int* target = reinterpret_cast<const int*>(d[kPrefixTarget]);
+  const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kPrefixMasks]);
+  const int64_t stride = d[kPrefixStride];
+  const bool vec_map = d[kPrefixFlags] & 1, vec_masks = d[kPrefixFlags] & 2;
+  const int* steps = step_q + d[kPrefixStepBegin];
+  int* delta_img = delta + d[kPrefixPairBegin];
+  u32* raw_img = raw + d[kPrefixRawBegin];
   const int64_t plane = (int64_t)G * (N + 1);
   const int lane = threadIdx.x & 31;
 
   int t[16];
   load16_maps(target, x, pixels, vec_map, t);
-  const bool bad = count_target(t, x, pixels, G, ga + d[kPSlotBegin], lane);
+  const bool bad = count_target(t, x, pixels, G, ga + d[kPrefixSlotBegin], lane);
   const LaneSlots ls = lane_slots(t, x, pixels, G);
   const LanePeers lp = lane_peers(ls, lane);
   const u32 valid = ls.e1 | ls.e2 | ls.emid;
@@ -445,16 +425,16 @@ prefix_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t to
         ok = false;
         break;
       }
-      const int64_t* d = pdesc(descs, find_image(descs, B, kPChunkBegin, chunk));
-      const int64_t pixels = d[kPPixels];
-      const int64_t x0 = (chunk - d[kPChunkBegin]) * (int64_t)kPxChunk;
+      const int64_t* d = pdesc(descs, find_image(descs, B, kPrefixChunkBegin, chunk));
+      const int64_t pixels = d[kPrefixPixels];
+      const int64_t x0 = (chunk - d[kPrefixChunkBegin]) * (int64_t)kPxChunk;
       const int64_t len = min((int64_t)kPxChunk, pixels - x0);
-      const int N = (int)d[kPN];
-      const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kPMasks]);
-      const int64_t stride = d[kPStride];
-      const int* target = reinterpret_cast<const int*>(d[kPTarget]);
+      const int N = (int)d[kPrefixN];
+      const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kPrefixMasks]);
+      const int64_t stride = d[kPrefixStride];
+      const int* target = reinterpret_cast<const int*>(d[kPrefixTarget]);
       const uint32_t map_bytes = (uint32_t)((len * 4) & ~15ll);
-      if ((d[kPFlags] & 1) && map_bytes) bulk_prefetch_l2(target + x0, map_bytes);
+      if ((d[kPrefixFlags] & 1) && map_bytes) bulk_prefetch_l2(target + x0, map_bytes);
       for (int r0 = 0; r0 < N; r0 += kPbStage) {
         const int slot = (int)(seq % kPbRing);
         const int64_t use = seq / kPbRing;
@@ -506,20 +486,20 @@ prefix_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t to
     if (lane == 0) mbar_arrive(&sm.chunk_empty[e]);
     ++taken;
     if (chunk < 0) break;
-    const int64_t* d = pdesc(descs, find_image(descs, B, kPChunkBegin, chunk));
-    const int64_t pixels = d[kPPixels];
-    const int64_t x0 = (chunk - d[kPChunkBegin]) * (int64_t)kPxChunk;
+    const int64_t* d = pdesc(descs, find_image(descs, B, kPrefixChunkBegin, chunk));
+    const int64_t pixels = d[kPrefixPixels];
+    const int64_t x0 = (chunk - d[kPrefixChunkBegin]) * (int64_t)kPxChunk;
     const int64_t x = x0 + (int64_t)threadIdx.x * 16;
-    const int N = (int)d[kPN], G = (int)d[kPG];
-    const int* steps = step_q + d[kPStepBegin];
+    const int N = (int)d[kPrefixN], G = (int)d[kPrefixG];
+    const int* steps = step_q + d[kPrefixStepBegin];
     const int64_t plane = (int64_t)G * (N + 1);
-    const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kPMasks]);
-    const int64_t stride = d[kPStride];
-    int* delta_img = delta + d[kPPairBegin];
-    u32* raw_img = raw + d[kPRawBegin];
+    const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kPrefixMasks]);
+    const int64_t stride = d[kPrefixStride];
+    int* delta_img = delta + d[kPrefixPairBegin];
+    u32* raw_img = raw + d[kPrefixRawBegin];
     int t[16];
-    load16_maps(reinterpret_cast<const int*>(d[kPTarget]), x, pixels, d[kPFlags] & 1, t);
-    bad |= count_target(t, x, pixels, G, ga + d[kPSlotBegin], lane);
+    load16_maps(reinterpret_cast<const int*>(d[kPrefixTarget]), x, pixels, d[kPrefixFlags] & 1, t);
+    bad |= count_target(t, x, pixels, G, ga + d[kPrefixSlotBegin], lane);
     const LaneSlots ls = lane_slots(t, x, pixels, G);
     const LanePeers lp = lane_peers(ls, lane);
     const u32 valid = ls.e1 | ls.e2 | ls.emid;  // pixels past the image end are not valid: stale bytes ignored
@@ -581,13 +561,13 @@ prefix_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t to
 __global__ void prefix_scan_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ ga,
                                    int* __restrict__ delta) {
   const int64_t* d = pdesc(descs, blockIdx.y);
-  const int N = (int)d[kPN], G = (int)d[kPG], Q = (int)d[kPQ];
+  const int N = (int)d[kPrefixN], G = (int)d[kPrefixG], Q = (int)d[kPrefixQ];
   const int64_t plane = (int64_t)G * (N + 1);
   const int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (cell >= plane) return;
-  int* base = delta + d[kPPairBegin] + cell;
+  int* base = delta + d[kPrefixPairBegin] + cell;
   const int g = (int)(cell / (N + 1)), j = (int)(cell % (N + 1));
-  int v = j == 0 ? (int)ga[d[kPSlotBegin] + g] : 0;
+  int v = j == 0 ? (int)ga[d[kPrefixSlotBegin] + g] : 0;
   for (int q = 0; q < Q; ++q) {
     v += base[(int64_t)q * plane];
     base[(int64_t)q * plane] = v;
@@ -606,14 +586,14 @@ prefix_score_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __r
                     double* __restrict__ sums, int64_t* __restrict__ confusion, int smem) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t row = blockIdx.x;
-  const int64_t b = find_image(descs, B, kPQBegin, row);
+  const int64_t b = find_image(descs, B, kPrefixQBegin, row);
   const int64_t* d = pdesc(descs, b);
-  const int N = (int)d[kPN], G = (int)d[kPG], P = N + 1;
-  const int q = (int)(row - d[kPQBegin]);
-  const u32* pq = reinterpret_cast<const u32*>(pairs + d[kPPairBegin] + (int64_t)q * G * P);
-  gc += d[kPSlotBegin];
-  crowd += d[kPSlotBegin];
-  classes += d[kPDetBegin];
+  const int N = (int)d[kPrefixN], G = (int)d[kPrefixG], P = N + 1;
+  const int q = (int)(row - d[kPrefixQBegin]);
+  const u32* pq = reinterpret_cast<const u32*>(pairs + d[kPrefixPairBegin] + (int64_t)q * G * P);
+  gc += d[kPrefixSlotBegin];
+  crowd += d[kPrefixSlotBegin];
+  classes += d[kPrefixDetBegin];
   ScoreOut out{reinterpret_cast<u64*>(tp + row * C), reinterpret_cast<u64*>(fp + row * C),
                reinterpret_cast<u64*>(fn + row * C), sums + row * C,
                reinterpret_cast<u64*>(confusion + row * C * (int64_t)(C + 1))};
@@ -658,14 +638,14 @@ prefix_match_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ g
                     int validate, int* __restrict__ error) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t* d = pdesc(descs, blockIdx.x);
-  const int N = (int)d[kPN], G = (int)d[kPG];
-  const int64_t qb = d[kPQBegin];
-  const int* steps = step_q + d[kPStepBegin];
-  ga += d[kPSlotBegin];
-  gc += d[kPSlotBegin];
-  crowd += d[kPSlotBegin];
-  classes += d[kPDetBegin];
-  raw += d[kPRawBegin];
+  const int N = (int)d[kPrefixN], G = (int)d[kPrefixG];
+  const int64_t qb = d[kPrefixQBegin];
+  const int* steps = step_q + d[kPrefixStepBegin];
+  ga += d[kPrefixSlotBegin];
+  gc += d[kPrefixSlotBegin];
+  crowd += d[kPrefixSlotBegin];
+  classes += d[kPrefixDetBegin];
+  raw += d[kPrefixRawBegin];
   const int words = (G + 31) / 32;
   u64* areas = reinterpret_cast<u64*>(smem_raw);                   // N mask areas on valid slots
   long long* iou_all = reinterpret_cast<long long*>(areas + N);    // candidate IoU bit patterns (kStaged)
@@ -894,7 +874,7 @@ __global__ void prefix_ratio_kernel(const int64_t* __restrict__ itp, const int64
 
 using namespace pe;
 
-PE_API int pe_prefix_desc_fields(void) { return kPFields; }
+PE_API int pe_prefix_desc_fields(void) { return kPrefixFields; }
 
 // Batched segmentation_prefixes (prefix.py:12-122; replaces the `prefix` op,
 // prefix_kernel.cu:142-199, for any number of images). Inputs: descriptor
@@ -920,19 +900,16 @@ PE_API int pe_prefix(const int64_t* descs, int64_t B, int64_t total_chunks, int6
   PE_REQUIRE(B >= 0 && total_rows >= 0 && C > 0 && C < INT_MAX && T > 0 && T <= 1024 && max_g >= 0 &&
                  max_p >= 1 && max_p < 65536,
              "invalid prefix batch (T must be 1..1024, masks per image < 65535)");
-  PE_CUDA(cudaMemsetAsync(error, 0, sizeof(int32_t), stream));
-  if (B == 0) return kOk;
-  if (ga_len) PE_CUDA(cudaMemsetAsync(ga, 0, 4 * ga_len, stream));
-  if (raw_len) PE_CUDA(cudaMemsetAsync(raw, 0, 4 * raw_len, stream));
-  if (pairs_len) PE_CUDA(cudaMemsetAsync(pairs, 0, 4 * pairs_len, stream));
-  if (counters_len) PE_CUDA(cudaMemsetAsync(counters, 0, 4 * counters_len, stream));
-  if (total_rows) {
-    PE_CUDA(cudaMemsetAsync(tp, 0, 8 * total_rows * C, stream));
-    PE_CUDA(cudaMemsetAsync(fp, 0, 8 * total_rows * C, stream));
-    PE_CUDA(cudaMemsetAsync(fn, 0, 8 * total_rows * C, stream));
-    PE_CUDA(cudaMemsetAsync(sums, 0, 8 * total_rows * C, stream));
-    PE_CUDA(cudaMemsetAsync(confusion, 0, 8 * total_rows * C * (C + 1), stream));
+  if (B == 0) {
+    PE_CUDA(cudaMemsetAsync(error, 0, sizeof(int32_t), stream));
+    return kOk;
   }
+  const int64_t rows = 8 * total_rows * C;
+  const int zeroed = zero_spans({{ga, 4 * ga_len}, {raw, 4 * raw_len}, {pairs, 4 * pairs_len},
+                                 {counters, 4 * counters_len}, {error, 4}, {tp, rows}, {fp, rows}, {fn, rows},
+                                 {sums, rows}, {confusion, rows * (C + 1)}},
+                                stream);
+  if (zeroed != kOk) return zeroed;
   if (total_chunks) {
     if (bulk) {
       const int64_t grid = std::min(total_chunks, (int64_t)sm_count() * 2);  // two CTAs per SM

@@ -39,6 +39,23 @@ int sm_count() {
   return g_sm_counts[device];
 }
 
+int zero_spans(std::initializer_list<ZeroSpan> spans, cudaStream_t stream) {
+  char* begin = nullptr;
+  int64_t bytes = 0;
+  for (const ZeroSpan& span : spans) {
+    if (span.bytes <= 0) continue;
+    if (bytes && static_cast<char*>(span.ptr) == begin + bytes) {
+      bytes += span.bytes;
+      continue;
+    }
+    if (bytes) PE_CUDA(cudaMemsetAsync(begin, 0, (size_t)bytes, stream));
+    begin = static_cast<char*>(span.ptr);
+    bytes = span.bytes;
+  }
+  if (bytes) PE_CUDA(cudaMemsetAsync(begin, 0, (size_t)bytes, stream));
+  return kOk;
+}
+
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
 }  // namespace pe

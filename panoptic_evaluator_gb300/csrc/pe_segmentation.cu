@@ -791,8 +791,9 @@ PE_API int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, co
   PE_REQUIRE(B >= 0 && total_chunks >= 0 && pairs_len >= 0 && dpairs_len >= 0, "invalid batch");
   // Keys of one image are G*P + D*G < 2^32 - 1 (pan_cap, det_cap: largest per-image G*P and D*G).
   PE_REQUIRE(pan_cap >= 0 && det_cap >= 0 && pan_cap + det_cap < (int64_t)UINT32_MAX, "histogram too large");
-  if (pairs_len) PE_CUDA(cudaMemsetAsync(pairs, 0, sizeof(uint32_t) * pairs_len, stream));
-  if (dpairs_len) PE_CUDA(cudaMemsetAsync(dpairs, 0, sizeof(uint32_t) * dpairs_len, stream));
+  const bool counted = bulk && schedule && B > 0 && total_chunks > 0;  // chunks from the counter
+  const int zeroed = zero_spans({{pairs, 4 * pairs_len}, {dpairs, 4 * dpairs_len}, {schedule, counted ? 8 : 0}}, stream);
+  if (zeroed != kOk) return zeroed;
   if (B == 0 || total_chunks == 0) return kOk;
   PE_REQUIRE(!cta_bounds || (ctas > 0 && ctas <= INT_MAX), "invalid CTA count");
   if (bulk) {
@@ -801,7 +802,6 @@ PE_API int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, co
     const int64_t per_cta = ceil_div(total_chunks, std::min(total_chunks, max_ctas));
     int64_t grid = cta_bounds ? ctas : ceil_div(total_chunks, per_cta);
     if (schedule) {  // chunks taken from the counter, `grab` at a time, by the chosen CTAs per SM
-      PE_CUDA(cudaMemsetAsync(schedule, 0, sizeof(uint64_t), stream));
       grid = std::min(ceil_div(total_chunks, choice.grab), (int64_t)sm_count() * choice.per_sm);
       cta_bounds = nullptr;
     }
