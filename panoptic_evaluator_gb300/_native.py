@@ -125,11 +125,47 @@ def on_device(device):
 
 def call(name, *args):
     """Invoke an entry point; negative statuses raise, others are returned."""
-    status = getattr(library(), name)(*args)
+    return check(name, getattr(library(), name)(*args))
+
+
+def check(name, status):
+    """Raise for a negative status of an entry point, else return it."""
     if status < 0:
         message = library().pe_last_error().decode(errors="replace")
         raise NativeError(f"{name}: {message} (status {status})")
     return status
+
+
+_call = call
+_host = None
+
+
+def host():
+    """The C++ host path (``_host.so``), or None while ``call`` is replaced.
+
+    Each of its functions takes a whole step (checks, tables, launches, result
+    views) for plain arguments and returns None for anything else, which then
+    takes the Python path. A replaced ``call`` (timing hooks, tests) sees every
+    entry point, so it gets the Python path too.
+    """
+    if call is not _call:
+        return None
+    return _host if _host is not None else _load_host()
+
+
+def _load_host():
+    global _host
+    lib = library()
+    with _lock:
+        if _host is None:
+            try:
+                from . import _host as module
+            except ImportError as error:
+                raise RuntimeError("_host.so is not built for this Python and torch; run "
+                                   "`python -m panoptic_evaluator_gb300.build`") from error
+            module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in SIGNATURES})
+            _host = module
+    return _host
 
 
 def size(name, *args) -> int:

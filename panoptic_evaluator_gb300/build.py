@@ -2,6 +2,8 @@
 
 Each ``csrc/*.cu`` translation unit is compiled in parallel with nvcc for
 ``sm_103a`` only, then linked into ``panoptic_evaluator_gb300/libpe_gb300.so``.
+Beside them ``csrc/host.cpp``, the evaluators' host path against torch's C++
+API, becomes the extension module ``panoptic_evaluator_gb300/_host.so``.
 Objects go to ``_build/`` at the repository root. Rebuilds only when a source
 or header is newer than the library.
 
@@ -23,6 +25,8 @@ CSRC = PACKAGE / "csrc"
 ROOT = PACKAGE.parent
 BUILD = ROOT / "_build"
 LIBRARY = PACKAGE / "libpe_gb300.so"
+HOST_SOURCE = CSRC / "host.cpp"
+HOST_MODULE = PACKAGE / "_host.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC,-fvisibility=hidden",
          "-I", str(CSRC), "-I", str(ROOT / "include")]
@@ -40,11 +44,36 @@ def sources():
 
 
 def stale() -> bool:
-    if not LIBRARY.exists():
+    if not LIBRARY.exists() or not HOST_MODULE.exists():
         return True
-    built = LIBRARY.stat().st_mtime
-    inputs = list(sources()) + list(CSRC.glob("*.cuh")) + list((ROOT / "include").glob("*.h")) + [Path(__file__)]
+    built = min(LIBRARY.stat().st_mtime, HOST_MODULE.stat().st_mtime)
+    inputs = [*sources(), HOST_SOURCE, *CSRC.glob("*.cuh"), *CSRC.glob("*.h"), *(ROOT / "include").glob("*.h"),
+              Path(__file__)]
     return any(path.stat().st_mtime > built for path in inputs)
+
+
+def compile_host(verbose: bool = False) -> Path:
+    """csrc/host.cpp -> _host.so, against the installed torch."""
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc()).resolve().parent.parent
+    include = [root / "include", root / "include/torch/csrc/api/include", sysconfig.get_paths()["include"],
+               cuda / "include", CSRC, ROOT / "include"]
+    libraries = [root / "lib", cuda / "lib64"]
+    tmp = HOST_MODULE.with_suffix(".so.tmp")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{p}" for p in include],
+           str(HOST_SOURCE), "-o", str(tmp), *[f"-L{p}" for p in libraries], "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-ltorch_python", "-lcudart"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    result = subprocess.run(cmd, capture_output=True, text=True)
+    if result.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed for {HOST_SOURCE.name}:\n{result.stdout}\n{result.stderr}")
+    os.replace(tmp, HOST_MODULE)
+    return HOST_MODULE
 
 
 def build(force: bool = False, verbose: bool = False, extra: list[str] | None = None) -> Path:
@@ -66,8 +95,10 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
             print(result.stdout + result.stderr, flush=True)
         return obj
 
-    with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+    with ThreadPoolExecutor(max_workers=min(9, os.cpu_count() or 1)) as pool:
+        host = pool.submit(compile_host, verbose)
         objects = list(pool.map(compile_one, sources()))
+        host.result()
     tmp = LIBRARY.with_suffix(".so.tmp")
     cmd = [compiler, *ARCH, "-shared", "-o", str(tmp), *map(str, objects), "-lcudart"]
     result = subprocess.run(cmd, capture_output=True, text=True)

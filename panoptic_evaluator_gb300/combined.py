@@ -41,6 +41,19 @@ _COMBINED_ERRORS = (
 )
 
 
+def _host():
+    """The C++ host path while the module's hooks and switches are at their defaults, else None."""
+    return N.host() if PASS_EVENTS is None and BULK_PASS and DYNAMIC_PASS else None
+
+
+def raise_combined_error(code: int):
+    if code & (8 | 16 | 32 | 64):
+        for bit, message in _COMBINED_ERRORS:
+            if code & bit:
+                raise ValueError(message)
+    raise_validation(code)
+
+
 class SegmentationEvaluator:
     """PQ/mIoU and mask AP/AR with separate predictions and one shared target (combined.py:18-167).
 
@@ -80,10 +93,19 @@ class SegmentationEvaluator:
             raise ValueError("instance_areas must be floating point B x S on evaluator device")
         return areas.to(torch.float64).contiguous()
 
-    @torch.no_grad()
     def update(self, prediction: PanopticBatch, detections: InstanceBatch, target: PanopticBatch, *,
                instance_areas: torch.Tensor | None = None):
         """Accumulate all metrics; optional annotation areas have shape B x S (combined.py:63-161)."""
+        host = _host() if instance_areas is None else None
+        if host is not None:
+            code = host.combined_update(self, prediction, detections, target)
+            if code is not None:
+                raise_combined_error(N.check("combined update", code))
+                return self
+        return self._update(prediction, detections, target, instance_areas)
+
+    @torch.no_grad()
+    def _update(self, prediction, detections, target, instance_areas):
         target = target.compact()
         prediction = prediction.compact()
         if target.crowd is None:
@@ -106,7 +128,6 @@ class SegmentationEvaluator:
                   [H * W] * B)
         return self
 
-    @torch.no_grad()
     def update_images(self, images):
         """Accumulate a batch of uneven images packed in a ``ragged.SegmentationImages`` arena.
 
@@ -119,6 +140,16 @@ class SegmentationEvaluator:
         if images.B == 0:
             return self
         table = images.table(self.instance._scratch)
+        host = _host()
+        if host is not None:
+            code = host.images_update(self, table, images.device, images.field_offsets)
+            if code is not None:
+                raise_combined_error(N.check("combined update", code))
+                return self
+        return self._update_images(images, table)
+
+    @torch.no_grad()
+    def _update_images(self, images, table):
         launch(self, table, images.tensor("target_classes"), images.tensor("pred_classes"), images.tensor("crowd"),
                images.tensor("det_classes"), images.tensor("scores"),
                images.tensor("areas") if images.has_areas else None)
@@ -132,6 +163,12 @@ class SegmentationEvaluator:
         both before this returns, so callers see one ordered stream (and a CUDA
         graph capture sees a fork and a join).
         """
+        host = N.host()
+        if host is not None:
+            outcome = host.combined_compute(self)
+            if outcome is not None:
+                N.check("combined compute", outcome[0])
+                return outcome[1]
         side = self._side
         if side is None:
             result = self.panoptic.compute()
@@ -248,10 +285,5 @@ def launch(ev, table, gc, pc, crowd_u8, det_classes, det_scores, ann):
                C, max_g, N.ptr(out_flags), 1, CHAINS, N.ptr(out_ranks), N.ptr(inst._counts), N.ptr(error),
                N.ptr(class_bits), stream)
     if ev.validate:
-        code = int(error.item())
-        if code & (8 | 16 | 32 | 64):
-            for bit, message in _COMBINED_ERRORS:
-                if code & bit:
-                    raise ValueError(message)
-        raise_validation(code)
+        raise_combined_error(int(error.item()))
     store.n += total_d

@@ -67,6 +67,14 @@ class PanopticBatch:
                 maps = decode_rgb(maps)
         elif maps.ndim != 3 or maps.dtype not in (torch.int32, torch.int64):
             raise ValueError("maps must be integer B x H x W tensors (or uint8 B x H x W x 3 RGB)")
+        host = N.host() if compact and maps.is_cuda else None
+        if host is not None:
+            slots = host.coco_slots(maps, segments_info, category_ids)
+            if slots is not None:
+                code, packed, table_classes, table_crowd = slots
+                if N.check("pe_pack_rgb" if packed.shape != maps.shape else "pe_pack", code):
+                    raise ValueError("map contains a segment absent from segments_info")
+                return PanopticBatch(packed, table_classes, table_crowd)
         if len(segments_info) != maps.shape[0] or len(set(category_ids)) != len(category_ids):
             raise ValueError("batch length or category IDs are invalid")
         index = {category: i for i, category in enumerate(category_ids)}
@@ -219,7 +227,9 @@ class PanopticEvaluator:
 
     def reset(self):
         if hasattr(self, "_state"):
-            self._state.zero_()  # one fill clears every accumulator (0.0 is the all-zero bit pattern)
+            host = N.host()  # one fill clears every accumulator (0.0 is the all-zero bit pattern)
+            if host is None or host.zero(self._state) is None:
+                self._state.zero_()
             return
         C = self.num_classes
         # tp, fp, fn [C], iou_sum [C] (float64) and confusion [C, C + 1] are views of one allocation. The last
@@ -246,8 +256,13 @@ class PanopticEvaluator:
             target.copy_(value.to(device=target.device, dtype=target.dtype))
         return self
 
-    @torch.no_grad()
     def update(self, prediction: PanopticBatch, target: PanopticBatch):
+        host = N.host()
+        if host is not None:
+            code = host.panoptic_update(self, prediction, target)
+            if code is not None:
+                raise_validation(N.check("pe_update", code))
+                return self
         return self._update(prediction, target)
 
     def _scratch_for(self, B, G, P, device):
@@ -289,9 +304,18 @@ class PanopticEvaluator:
         raise_validation(code)
         return scratch[1][:, :G] if return_areas else self
 
-    @torch.no_grad()
     def compute(self) -> dict:
         """Device tensors in [0, 1]; absent classes have zero PQ and NaN IoU (evaluator.py:419-447)."""
+        host = N.host()
+        if host is not None:
+            outcome = host.panoptic_compute(self)
+            if outcome is not None:
+                N.check("pe_compute", outcome[0])
+                return outcome[1]
+        return self._compute()
+
+    @torch.no_grad()
+    def _compute(self) -> dict:
         rows, s, n, miou, copies = native.compute_one(self.tp, self.fp, self.fn, self.iou_sum, self.confusion,
                                                       self.isthing, self.num_classes)
         tp, fp, fn, sums, confusion = copies
@@ -302,7 +326,6 @@ class PanopticEvaluator:
         return result
 
 
-@torch.no_grad()
 def panoptic_quality(prediction: PanopticBatch, target: PanopticBatch, num_classes: int, reduction: str = "none",
                      *, validate: bool = True, return_stats: bool = False) -> torch.Tensor:
     """Stateless mean-class PQ per image, float64 on the input device (evaluator.py:471-544).
@@ -314,6 +337,17 @@ def panoptic_quality(prediction: PanopticBatch, target: PanopticBatch, num_class
         raise ValueError("num_classes must be a positive integer")
     if reduction != "none":
         raise ValueError('reduction must be "none"')
+    host = N.host() if not return_stats and target.segment_map.is_cuda else None
+    if host is not None:
+        outcome = host.reward(prediction, target, num_classes, validate)
+        if outcome is not None:
+            raise_validation(N.check("pe_update", outcome[0]))
+            return outcome[1]
+    return _panoptic_quality(prediction, target, num_classes, validate, return_stats)
+
+
+@torch.no_grad()
+def _panoptic_quality(prediction, target, num_classes, validate, return_stats):
     gt, gc, crowd = _prepare(target, num_classes)
     pred, pc, _ = _prepare(prediction, num_classes, ignore_crowd=True)
     if gt.shape != pred.shape or gt.device != pred.device:

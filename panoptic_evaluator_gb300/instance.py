@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from . import _native as N
-from ._batch import (CHAINS, CHUNK_BEGIN, D, DET_BEGIN, DPAIR_BEGIN, FLAGS, G, INST_CHUNK, MASK_STRIDE, MASKS, PIXELS,
+from ._batch import (CHAINS, CHUNK_BEGIN, CONTRACT_TMA_COST, D, DET_BEGIN, DPAIR_BEGIN, FLAGS, G, INST_CHUNK, MASK_STRIDE, MASKS, PIXELS,
                      SLOT_BEGIN, TARGET, DescTable, RecordStore, Scratch, aligned, contract_blocks)
 
 # Mask-vs-mask counts: "tensor" runs the tcgen05 contraction (pe_inst_contract),
@@ -241,12 +241,15 @@ class InstanceEvaluator:
             self.device = torch.device("cuda", torch.cuda.current_device())
         self.validate = validate
         self._scratch = Scratch(self.device)
+        self._arena = None  # the C++ host path's scratch
         self._store = RecordStore(self.device)
-        self.reset()
+        self._counts = torch.zeros((num_classes, 4), dtype=torch.int64, device=self.device)
 
     def reset(self):
         self._store.reset()
-        self._counts = torch.zeros((self.num_classes, 4), dtype=torch.int64, device=self.device)
+        host = N.host()
+        if host is None or host.zero(self._counts) is None:
+            self._counts.zero_()
 
     @property
     def num_records(self):
@@ -280,8 +283,18 @@ class InstanceEvaluator:
         self._counts.copy_(counts.to(dev, torch.int64))
         return self
 
-    @torch.no_grad()
     def update(self, prediction: InstanceBatch, target: InstanceBatch):
+        host = N.host() if CONTRACTION == "tensor" and DIRECT_CONTRACTION else None
+        if host is not None:
+            from . import tuning
+            code = host.instance_update(self, prediction, target, tuning.contract_costs(), CONTRACT_TMA_COST)
+            if code is not None:
+                raise_instance_error(N.check("instance update", code))
+                return self
+        return self._update(prediction, target)
+
+    @torch.no_grad()
+    def _update(self, prediction: InstanceBatch, target: InstanceBatch):
         pred_shapes, pred_kinds = check_instance_batch(prediction, self.device, prediction=True)
         gt_shapes, gt_kinds = check_instance_batch(target, self.device, prediction=False)
         B = len(prediction.masks)
@@ -380,9 +393,18 @@ class InstanceEvaluator:
         store.n += total_d
         return self
 
-    @torch.no_grad()
     def compute(self):
         """COCO AP/AR summaries plus full precision / recall arrays."""
+        host = N.host()
+        if host is not None:
+            outcome = host.instance_compute(self)
+            if outcome is not None:
+                N.check("pe_instance_accumulate", outcome[0])
+                return outcome[1]
+        return self._compute()
+
+    @torch.no_grad()
+    def _compute(self):
         return accumulate_records(self._store, self._counts, self.num_classes, self._scratch)
 
 

@@ -13,6 +13,7 @@ from __future__ import annotations
 import itertools
 import math
 from collections.abc import Mapping
+from functools import partial
 
 import numpy as np
 import torch
@@ -96,10 +97,10 @@ def _output_layout(R, T, C):
 class PackedOutputs(Mapping):
     """pe_prefix's outputs: named views of one int64 allocation, each made on first access and kept."""
 
-    __slots__ = ("flat", "_layout", "_views")
+    __slots__ = ("flat", "_layout", "_views", "_rows")
 
     def __init__(self, flat, layout):
-        self.flat, self._layout, self._views = flat, layout, {}
+        self.flat, self._layout, self._views, self._rows = flat, layout, {}, {}
 
     def __getitem__(self, key):
         view = self._views.get(key)
@@ -108,6 +109,13 @@ class PackedOutputs(Mapping):
             part = self.flat[offset: offset + math.prod(shape)]
             view = self._views[key] = (part if dtype is torch.int64 else part.view(dtype)).view(shape)
         return view
+
+    def rows(self, key):
+        """The rows of a field as a tuple of views, all made when the first one is read."""
+        rows = self._rows.get(key)
+        if rows is None:
+            rows = self._rows[key] = self[key].unbind(0)
+        return rows
 
     def __iter__(self):
         return iter(self._layout)
@@ -212,6 +220,11 @@ _METRICS = ("pq", "sq", "rq", "iou")
 _ROW_FIELDS = {"tp": "tp", "fp": "fp", "fn": "fn", "iou_sum": "sums", "confusion": "confusion", "miou": "miou"}
 
 
+def _row_of(out, r, key):
+    """Row r of a field (packed outputs keep the rows they have made)."""
+    return out.rows(key)[r] if type(out) is PackedOutputs else out[key][r]
+
+
 class Snapshot(Mapping):
     """One checkpoint's result dict (prefix.py:125-142), built lazily from the call's packed outputs.
 
@@ -236,20 +249,21 @@ class Snapshot(Mapping):
         cache = self._cache
         if key in cache:
             return cache[key]
-        out, r = self._out, self._row
+        r = self._row
+        row = partial(_row_of, self._out, r)
         if key == "prefix":
             value = self._prefix
         elif key in _ROW_FIELDS:
-            value = out[_ROW_FIELDS[key]][r]
+            value = row(_ROW_FIELDS[key])
         elif key in _GROUPS:
             i = _GROUPS.index(key)
-            summary, counts = out["summaries"][r, i], out["counts"][r]
-            value = dict(pq=summary[0], sq=summary[1], rq=summary[2], n=counts[i])
+            pq, sq, rq = row("summaries")[i].unbind(0)
+            value = dict(pq=pq, sq=sq, rq=rq, n=row("counts")[i])
         elif key == "per_class":
-            value = dict(zip(_METRICS, out["values"][r].unbind(0)))
+            value = dict(zip(_METRICS, row("values").unbind(0)))
         elif key == "instance":
-            value = dict(iou_thresholds=self._thr, tp=out["itp"][r], fp=out["ifp"][r], fn=out["ifn"][r],
-                         precision=out["precision"][r], recall=out["recall"][r])
+            value = dict(iou_thresholds=self._thr, tp=row("itp"), fp=row("ifp"), fn=row("ifn"),
+                         precision=row("precision"), recall=row("recall"))
         else:
             raise KeyError(key)
         cache[key] = value
@@ -291,7 +305,6 @@ def check_prefix_inputs(masks, classes, maps_shape, device, requested):
     return counts
 
 
-@torch.no_grad()
 def segmentation_prefixes(prediction: InstanceBatch, target: PanopticBatch, num_classes, *, isthing=None,
                           checkpoints=None, iou_thresholds=(0.5, 0.75), validate=True):
     """Evaluate independent masks in generation order, later masks drawn on top (prefix.py:12-27).
@@ -310,6 +323,25 @@ def segmentation_prefixes(prediction: InstanceBatch, target: PanopticBatch, num_
                               torch.uint8, device)
     if len(things) != num_classes:
         raise ValueError("isthing must contain one flag per category")
+    host = N.host() if BULK_PASS else None
+    if host is not None:
+        outcome = host.prefixes(prediction, target, num_classes, things, thresholds, requested, validate)
+        if outcome is not None:
+            code, flat, thr = outcome
+            N.check("pe_prefix", code)
+            if validate:
+                raise_prefix_error(code)
+            points = [requested if requested is not None else (range(1, len(m) + 1) if len(m) else (0,))
+                      for m in prediction.masks]
+            rows = list(itertools.accumulate(map(len, points), initial=0))
+            out = PackedOutputs(flat, _output_layout(rows[-1], len(thresholds), num_classes)[0])
+            return [unpack(out, row, image, thr) for row, image in zip(rows, points)]
+    return _segmentation_prefixes(prediction, target, num_classes, things, thresholds, requested, validate)
+
+
+@torch.no_grad()
+def _segmentation_prefixes(prediction, target, num_classes, things, thresholds, requested, validate):
+    device = target.segment_map.device
     target = target.compact()
     if target.crowd is None:
         from dataclasses import replace

@@ -77,6 +77,9 @@ class SegmentationImages:
             reserve("areas", self.G.sum(), np.float64)
         self.nbytes = _round(cursor)
         self.layout = layout
+        # Byte offsets of the flat metadata in the arena (annotation areas: -1 when there are none).
+        self.field_offsets = tuple(layout[name].offset if name in layout else -1 for name in (
+            "target_classes", "crowd", "pred_classes", "det_classes", "scores", "areas"))
         self.host = torch.empty(self.nbytes, dtype=torch.uint8, pin_memory=pin)
         buf = self.host.numpy()
         self.map_offset = np.zeros(B, np.int64)  # element offsets into the map arrays

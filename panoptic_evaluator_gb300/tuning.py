@@ -271,6 +271,11 @@ def forget_contract(tma_bucket: int) -> None:
     _contract_costs.pop(int(tma_bucket), None)
 
 
+def contract_costs() -> dict[int, float]:
+    """The tuned TMA block weights by bucket (not a copy)."""
+    return _contract_costs
+
+
 def contract_cost(tma_bucket: int) -> float:
     """The TMA block weight a batch in this bucket uses now (the built-in CONTRACT_TMA_COST without an entry)."""
     from ._batch import CONTRACT_TMA_COST
