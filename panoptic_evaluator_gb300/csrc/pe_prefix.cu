@@ -43,29 +43,6 @@ __device__ __forceinline__ int64_t find_image(const int64_t* descs, int64_t B, i
   return lo;
 }
 
-// Target areas of one lane's 16 pixels, run-combined per lane and warp-aggregated; false on a slot
-// outside [0, G).
-__device__ __forceinline__ bool count_target(const int (&t)[16], int64_t x, int64_t pixels, int G, u32* ga_img,
-                                             int lane) {
-  bool bad = false;
-  u32 key = kEmpty, n = 0;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    if (x + j >= pixels) continue;
-    if (t[j] < 0 || t[j] >= G) { bad = true; continue; }
-    if ((u32)t[j] != key) {
-      if (n) atomicAdd(ga_img + key, n);
-      key = (u32)t[j];
-      n = 0;
-    }
-    ++n;
-  }
-  const u32 peers = __match_any_sync(0xffffffffu, key);
-  const u32 total = __reduce_add_sync(peers, n);
-  if (lane == (int)(__ffs(peers) - 1) && total) atomicAdd(ga_img + key, total);
-  return bad;
-}
-
 // Visible owner (1-based mask index, 0 = none) of one lane's 16 pixels, now and at the previous
 // checkpoint: one byte per pixel when every image of the batch has at most 255 masks (kBytes), else
 // 16 bits per pixel. Drawing a mask is a byte (or half-word) select per register, so its cost does not
@@ -110,33 +87,15 @@ struct Owners {
   }
 };
 
-// True when some lane of the warp may hold a covered pixel in these staged words (a superset test on
-// the raw words, before they are re-aligned). Warp-uniform.
-__device__ __forceinline__ bool warp_may_cover(uint4 a, uint4 b, bool two) {
-  u32 any = a.x | a.y | a.z | a.w;
-  if (two) any |= b.x | b.y | b.z | b.w;
-  return __any_sync(0xffffffffu, (any & 0x01010101u) != 0);
-}
-
 // Draw mask i (its 16 bytes for this lane in w) over the lane's pixels: the raw mask x slot
 // intersections raw_row[slot] and the new owners. Called by every lane of the warp.
 template <bool kBytes>
-__device__ __forceinline__ void draw_mask(int i, uint4 w, const int (&t)[16], const LaneSlots& ls,
-                                          const LanePeers& lp, u32 valid, u32* raw_row, Owners<kBytes>& s) {
+__device__ __forceinline__ void draw_mask(int i, uint4 w, const int (&t)[16], const LaneSlots& ls, u32* raw_row,
+                                          Owners<kBytes>& s) {
   const u32 lsb[4] = {w.x & 0x01010101u, w.y & 0x01010101u, w.z & 0x01010101u, w.w & 0x01010101u};
   const auto pack4 = [](u32 v) { return (v * 0x01020408u) >> 24; };
-  const u32 m = (pack4(lsb[0]) | pack4(lsb[1]) << 4 | pack4(lsb[2]) << 8 | pack4(lsb[3]) << 12) & valid;
-  const u32 c1 = __popc(m & ls.e1), c2 = __popc(m & ls.e2);
-  const u32 t1 = __reduce_add_sync(lp.peers1, c1);
-  const u32 t2 = __reduce_add_sync(lp.peers2, c2);
-  if (lp.lead1 && t1) atomicAdd(raw_row + ls.s1, t1);
-  if (lp.lead2 && t2) atomicAdd(raw_row + ls.s2, t2);
-  const u32 mid = m & ls.emid;  // a third slot inside 16 pixels: rare
-  if (mid) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if ((mid >> j) & 1u) atomicAdd(raw_row + t[j], 1u);
-  }
+  const u32 m = pack4(lsb[0]) | pack4(lsb[1]) << 4 | pack4(lsb[2]) << 8 | pack4(lsb[3]) << 12;
+  add_slots(t, ls, m & ls.valid(), raw_row);
   s.draw(lsb, (u32)(i + 1));
 }
 
@@ -180,14 +139,40 @@ __device__ __forceinline__ int byte_at(const u32 (&v)[4], int j) {
   return (int)((w >> (8 * (j & 3))) & 0xffu);
 }
 
+// The lanes' first runs of equal (slot, old owner, new owner): summed over the lanes of the warp that share
+// one when many have a run (inside a large region every lane has the same transition), else lane by lane.
+__device__ __forceinline__ void add_first_run(int g, int o, int n, int count, int* dq, int N) {
+  if (__popc(__ballot_sync(0xffffffffu, count != 0)) >= kGroupLanes) {
+    // Owners are below 65536 (N < 65535), so (slot, old, new) packs into 64 bits.
+    const unsigned long long key =
+        count ? ((unsigned long long)(u32)g << 32) | ((unsigned long long)o << 16) | (unsigned long long)n : ~0ull;
+    const u32 peers = __match_any_sync(0xffffffffu, key);
+    const int total = (int)__reduce_add_sync(peers, (u32)count);
+    if ((threadIdx.x & 31) != (int)(__ffs(peers) - 1)) count = 0;
+    else if (count) count = total;
+  }
+  if (count) {
+    atomicAdd(dq + (int64_t)g * (N + 1) + o, -count);
+    atomicAdd(dq + (int64_t)g * (N + 1) + n, count);
+  }
+}
+
+// Slot changes between neighbouring pixels of a lane (bit j: pixel j's slot differs from pixel j - 1's).
+__device__ __forceinline__ u32 slot_changes(const int (&t)[16]) {
+  u32 bits = 1u;
+#pragma unroll
+  for (int j = 1; j < 16; ++j) bits |= (u32)(t[j] != t[j - 1]) << j;
+  return bits;
+}
+
 // Byte-owner transitions of a lane, run by run rather than pixel by pixel: the changed valid pixels
 // (cv) split into runs wherever the slot (gchg, fixed for the chunk), the old owner or the new owner
 // changes from one pixel to the next; a lane usually has one to three runs. The first run is summed
 // over the warp's lanes that share it, later runs go to memory directly.
-__device__ __forceinline__ void emit_transitions_bytes(const int (&t)[16], const LaneSlots& ls, u32 valid, u32 gchg,
-                                                       int* dq, int N, Owners<true>& s) {
-  const u32 cv = byte_differs(s.now, s.prev) & valid;
-  const u32 kchg = gchg | byte_changes(s.now) | byte_changes(s.prev) | 1u;
+__device__ __forceinline__ void emit_transitions_bytes(const int (&t)[16], const LaneSlots& ls, int* dq, int N,
+                                                       Owners<true>& s) {
+  const u32 cv = byte_differs(s.now, s.prev) & ls.valid();
+  const u32 kchg = slot_changes(t) | byte_changes(s.now) | byte_changes(s.prev) | 1u;
   u32 starts = cv & (~(cv << 1) | kchg);
   int fg = -1, fo = 0, fn = 0, fcnt = 0;
   while (starts) {
@@ -200,7 +185,9 @@ __device__ __forceinline__ void emit_transitions_bytes(const int (&t)[16], const
       g = ls.s1;
     } else if ((ls.e2 >> j) & 1u) {
       g = ls.s2;
-    } else {  // a third slot inside the lane: rare
+    } else if ((ls.e0 >> j) & 1u) {
+      g = 0;
+    } else {  // another slot inside the lane: rare
       g = t[0];
 #pragma unroll
       for (int k = 1; k < 16; ++k) g = k == j ? t[k] : g;
@@ -213,34 +200,12 @@ __device__ __forceinline__ void emit_transitions_bytes(const int (&t)[16], const
       atomicAdd(dq + (int64_t)g * (N + 1) + n, cnt);
     }
   }
-  const unsigned long long key =
-      fcnt ? ((unsigned long long)(u32)fg << 32) | ((unsigned long long)fo << 16) | (unsigned long long)fn : ~0ull;
-  const u32 peers = __match_any_sync(0xffffffffu, key);
-  const int total = (int)__reduce_add_sync(peers, (u32)fcnt);
-  if (fcnt && (threadIdx.x & 31) == (int)(__ffs(peers) - 1)) {
-    atomicAdd(dq + (int64_t)fg * (N + 1) + fo, -total);
-    atomicAdd(dq + (int64_t)fg * (N + 1) + fn, total);
-  }
+  add_first_run(fg, fo, fn, fcnt, dq, N);
 #pragma unroll
   for (int k = 0; k < 4; ++k) s.prev[k] = s.now[k];
 }
 
-// Slot changes between neighbouring pixels of a lane (bit j: pixel j's slot differs from pixel j - 1's).
-__device__ __forceinline__ u32 slot_changes(const int (&t)[16]) {
-  u32 bits = 1u;
-#pragma unroll
-  for (int j = 1; j < 16; ++j) bits |= (u32)(t[j] != t[j - 1]) << j;
-  return bits;
-}
-
-// Transitions at a checkpoint: the run form for byte owners, the pixel loop for 16-bit owners.
-template <bool kBytes>
-__device__ __forceinline__ void emit_at_checkpoint(const int (&t)[16], const LaneSlots& ls, u32 valid, u32 gchg,
-                                                   int* dq, int N, Owners<kBytes>& s);
-
-// Each lane's first run of equal (slot, old owner, new owner) is summed over the lanes of the warp that
-// share it (one pair of atomics per distinct run instead of one per lane: inside a large region every
-// lane has the same transition); later runs, at region borders, go to memory directly.
+// Later runs, at region borders, go to memory directly.
 template <bool kBytes>
 __device__ __forceinline__ void emit_transitions(const int (&t)[16], u32 valid, int* dq, int N, Owners<kBytes>& s) {
   int rg = -1, ro = -1, rn = -1, cnt = 0;
@@ -272,29 +237,17 @@ __device__ __forceinline__ void emit_transitions(const int (&t)[16], u32 valid, 
       atomicAdd(dq + (int64_t)rg * (N + 1) + rn, cnt);
     }
   }
-  // Owners are below 65536 (N < 65535), so (slot, old, new) packs into 64 bits.
-  const unsigned long long key =
-      fcnt ? ((unsigned long long)(u32)fg << 32) | ((unsigned long long)fo << 16) | (unsigned long long)fn : ~0ull;
-  const u32 peers = __match_any_sync(0xffffffffu, key);
-  const int total = (int)__reduce_add_sync(peers, (u32)fcnt);
-  if (fcnt && (threadIdx.x & 31) == (int)(__ffs(peers) - 1)) {
-    atomicAdd(dq + (int64_t)fg * (N + 1) + fo, -total);
-    atomicAdd(dq + (int64_t)fg * (N + 1) + fn, total);
-  }
+  add_first_run(fg, fo, fn, fcnt, dq, N);
 #pragma unroll
   for (int k = 0; k < Owners<kBytes>::kWords; ++k) s.prev[k] = s.now[k];
 }
 
-template <>
-__device__ __forceinline__ void emit_at_checkpoint<true>(const int (&t)[16], const LaneSlots& ls, u32 valid, u32 gchg,
-                                                         int* dq, int N, Owners<true>& s) {
-  emit_transitions_bytes(t, ls, valid, gchg, dq, N, s);
-}
-
-template <>
-__device__ __forceinline__ void emit_at_checkpoint<false>(const int (&t)[16], const LaneSlots&, u32 valid, u32,
-                                                          int* dq, int N, Owners<false>& s) {
-  emit_transitions<false>(t, valid, dq, N, s);
+// Transitions at a checkpoint: the run form for byte owners, the pixel loop for 16-bit owners.
+template <bool kBytes>
+__device__ __forceinline__ void emit_at_checkpoint(const int (&t)[16], const LaneSlots& ls, int* dq, int N,
+                                                   Owners<kBytes>& s) {
+  if constexpr (kBytes) emit_transitions_bytes(t, ls, dq, N, s);
+  else emit_transitions<false>(t, ls.valid(), dq, N, s);
 }
 
 // One CTA per 4096-pixel chunk, masks read with plain loads (rows at any alignment).
@@ -319,11 +272,9 @@ prefix_pass_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __re
 
   int t[16];
   load16_maps(target, x, pixels, vec_map, t);
-  const bool bad = count_target(t, x, pixels, G, ga + d[kPrefixSlotBegin], lane);
-  const LaneSlots ls = lane_slots(t, x, pixels, G);
-  const LanePeers lp = lane_peers(ls, lane);
-  const u32 valid = ls.e1 | ls.e2 | ls.emid;
-  const u32 gchg = slot_changes(t);
+  bool bad = false;
+  const LaneSlots ls = lane_slots(t, x, pixels, G, bad);
+  add_slots<true>(t, ls, ls.valid(), ga + d[kPrefixSlotBegin]);
   Owners<kBytes> s;
   s.clear();
   const int64_t xm = x < pixels ? x : pixels;
@@ -339,10 +290,11 @@ prefix_pass_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __re
 #pragma unroll
     for (int k = 1; k < kPxWindow; ++k)
       if (i % kPxWindow == k) w = window[k];
-    if (warp_may_cover(w, w, false)) draw_mask<kBytes>(i, w, t, ls, lp, valid, raw_img + (int64_t)i * G, s);
+    if (__any_sync(0xffffffffu, (w.x | w.y | w.z | w.w) != 0))
+      draw_mask<kBytes>(i, w, t, ls, raw_img + (int64_t)i * G, s);
     const int q = steps[i + 1];  // uniform across the CTA
     if (q >= 0 && __any_sync(0xffffffffu, s.changed()))
-      emit_at_checkpoint<kBytes>(t, ls, valid, gchg, delta_img + q * plane, N, s);
+      emit_at_checkpoint<kBytes>(t, ls, delta_img + q * plane, N, s);
   }
   if (bad) atomicOr(error, 1);
 }
@@ -350,8 +302,13 @@ prefix_pass_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __re
 // Persistent form: a producer warp streams every mask's segment of the current 4096-pixel chunk into a
 // shared-memory ring with cp.async.bulk (one copy per mask row and chunk: the 16-byte-aligned words
 // covering the segment, since rows may start at any byte; completion on the stage's mbarrier) while
-// 8 consumer warps draw the masks in order from shared memory, re-aligning each lane's 16 bytes from
-// two staged words when the row is not aligned (the offset is per row, uniform across a warp). Each
+// 8 consumer warps draw the masks in order from shared memory. What bounds them is instructions: most
+// masks leave most warps' 512 pixels alone, so a stage of four masks costs a warp four loads, one
+// warp-wide OR of "has a pixel here" and a barrier, and only masks with a pixel (a superset: the staged
+// words as they lie) are re-aligned and drawn; checkpoints are a bit mask read 32 masks at a time, and
+// only warps drawn to since the last one look for transitions. 16 images of 845 x 845 with 64 masks:
+// 151 us (308 with a test, a step lookup and two loads per mask and one reduction per lane and slot for
+// the target areas: those met on the bins of void and of large segments), 45 for one of 256 x 384 (69). Each
 // wait is bounded; a timeout sets bit 30 of *error, the producer waits (bounded) for its copies in
 // flight, and every role returns.
 constexpr int kPbConsumers = kPxThreads;
@@ -367,7 +324,8 @@ constexpr int kPbChunkRing = 4;  // published chunks in flight per CTA
 
 struct PrefixShared {
   unsigned char ring[kPbRing][kPbStage][kPbSlot];
-  int64_t chunk[kPbChunkRing];  // chunk published to the consumers; -1 ends the CTA's work
+  int64_t x0[kPbChunkRing];     // first pixel of the chunk published to the consumers
+  int64_t image[kPbChunkRing];  // its image; -1 ends the CTA's work
   uint64_t full[kPbRing];
   uint64_t empty[kPbRing];
   uint64_t chunk_full[kPbChunkRing];
@@ -407,13 +365,14 @@ prefix_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t to
     if (threadIdx.x != kPbConsumers) return;
     int64_t seq = 0, published = 0, next = c_begin;
     bool ok = true;
-    // Publish a chunk to the consumers (-1: no more work); false when the wait for a free entry fails.
-    auto publish = [&](int64_t chunk) {
+    // Publish a chunk to the consumers (image -1: no more work); false when the wait for a free entry fails.
+    auto publish = [&](int64_t image, int64_t x0) {
       const int e = (int)(published % kPbChunkRing);
       const int64_t use = published / kPbChunkRing;
       if ((use > 0 && !mbar_wait(&sm.chunk_empty[e], (uint32_t)((use - 1) & 1), kPbWaitLimit)) || *abort)
         return false;
-      sm.chunk[e] = chunk;
+      sm.x0[e] = x0;
+      sm.image[e] = image;
       mbar_arrive(&sm.chunk_full[e]);  // release: the entry is visible to consumers that see the phase
       ++published;
       return true;
@@ -421,13 +380,14 @@ prefix_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t to
     while (ok) {
       const int64_t chunk = schedule ? (int64_t)atomicAdd(schedule, 1ull) : (next < c_end ? next++ : total_chunks);
       if (chunk >= total_chunks) break;
-      if (!publish(chunk)) {
+      const int64_t image = find_image(descs, B, kPrefixChunkBegin, chunk);
+      const int64_t* d = pdesc(descs, image);
+      const int64_t pixels = d[kPrefixPixels];
+      const int64_t x0 = (chunk - d[kPrefixChunkBegin]) * (int64_t)kPxChunk;
+      if (!publish(image, x0)) {
         ok = false;
         break;
       }
-      const int64_t* d = pdesc(descs, find_image(descs, B, kPrefixChunkBegin, chunk));
-      const int64_t pixels = d[kPrefixPixels];
-      const int64_t x0 = (chunk - d[kPrefixChunkBegin]) * (int64_t)kPxChunk;
       const int64_t len = min((int64_t)kPxChunk, pixels - x0);
       const int N = (int)d[kPrefixN];
       const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kPrefixMasks]);
@@ -460,7 +420,7 @@ prefix_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t to
         ++seq;
       }
     }
-    if (ok) ok = publish(-1);
+    if (ok) ok = publish(-1, 0);
     if (!ok) {
       *abort = 1;
       atomicOr(error, kPbTimeoutBit);
@@ -481,69 +441,71 @@ prefix_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t to
       ok = false;
       break;
     }
-    const int64_t chunk = sm.chunk[e];
+    const int64_t image = sm.image[e], x0 = sm.x0[e];
     __syncwarp();
     if (lane == 0) mbar_arrive(&sm.chunk_empty[e]);
     ++taken;
-    if (chunk < 0) break;
-    const int64_t* d = pdesc(descs, find_image(descs, B, kPrefixChunkBegin, chunk));
+    if (image < 0) break;
+    const int64_t* d = pdesc(descs, image);
     const int64_t pixels = d[kPrefixPixels];
-    const int64_t x0 = (chunk - d[kPrefixChunkBegin]) * (int64_t)kPxChunk;
     const int64_t x = x0 + (int64_t)threadIdx.x * 16;
     const int N = (int)d[kPrefixN], G = (int)d[kPrefixG];
     const int* steps = step_q + d[kPrefixStepBegin];
     const int64_t plane = (int64_t)G * (N + 1);
-    const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kPrefixMasks]);
     const int64_t stride = d[kPrefixStride];
+    // Row r of the chunk starts (first + r * stride) mod 16 bytes into its first staged word.
+    const uint32_t first = (uint32_t)d[kPrefixMasks] & 15u, o_step = (uint32_t)stride & 15u;
     int* delta_img = delta + d[kPrefixPairBegin];
     u32* raw_img = raw + d[kPrefixRawBegin];
     int t[16];
     load16_maps(reinterpret_cast<const int*>(d[kPrefixTarget]), x, pixels, d[kPrefixFlags] & 1, t);
-    bad |= count_target(t, x, pixels, G, ga + d[kPrefixSlotBegin], lane);
-    const LaneSlots ls = lane_slots(t, x, pixels, G);
-    const LanePeers lp = lane_peers(ls, lane);
-    const u32 valid = ls.e1 | ls.e2 | ls.emid;  // pixels past the image end are not valid: stale bytes ignored
-    const u32 gchg = slot_changes(t);
+    // Pixels past the image end are not valid: stale staged bytes under them are ignored.
+    const LaneSlots ls = lane_slots(t, x, pixels, G, bad);
+    add_slots<true>(t, ls, ls.valid(), ga + d[kPrefixSlotBegin]);
     Owners<kBytes> s;
     s.clear();
+    u32 checks = 0;      // bit k: a checkpoint follows mask 32 (r0 / 32) + k
+    bool drawn = false;  // since the last checkpoint, anywhere in the warp
     for (int r0 = 0; r0 < N; r0 += kPbStage) {
+      if ((r0 & 31) == 0) checks = __ballot_sync(0xffffffffu, r0 + lane < N && steps[r0 + 1 + lane] >= 0);
       const int slot = (int)(seq % kPbRing);
       const bool got = mbar_wait(&sm.full[slot], (uint32_t)((seq / kPbRing) & 1), kPbWaitLimit);
       if (!__all_sync(0xffffffffu, got && !*abort)) {  // warp-uniform decision
         ok = false;
         break;
       }
-      const int n = min(kPbStage, N - r0);
-      // One mask at a time, not unrolled: the drawing code is large and unrolled copies of it missed
-      // the instruction cache. The next mask's staged words and checkpoint index are loaded before the
-      // current mask is drawn, so their latency overlaps the drawing. Row offsets advance by the row
-      // stride mod 16 (the same for the whole warp).
-      int o = (int)(reinterpret_cast<uintptr_t>(masks + (int64_t)r0 * stride) & 15);
-      const int o_step = (int)(stride & 15);
       const uint4* words = reinterpret_cast<const uint4*>(&sm.ring[slot][0][threadIdx.x * 16]);
-      uint4 a = words[0];
-      uint4 b = o ? words[1] : a;
-      int q = steps[r0 + 1];
-#pragma unroll 1
-      for (int k = 0; k < n; ++k) {
-        const int i = r0 + k;
-        const int o_next = (o + o_step) & 15;
-        uint4 a_next = a, b_next = b;
-        int q_next = -1;
-        if (k + 1 < n) {
-          const uint4* next = reinterpret_cast<const uint4*>(&sm.ring[slot][k + 1][threadIdx.x * 16]);
-          a_next = next[0];
-          b_next = o_next ? next[1] : a_next;
-          q_next = steps[i + 2];
+      u32 hit = 0;
+#pragma unroll
+      for (int k = 0; k < kPbStage; ++k) {
+        const uint4 a = words[k * (kPbSlot / 16)];
+        u32 any = a.x | a.y | a.z | a.w;
+        if (lane == 31 && ((first + (r0 + k) * o_step) & 15u)) {  // the warp's pixels end in the next word
+          const uint4 b = words[k * (kPbSlot / 16) + 1];
+          any |= b.x | b.y | b.z | b.w;
         }
-        if (warp_may_cover(a, b, o != 0))
-          draw_mask<kBytes>(i, o ? realign16(a, b, o) : a, t, ls, lp, valid, raw_img + (int64_t)i * G, s);
-        if (q >= 0 && __any_sync(0xffffffffu, s.changed()))  // q: uniform across the CTA
-          emit_at_checkpoint<kBytes>(t, ls, valid, gchg, delta_img + q * plane, N, s);
-        a = a_next;
-        b = b_next;
-        q = q_next;
-        o = o_next;
+        hit |= (u32)(any != 0) << k;
+      }
+      const u32 present = (1u << min(kPbStage, N - r0)) - 1u;
+      hit = __reduce_or_sync(0xffffffffu, hit) & present;
+      const u32 check = (checks >> (r0 & 31)) & present;
+      // One mask at a time, not unrolled: the drawing code is large and unrolled copies of it missed the
+      // instruction cache.
+#pragma unroll 1
+      for (u32 todo = hit | check; todo; todo &= todo - 1) {
+        const int k = __ffs(todo) - 1, i = r0 + k;
+        if ((hit >> k) & 1u) {
+          const int o = (int)((first + i * o_step) & 15u);
+          const uint4 a = words[k * (kPbSlot / 16)];
+          draw_mask<kBytes>(i, o ? realign16(a, words[k * (kPbSlot / 16) + 1], o) : a, t, ls,
+                            raw_img + (int64_t)i * G, s);
+          drawn = true;
+        }
+        if (drawn && ((check >> k) & 1u)) {
+          drawn = false;
+          if (__any_sync(0xffffffffu, s.changed()))
+            emit_at_checkpoint<kBytes>(t, ls, delta_img + (int64_t)steps[i + 1] * plane, N, s);
+        }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.empty[slot]);

@@ -118,7 +118,8 @@ seg_pass_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chun
     const int64_t stride = d[kMaskStride];
     const int64_t* ord = order + d[kDetBegin];
     const bool vec_maps = d[kFlags] & 1, vec_masks = d[kFlags] & 2;
-    const ImageOut out{pairs + d[kPairBegin], dpairs + d[kDPairBegin], (u32)(G * P)};
+    u32* image_pairs = pairs + d[kPairBegin];
+    u32* image_dpairs = dpairs + d[kDPairBegin];
     const int64_t stop = min(last, c_end);
     for (; chunk < stop; ++chunk) {
       const int64_t x = (chunk - first) * kChunk + (int64_t)threadIdx.x * kPassPixels;
@@ -133,28 +134,9 @@ seg_pass_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chun
       {
         int p[16];
         load16_maps(target, x, pixels, vec_maps, t);
-        if (pred) load16_maps(pred, x, pixels, vec_maps, p);
-        u32 run_key = kEmpty, run_count = 0;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (x + j >= pixels) continue;
-          const bool tv = t[j] >= 0 && t[j] < G;
-          const bool pv = !pred || (p[j] >= 0 && p[j] < P);
-          if (!tv || !pv) { bad = true; continue; }
-          if (pred) {
-            const u32 key = (u32)(t[j] * P + p[j]);
-            if (key != run_key) {
-              if (run_count) global_add(out, run_key, run_count);
-              run_key = key;
-              run_count = 0;
-            }
-            ++run_count;
-          }
-        }
         if (pred) {
-          const u32 peers = __match_any_sync(0xffffffffu, run_key);
-          const u32 total = __reduce_add_sync(peers, run_count);
-          if (lane == (int)(__ffs(peers) - 1) && total) global_add(out, run_key, total);
+          load16_maps(pred, x, pixels, vec_maps, p);
+          add_pairs(t, p, x, pixels, G, P, image_pairs, bad);
         }
       }
       if (!PE_PASS_PRELOAD) {
@@ -162,7 +144,7 @@ seg_pass_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chun
         for (int k = 0; k < kGroup; ++k)
           cur[k] = k < D ? load16_stream(masks + ord[k] * stride, xm, pixels, vec_masks) : make_uint4(0, 0, 0, 0);
       }
-      const LaneSlots ls = lane_slots(t, x, pixels, G);
+      const LaneSlots ls = lane_slots(t, x, pixels, G, bad);
       // Detections: groups of kGroup masks with one group of look-ahead; one
       // warp-wide OR tells which masks of the group have any pixel here.
       for (int r0 = 0; r0 < D; r0 += kGroup) {
@@ -177,7 +159,8 @@ seg_pass_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chun
         const u32 warp_bits = __reduce_or_sync(0xffffffffu, bits);
 #pragma unroll
         for (int k = 0; k < kGroup; ++k)
-          if ((warp_bits >> k) & 1u) bin_detection(out, ls, t, cur[k], r0 + k, G, lane);  // uniform across the warp
+          if ((warp_bits >> k) & 1u)   // uniform across the warp
+            add_slots(t, ls, pack16(cur[k]), image_dpairs + (int64_t)(r0 + k) * G);
 #pragma unroll
         for (int k = 0; k < kGroup; ++k) cur[k] = nxt[k];
       }
@@ -372,39 +355,21 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
     const int* target = reinterpret_cast<const int*>(d[kTarget]);
     const int* pred = reinterpret_cast<const int*>(d[kPred]);
     const bool vec_maps = d[kFlags] & 1;
-    const ImageOut out{pairs + d[kPairBegin], dpairs + d[kDPairBegin], (u32)(G * P)};
+    u32* image_pairs = pairs + d[kPairBegin];
+    u32* image_dpairs = dpairs + d[kDPairBegin];
     const int64_t len = min((int64_t)kHalf, pixels - x0);
     const int64_t x = x0 + (int64_t)ctid * kPassPixels;
     int t[16];
     {
       int p[16];
       load16_maps(target, x, pixels, vec_maps, t);
-      if (pred) load16_maps(pred, x, pixels, vec_maps, p);
-      u32 run_key = kEmpty, run_count = 0;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        if (x + j >= pixels) continue;
-        const bool tv = t[j] >= 0 && t[j] < G;
-        const bool pv = !pred || (p[j] >= 0 && p[j] < P);
-        if (!tv || !pv) { bad = true; continue; }
-        if (pred) {
-          const u32 key = (u32)(t[j] * P + p[j]);
-          if (key != run_key) {
-            if (run_count) global_add(out, run_key, run_count);
-            run_key = key;
-            run_count = 0;
-          }
-          ++run_count;
-        }
-      }
       if (pred) {
-        const u32 peers = __match_any_sync(0xffffffffu, run_key);
-        const u32 total = __reduce_add_sync(peers, run_count);
-        if (lane == (int)(__ffs(peers) - 1) && total) global_add(out, run_key, total);
+        load16_maps(pred, x, pixels, vec_maps, p);
+        add_pairs(t, p, x, pixels, G, P, image_pairs, bad);
       }
     }
     const bool in_range = x < x0 + len;
-    const LaneSlots ls = lane_slots(t, x, pixels, G);
+    const LaneSlots ls = lane_slots(t, x, pixels, G, bad);
     for (int r0 = 0; r0 < D; r0 += kStageMasks) {
       const int slot = (int)(seq % kRing);
       const bool got = mbar_wait(&sm.full[slot], (uint32_t)((seq / kRing) & 1), kWaitLimit);
@@ -436,7 +401,8 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
       if (!warp_bits) continue;
 #pragma unroll
       for (int k = 0; k < kStageMasks; ++k)
-        if ((warp_bits >> k) & 1u) bin_detection(out, ls, t, w[k], r0 + k, G, lane);  // uniform across the warp
+        if ((warp_bits >> k) & 1u)  // uniform across the warp
+          add_slots(t, ls, pack16(w[k]), image_dpairs + (int64_t)(r0 + k) * G);
     }
   }
   if (!ok) {
