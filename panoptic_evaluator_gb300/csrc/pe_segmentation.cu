@@ -174,13 +174,13 @@ seg_pass_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chun
 // row starts on a 16-byte boundary (e.g. a ragged.SegmentationImages arena);
 // true: rows at any byte offset, the producer copies the aligned 16-byte words
 // covering each row segment and the consumers re-align them by the row's offset.
-// Warp 8 is the producer: one lane takes 8192-pixel chunks, publishes each
-// 4096-pixel half (image, first pixel) in a small queue of kHalfRing entries,
+// Warp 8 is the producer: one lane takes 4096-pixel halves of 8192-pixel chunks,
+// publishes each (image, first pixel) in a small queue of kHalfRing entries,
 // prefetches its slot maps into L2 and streams its 4096-byte mask-row segments
 // into a ring of kRing shared-memory slots with cp.async.bulk, completing on
-// per-slot "full" mbarriers. Chunks come from a global counter (`schedule`,
-// one atomicAdd per chunk), so CTAs that run faster take more of them, or,
-// without a counter, from a contiguous range per CTA. Warps 0-7 consume: they
+// per-slot "full" mbarriers. Halves come from a global counter (`schedule`,
+// one atomicAdd per `grab` of them), so CTAs that run faster take more of them,
+// or, without a counter, from a contiguous range of chunks per CTA. Warps 0-7 consume: they
 // take the next half from the queue, read the target/prediction slots of their
 // 16 pixels with plain loads (kept in registers), then take each mask segment
 // from the ring, bin it exactly as the register path does and release the slot
@@ -192,7 +192,7 @@ constexpr int kBulkConsumers = 256;
 constexpr int kBulkThreads = kBulkConsumers + 32;
 constexpr int kHalf = kBulkConsumers * kPassPixels;  // 4096 pixels per step
 constexpr int kStageMasks = 4;  // mask-row segments per ring stage (one barrier each)
-constexpr int kRing = 4;        // stages in flight per CTA
+constexpr int kRing = 6;        // stages in flight per CTA (two CTAs hold 197 KB; 4 stages: 310 us where 6 take 293)
 constexpr int kHalfRing = 4;    // published halves in flight per CTA
 constexpr long long kWaitLimit = 4000000000ll;  // about two seconds of SM clock
 constexpr int kTimeoutBit = 1 << 30;
@@ -239,8 +239,8 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
   if (threadIdx.x >= kBulkConsumers) {
     // ---- producer --------------------------------------------------------
     if (threadIdx.x != kBulkConsumers) return;
-    int64_t seq = 0, halves = 0, next = c_begin;
-    int64_t grabbed = 0, grab_end = 0;  // with a counter: the current grab of `grab` consecutive chunks
+    int64_t seq = 0, halves = 0, next = 2 * c_begin;  // work is taken in halves, two per chunk
+    int64_t grabbed = 0, grab_end = 0;  // with a counter: the current grab of `grab` consecutive halves
     bool ok = true;
     // Publish the next half (image -1: no more work); false when the wait for a free entry fails.
     auto publish = [&](int64_t image, int64_t x0) {
@@ -254,20 +254,23 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
       return true;
     };
     while (ok) {
-      int64_t chunk;
+      int64_t unit;
       if (schedule) {
         if (grabbed == grab_end) {
           grabbed = (int64_t)atomicAdd(schedule, (unsigned long long)grab);
-          grab_end = min(grabbed + grab, total_chunks);
+          grab_end = min(grabbed + grab, 2 * total_chunks);
         }
-        chunk = grabbed < grab_end ? grabbed++ : total_chunks;
+        unit = grabbed < grab_end ? grabbed++ : 2 * total_chunks;
       } else {
-        chunk = next < c_end ? next++ : total_chunks;
+        unit = next < 2 * c_end ? next++ : 2 * total_chunks;
       }
-      if (chunk >= total_chunks) break;
+      if (unit >= 2 * total_chunks) break;
+      const int64_t chunk = unit >> 1;
       const int64_t b = image_of_chunk(descs, B, chunk);
       const int64_t* d = desc_of(descs, b);
-      const int64_t first = d[kChunkBegin], pixels = d[kPixels];
+      const int64_t pixels = d[kPixels];
+      const int64_t x0 = (chunk - d[kChunkBegin]) * kChunk + (unit & 1) * kHalf;
+      if (x0 >= pixels) continue;  // the second half of an image's last chunk
       const int D = (int)d[kD];
       const int* target = reinterpret_cast<const int*>(d[kTarget]);
       const int* pred = reinterpret_cast<const int*>(d[kPred]);
@@ -275,51 +278,47 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
       const int64_t stride = d[kMaskStride];
       const int64_t* ord = order + d[kDetBegin];
       const bool vec_maps = d[kFlags] & 1;
-      for (int half = 0; half < kChunk / kHalf && ok; ++half) {
-        const int64_t x0 = (chunk - first) * kChunk + (int64_t)half * kHalf;
-        if (x0 >= pixels) break;
-        if (!publish(b, x0)) {
+      if (!publish(b, x0)) {
+        ok = false;
+        break;
+      }
+      const int64_t len = min((int64_t)kHalf, pixels - x0);
+      const uint32_t map_bytes = (uint32_t)((len * 4) & ~15ll);
+      if (vec_maps && map_bytes) {
+        bulk_prefetch_l2(target + x0, map_bytes);
+        if (pred) bulk_prefetch_l2(pred + x0, map_bytes);
+      }
+      for (int r0 = 0; r0 < D; r0 += kStageMasks) {
+        const int slot = (int)(seq % kRing);
+        const int64_t use = seq / kRing;
+        if ((use > 0 && !mbar_wait(&sm.empty[slot], (uint32_t)((use - 1) & 1), kWaitLimit)) || *abort) {
           ok = false;
           break;
         }
-        const int64_t len = min((int64_t)kHalf, pixels - x0);
-        const uint32_t map_bytes = (uint32_t)((len * 4) & ~15ll);
-        if (vec_maps && map_bytes) {
-          bulk_prefetch_l2(target + x0, map_bytes);
-          if (pred) bulk_prefetch_l2(pred + x0, map_bytes);
-        }
-        for (int r0 = 0; r0 < D; r0 += kStageMasks) {
-          const int slot = (int)(seq % kRing);
-          const int64_t use = seq / kRing;
-          if ((use > 0 && !mbar_wait(&sm.empty[slot], (uint32_t)((use - 1) & 1), kWaitLimit)) || *abort) {
-            ok = false;
-            break;
+        const int n = min(kStageMasks, D - r0);
+        // Rows may start at any byte: copy the aligned words from the one holding pixel x0 to the
+        // one holding the segment's last byte; the consumers re-align by the row's offset.
+        if constexpr (ANY_ALIGN) {
+          const uint8_t* rows[kStageMasks];
+          uint32_t total = 0;
+          for (int k = 0; k < n; ++k) {
+            rows[k] = masks + ord[r0 + k] * stride + x0;
+            const int o = (int)(reinterpret_cast<uintptr_t>(rows[k]) & 15);
+            sm.shift[slot][k] = (unsigned char)o;
+            total += (uint32_t)round_up(len + o, 16);
           }
-          const int n = min(kStageMasks, D - r0);
-          // Rows may start at any byte: copy the aligned words from the one holding pixel x0 to the
-          // one holding the segment's last byte; the consumers re-align by the row's offset.
-          if constexpr (ANY_ALIGN) {
-            const uint8_t* rows[kStageMasks];
-            uint32_t total = 0;
-            for (int k = 0; k < n; ++k) {
-              rows[k] = masks + ord[r0 + k] * stride + x0;
-              const int o = (int)(reinterpret_cast<uintptr_t>(rows[k]) & 15);
-              sm.shift[slot][k] = (unsigned char)o;
-              total += (uint32_t)round_up(len + o, 16);
-            }
-            mbar_arrive_expect_tx(&sm.full[slot], total);  // release: the offsets are visible with the phase
-            for (int k = 0; k < n; ++k) {
-              const int o = sm.shift[slot][k];
-              bulk_copy_g2s(sm.ring[slot][k], rows[k] - o, (uint32_t)round_up(len + o, 16), &sm.full[slot]);
-            }
-          } else {  // every row starts on a 16-byte boundary
-            const uint32_t bytes = (uint32_t)round_up(len, 16);
-            mbar_arrive_expect_tx(&sm.full[slot], bytes * (uint32_t)n);
-            for (int k = 0; k < n; ++k)
-              bulk_copy_g2s(sm.ring[slot][k], masks + ord[r0 + k] * stride + x0, bytes, &sm.full[slot]);
+          mbar_arrive_expect_tx(&sm.full[slot], total);  // release: the offsets are visible with the phase
+          for (int k = 0; k < n; ++k) {
+            const int o = sm.shift[slot][k];
+            bulk_copy_g2s(sm.ring[slot][k], rows[k] - o, (uint32_t)round_up(len + o, 16), &sm.full[slot]);
           }
-          ++seq;
+        } else {  // every row starts on a 16-byte boundary
+          const uint32_t bytes = (uint32_t)round_up(len, 16);
+          mbar_arrive_expect_tx(&sm.full[slot], bytes * (uint32_t)n);
+          for (int k = 0; k < n; ++k)
+            bulk_copy_g2s(sm.ring[slot][k], masks + ord[r0 + k] * stride + x0, bytes, &sm.full[slot]);
         }
+        ++seq;
       }
     }
     if (ok) ok = publish(-1, 0);
@@ -377,32 +376,36 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
         ok = false;
         break;
       }
-      const int n = min(kStageMasks, D - r0);
-      uint4 w[kStageMasks];
-      u32 bits = 0;
+      // One warp-wide OR tells which masks of the stage have a pixel here (a superset for rows at any
+      // offset: the staged words as they lie); only those are re-aligned and counted, by one copy of the
+      // counting code.
+      const unsigned char* staged = &sm.ring[slot][0][ctid * kPassPixels];
+      constexpr int kRowBytes = kHalf + 16;
+      u32 hit = 0;
 #pragma unroll
       for (int k = 0; k < kStageMasks; ++k) {
-        w[k] = make_uint4(0, 0, 0, 0);
-        if (in_range && k < n) {
-          const uint4* words = reinterpret_cast<const uint4*>(&sm.ring[slot][k][ctid * kPassPixels]);
-          if constexpr (ANY_ALIGN) {
-            const int o = sm.shift[slot][k];  // the same for the whole warp
-            w[k] = o ? realign16(words[0], words[1], o) : words[0];
-          } else {
-            w[k] = words[0];
-          }
+        const uint4 a = *reinterpret_cast<const uint4*>(staged + k * kRowBytes);
+        u32 any = a.x | a.y | a.z | a.w;
+        if (ANY_ALIGN && lane == 31 && sm.shift[slot][k]) {  // the warp's pixels end in the next word
+          const uint4 c = *reinterpret_cast<const uint4*>(staged + k * kRowBytes + 16);
+          any |= c.x | c.y | c.z | c.w;
         }
-        bits |= (u32)((w[k].x | w[k].y | w[k].z | w[k].w) != 0) << k;
+        hit |= (u32)(any != 0) << k;
+      }
+      hit = __reduce_or_sync(0xffffffffu, in_range ? hit : 0u) & ((1u << min(kStageMasks, D - r0)) - 1u);
+#pragma unroll 1
+      for (; hit; hit &= hit - 1) {
+        const int k = __ffs(hit) - 1;
+        uint4 w = *reinterpret_cast<const uint4*>(staged + k * kRowBytes);
+        if constexpr (ANY_ALIGN) {
+          const int o = sm.shift[slot][k];  // the same for the whole warp
+          if (o) w = realign16(w, *reinterpret_cast<const uint4*>(staged + k * kRowBytes + 16), o);
+        }
+        add_slots(t, ls, pack16(w), image_dpairs + (int64_t)(r0 + k) * G);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.empty[slot]);
       ++seq;
-      const u32 warp_bits = __reduce_or_sync(0xffffffffu, bits);
-      if (!warp_bits) continue;
-#pragma unroll
-      for (int k = 0; k < kStageMasks; ++k)
-        if ((warp_bits >> k) & 1u)  // uniform across the warp
-          add_slots(t, ls, pack16(w[k]), image_dpairs + (int64_t)(r0 + k) * G);
     }
   }
   if (!ok) {
@@ -767,15 +770,22 @@ PE_API int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, co
     const int64_t max_ctas = (int64_t)sm_count() * 2;
     const int64_t per_cta = ceil_div(total_chunks, std::min(total_chunks, max_ctas));
     int64_t grid = cta_bounds ? ctas : ceil_div(total_chunks, per_cta);
-    if (schedule) {  // chunks taken from the counter, `grab` at a time, by the chosen CTAs per SM
-      grid = std::min(ceil_div(total_chunks, choice.grab), (int64_t)sm_count() * choice.per_sm);
+    // Chunks taken from the counter, `grab` at a time, by the chosen CTAs per SM; half a chunk at a time
+    // while the halves are fewer than kFewHalves per CTA, where a CTA left with one chunk more than the
+    // others is a large part of the launch (384 chunks on 304 CTAs: 207 us by chunks, 161 by halves).
+    int grab = 2 * choice.grab;
+    if (schedule) {
+      constexpr int64_t kFewHalves = 16;
+      const int64_t all = (int64_t)sm_count() * choice.per_sm;
+      if (2 * total_chunks < kFewHalves * all) grab = 1;
+      grid = std::min(ceil_div(2 * total_chunks, grab), all);
       cta_bounds = nullptr;
     }
     const size_t smem = sizeof(BulkShared) + 128;
     auto kernel = bulk == 2 ? seg_pass_bulk_kernel<true> : seg_pass_bulk_kernel<false>;
     PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<(unsigned)grid, kBulkThreads, smem, stream>>>(
-        descs, B, total_chunks, per_cta, cta_bounds, reinterpret_cast<unsigned long long*>(schedule), choice.grab,
+        descs, B, total_chunks, per_cta, cta_bounds, reinterpret_cast<unsigned long long*>(schedule), grab,
         order, pairs, dpairs, error);
     PE_LAUNCHED("seg_pass_bulk");
     count_launch();
