@@ -29,24 +29,28 @@
 //    tensor maps (pe_contract_maps; descriptor flags bit 2) are loaded by TMA:
 //    one 2-D tile load per operand and stage (127 x 128 and 63 x 128 bytes,
 //    hardware 128-byte swizzle, zero fill past the last row and pixel) into an
-//    eight-deep ring (the three operand slots and five slots carved from the
+//    eight-deep ring (the four operand slots and four slots carved from the
 //    raw ring, idle once a CTA's staged blocks are done), issued by one thread.
 //  - Other rows may start at any byte. Four copy warps stream, per stage and
 //    row, the nine aligned 16-byte words covering the row's 128 bytes into a
-//    five-deep raw ring with cp.async (completion on the stage's mbarrier);
-//    words that start past the row end are not copied. Seven converter warps
+//    four-deep raw ring with cp.async (completion on the stage's mbarrier);
+//    words that start past the row end are not copied. Six converter warps
 //    take each row's bytes [o, o + 128) from the raw words (o = the row's start
 //    offset mod 16; funnel shifts and selects; a lane turns five words into
 //    four chunks, so shared-memory reads stay at 1.25x the bytes produced),
-//    zero bytes past the row end and store them swizzled into a three-deep
-//    operand ring.
+//    zero bytes past the row end and store them swizzled into a four-deep
+//    operand ring. Two teams of three convert every other stage: a stage is a
+//    chain (wait, load, shift, store, proxy fence, arrive), and with every warp
+//    in every stage the chains came one after another. 16 images of 641 x 639,
+//    100 x 50 masks: 233 -> 226 us; 120 x 80: 498 -> 442; 32 images, 100 x 8:
+//    359 -> 350 (at 4.0 TB/s; rows on 16-byte boundaries, by TMA: 5.4).
 // The host puts every TMA block after every staged block in chunk order, so a
 // CTA switches kinds at most once (staged, then TMA). CTAs take contiguous
 // chunk ranges of equal cost (rows x pixels).
 //
-// Roles per CTA (16 warps): warps 0-3 read the accumulator (TMEM lanes
+// Roles per CTA (15 warps): warps 0-3 read the accumulator (TMEM lanes
 // 32w..32w+31), warp 4 allocates TMEM and issues the MMAs, warps 5-8 copy,
-// warps 9-15 convert (converter 0 also issues the TMA loads). Every mbarrier
+// warps 9-14 convert (converter 0 also issues the TMA loads). Every mbarrier
 // wait is bounded; a timeout sets bit 30 of *error (and bit 20 + the wait's
 // site), every role leaves its loop, copies and TMA loads in flight land
 // before the CTA exits, the MMA thread waits (bounded) for its MMAs to retire
@@ -74,12 +78,14 @@ constexpr int kInterval = 4096;         // pixels of one work chunk
 constexpr int kSegmentChunks = 1024;    // chunks per accumulator read-back at most (2^22 pixels)
 constexpr int kRawWords = kAtom / 16 + 1;  // aligned words covering 128 row bytes at any offset
 constexpr int kRawRow = kRawWords * 16;
-constexpr int kRawRing = 5;
-constexpr int kRing = 3;
+constexpr int kRawRing = 4;
+constexpr int kRing = 4;
 constexpr int kEpilogueWarps = 4;
 constexpr int kMmaWarp = 4;
 constexpr int kCopyWarps = 4;
-constexpr int kConvertWarps = 7;
+constexpr int kTeams = 2;      // converter teams; each takes every kTeams-th stage
+constexpr int kTeamWarps = 3;
+constexpr int kConvertWarps = kTeams * kTeamWarps;
 constexpr int kFirstCopyWarp = kMmaWarp + 1;
 constexpr int kFirstConvertWarp = kFirstCopyWarp + kCopyWarps;
 constexpr int kThreads = (kEpilogueWarps + 1 + kCopyWarps + kConvertWarps) * 32;
@@ -92,11 +98,11 @@ constexpr int kCopyItems = (kCopyRows * kRawWords + 31) / 32;             // 16-
 constexpr int kConvertChunks = 4;
 constexpr int kLanesPerRow = (kAtom / 16) / kConvertChunks;
 constexpr int kConvertRowsPerWarp = 32 / kLanesPerRow;
-constexpr int kConvertRowsPerRound = kConvertWarps * kConvertRowsPerWarp;
+constexpr int kConvertRowsPerRound = kTeamWarps * kConvertRowsPerWarp;
 constexpr int kConvertRounds = (kRows + kConvertRowsPerRound - 1) / kConvertRowsPerRound;
 constexpr int kTmemCols = 2 * kN;       // two accumulator buffers
 constexpr int kTmaSlotBytes = (kM + kN) * kAtom;               // one TMA stage: A tile, then B tile
-constexpr int kTmaExtra = 5;                                   // TMA slots carved from the raw ring
+constexpr int kTmaExtra = 4;                                   // TMA slots carved from the raw ring
 constexpr int kTmaRing = kRing + kTmaExtra;
 constexpr uint32_t kTmaBytes = (uint32_t)(kRowsA + kRowsB) * kAtom;  // both tile loads of a stage
 constexpr long long kWaitLimit = 4000000000ll;  // ~2 s at 2 GHz
@@ -106,7 +112,7 @@ constexpr int kOrderBit = 1 << 28;  // a CTA range has staged blocks after TMA b
 enum : int { kSiteBit = 20, kAtAccEmpty = 0, kAtFull, kAtFullTma, kAtTmaSlot, kAtStageSlot, kAtAccFull, kAtRaw };
 constexpr float kCountScale = 262144.0f;  // 2^18: one product of two mask bytes (e4m3 2^-9 each)
 
-static_assert(kThreads == 512, "16 warps");
+static_assert(kRing % kTeams == 0 && kRawRing % kTeams == 0, "a ring slot is always the same team's");
 static_assert(kConvertRounds * kConvertRowsPerRound >= kRows, "converter rounds cover every row");
 static_assert(kCopyItems <= 32, "copy items fit the live mask");
 static_assert(kTmaExtra * kTmaSlotBytes <= kRawRing * kRows * kRawRow, "TMA slots fit the raw ring");
@@ -358,12 +364,12 @@ inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restric
   }
   if (threadIdx.x == 0) {
     for (int i = 0; i < kRing; ++i) {
-      mbar_init(&sm.full[i], kConvertWarps);
+      mbar_init(&sm.full[i], kTeamWarps);
       mbar_init(&sm.empty[i], 1);
     }
     for (int i = 0; i < kRawRing; ++i) {
       mbar_init(&sm.raw_full[i], kCopyWarps * 32);
-      mbar_init(&sm.raw_empty[i], kConvertWarps);
+      mbar_init(&sm.raw_empty[i], kTeamWarps);
     }
     for (int i = 0; i < kTmaRing; ++i) {
       mbar_init(&sm.tma_full[i], 1);
@@ -447,9 +453,8 @@ inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restric
     const int c = warp - kFirstCopyWarp;
     const int r0 = c * kCopyRows;
     const uint8_t* src[kCopyItems];  // the item's aligned word at x = 0
-    int64_t room[kCopyItems];        // the word holds a row byte while x0 < room
-    uint32_t dst[kCopyItems];        // byte offset in a raw stage
-    uint32_t live = 0;               // bit k: item k exists in this block
+    int first[kCopyItems];           // the word's first byte, counted from the row's byte at x = 0
+    int items = 0;                   // words of the warp's rows in this block
     Block blk;
     int64_t seg_start = 0, cached = -1;
     Ring<kRawRing> ring;
@@ -464,21 +469,18 @@ inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restric
       if (blk.index != cached) {
         cached = blk.index;
         const Rows rows = rows_of(descs, blocks, blk.index);
-        const int items = max(0, min(kCopyRows, rows.Dm + rows.Gn - r0)) * kRawWords;
-        live = 0;
+        items = max(0, min(kCopyRows, rows.Dm + rows.Gn - r0)) * kRawWords - lane;
 #pragma unroll
         for (int k = 0; k < kCopyItems; ++k) {
           const int i = lane + 32 * k;
           const int r = i / kRawWords, w = i - r * kRawWords;
           src[k] = nullptr;
-          room[k] = 0;
-          dst[k] = (uint32_t)((r0 + r) * kRawRow + 16 * w);
-          if (i < items) {
+          first[k] = 0;
+          if (32 * k < items) {
             const uint8_t* p = rows.row(r0 + r);
             const int o = (int)(reinterpret_cast<uintptr_t>(p) & 15);
             src[k] = p - o + 16 * w;
-            room[k] = blk.pixels + o - 16 * w;
-            live |= 1u << k;
+            first[k] = 16 * w - o;
           }
         }
       }
@@ -492,12 +494,11 @@ inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restric
           break;
         }
         const int64_t x0 = x_begin + (int64_t)st * kAtom;
-        uint8_t* stage = sm.raw[slot];
+        const int left = (int)min((int64_t)kRawRow, blk.pixels - x0);
+        uint8_t* stage = sm.raw[slot] + r0 * kRawRow + 16 * lane;
 #pragma unroll
-        for (int k = 0; k < kCopyItems; ++k) {
-          if (!((live >> k) & 1u)) continue;
-          if (x0 < room[k]) cp_async16(stage + dst[k], src[k] + x0);  // words past the row end stay stale
-        }
+        for (int k = 0; k < kCopyItems; ++k)  // words past the row end stay stale
+          if (32 * k < items && first[k] < left) cp_async16(stage + 512 * k, src[k] + x0);
         cp_async_arrive(&sm.raw_full[slot]);
       }
     }
@@ -507,75 +508,29 @@ inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restric
     // Lane = kLanesPerRow * q + h: row q of the warp's kConvertRowsPerWarp rows in a round, 16-byte chunks
     // c0 = h * kConvertChunks ... of the row's 128 bytes. Converter 0 also issues the TMA loads of TMA blocks.
     const int cw = warp - kFirstConvertWarp;
+    const int team = cw / kTeamWarps, tw = cw % kTeamWarps;
+    int turn = 0;  // the team whose stage is next
     const int q = lane / kLanesPerRow, c0 = (lane % kLanesPerRow) * kConvertChunks;
     Block blk;
     int64_t seg_start = 0, cached = -1;
     Ring<kRawRing> raw_ring;
     Ring<kRing> ring;
-    Ring<kTmaRing> tring;  // converter 0 lane 0: TMA stages issued
-    bool tma_started = false;
     uint32_t dst_row[kConvertRounds];  // this lane's tile row (bits 0-30), B tile (bit 31)
     int shift[kConvertRounds];
     bool valid[kConvertRounds];
     bool ok = true;
-    for (int64_t chunk = c_begin; chunk < c_end && ok; ++chunk) {
+    int64_t chunk = c_begin;
+    for (; chunk < c_end && ok; ++chunk) {
       advance(blk, seg_start, descs, blocks, n_blocks, chunk, has_maps);
+      if (blk.tma) break;
       int64_t x_begin;
       const int stages = stages_of(blk, chunk, &x_begin);
-      if (blk.tma) {
-        if (cw != 0) continue;
-        if (!tma_started) {
-          // The staged stages before are done: the MMA has read every staged operand stage and the
-          // converters every raw stage (last phases, which cannot alias). Then the ones rows of the
-          // slots carved from the raw ring.
-          tma_started = true;
-          bool got = true;
-          if (lane == 0)
-            got = drain(sm.empty, ring, abort, error, kAtStageSlot) && drain(sm.raw_empty, raw_ring, abort, error, kAtRaw);
-          if (!__shfl_sync(0xffffffffu, (int)got, 0)) {
-            ok = false;
-            break;
-          }
-          const uint4 ones = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
-          for (int i = lane; i < kTmaExtra * (kAtom / 16); i += 32) {
-            const int s = kRing + i / (kAtom / 16), c16 = i % (kAtom / 16);
-            *reinterpret_cast<uint4*>(tma_tile_a(sm, s) + kRowsA * kAtom + 16 * c16) = ones;
-            *reinterpret_cast<uint4*>(tma_tile_b(sm, s) + kRowsB * kAtom + 16 * c16) = ones;
-          }
-          fence_async_smem();  // generic stores before the tensor core reads them
-          __syncwarp();
-        }
-        bool got = true;
-        if (lane == 0) {
-          const int64_t* r = blocks + blk.index * kBlkFields;
-          const CUtensorMap* m = maps + 2 * r[kBlkImage];
-          for (int st = 0; st < stages; ++st, tring.next()) {
-            const int slot = tring.slot;
-            if (tring.reused && !wait_bar(&sm.tma_empty[slot], tring.phase ^ 1u, abort, error, kAtTmaSlot)) {
-              got = false;
-              break;
-            }
-            const int x = (int)(x_begin + (int64_t)st * kAtom);
-            mbar_arrive_expect_tx(&sm.tma_full[slot], kTmaBytes);  // release: the ones rows above
-            tma_load_2d(tma_tile_a(sm, slot), m, x, (int)r[kBlkM0], &sm.tma_full[slot]);
-            tma_load_2d(tma_tile_b(sm, slot), m + 1, x, (int)r[kBlkN0], &sm.tma_full[slot]);
-          }
-        }
-        if (!__shfl_sync(0xffffffffu, (int)got, 0)) ok = false;
-        continue;
-      }
-      if (tma_started) {  // a staged block after a TMA block: the host orders them the other way
-        if (lane == 0) atomicOr(error, kOrderBit);
-        *abort = 1;
-        ok = false;
-        break;
-      }
       if (blk.index != cached) {
         cached = blk.index;
         const Rows rows = rows_of(descs, blocks, blk.index);
 #pragma unroll
         for (int k = 0; k < kConvertRounds; ++k) {
-          const int row = cw * kConvertRowsPerWarp + q + kConvertRowsPerRound * k;
+          const int row = tw * kConvertRowsPerWarp + q + kConvertRowsPerRound * k;
           valid[k] = row < rows.Dm + rows.Gn;
           shift[k] = valid[k] ? (int)(reinterpret_cast<uintptr_t>(rows.row(row)) & 15) : 0;
           const int t = row < rows.Dm ? row : row - rows.Dm;
@@ -583,6 +538,9 @@ inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restric
         }
       }
       for (int st = 0; st < stages; ++st, raw_ring.next(), ring.next()) {
+        const bool mine = turn == team;  // the slots then are the team's too: it awaits each of their phases
+        turn = turn + 1 == kTeams ? 0 : turn + 1;
+        if (!mine) continue;
         const int rslot = raw_ring.slot, slot = ring.slot;
         bool got = wait_bar(&sm.raw_full[rslot], raw_ring.phase, abort, error, kAtRaw);
         got = got && (!ring.reused || wait_bar(&sm.empty[slot], ring.phase ^ 1u, abort, error, kAtStageSlot));
@@ -602,7 +560,7 @@ inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restric
 #pragma unroll
           for (int k = 0; k < kConvertRounds; ++k) {
             if (!valid[k]) continue;
-            const int row = cw * kConvertRowsPerWarp + q + kConvertRowsPerRound * k;
+            const int row = tw * kConvertRowsPerWarp + q + kConvertRowsPerRound * k;
             const uint4* words = reinterpret_cast<const uint4*>(raw + row * kRawRow) + c0;
             uint4 wv[kConvertChunks + 1];
 #pragma unroll
@@ -632,11 +590,53 @@ inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restric
         }
       }
     }
-    if (cw == 0 && lane == 0 && tma_started)  // the last TMA load into every slot lands before the CTA exits
-      for (int s = 0; s < kTmaRing; ++s) {
-        if (s < tring.slot) mbar_wait(&sm.tma_full[s], tring.phase, kWaitLimit);
-        else if (tring.reused) mbar_wait(&sm.tma_full[s], tring.phase ^ 1u, kWaitLimit);
+    // Every converter has stored its last stage (or gave up): of every operand slot only the last phase can be
+    // open, and the raw ring is free.
+    asm volatile("bar.sync 1, %0;" ::"n"(kConvertWarps * 32) : "memory");
+    if (cw == 0 && ok && chunk < c_end) {
+      bool got = true;
+      if (lane == 0) got = drain(sm.empty, ring, abort, error, kAtStageSlot);
+      got = __shfl_sync(0xffffffffu, (int)got, 0);
+      // Ones rows of the slots carved from the raw ring, in memory before the tensor core reads them.
+      const uint4 ones = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
+      for (int i = lane; i < kTmaExtra * (kAtom / 16); i += 32) {
+        const int s = kRing + i / (kAtom / 16), c16 = i % (kAtom / 16);
+        *reinterpret_cast<uint4*>(tma_tile_a(sm, s) + kRowsA * kAtom + 16 * c16) = ones;
+        *reinterpret_cast<uint4*>(tma_tile_b(sm, s) + kRowsB * kAtom + 16 * c16) = ones;
       }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        Ring<kTmaRing> tring;
+        for (; chunk < c_end && got; ++chunk) {
+          advance(blk, seg_start, descs, blocks, n_blocks, chunk, has_maps);
+          if (!blk.tma) {  // a staged block after a TMA block: the host orders them the other way
+            atomicOr(error, kOrderBit);
+            *abort = 1;
+            break;
+          }
+          int64_t x_begin;
+          const int stages = stages_of(blk, chunk, &x_begin);
+          const int64_t* r = blocks + blk.index * kBlkFields;
+          const CUtensorMap* m = maps + 2 * r[kBlkImage];
+          for (int st = 0; st < stages; ++st, tring.next()) {
+            const int slot = tring.slot;
+            if (tring.reused && !wait_bar(&sm.tma_empty[slot], tring.phase ^ 1u, abort, error, kAtTmaSlot)) {
+              got = false;
+              break;
+            }
+            const int x = (int)(x_begin + (int64_t)st * kAtom);
+            mbar_arrive_expect_tx(&sm.tma_full[slot], kTmaBytes);  // release: the ones rows above
+            tma_load_2d(tma_tile_a(sm, slot), m, x, (int)r[kBlkM0], &sm.tma_full[slot]);
+            tma_load_2d(tma_tile_b(sm, slot), m + 1, x, (int)r[kBlkN0], &sm.tma_full[slot]);
+          }
+        }
+        for (int s = 0; s < kTmaRing; ++s) {  // the last TMA load into every slot lands before the CTA exits
+          if (s < tring.slot) mbar_wait(&sm.tma_full[s], tring.phase, kWaitLimit);
+          else if (tring.reused) mbar_wait(&sm.tma_full[s], tring.phase ^ 1u, kWaitLimit);
+        }
+      }
+    }
     __syncwarp();
   } else {
     // ---- epilogue: accumulator -> integer counts -> global counters ------------
