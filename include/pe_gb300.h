@@ -274,6 +274,25 @@ int pe_inst_contract(const int64_t* descs, const int64_t* blocks, int64_t n_bloc
                      int64_t inter_len, uint64_t* pa, int64_t pa_len, uint64_t* ga, int64_t ga_len, const void* maps,
                      int32_t* error, cudaStream_t stream);
 /*
+ * How long streaming a batch may take (picoseconds, as pe_inst_intersect estimates
+ * it) to be faster than its contraction; 0: contract whatever the masks hold.
+ * tma (optional) marks the images with tensor maps; sms: the device's SMs. Host
+ * side, no GPU work.
+ */
+int64_t pe_stream_limit(const int64_t* dets, const int64_t* gts, const int64_t* pixels, const uint8_t* tma, int64_t B,
+                        int64_t sms);
+/*
+ * pe_inst_contract's counts, with the way chosen on the device: a sample of the
+ * masks estimates how long streaming them through CUDA cores would take; above
+ * `limit` (pe_stream_limit) they are contracted instead.
+ * pair_chunks: 4096-pixel chunks of the table (kChunkBegin); work: 8 B + 1 u64,
+ * device scratch. A wait that times out sets bit 30 of *error.
+ */
+int pe_inst_intersect(const int64_t* descs, int64_t B, int64_t pair_chunks, const int64_t* blocks, int64_t n_blocks,
+                      int64_t total_chunks, const int64_t* cta_bounds, int64_t ctas, const int64_t* order,
+                      uint32_t* inter, int64_t inter_len, uint64_t* pa, int64_t pa_len, uint64_t* ga, int64_t ga_len,
+                      const void* maps, int64_t limit, uint64_t* work, int32_t* error, cudaStream_t stream);
+/*
  * Host-side companion of pe_inst_contract (no GPU work): for each image of the
  * HOST descriptor table whose mask rows start on 16-byte boundaries (flags
  * bit 1), with detections and targets, encodes two CUtensorMap (detection

@@ -51,6 +51,8 @@ SIGNATURES = {
     "pe_inst_overlap": [P, I64, I64, I64, P, P, P, P, I64, P, I64, P, I64, P],
     "pe_pack_rgb": [P, I64, I64, P, P, I64, P, P, P],
     "pe_inst_contract": [P, P, I64, I64, P, I64, P, P, I64, P, I64, P, I64, P, P, P],
+    "pe_inst_intersect": [P, I64, I64, P, I64, I64, P, I64, P, P, I64, P, I64, P, I64, P, I64, P, P, P],
+    "pe_stream_limit": [P, P, P, P, I64, I64],
     "pe_contract_maps": [P, I64, P],
     "pe_contract_blocks": [P, P, P, P, I64, D, I64, P, I64, P, P, P],
     "pe_inst_gather": [P, P, I64, P, P, P, P, P, P],
@@ -61,7 +63,8 @@ SIGNATURES = {
 }
 
 # Entry points that return a size instead of a status.
-INT64_RESULTS = {"pe_instance_accumulate_workspace", "pe_seg_sort_workspace", "pe_contract_blocks"}
+INT64_RESULTS = {"pe_instance_accumulate_workspace", "pe_seg_sort_workspace", "pe_contract_blocks",
+                 "pe_stream_limit"}
 
 _lock = threading.Lock()
 _lib = None

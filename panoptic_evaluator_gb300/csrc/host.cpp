@@ -39,7 +39,7 @@ using namespace pe;
 #define PE_HOST_API(X)                                                                              \
   X(pe_update) X(pe_compute) X(pe_reward_pq) X(pe_pack) X(pe_pack_rgb) X(pe_contract_maps)          \
   X(pe_contract_blocks) X(pe_inst_gather) X(pe_seg_sort) X(pe_seg_sort_workspace)                   \
-  X(pe_inst_contract) X(pe_inst_prepare) X(pe_seg_match) X(pe_instance_accumulate)                  \
+  X(pe_inst_contract) X(pe_inst_intersect) X(pe_stream_limit) X(pe_inst_prepare) X(pe_seg_match) X(pe_instance_accumulate)                  \
   X(pe_instance_accumulate_workspace) X(pe_seg_pass) X(pe_seg_score) X(pe_prefix)
 
 struct Api {
@@ -639,7 +639,7 @@ struct InstancePlan {
   std::vector<int64_t> dets, gts;
   Metadata pc, scores, gc, crowd, areas;
   int64_t B = 0, total_d = 0, total_g = 0, pairs = 0, max_g = 1;
-  int64_t n_blocks = 0, total_chunks = 0, ranges = 0;
+  int64_t n_blocks = 0, total_chunks = 0, ranges = 0, chunks = 0, stream_limit = 0;
   int64_t bounds_at = 0, blocks_at = 0, maps_at = -1, rows_at = 0, words = 0;
   Tensor host;
 };
@@ -719,6 +719,9 @@ bool plan_instances(PyObject* prediction, PyObject* target, int index, PyObject*
   p.n_blocks = api.pe_contract_blocks(p.dets.data(), p.gts.data(), pixels.data(), given ? tma.data() : nullptr, B, cost,
                                       ctas, words + p.blocks_at, cap, words + p.bounds_at, &p.total_chunks, &p.ranges);
   if (p.n_blocks < 0) return false;
+  p.chunks = chunks;
+  p.stream_limit = api.pe_stream_limit(p.dets.data(), p.gts.data(), pixels.data(), given ? tma.data() : nullptr, B, ctas);
+  if (p.stream_limit < 0) return false;
   std::memcpy(words, table.data(), 8 * B * kDescFields);
   fill_offsets(words, B);
   for (int64_t b = 0; b < B; ++b) {
@@ -770,7 +773,7 @@ PyObject* instance_update(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int64_t table_at = l.add(8 * p.words), pc_at = l.add(4 * D), scores_at = l.add(8 * D), gc_at = l.add(4 * G);
   const int64_t crowd_at = l.add(G), ann_in_at = l.add(8 * G), order_at = l.add(8 * D), sort_at = l.add(sort_bytes);
   const int64_t pa_d_at = l.add(8 * D), ga_d_at = l.add(8 * G), ann_at = l.add(8 * G);
-  const int64_t bits_at = l.add(4 * B * ((*C + 31) / 32));
+  const int64_t bits_at = l.add(4 * B * ((*C + 31) / 32)), stream_at = l.add(8 * (8 * B + 1));
   // Intersections, the error word, then both area counters, without gaps: the contraction clears them at once.
   const int64_t inter_len = round_up(p.pairs, 2) + 2, counts_at = l.add(4 * inter_len + 8 * (D + G));
   Tensor work = arena(self, index, l.size);
@@ -799,11 +802,16 @@ PyObject* instance_update(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (!code)
       code = api.pe_seg_sort(descs, B, scores, pc, D, order, tail.scores, tail.classes, at_address<void>(base + sort_at),
                              sort_bytes, stream);
-    if (!code)
-      code = api.pe_inst_contract(descs, p.total_chunks ? descs + p.blocks_at : nullptr, p.n_blocks, p.total_chunks,
-                                  p.total_chunks ? descs + p.bounds_at : nullptr, p.ranges, order, inter, inter_len, pa,
-                                  D, pa + D, G, p.maps_at >= 0 && p.total_chunks ? descs + p.maps_at : nullptr, error,
-                                  stream);
+    const int64_t* blocks = p.total_chunks ? descs + p.blocks_at : nullptr;
+    const int64_t* bounds = p.total_chunks ? descs + p.bounds_at : nullptr;
+    const int64_t* maps = p.maps_at >= 0 && p.total_chunks ? descs + p.maps_at : nullptr;
+    if (!code && p.stream_limit > 0)  // sparse masks may be counted faster by streaming them
+      code = api.pe_inst_intersect(descs, B, p.chunks, blocks, p.n_blocks, p.total_chunks, bounds, p.ranges, order, inter,
+                                   inter_len, pa, D, pa + D, G, maps, p.stream_limit,
+                                   at_address<uint64_t>(base + stream_at), error, stream);
+    else if (!code)
+      code = api.pe_inst_contract(descs, blocks, p.n_blocks, p.total_chunks, bounds, p.ranges, order, inter, inter_len,
+                                  pa, D, pa + D, G, maps, error, stream);
     if (!code)
       code = api.pe_inst_prepare(descs, B, pa, pa + D, pa_d, ga_d, tail.classes, gc, tail.scores, ann_in, ann, *C, check,
                                  bits, error, stream);

@@ -62,6 +62,7 @@
 #include <type_traits>
 
 #include "pe_common.cuh"
+#include "pe_contract.cuh"
 #include "pe_desc.cuh"
 
 namespace pe {
@@ -345,10 +346,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restrict__ blocks, int64_t n_blocks,
                      int64_t total_chunks, int64_t chunks_per_cta, const int64_t* __restrict__ bounds,
                      const int64_t* __restrict__ order, u32* __restrict__ inter, u64* __restrict__ pa,
-                     u64* __restrict__ ga, const CUtensorMap* __restrict__ maps, int* __restrict__ error) {
+                     u64* __restrict__ ga, const CUtensorMap* __restrict__ maps, Choice choice,
+                     int* __restrict__ error) {
   extern __shared__ unsigned char smem_raw[];
   ContractShared& sm = *reinterpret_cast<ContractShared*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  if (streams(choice)) return;  // the batch is counted by inst_pairs_kernel
   const int64_t c_begin = bounds ? bounds[blockIdx.x] : (int64_t)blockIdx.x * chunks_per_cta;
   const int64_t c_end = bounds ? min(bounds[blockIdx.x + 1], total_chunks) : min(c_begin + chunks_per_cta, total_chunks);
   if (c_begin >= c_end) return;
@@ -740,6 +743,28 @@ bool encode_rows(CUtensorMap* map, const void* base, int64_t pixels, int64_t row
 }
 
 }  // namespace
+
+int launch_contract(const int64_t* descs, const int64_t* blocks, int64_t n_blocks, int64_t total_chunks,
+                    const int64_t* cta_bounds, int64_t ctas, const int64_t* order, uint32_t* inter, uint64_t* pa,
+                    uint64_t* ga, const void* maps, Choice choice, int32_t* error, cudaStream_t stream) {
+  PE_REQUIRE(n_blocks >= 0 && total_chunks >= 0, "invalid batch");
+  PE_REQUIRE(n_blocks > 0 || total_chunks == 0, "chunks without blocks");
+  PE_REQUIRE((reinterpret_cast<uintptr_t>(maps) & 63) == 0, "tensor maps must be 64-byte aligned");
+  if (total_chunks == 0) return kOk;
+  PE_REQUIRE(!cta_bounds || (ctas > 0 && ctas <= INT_MAX), "invalid CTA count");
+  const int64_t even = std::min<int64_t>(total_chunks, sm_count());
+  const int64_t per_cta = ceil_div(total_chunks, even);
+  const int64_t grid = cta_bounds ? ctas : ceil_div(total_chunks, per_cta);
+  const size_t smem = sizeof(ContractShared) + 1024;
+  PE_CUDA(cudaFuncSetAttribute(inst_contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  inst_contract_kernel<<<(unsigned)grid, kThreads, smem, stream>>>(
+      descs, blocks, n_blocks, total_chunks, per_cta, cta_bounds, order, reinterpret_cast<u32*>(inter),
+      reinterpret_cast<u64*>(pa), reinterpret_cast<u64*>(ga), reinterpret_cast<const CUtensorMap*>(maps), choice, error);
+  PE_LAUNCHED("inst_contract");
+  count_launch();
+  return kOk;
+}
+
 }  // namespace pe
 
 using namespace pe;
@@ -878,17 +903,6 @@ PE_API int pe_inst_contract(const int64_t* descs, const int64_t* blocks, int64_t
   PE_REQUIRE((reinterpret_cast<uintptr_t>(maps) & 63) == 0, "tensor maps must be 64-byte aligned");
   const int zeroed = zero_spans({{inter, 4 * inter_len}, {pa, 8 * pa_len}, {ga, 8 * ga_len}}, stream);
   if (zeroed != kOk) return zeroed;
-  if (total_chunks == 0) return kOk;
-  PE_REQUIRE(!cta_bounds || (ctas > 0 && ctas <= INT_MAX), "invalid CTA count");
-  const int64_t even = std::min<int64_t>(total_chunks, sm_count());
-  const int64_t per_cta = ceil_div(total_chunks, even);
-  const int64_t grid = cta_bounds ? ctas : ceil_div(total_chunks, per_cta);
-  const size_t smem = sizeof(ContractShared) + 1024;
-  PE_CUDA(cudaFuncSetAttribute(inst_contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  inst_contract_kernel<<<(unsigned)grid, kThreads, smem, stream>>>(
-      descs, blocks, n_blocks, total_chunks, per_cta, cta_bounds, order, reinterpret_cast<u32*>(inter),
-      reinterpret_cast<u64*>(pa), reinterpret_cast<u64*>(ga), reinterpret_cast<const CUtensorMap*>(maps), error);
-  PE_LAUNCHED("inst_contract");
-  count_launch();
-  return kOk;
+  return launch_contract(descs, blocks, n_blocks, total_chunks, cta_bounds, ctas, order, inter, pa, ga, maps,
+                         Choice{nullptr, 0, 0}, error, stream);
 }
