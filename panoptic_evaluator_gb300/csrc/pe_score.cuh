@@ -136,8 +136,8 @@ __device__ void score_accumulate(const Count* __restrict__ pairs, const int* __r
 // same-class crowd target is the largest such index. Same results as
 // score_accumulate, the class sums added in the same order. Counts of one image
 // are below 2^32, slots below 2^16 (the tables' shared memory holds fewer).
-// 16 images of 101 x 121 slots: 44.7 -> 10.7 us; 8 of 257 x 277: 132 -> 42; 64
-// of up to 150 x 170: 41 -> 21. Staging all counts and matching column by column
+// 16 images of 101 x 121 slots: 44.7 -> 10.3 us; 8 of 257 x 277: 132 -> 32; 64
+// of up to 150 x 170: 41 -> 17.6. Staging all counts and matching column by column
 // instead of by list took 18, 71 and 33.
 struct ScoreTables {
   double* acc;   // C per-class IoU sums
@@ -223,19 +223,32 @@ __device__ void score_totals(const Count* __restrict__ pairs, const ScoreTables&
       for (int j = 0; j < kScoreRows; ++j)
         v[j] = g + j < g1 && p < P ? (u32)column[(int64_t)(g + j) * P] : 0u;
       if (g == 0 && p < P) t.over[p] = v[0];
+      // One place in the list for the entries of all these rows: every atomic on its length waits for the last.
+      u32 some[kScoreRows];
+      int count = 0;
 #pragma unroll
       for (int j = 0; j < kScoreRows; ++j) {
-        const u32 some = __ballot_sync(0xffffffffu, v[j] != 0);
-        if (!some) continue;  // the whole warp: most rows have no pixel in these columns
+        some[j] = __ballot_sync(0xffffffffu, v[j] != 0);
+        count += __popc(some[j]);
+      }
+      if (!count) continue;
+      int at = 0;
+      if (lane == 0) at = atomicAdd(t.n, count);
+      u32 total = 0;  // lane j: row g + j
+#pragma unroll
+      for (int j = 0; j < kScoreRows; ++j) {
+        if (!some[j]) continue;  // the whole warp: most rows have no pixel in these columns
         sum += v[j];
-        const u32 total = __reduce_add_sync(0xffffffffu, v[j]);
-        int at = 0;
-        if (lane == 0) {
-          atomicAdd(t.row + g + j, total);
-          at = atomicAdd(t.n, __popc(some));
-        }
-        at = __shfl_sync(0xffffffffu, at, 0) + __popc(some & below);
-        if (v[j] && at < t.cap) t.list[at] = make_uint2((u32)(g + j) << 16 | (u32)p, v[j]);
+        const u32 row = __reduce_add_sync(0xffffffffu, v[j]);
+        total = lane == j ? row : total;
+      }
+      if (total) atomicAdd(t.row + g + lane, total);
+      at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+      for (int j = 0; j < kScoreRows; ++j) {
+        const int e = at + __popc(some[j] & below);
+        if (v[j] && e < t.cap) t.list[e] = make_uint2((u32)(g + j) << 16 | (u32)p, v[j]);
+        at += __popc(some[j]);
       }
     }
     if (sum) atomicAdd(t.col + p, sum);
