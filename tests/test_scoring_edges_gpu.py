@@ -102,3 +102,23 @@ def test_out_of_range_slots_are_reported_and_not_counted():
     with pytest.raises(ValueError, match="unknown segment ID or a slot outside"):
         ev.update(pe.PanopticBatch(dev(pred), dev(classes)), pe.PanopticBatch(dev(gt), dev(classes)))
     assert all(torch.equal(v, before[k]) for k, v in ev.state_dict().items())
+
+
+@pytest.mark.parametrize("validate", (False, True))
+@pytest.mark.parametrize("images", (1, 7, 77, 160))
+def test_detection_areas_beside_the_scoring(images, validate):
+    """Few images leave SMs that sum detection areas in blocks of their own; more than SMs share their blocks."""
+    import panoptic_evaluator_gb300 as pe
+    from oracle import combined as ocomb
+    from panoptic_evaluator_gb300 import synthetic
+    from panoptic_evaluator_gb300.ragged import SegmentationImages
+    batch = synthetic.segmentation_batch(seed=images, images=images, side=(20, 60), slots=(3, 60), dets=(0, 40))
+    isthing = list(np.arange(133) < 80)
+    oracle = ocomb.SegmentationOracle(133, isthing)
+    for i in batch:
+        oracle.update(i.pred[None], i.pred_classes[None], [i.det_masks], [i.det_classes], [i.scores], i.target[None],
+                      i.target_classes[None], i.crowd[None])
+    fields = ("target", "target_classes", "crowd", "pred", "pred_classes", "det_masks", "det_classes", "scores")
+    joint = pe.SegmentationEvaluator(133, isthing=isthing, validate=validate)
+    joint.update_images(SegmentationImages(*([getattr(i, f) for i in batch] for f in fields)))
+    assert_tree(joint.compute(), oracle.compute())
