@@ -176,4 +176,38 @@ __device__ __forceinline__ uint4 realign16(uint4 lo, uint4 hi, int o) {
                     __funnelshift_r(u3, u4, sh));
 }
 
+// ---- kernels behind one another -------------------------------------------------
+// An evaluator call is a chain of short kernels, and each launch that is prepared only when the kernel before it
+// has ended and its writes are out costs 2 us of an idle chip. Every kernel of this library is launched with
+// programmatic stream serialization and begins with wait_for_earlier_kernels(): its launch is under way while the
+// kernel before ends, its blocks start when the last block before has left, and they go on once that kernel's
+// writes are visible. No access comes before the wait, so a kernel that completed also stands for all before it.
+// No kernel lets the next one start earlier (griddepcontrol.launch_dependents): the next one's read-only loads
+// then never see memory that a running kernel writes, and it measured the same. Per call, us: 16 reward images
+// 36.5 -> 28.8, 16 COCO-like panoptic images 48.6 -> 43.1, instance updates of 32 images 333 -> 312 and
+// 259 -> 242, joint updates 300 -> 285 and 405 -> 389, prefixes of 8 images 260 -> 246.
+__device__ __forceinline__ void wait_for_earlier_kernels() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+inline cudaLaunchAttribute early_launch() {
+  cudaLaunchAttribute attribute = {};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  return attribute;
+}
+
+// kernel<<<grid, block, smem, stream>>>(args...), launched ahead. Errors are left to PE_LAUNCHED.
+template <typename... Params, typename... Args>
+void launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  static_assert(sizeof...(Params) == sizeof...(Args), "one argument per kernel parameter");
+  cudaLaunchAttribute attribute = early_launch();
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 }  // namespace pe

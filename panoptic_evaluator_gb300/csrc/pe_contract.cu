@@ -348,6 +348,7 @@ inst_contract_kernel(const int64_t* __restrict__ descs, const int64_t* __restric
                      const int64_t* __restrict__ order, u32* __restrict__ inter, u64* __restrict__ pa,
                      u64* __restrict__ ga, const CUtensorMap* __restrict__ maps, Choice choice,
                      int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ unsigned char smem_raw[];
   ContractShared& sm = *reinterpret_cast<ContractShared*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -757,9 +758,9 @@ int launch_contract(const int64_t* descs, const int64_t* blocks, int64_t n_block
   const int64_t grid = cta_bounds ? ctas : ceil_div(total_chunks, per_cta);
   const size_t smem = sizeof(ContractShared) + 1024;
   PE_CUDA(cudaFuncSetAttribute(inst_contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  inst_contract_kernel<<<(unsigned)grid, kThreads, smem, stream>>>(
-      descs, blocks, n_blocks, total_chunks, per_cta, cta_bounds, order, reinterpret_cast<u32*>(inter),
-      reinterpret_cast<u64*>(pa), reinterpret_cast<u64*>(ga), reinterpret_cast<const CUtensorMap*>(maps), choice, error);
+  launch_kernel(inst_contract_kernel, (unsigned)grid, kThreads, smem, stream, descs, blocks, n_blocks, total_chunks,
+      per_cta, cta_bounds, order, reinterpret_cast<u32*>(inter), reinterpret_cast<u64*>(pa), reinterpret_cast<u64*>(ga),
+      reinterpret_cast<const CUtensorMap*>(maps), choice, error);
   PE_LAUNCHED("inst_contract");
   count_launch();
   return kOk;

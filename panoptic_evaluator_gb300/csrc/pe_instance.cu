@@ -98,6 +98,7 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
              const double* __restrict__ areas, int C, int g_max, FlagLayout flags, int* __restrict__ ranks,
              int64_t* __restrict__ counts, const int* __restrict__ gate,
              const u32* __restrict__ class_bits) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (gate && *reinterpret_cast<const volatile int*>(gate)) return;  // validation failed upstream
   // Image b covers detections [d_off[b], d_off[b+1]) and targets [g_off[b], g_off[b+1]);
@@ -345,6 +346,7 @@ constexpr int kRankSort = 192;  // records of a class sorted by counting rather 
 constexpr int64_t kScanRecords = 8192;
 
 __global__ void class_histogram_kernel(const int* __restrict__ classes, int64_t n, int C, int* __restrict__ hist) {
+  wait_for_earlier_kernels();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int c = classes[i];
     if (c >= 0 && c < C) atomicAdd(hist + c, 1);
@@ -354,6 +356,7 @@ __global__ void class_histogram_kernel(const int* __restrict__ classes, int64_t 
 // Exclusive scan of the class histogram into `cursor` (one CTA): cursor[c] is
 // where class c's record indices start in the per-class list.
 __global__ void __launch_bounds__(1024) class_offsets_kernel(const int* __restrict__ hist, int C, int* cursor) {
+  wait_for_earlier_kernels();
   __shared__ int s_warp[32];
   const int per = (C + blockDim.x - 1) / blockDim.x;
   const int c0 = min(C, (int)threadIdx.x * per), c1 = min(C, c0 + per);
@@ -389,6 +392,7 @@ __global__ void __launch_bounds__(1024) class_offsets_kernel(const int* __restri
 // accumulation sorts each class by score, then record index).
 __global__ void class_scatter_kernel(const int* __restrict__ classes, int64_t n, int C, int* cursor,
                                      int* __restrict__ list) {
+  wait_for_earlier_kernels();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int c = classes[i];
     if (c >= 0 && c < C) list[atomicAdd(cursor + c, 1)] = (int)i;
@@ -465,6 +469,7 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
                   unsigned long long* __restrict__ ws_key, int* __restrict__ ws_idx,
                   int C, int* __restrict__ env_ws, double* __restrict__ precision,
                   double* __restrict__ recall, double* __restrict__ chain_stats, int above) {
+  wait_for_earlier_kernels();
   // The bitonic sort pads a class's records to the next power of two inside the kCap-entry stage.
   static_assert(kCap > 0 && (kCap & (kCap - 1)) == 0, "a stage cap must be a power of two");
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -722,6 +727,7 @@ constexpr int kSummarizeLoads = 4;  // loads in flight per thread and round
 
 __global__ void __launch_bounds__(kSummarizeThreads)
 summarize_chains_kernel(const double* __restrict__ chain_stats, int C, double* __restrict__ out) {
+  wait_for_earlier_kernels();
   const int q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // summary -> (uses precision sums?, area, maxDets index, single threshold or -1)
   const bool is_ap = q < 4 || q == 5 || q == 7;
@@ -781,6 +787,7 @@ summarize_chains_kernel(const double* __restrict__ chain_stats, int C, double* _
 __global__ void __launch_bounds__(256)
 summarize_kernel(const double* __restrict__ precision, const double* __restrict__ recall, int C,
                  double* __restrict__ out) {
+  wait_for_earlier_kernels();
   // out: ap, ap50, ap75, ap_small, ar_small, ap_medium, ar_medium, ap_large, ar_large, ar1, ar10, ar100
   __shared__ double s_sum[256];
   __shared__ int s_cnt[256];
@@ -856,6 +863,7 @@ template <bool SMEM>
 __global__ void __launch_bounds__(kDetThreads)
 detection_histogram_kernel(const uint8_t* __restrict__ masks, int64_t pixels, int D, const int* __restrict__ target,
                            const int64_t* __restrict__ order, int S, int align, u64* __restrict__ pairs) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   u32* bins = reinterpret_cast<u32*>(smem_raw);
   const int bins_count = D * S;
@@ -920,6 +928,7 @@ __device__ __forceinline__ uint32_t pack4(uint32_t w) { return ((w & 0x01010101u
 __global__ void __launch_bounds__(kOvThreads)
 mask_overlap_kernel(const uint8_t* __restrict__ pm, int D, const uint8_t* __restrict__ gm, int G, int64_t pixels,
                     int align, const int* __restrict__ pc, const int* __restrict__ gc, u64* __restrict__ inter) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int rows = D + G;
   uint32_t* bits = reinterpret_cast<uint32_t*>(smem_raw);            // rows x kOvWords
@@ -994,15 +1003,13 @@ int launch_match(const void* pairs, bool pairs_u32, const int64_t* pair_off, con
   if (pairs_u32) {
     auto kernel = match_kernel<u32>;
     if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, kMatchThreads, smem, stream>>>(static_cast<const u32*>(pairs), pair_off, d_off, g_off, single_d,
-                                                      single_g, pc, pa, gc, ga, crowd, areas, C, g_max, layout, ranks,
-                                                      counts, gate, class_bits);
+    launch_kernel(kernel, grid, kMatchThreads, smem, stream, static_cast<const u32*>(pairs), pair_off, d_off, g_off,
+        single_d, single_g, pc, pa, gc, ga, crowd, areas, C, g_max, layout, ranks, counts, gate, class_bits);
   } else {
     auto kernel = match_kernel<int64_t>;
     if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, kMatchThreads, smem, stream>>>(static_cast<const int64_t*>(pairs), pair_off, d_off, g_off,
-                                                      single_d, single_g, pc, pa, gc, ga, crowd, areas, C, g_max,
-                                                      layout, ranks, counts, gate, class_bits);
+    launch_kernel(kernel, grid, kMatchThreads, smem, stream, static_cast<const int64_t*>(pairs), pair_off, d_off, g_off,
+        single_d, single_g, pc, pa, gc, ga, crowd, areas, C, g_max, layout, ranks, counts, gate, class_bits);
   }
   PE_LAUNCHED("match");
   count_launch();
@@ -1035,9 +1042,9 @@ int launch_accumulate_cap(const int* classes, int64_t n, const int* list, const 
   auto kernel = accumulate_kernel<kCap>;
   const size_t smem = sizeof(AccShared<kCap>);
   PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<(unsigned)(C * kAccParts), kAccThreads, smem, stream>>>(
-      classes, n, list, cursor, hist, ranks, flags, chain_stride, det_stride, scores, positives, ws_key, ws_idx, C,
-      env_ws, precision, recall, chain_stats, above);
+  launch_kernel(kernel, (unsigned)(C * kAccParts), kAccThreads, smem, stream, classes, n, list, cursor, hist, ranks,
+      flags, chain_stride, det_stride, scores, positives, ws_key, ws_idx, C, env_ws, precision, recall, chain_stats,
+      above);
   PE_LAUNCHED("accumulate");
   count_launch();
   return kOk;
@@ -1062,11 +1069,11 @@ int launch_accumulate(const int* classes, const int* ranks, const int8_t* flags,
   } else {
     PE_CUDA(cudaMemsetAsync(hist, 0, sizeof(int) * C, stream));
     const int64_t blocks = std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 4);
-    class_histogram_kernel<<<(unsigned)blocks, 256, 0, stream>>>(classes, n, C, hist);
+    launch_kernel(class_histogram_kernel, (unsigned)blocks, 256, 0, stream, classes, n, C, hist);
     PE_LAUNCHED("class_histogram");
-    class_offsets_kernel<<<1, 1024, 0, stream>>>(hist, C, cursor);
+    launch_kernel(class_offsets_kernel, 1, 1024, 0, stream, hist, C, cursor);
     PE_LAUNCHED("class_offsets");
-    class_scatter_kernel<<<(unsigned)blocks, 256, 0, stream>>>(classes, n, C, cursor, list);
+    launch_kernel(class_scatter_kernel, (unsigned)blocks, 256, 0, stream, classes, n, C, cursor, list);
     PE_LAUNCHED("class_scatter");
     count_launch(3);
   }
@@ -1081,7 +1088,7 @@ int launch_accumulate(const int* classes, const int* ranks, const int8_t* flags,
                                              chain_stats, kSmallCap, stream);
   if (status != kOk) return status;
   if (summary) {
-    summarize_chains_kernel<<<12, kSummarizeThreads, 0, stream>>>(chain_stats, C, summary);
+    launch_kernel(summarize_chains_kernel, 12, kSummarizeThreads, 0, stream, chain_stats, C, summary);
     PE_LAUNCHED("summarize_chains");
     count_launch();
   }
@@ -1089,7 +1096,7 @@ int launch_accumulate(const int* classes, const int* ranks, const int8_t* flags,
 }
 
 int launch_summarize(const double* precision, const double* recall, int C, double* out, cudaStream_t stream) {
-  summarize_kernel<<<12, 256, 0, stream>>>(precision, recall, C, out);
+  launch_kernel(summarize_kernel, 12, 256, 0, stream, precision, recall, C, out);
   PE_LAUNCHED("summarize");
   count_launch();
   return kOk;
@@ -1118,11 +1125,11 @@ PE_API int pe_instance_histogram(const uint8_t* masks, int64_t D, int64_t pixels
     if (smem_bytes > 48 * 1024)
       PE_CUDA(cudaFuncSetAttribute(detection_histogram_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)smem_bytes));
-    detection_histogram_kernel<true><<<(unsigned)grid, kDetThreads, smem_bytes, stream>>>(
-        masks, pixels, (int)D, target, order, (int)S, align, out);
+    launch_kernel(detection_histogram_kernel<true>, (unsigned)grid, kDetThreads, smem_bytes, stream, masks, pixels,
+        (int)D, target, order, (int)S, align, out);
   } else {
-    detection_histogram_kernel<false><<<(unsigned)grid, kDetThreads, 0, stream>>>(masks, pixels, (int)D, target, order,
-                                                                                  (int)S, align, out);
+    launch_kernel(detection_histogram_kernel<false>, (unsigned)grid, kDetThreads, 0, stream, masks, pixels, (int)D,
+        target, order, (int)S, align, out);
   }
   PE_LAUNCHED("detection_histogram");
   count_launch();
@@ -1160,8 +1167,8 @@ PE_API int pe_mask_overlap(const uint8_t* pm, int64_t D, const uint8_t* gm, int6
   if (smem > 48 * 1024)
     PE_CUDA(cudaFuncSetAttribute(mask_overlap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t grid = ceil_div(pixels, (int64_t)kOvWords * 32);
-  mask_overlap_kernel<<<(unsigned)grid, kOvThreads, smem, stream>>>(pm, (int)D, gm, (int)G, pixels, align, pc, gc,
-                                                                     reinterpret_cast<u64*>(inter));
+  launch_kernel(mask_overlap_kernel, (unsigned)grid, kOvThreads, smem, stream, pm, (int)D, gm, (int)G, pixels, align,
+      pc, gc, reinterpret_cast<u64*>(inter));
   PE_LAUNCHED("mask_overlap");
   count_launch();
   return kOk;

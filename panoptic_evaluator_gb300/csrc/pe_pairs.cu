@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kSampleThreads)
 inst_sample_kernel(const int64_t* __restrict__ descs, int64_t B, u64* __restrict__ costs, u32* __restrict__ inter,
                    int64_t inter_len, u64* __restrict__ pa, int64_t pa_len, u64* __restrict__ ga, int64_t ga_len,
                    unsigned long long* __restrict__ schedule) {
+  wait_for_earlier_kernels();
   const int64_t image = blockIdx.x / kSampleParts;
   if (image >= B) {
     const int64_t first = (blockIdx.x - B * kSampleParts) * kSampleThreads + threadIdx.x;
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kPairThreads, 2)
 inst_pairs_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chunks, Choice choice,
                   unsigned long long* __restrict__ schedule, const int64_t* __restrict__ order,
                   u32* __restrict__ inter, u64* __restrict__ pa, u64* __restrict__ ga, int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PairShared& sm = *reinterpret_cast<PairShared*>(smem_raw);
   if (!streams(choice)) return;
@@ -356,14 +358,13 @@ PE_API int pe_inst_intersect(const int64_t* descs, int64_t B, int64_t pair_chunk
                              const int64_t* order, uint32_t* inter, int64_t inter_len, uint64_t* pa, int64_t pa_len,
                              uint64_t* ga, int64_t ga_len, const void* maps, int64_t limit, uint64_t* work,
                              int32_t* error, cudaStream_t stream) {
-  PE_REQUIRE(B >= 0 && B <= INT_MAX / kSampleParts - kZeroBlocks && pair_chunks >= 0 && inter_len >= 0 && pa_len >= 0 && ga_len >= 0 &&
-                 work,
-             "invalid batch");
+  PE_REQUIRE(B >= 0 && B <= INT_MAX / kSampleParts - kZeroBlocks && pair_chunks >= 0 && work, "invalid batch");
+  PE_REQUIRE(inter_len >= 0 && pa_len >= 0 && ga_len >= 0, "invalid batch");
   u64* costs = reinterpret_cast<u64*>(work);
   unsigned long long* schedule = reinterpret_cast<unsigned long long*>(work + B * kSampleParts);
-  inst_sample_kernel<<<(unsigned)(B * kSampleParts + kZeroBlocks), kSampleThreads, 0, stream>>>(
-      descs, B, costs, reinterpret_cast<u32*>(inter), inter_len, reinterpret_cast<u64*>(pa), pa_len,
-      reinterpret_cast<u64*>(ga), ga_len, schedule);
+  launch_kernel(inst_sample_kernel, (unsigned)(B * kSampleParts + kZeroBlocks), kSampleThreads, 0, stream, descs, B,
+      costs, reinterpret_cast<u32*>(inter), inter_len, reinterpret_cast<u64*>(pa), pa_len, reinterpret_cast<u64*>(ga),
+      ga_len, schedule);
   PE_LAUNCHED("inst_sample");
   count_launch();
   if (B == 0 || pair_chunks == 0) return kOk;
@@ -371,9 +372,8 @@ PE_API int pe_inst_intersect(const int64_t* descs, int64_t B, int64_t pair_chunk
   const size_t smem = sizeof(PairShared);
   PE_CUDA(cudaFuncSetAttribute(inst_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t grid = std::min(pair_chunks, (int64_t)sm_count() * 2);
-  inst_pairs_kernel<<<(unsigned)grid, kPairThreads, smem, stream>>>(
-      descs, B, pair_chunks, choice, schedule, order, reinterpret_cast<u32*>(inter), reinterpret_cast<u64*>(pa),
-      reinterpret_cast<u64*>(ga), error);
+  launch_kernel(inst_pairs_kernel, (unsigned)grid, kPairThreads, smem, stream, descs, B, pair_chunks, choice, schedule,
+      order, reinterpret_cast<u32*>(inter), reinterpret_cast<u64*>(pa), reinterpret_cast<u64*>(ga), error);
   PE_LAUNCHED("inst_pairs");
   count_launch();
   return launch_contract(descs, blocks, n_blocks, total_chunks, cta_bounds, ctas, order, inter, pa, ga, maps, choice,

@@ -84,6 +84,7 @@ pair_histogram(const GT* __restrict__ gt, const PR* __restrict__ pred, int64_t p
                const int64_t* __restrict__ gt_ids, const int* __restrict__ gt_slots,
                const int64_t* __restrict__ pred_ids, const int* __restrict__ pred_slots,
                u64* __restrict__ pairs, int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   u32* bins = reinterpret_cast<u32*>(smem_raw);
   const int bins_count = G * P;
@@ -178,6 +179,7 @@ template <bool SMEM>
 __global__ void __launch_bounds__(kHistThreads, 2)
 slot_histogram(const int* __restrict__ gt, const int* __restrict__ pred, int64_t pixels, int64_t B, int G, int P,
                int64_t tiles_per_image, int64_t tiles_per_cta, u64* __restrict__ pairs, int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   u32* bins = reinterpret_cast<u32*>(smem_raw);
   const int bins_count = G * P;
@@ -301,6 +303,7 @@ score_blocks(const u64* __restrict__ pairs, const int* __restrict__ gc, const in
              const uint8_t* __restrict__ crowd, u64* __restrict__ areas, int* __restrict__ matched,
              u64* __restrict__ tp, u64* __restrict__ fp, u64* __restrict__ fn, double* __restrict__ iou_sum,
              u64* __restrict__ confusion, int G, int P, int C, int flags, int smem, int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t b = blockIdx.x;
   if ((flags & 8) && *reinterpret_cast<volatile int*>(error)) return;
@@ -333,6 +336,7 @@ score(const u64* __restrict__ pairs, const int* __restrict__ gc, const int* __re
       const uint8_t* __restrict__ crowd, u64* __restrict__ areas, int* __restrict__ matched,
       u64* __restrict__ tp, u64* __restrict__ fp, u64* __restrict__ fn, double* __restrict__ iou_sum,
       u64* __restrict__ confusion, int G, int P, int C, int flags, int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t b = blockIdx.x;
   if ((flags & 8) && *reinterpret_cast<volatile int*>(error)) return;
@@ -356,6 +360,7 @@ score(const u64* __restrict__ pairs, const int* __restrict__ gc, const int* __re
 __global__ void pack_slots_kernel(const void* maps, int is64, int64_t pixels, int64_t total,
                                   const int64_t* __restrict__ ids, const int* __restrict__ slots, int S,
                                   int* __restrict__ out, int* __restrict__ error) {
+  wait_for_earlier_kernels();
   bool bad = false;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -382,6 +387,7 @@ constexpr int kRgbPixels = 16;
 __global__ void __launch_bounds__(kRgbThreads)
 rgb_slots_kernel(const uint8_t* __restrict__ rgb, int64_t pixels, const int64_t* __restrict__ ids,
                  const int* __restrict__ slots, int S, int vec, int* __restrict__ out, int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int64_t* s_ids = reinterpret_cast<int64_t*>(smem_raw);
   int* s_slots = reinterpret_cast<int*>(s_ids + S);
@@ -477,6 +483,7 @@ compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, c
                const bool* __restrict__ things, double* per_class, double* summaries, int64_t* counts,
                double* miou, int64_t* out_tp, int64_t* out_fp, int64_t* out_fn, double* out_sums,
                int64_t* out_confusion, int C) {
+  wait_for_earlier_kernels();
   const int64_t k = blockIdx.x / CL;
   const int rank = blockIdx.x % CL;
   tp += k * C; fp += k * C; fn += k * C; sums += k * C;
@@ -655,8 +662,8 @@ int launch_slot_histogram(const int* gt, const int* pred, int64_t B, int64_t pix
   auto kernel = choice.smem ? slot_histogram<true> : slot_histogram<false>;
   if (smem_bytes > 48 * 1024)
     PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
-  kernel<<<(unsigned)grid.ctas, kHistThreads, smem_bytes, stream>>>(gt, pred, pixels, B, G, P, tiles_per_image,
-                                                                    grid.per_cta, pairs, error);
+  launch_kernel(kernel, (unsigned)grid.ctas, kHistThreads, smem_bytes, stream, gt, pred, pixels, B, G, P,
+      tiles_per_image, grid.per_cta, pairs, error);
   PE_LAUNCHED("slot_histogram");
   count_launch();
   return kOk;
@@ -679,7 +686,7 @@ int launch_histogram(const void* gt, const void* pred, int64_t B, int64_t pixels
     auto kernel = pair_histogram<GT, PR, SM, VC>;                                                      \
     if (smem_bytes > 48 * 1024)                                                                        \
       PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes)); \
-    kernel<<<(unsigned)grid.ctas, kHistThreads, smem_bytes, stream>>>(g, p, pixels, B, G, P, tiles_per_image, \
+    launch_kernel(kernel, (unsigned)grid.ctas, kHistThreads, smem_bytes, stream, g, p, pixels, B, G, P, tiles_per_image, \
                                                                       grid.per_cta, gi, gs, pi, ps, pairs, error); \
   } while (0)
   if (smem) {
@@ -759,12 +766,11 @@ PE_API int pe_update(const void* gt, int gt_is_int64, const void* pred, int pred
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   auto launch = [&](int flags, int* word) {
     if (blocks)
-      by_blocks<<<(unsigned)B, score_threads, smem, stream>>>(upairs, gc, pc, crowd, ua, matched, utp, ufp, ufn,
-                                                              iou_sum, uconf, (int)G, (int)P, (int)C, flags,
-                                                              (int)smem, word);
+      launch_kernel(by_blocks, (unsigned)B, score_threads, smem, stream, upairs, gc, pc, crowd, ua, matched, utp, ufp,
+          ufn, iou_sum, uconf, (int)G, (int)P, (int)C, flags, (int)smem, word);
     else
-      in_place<<<(unsigned)B, score_threads, smem, stream>>>(upairs, gc, pc, crowd, ua, matched, utp, ufp, ufn,
-                                                             iou_sum, uconf, (int)G, (int)P, (int)C, flags, word);
+      launch_kernel(in_place, (unsigned)B, score_threads, smem, stream, upairs, gc, pc, crowd, ua, matched, utp, ufp,
+          ufn, iou_sum, uconf, (int)G, (int)P, (int)C, flags, word);
     count_launch();
   };
   if (validate) {
@@ -792,6 +798,7 @@ __global__ void __launch_bounds__(kRewardThreads)
 reward_pq_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, const int64_t* __restrict__ fn,
                  const double* __restrict__ sums, int C, double* __restrict__ pq, int64_t* __restrict__ tot_tp,
                  int64_t* __restrict__ tot_fp, int64_t* __restrict__ tot_fn, double* __restrict__ tot_sums) {
+  wait_for_earlier_kernels();
   __shared__ double s_total[kRewardThreads / 32];
   __shared__ int s_active[kRewardThreads / 32];
   const int64_t o = (int64_t)blockIdx.x * C;
@@ -859,12 +866,13 @@ PE_API int pe_compute(const int64_t* tp, const int64_t* fp, const int64_t* fn, c
   config.blockDim = dim3(kComputeThreads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute cluster;
-  cluster.id = cudaLaunchAttributeClusterDimension;
-  cluster.val.clusterDim.x = kComputeCluster;
-  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-  config.attrs = &cluster;
-  config.numAttrs = shared_rows ? 1 : 0;
+  cudaLaunchAttribute attributes[2];
+  attributes[0] = early_launch();
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = kComputeCluster;
+  attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
+  config.attrs = attributes;
+  config.numAttrs = shared_rows ? 2 : 1;
   PE_CUDA(cudaLaunchKernelEx(&config, kernel, tp, fp, fn, sums, confusion, reinterpret_cast<const bool*>(things),
                              per_class, summaries, counts, miou, out_tp, out_fp, out_fn, out_sums, out_confusion,
                              (int)C));
@@ -881,8 +889,8 @@ PE_API int pe_reward_pq(const int64_t* tp, const int64_t* fp, const int64_t* fn,
   PE_REQUIRE(B >= 0 && C > 0 && C < INT_MAX, "invalid reward shapes");
   if (B == 0) return kOk;
   PE_REQUIRE(B <= INT_MAX, "too many images");
-  reward_pq_kernel<<<(unsigned)B, kRewardThreads, 0, stream>>>(tp, fp, fn, sums, (int)C, pq, tot_tp, tot_fp, tot_fn,
-                                                              tot_sums);
+  launch_kernel(reward_pq_kernel, (unsigned)B, kRewardThreads, 0, stream, tp, fp, fn, sums, (int)C, pq, tot_tp, tot_fp,
+      tot_fn, tot_sums);
   PE_LAUNCHED("reward_pq");
   count_launch();
   return kOk;
@@ -897,8 +905,8 @@ PE_API int pe_pack(const void* maps, int maps_is_int64, int64_t B, int64_t pixel
   const int64_t total = B * pixels;
   if (total == 0) return kOk;
   const int64_t blocks = std::min<int64_t>(ceil_div(total, 256), (int64_t)sm_count() * 8);
-  pack_slots_kernel<<<(unsigned)blocks, 256, 0, stream>>>(maps, maps_is_int64, pixels, total, ids, slots, (int)S,
-                                                          out, error);
+  launch_kernel(pack_slots_kernel, (unsigned)blocks, 256, 0, stream, maps, maps_is_int64, pixels, total, ids, slots,
+      (int)S, out, error);
   PE_LAUNCHED("pack");
   count_launch();
   return kOk;
@@ -923,8 +931,8 @@ PE_API int pe_pack_rgb(const uint8_t* rgb, int64_t B, int64_t pixels, const int6
   const int64_t per_block = (int64_t)kRgbThreads * kRgbPixels;
   const int64_t want = std::max<int64_t>(1, (int64_t)sm_count() * 8 / std::max<int64_t>(B, 1));
   const int64_t gx = std::min<int64_t>(ceil_div(pixels, per_block), want);
-  rgb_slots_kernel<<<dim3((unsigned)gx, (unsigned)B), kRgbThreads, smem, stream>>>(rgb, pixels, ids, slots, (int)S,
-                                                                                    vec, out, error);
+  launch_kernel(rgb_slots_kernel, dim3((unsigned)gx, (unsigned)B), kRgbThreads, smem, stream, rgb, pixels, ids, slots,
+      (int)S, vec, out, error);
   PE_LAUNCHED("pack_rgb");
   count_launch();
   return kOk;

@@ -255,6 +255,7 @@ template <bool kBytes>
 __global__ void __launch_bounds__(kPxThreads, 2)
 prefix_pass_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __restrict__ step_q, u32* __restrict__ ga,
                    u32* __restrict__ raw, int* __restrict__ delta, int* __restrict__ error) {
+  wait_for_earlier_kernels();
   const int64_t b = find_image(descs, B, kPrefixChunkBegin, blockIdx.x);
   const int64_t* d = pdesc(descs, b);
   const int64_t pixels = d[kPrefixPixels];
@@ -339,6 +340,7 @@ prefix_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t to
                         unsigned long long* __restrict__ schedule, const int* __restrict__ step_q,
                         u32* __restrict__ ga, u32* __restrict__ raw, int* __restrict__ delta,
                         int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PrefixShared& sm = *reinterpret_cast<PrefixShared*>(smem_raw);
   // Without a counter: contiguous chunk ranges whose sizes differ by at most one chunk.
@@ -522,6 +524,7 @@ prefix_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t to
 // Running sums over checkpoints: delta[q] -> pairs[q] in place.
 __global__ void prefix_scan_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ ga,
                                    int* __restrict__ delta) {
+  wait_for_earlier_kernels();
   const int64_t* d = pdesc(descs, blockIdx.y);
   const int N = (int)d[kPrefixN], G = (int)d[kPrefixG], Q = (int)d[kPrefixQ];
   const int64_t plane = (int64_t)G * (N + 1);
@@ -546,6 +549,7 @@ prefix_score_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __r
                     const int* __restrict__ classes, const int* __restrict__ gc, const uint8_t* __restrict__ crowd,
                     int C, int64_t* __restrict__ tp, int64_t* __restrict__ fp, int64_t* __restrict__ fn,
                     double* __restrict__ sums, int64_t* __restrict__ confusion, int smem) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t row = blockIdx.x;
   const int64_t b = find_image(descs, B, kPrefixQBegin, row);
@@ -598,6 +602,7 @@ prefix_match_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ g
                     const int* __restrict__ step_q, int64_t* __restrict__ itp, int64_t* __restrict__ ifp,
                     int64_t* __restrict__ ifn, double* __restrict__ precision, double* __restrict__ recall,
                     int validate, int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t* d = pdesc(descs, blockIdx.x);
   const int N = (int)d[kPrefixN], G = (int)d[kPrefixG];
@@ -824,6 +829,7 @@ prefix_match_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ g
 __global__ void prefix_ratio_kernel(const int64_t* __restrict__ itp, const int64_t* __restrict__ ifp,
                                     const int64_t* __restrict__ ifn, int64_t entries, double* __restrict__ precision,
                                     double* __restrict__ recall) {
+  wait_for_earlier_kernels();
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < entries; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t a = itp[e], f = ifp[e], n = a + ifn[e];
     precision[e] = (double)a / (double)(a + f > 1 ? a + f : 1);
@@ -880,18 +886,18 @@ PE_API int pe_prefix(const int64_t* descs, int64_t B, int64_t total_chunks, int6
       // Owners fit in a byte per pixel when no image has more than 255 masks.
       auto kernel = max_p <= 256 ? prefix_pass_bulk_kernel<true> : prefix_pass_bulk_kernel<false>;
       PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      kernel<<<(unsigned)grid, kPbThreads, smem, stream>>>(descs, B, total_chunks,
-                                                          reinterpret_cast<unsigned long long*>(schedule), step_q, ga,
-                                                          raw, pairs, error);
+      launch_kernel(kernel, (unsigned)grid, kPbThreads, smem, stream, descs, B, total_chunks,
+          reinterpret_cast<unsigned long long*>(schedule), step_q, ga, raw, pairs, error);
     } else {
       auto kernel = max_p <= 256 ? prefix_pass_kernel<true> : prefix_pass_kernel<false>;
-      kernel<<<(unsigned)total_chunks, kPxThreads, 0, stream>>>(descs, B, step_q, ga, raw, pairs, error);
+      launch_kernel(kernel, (unsigned)total_chunks, kPxThreads, 0, stream, descs, B, step_q, ga, raw, pairs, error);
     }
     PE_LAUNCHED("prefix_pass");
     count_launch();
   }
   if (max_cells > 0) {
-    prefix_scan_kernel<<<dim3((unsigned)ceil_div(max_cells, 256), (unsigned)B), 256, 0, stream>>>(descs, ga, pairs);
+    launch_kernel(prefix_scan_kernel, dim3((unsigned)ceil_div(max_cells, 256), (unsigned)B), 256, 0, stream, descs, ga,
+        pairs);
     PE_LAUNCHED("prefix_scan");
     count_launch();
   }
@@ -905,8 +911,8 @@ PE_API int pe_prefix(const int64_t* descs, int64_t B, int64_t total_chunks, int6
     const size_t smem = std::max(in_place, std::min<size_t>(want, 110 * 1024));
     if (smem > 48 * 1024)
       PE_CUDA(cudaFuncSetAttribute(prefix_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    prefix_score_kernel<<<(unsigned)total_rows, kPrefixScoreThreads, smem, stream>>>(
-        descs, B, pairs, classes, gc, crowd, (int)C, tp, fp, fn, sums, confusion, (int)smem);
+    launch_kernel(prefix_score_kernel, (unsigned)total_rows, kPrefixScoreThreads, smem, stream, descs, B, pairs,
+        classes, gc, crowd, (int)C, tp, fp, fn, sums, confusion, (int)smem);
     PE_LAUNCHED("prefix_score");
     count_launch();
   }
@@ -923,16 +929,15 @@ PE_API int pe_prefix(const int64_t* descs, int64_t B, int64_t total_chunks, int6
                (long long)T, (long long)C);
     auto kernel = stage ? prefix_match_kernel<true> : prefix_match_kernel<false>;
     if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<(unsigned)B, kPrefixMatchThreads, smem, stream>>>(descs, ga, raw, classes, gc, crowd, isthing, thresholds,
-                                                               (int)T, (int)C,
-                                               step_q, itp, ifp, ifn, precision, recall, validate, error);
+    launch_kernel(kernel, (unsigned)B, kPrefixMatchThreads, smem, stream, descs, ga, raw, classes, gc, crowd, isthing,
+        thresholds, (int)T, (int)C, step_q, itp, ifp, ifn, precision, recall, validate, error);
     PE_LAUNCHED("prefix_match");
     count_launch();
   }
   if (total_rows) {
     const int64_t entries = total_rows * T * C;
     const int64_t blocks = std::min<int64_t>(ceil_div(entries, 256), (int64_t)sm_count() * 4);
-    prefix_ratio_kernel<<<(unsigned)blocks, 256, 0, stream>>>(itp, ifp, ifn, entries, precision, recall);
+    launch_kernel(prefix_ratio_kernel, (unsigned)blocks, 256, 0, stream, itp, ifp, ifn, entries, precision, recall);
     PE_LAUNCHED("prefix_ratio");
     count_launch();
   }

@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(kSortThreads)
 seg_sort_kernel(const int64_t* __restrict__ descs, const double* __restrict__ scores, const int* __restrict__ classes,
                 int64_t* __restrict__ order, double* __restrict__ sorted_scores, int* __restrict__ sorted_classes,
                 u64* __restrict__ ws_key, int* __restrict__ ws_idx) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t* d = desc_of(descs, blockIdx.x);
   const int D = (int)d[kD];
@@ -97,6 +98,7 @@ seg_pass_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chun
                 const int64_t* __restrict__ bounds,
                 const int64_t* __restrict__ order, u32* __restrict__ pairs, u32* __restrict__ dpairs,
                 int* __restrict__ error) {
+  wait_for_earlier_kernels();
   // Contiguous chunk range of this CTA: host-balanced bounds, or an even split.
   const int64_t c_begin = bounds ? bounds[blockIdx.x] : (int64_t)blockIdx.x * chunks_per_cta;
   const int64_t c_end = bounds ? min(bounds[blockIdx.x + 1], total_chunks) : min(c_begin + chunks_per_cta, total_chunks);
@@ -215,6 +217,7 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
                      const int64_t* __restrict__ bounds, unsigned long long* __restrict__ schedule, int grab,
                      const int64_t* __restrict__ order, u32* __restrict__ pairs, u32* __restrict__ dpairs,
                      int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   BulkShared& sm = *reinterpret_cast<BulkShared*>(smem_raw);
   // Without a counter: a contiguous chunk range per CTA (host-balanced bounds, or an even split).
@@ -427,6 +430,7 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
                  int* __restrict__ slot_class, const double* __restrict__ ann_in, double* __restrict__ ann_out,
                  int mode, int validate, int reward, int smem, u32* __restrict__ class_bits,
                  int* __restrict__ error) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if ((mode & 4) && *reinterpret_cast<volatile int*>(error)) return;
   const int64_t* d = desc_of(descs, blockIdx.x);
@@ -547,6 +551,7 @@ __global__ void __launch_bounds__(kOvThreads)
 inst_overlap_kernel(const int64_t* __restrict__ descs, int64_t B, const int64_t* __restrict__ order,
                     const int* __restrict__ pc, const int* __restrict__ gc, u32* __restrict__ inter,
                     u64* __restrict__ pa, u64* __restrict__ ga) {
+  wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t b = image_of_chunk(descs, B, blockIdx.x);
   const int64_t* d = desc_of(descs, b);
@@ -617,6 +622,7 @@ __global__ void __launch_bounds__(128)
 inst_gather_kernel(const int64_t* __restrict__ descs, const int64_t* __restrict__ fields, int* __restrict__ pc,
                    double* __restrict__ scores, int* __restrict__ gc, uint8_t* __restrict__ crowd,
                    double* __restrict__ areas) {
+  wait_for_earlier_kernels();
   const int64_t* d = desc_of(descs, blockIdx.x);
   const int64_t* f = fields + (int64_t)blockIdx.x * kGatherFields;
   const int D = (int)d[kD], G = (int)d[kG];
@@ -641,6 +647,7 @@ __global__ void inst_prepare_kernel(const int64_t* __restrict__ descs, const u64
                                     const double* __restrict__ scores, const double* __restrict__ ann_in,
                                     double* __restrict__ ann_out, int C, int validate, u32* __restrict__ class_bits,
                                     int* __restrict__ error) {
+  wait_for_earlier_kernels();
   const int64_t* d = desc_of(descs, blockIdx.x);
   const int D = (int)d[kD], G = (int)d[kG];
   const int64_t db = d[kDetBegin], gb = d[kSlotBegin];
@@ -712,8 +719,8 @@ PE_API int pe_seg_sort(const int64_t* descs, int64_t B, const double* scores, co
   int* ws_idx = reinterpret_cast<int*>(ws_key + entries);
   const size_t smem = (sizeof(u64) + sizeof(int)) * kSortCap;
   PE_CUDA(cudaFuncSetAttribute(seg_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  seg_sort_kernel<<<(unsigned)B, kSortThreads, smem, stream>>>(descs, scores, classes, order, sorted_scores, sorted_classes,
-                                                      ws_key, ws_idx);
+  launch_kernel(seg_sort_kernel, (unsigned)B, kSortThreads, smem, stream, descs, scores, classes, order, sorted_scores,
+      sorted_classes, ws_key, ws_idx);
   PE_LAUNCHED("seg_sort");
   count_launch();
   return kOk;
@@ -794,9 +801,8 @@ PE_API int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, co
     const size_t smem = sizeof(BulkShared) + 128;
     auto kernel = bulk == 2 ? seg_pass_bulk_kernel<true> : seg_pass_bulk_kernel<false>;
     PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<(unsigned)grid, kBulkThreads, smem, stream>>>(
-        descs, B, total_chunks, per_cta, cta_bounds, reinterpret_cast<unsigned long long*>(schedule), grab,
-        order, pairs, dpairs, error);
+    launch_kernel(kernel, (unsigned)grid, kBulkThreads, smem, stream, descs, B, total_chunks, per_cta, cta_bounds,
+        reinterpret_cast<unsigned long long*>(schedule), grab, order, pairs, dpairs, error);
     PE_LAUNCHED("seg_pass_bulk");
     count_launch();
     return kOk;
@@ -804,8 +810,8 @@ PE_API int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, co
   const int64_t max_ctas = (int64_t)sm_count() * PE_PASS_MIN_BLOCKS;
   const int64_t per_cta = ceil_div(total_chunks, std::min(total_chunks, max_ctas));
   const int64_t grid = cta_bounds ? ctas : ceil_div(total_chunks, per_cta);
-  seg_pass_kernel<<<(unsigned)grid, kPassThreads, 0, stream>>>(descs, B, total_chunks, per_cta, cta_bounds, order,
-                                                               pairs, dpairs, error);
+  launch_kernel(seg_pass_kernel, (unsigned)grid, kPassThreads, 0, stream, descs, B, total_chunks, per_cta, cta_bounds,
+      order, pairs, dpairs, error);
   PE_LAUNCHED("seg_pass");
   count_launch();
   return kOk;
@@ -845,23 +851,20 @@ PE_API int pe_seg_score(const int64_t* descs, int64_t B, int64_t max_p, int64_t 
                reinterpret_cast<u64*>(confusion)};
   auto* ua = reinterpret_cast<u64*>(areas);
   if (validate) {
-    seg_score_kernel<<<areas_grid, threads, smem, stream>>>(descs, pairs, dpairs, gc, pc, crowd, ua, matched,
-                                                            out, (int)C, isthing, det_classes, det_scores,
-                                                            det_pa, slot_ga, slot_class, ann_in, ann_out, 1, 1,
-                                                                   reward, (int)smem, nullptr, error);
+    launch_kernel(seg_score_kernel, areas_grid, threads, smem, stream, descs, pairs, dpairs, gc, pc, crowd, ua, matched,
+        out, (int)C, isthing, det_classes, det_scores, det_pa, slot_ga, slot_class, ann_in, ann_out, 1, 1, reward,
+        (int)smem, nullptr, error);
     PE_LAUNCHED("seg_score(areas)");
-    seg_score_kernel<<<(unsigned)B, threads, smem, stream>>>(descs, pairs, dpairs, gc, pc, crowd, ua, matched,
-                                                                   out, (int)C, isthing, det_classes, det_scores,
-                                                                   det_pa, slot_ga, slot_class, ann_in, ann_out, 2 | 4,
-                                                                   1, reward, (int)smem, bits, error);
+    launch_kernel(seg_score_kernel, (unsigned)B, threads, smem, stream, descs, pairs, dpairs, gc, pc, crowd, ua,
+        matched, out, (int)C, isthing, det_classes, det_scores, det_pa, slot_ga, slot_class, ann_in, ann_out, 2 | 4, 1,
+        reward, (int)smem, bits, error);
     PE_LAUNCHED("seg_score(accumulate)");
     count_launch(2);
     return kOk;
   }
-  seg_score_kernel<<<areas_grid, threads, smem, stream>>>(descs, pairs, dpairs, gc, pc, crowd, ua, matched, out,
-                                                                 (int)C, isthing, det_classes, det_scores, det_pa,
-                                                                 slot_ga, slot_class, ann_in, ann_out, 1 | 2, 0,
-                                                                 reward, (int)smem, bits, error);
+  launch_kernel(seg_score_kernel, areas_grid, threads, smem, stream, descs, pairs, dpairs, gc, pc, crowd, ua, matched,
+      out, (int)C, isthing, det_classes, det_scores, det_pa, slot_ga, slot_class, ann_in, ann_out, 1 | 2, 0, reward,
+      (int)smem, bits, error);
   PE_LAUNCHED("seg_score");
   count_launch();
   return kOk;
@@ -898,9 +901,8 @@ PE_API int pe_inst_overlap(const int64_t* descs, int64_t B, int64_t total_chunks
   PE_REQUIRE(smem <= 220 * 1024, "too many masks per image for the overlap kernel (%lld)", (long long)max_rows);
   if (smem > 48 * 1024)
     PE_CUDA(cudaFuncSetAttribute(inst_overlap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  inst_overlap_kernel<<<(unsigned)total_chunks, kOvThreads, smem, stream>>>(descs, B, order, pc, gc, inter,
-                                                                            reinterpret_cast<u64*>(pa),
-                                                                            reinterpret_cast<u64*>(ga));
+  launch_kernel(inst_overlap_kernel, (unsigned)total_chunks, kOvThreads, smem, stream, descs, B, order, pc, gc, inter,
+      reinterpret_cast<u64*>(pa), reinterpret_cast<u64*>(ga));
   PE_LAUNCHED("inst_overlap");
   count_launch();
   return kOk;
@@ -914,7 +916,7 @@ PE_API int pe_inst_gather(const int64_t* descs, const int64_t* fields, int64_t B
                           int32_t* gc, uint8_t* crowd, double* areas, cudaStream_t stream) {
   PE_REQUIRE(B >= 0 && B <= INT_MAX, "invalid batch");
   if (B == 0) return kOk;
-  inst_gather_kernel<<<(unsigned)B, 128, 0, stream>>>(descs, fields, pc, scores, gc, crowd, areas);
+  launch_kernel(inst_gather_kernel, (unsigned)B, 128, 0, stream, descs, fields, pc, scores, gc, crowd, areas);
   PE_LAUNCHED("inst_gather");
   count_launch();
   return kOk;
@@ -926,10 +928,9 @@ PE_API int pe_inst_prepare(const int64_t* descs, int64_t B, const uint64_t* pa_c
                            int32_t* error, cudaStream_t stream) {
   PE_REQUIRE(B >= 0 && C > 0 && C < INT_MAX, "invalid batch");
   if (B == 0) return kOk;
-  inst_prepare_kernel<<<(unsigned)B, 128, 0, stream>>>(descs, reinterpret_cast<const u64*>(pa_count),
-                                                      reinterpret_cast<const u64*>(ga_count), pa, ga, pc, gc, scores,
-                                                      ann_in, ann_out, (int)C, validate,
-                                                      reinterpret_cast<u32*>(class_bits), error);
+  launch_kernel(inst_prepare_kernel, (unsigned)B, 128, 0, stream, descs, reinterpret_cast<const u64*>(pa_count),
+      reinterpret_cast<const u64*>(ga_count), pa, ga, pc, gc, scores, ann_in, ann_out, (int)C, validate,
+      reinterpret_cast<u32*>(class_bits), error);
   PE_LAUNCHED("inst_prepare");
   count_launch();
   return kOk;
