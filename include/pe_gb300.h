@@ -37,6 +37,8 @@ extern "C" {
 
 /* Text of the last failure on the calling host thread. */
 const char* pe_last_error(void);
+/* Zeroes `bytes` bytes at device address `ptr` on the stream. */
+int pe_zero(void* ptr, int64_t bytes, cudaStream_t stream);
 /* Kernels launched by this library since load or the last reset. */
 long long pe_launch_count(void);
 void pe_reset_launch_count(void);

@@ -49,6 +49,7 @@ SIGNATURES = {
     "pe_seg_score": [P, I64, I64, I64, P, P, P, P, P, P, P, P, P, P, P, P, I64, P, P, P, P, P, P, P, P, I32, I32, P, P, P],
     "pe_seg_match": [P, P, P, P, I64, P, P, P, P, P, P, I64, I64, P, I64, I64, P, P, P, P, P],
     "pe_inst_overlap": [P, I64, I64, I64, P, P, P, P, I64, P, I64, P, I64, P],
+    "pe_zero": [P, I64, P],
     "pe_pack_rgb": [P, I64, I64, P, P, I64, P, P, P],
     "pe_inst_contract": [P, P, I64, I64, P, I64, P, P, I64, P, I64, P, I64, P, P, P],
     "pe_inst_intersect": [P, I64, I64, P, I64, I64, P, I64, P, P, I64, P, I64, P, I64, P, I64, P, P, P],

@@ -37,7 +37,7 @@ using namespace pe;
 // ---- the C ABI, bound to the addresses of the library that the Python layer loaded ------------------
 
 #define PE_HOST_API(X)                                                                              \
-  X(pe_update) X(pe_compute) X(pe_reward_pq) X(pe_pack) X(pe_pack_rgb) X(pe_contract_maps)          \
+  X(pe_update) X(pe_zero) X(pe_compute) X(pe_reward_pq) X(pe_pack) X(pe_pack_rgb) X(pe_contract_maps)          \
   X(pe_contract_blocks) X(pe_inst_gather) X(pe_seg_sort) X(pe_seg_sort_workspace)                   \
   X(pe_inst_contract) X(pe_inst_intersect) X(pe_stream_limit) X(pe_inst_prepare) X(pe_seg_match) X(pe_instance_accumulate)                  \
   X(pe_instance_accumulate_workspace) X(pe_seg_pass) X(pe_seg_score) X(pe_prefix)
@@ -376,7 +376,7 @@ PyObject* zero(PyObject*, PyObject* object) {
   const int index = c10::cuda::current_device();
   auto t = plain(object, index);
   if (!t) return none();
-  if (t->nbytes() && cudaMemsetAsync(t->data_ptr(), 0, t->nbytes(), current_stream(index)) != cudaSuccess) {
+  if (api.pe_zero(t->data_ptr(), (int64_t)t->nbytes(), current_stream(index)) != 0) {
     PyErr_SetString(PyExc_RuntimeError, "clearing the accumulators failed");
     return nullptr;
   }
@@ -417,7 +417,7 @@ PyObject* reward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   int code = 0;
   {
     ReleaseGil released;
-    if (zeroed && cudaMemsetAsync(stats, 0, (size_t)zeroed, stream) != cudaSuccess) code = -2;
+    code = api.pe_zero(stats, zeroed, stream);
     if (!code)
       code = api.pe_update(gt.maps.data_ptr(), 0, pred.maps.data_ptr(), 0, B, gt.maps.size(1) * gt.maps.size(2),
                            data<int32_t>(gt.classes), data<int32_t>(pred.classes), flags, G, P, C, pairs,

@@ -59,8 +59,9 @@ void set_error(const char* fmt, ...);
 
 int sm_count();            // SMs of the current device (cached per device)
 int current_device();
-// Zeroes buffers on the stream, those that follow one another in memory with one memset (a memset costs
-// about 2 us of host time and 1.4 us of the stream). A Status.
+// Zeroes buffers on the stream, all with one kernel: a memset per buffer costs about 2 us of host time and 1.4 us
+// of the stream, and breaks the chain of kernels launched ahead (below). Per call: 16 reward
+// images 27.7 -> 23.2 us, 16 panoptic images 43.1 -> 38.0, one instance image 112 -> 105. A Status.
 struct ZeroSpan {
   void* ptr;
   int64_t bytes;

@@ -1067,7 +1067,8 @@ int launch_accumulate(const int* classes, const int* ranks, const int8_t* flags,
   if (n <= kScanRecords) {
     list = nullptr;
   } else {
-    PE_CUDA(cudaMemsetAsync(hist, 0, sizeof(int) * C, stream));
+    const int zeroed = zero_spans({{hist, 4 * C}}, stream);
+    if (zeroed != kOk) return zeroed;
     const int64_t blocks = std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 4);
     launch_kernel(class_histogram_kernel, (unsigned)blocks, 256, 0, stream, classes, n, C, hist);
     PE_LAUNCHED("class_histogram");
@@ -1114,7 +1115,8 @@ PE_API int pe_instance_histogram(const uint8_t* masks, int64_t D, int64_t pixels
   PE_REQUIRE(D >= 0 && D < INT_MAX && pixels > 0 && S > 0 && S < INT_MAX && D * S < INT_MAX,
              "invalid shared ground-truth inputs");
   if (D == 0) return kOk;
-  PE_CUDA(cudaMemsetAsync(pairs, 0, sizeof(int64_t) * D * S, stream));
+  const int zeroed = zero_spans({{pairs, 8 * D * S}}, stream);
+  if (zeroed != kOk) return zeroed;
   const int64_t bins = D * S;
   const bool smem = bins <= 48 * 1024;
   const size_t smem_bytes = smem ? sizeof(u32) * bins : 0;
@@ -1147,7 +1149,8 @@ PE_API int pe_instance_match(const int64_t* pairs, int64_t D, int64_t G, const i
                              int64_t C, int8_t* flags, int32_t* ranks, int64_t* counts, cudaStream_t stream) {
   PE_REQUIRE(D >= 0 && G >= 0 && D < INT_MAX && G < INT_MAX && D * G < INT_MAX, "too many instance pairs");
   PE_REQUIRE(C > 0 && C <= INT_MAX / 120, "invalid category count");
-  PE_CUDA(cudaMemsetAsync(counts, 0, sizeof(int64_t) * C * 4, stream));
+  const int zeroed = zero_spans({{counts, 32 * C}}, stream);
+  if (zeroed != kOk) return zeroed;
   if (D == 0 && G == 0) return kOk;
   return launch_match(pairs, false, nullptr, nullptr, nullptr, (int)D, (int)G, 1, pc, pa, gc, ga, crowd, areas,
                       (int)C, (int)std::max<int64_t>(G, 1), flags, D, 1, ranks, counts, stream);
@@ -1160,7 +1163,8 @@ PE_API int pe_mask_overlap(const uint8_t* pm, int64_t D, const uint8_t* gm, int6
                            const int32_t* pc, const int32_t* gc, int64_t* inter, cudaStream_t stream) {
   PE_REQUIRE(D >= 0 && G >= 0 && pixels > 0 && D * G < INT_MAX, "invalid instance masks");
   if (D == 0 || G == 0) return kOk;
-  PE_CUDA(cudaMemsetAsync(inter, 0, sizeof(int64_t) * D * G, stream));
+  const int zeroed = zero_spans({{inter, 8 * D * G}}, stream);
+  if (zeroed != kOk) return zeroed;
   const size_t smem = (size_t)(D + G) * (kOvWords * sizeof(uint32_t) + sizeof(int2));
   PE_REQUIRE(smem <= 220 * 1024, "too many masks per image for the overlap kernel (D+G=%lld)", (long long)(D + G));
   const int align = std::min(alignment_of(pm, pixels), alignment_of(gm, pixels));

@@ -722,8 +722,8 @@ PE_API int pe_update(const void* gt, int gt_is_int64, const void* pred, int pred
   if (B == 0) return kOk;
   PE_REQUIRE(gc && pc && crowd && pairs && areas && matched && tp && fp && fn && iou_sum, "null state pointer");
   const int64_t total = B * pixels;
-  PE_CUDA(cudaMemsetAsync(pairs, 0, sizeof(int64_t) * B * G * P, stream));
-  if (validate) PE_CUDA(cudaMemsetAsync(error, 0, sizeof(int32_t), stream));
+  const int zeroed = zero_spans({{pairs, 8 * B * G * P}, {error, validate ? 4 : 0}}, stream);
+  if (zeroed != kOk) return zeroed;
   auto* upairs = reinterpret_cast<u64*>(pairs);
   int* err = validate ? error : nullptr;
   if (total > 0) {
@@ -901,7 +901,8 @@ PE_API int pe_reward_pq(const int64_t* tp, const int64_t* fp, const int64_t* fn,
 PE_API int pe_pack(const void* maps, int maps_is_int64, int64_t B, int64_t pixels, const int64_t* ids,
                    const int32_t* slots, int64_t S, int32_t* out, int32_t* error, cudaStream_t stream) {
   PE_REQUIRE(B >= 0 && pixels >= 0 && S > 0 && S < INT_MAX, "invalid lookup shapes");
-  PE_CUDA(cudaMemsetAsync(error, 0, sizeof(int32_t), stream));
+  const int zeroed = zero_spans({{error, 4}}, stream);
+  if (zeroed != kOk) return zeroed;
   const int64_t total = B * pixels;
   if (total == 0) return kOk;
   const int64_t blocks = std::min<int64_t>(ceil_div(total, 256), (int64_t)sm_count() * 8);
@@ -921,7 +922,8 @@ PE_API int pe_pack_rgb(const uint8_t* rgb, int64_t B, int64_t pixels, const int6
   PE_REQUIRE(B >= 0 && B <= 65535 && pixels >= 0, "invalid RGB batch (at most 65535 images per call)");
   PE_REQUIRE((ids == nullptr) == (slots == nullptr), "lookup IDs and slots go together");
   PE_REQUIRE(!ids || (S > 0 && S <= 16384), "lookup tables must have 1..16384 entries per image");
-  if (error) PE_CUDA(cudaMemsetAsync(error, 0, sizeof(int32_t), stream));
+  const int zeroed = zero_spans({{error, error ? 4 : 0}}, stream);
+  if (zeroed != kOk) return zeroed;
   if (B == 0 || pixels == 0) return kOk;
   const size_t smem = ids ? (size_t)S * (sizeof(int64_t) + sizeof(int)) : 0;
   if (smem > 48 * 1024)

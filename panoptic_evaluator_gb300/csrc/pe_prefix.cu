@@ -868,20 +868,16 @@ PE_API int pe_prefix(const int64_t* descs, int64_t B, int64_t total_chunks, int6
   PE_REQUIRE(B >= 0 && total_rows >= 0 && C > 0 && C < INT_MAX && T > 0 && T <= 1024 && max_g >= 0 &&
                  max_p >= 1 && max_p < 65536,
              "invalid prefix batch (T must be 1..1024, masks per image < 65535)");
-  if (B == 0) {
-    PE_CUDA(cudaMemsetAsync(error, 0, sizeof(int32_t), stream));
-    return kOk;
-  }
+  if (B == 0) return zero_spans({{error, 4}}, stream);
   const int64_t rows = 8 * total_rows * C;
   const int zeroed = zero_spans({{ga, 4 * ga_len}, {raw, 4 * raw_len}, {pairs, 4 * pairs_len},
                                  {counters, 4 * counters_len}, {error, 4}, {tp, rows}, {fp, rows}, {fn, rows},
-                                 {sums, rows}, {confusion, rows * (C + 1)}},
+                                 {sums, rows}, {confusion, rows * (C + 1)}, {schedule, schedule ? 8 : 0}},
                                 stream);
   if (zeroed != kOk) return zeroed;
   if (total_chunks) {
     if (bulk) {
       const int64_t grid = std::min(total_chunks, (int64_t)sm_count() * 2);  // two CTAs per SM
-      if (schedule) PE_CUDA(cudaMemsetAsync(schedule, 0, sizeof(uint64_t), stream));
       const size_t smem = sizeof(PrefixShared);
       // Owners fit in a byte per pixel when no image has more than 255 masks.
       auto kernel = max_p <= 256 ? prefix_pass_bulk_kernel<true> : prefix_pass_bulk_kernel<false>;

@@ -39,21 +39,62 @@ int sm_count() {
   return g_sm_counts[device];
 }
 
+namespace {
+constexpr int kZeroSpans = 8;
+constexpr int kZeroThreads = 256;
+struct ZeroSpans {
+  unsigned char* ptr[kZeroSpans];
+  int64_t bytes[kZeroSpans];
+  int count;
+};
+
+__global__ void __launch_bounds__(kZeroThreads) zero_kernel(ZeroSpans spans) {
+  wait_for_earlier_kernels();
+  const int64_t first = (int64_t)blockIdx.x * kZeroThreads + threadIdx.x, step = (int64_t)gridDim.x * kZeroThreads;
+  for (int s = 0; s < spans.count; ++s) {
+    unsigned char* p = spans.ptr[s];
+    const int64_t bytes = spans.bytes[s];
+    const int64_t head = min(bytes, (int64_t)(-reinterpret_cast<uintptr_t>(p) & 15)), words = (bytes - head) / 16;
+    const int64_t tail = bytes - head - 16 * words;
+    uint4* q = reinterpret_cast<uint4*>(p + head);
+    for (int64_t i = first; i < words; i += step) q[i] = make_uint4(0, 0, 0, 0);
+    if (first < head) p[first] = 0;
+    if (first < tail) p[head + 16 * words + first] = 0;
+  }
+}
+}  // namespace
+
 int zero_spans(std::initializer_list<ZeroSpan> spans, cudaStream_t stream) {
-  char* begin = nullptr;
-  int64_t bytes = 0;
+  ZeroSpans z = {};
+  int64_t total = 0;
+  const auto launch = [&]() -> int {
+    if (!z.count) return kOk;
+    const int64_t blocks = std::min<int64_t>(ceil_div(total, 16 * kZeroThreads), (int64_t)sm_count() * 8);
+    launch_kernel(zero_kernel, (unsigned)blocks, kZeroThreads, 0, stream, z);
+    PE_LAUNCHED("zero");
+    count_launch();
+    z.count = 0;
+    total = 0;
+    return kOk;
+  };
   for (const ZeroSpan& span : spans) {
     if (span.bytes <= 0) continue;
-    if (bytes && static_cast<char*>(span.ptr) == begin + bytes) {
-      bytes += span.bytes;
+    unsigned char* p = static_cast<unsigned char*>(span.ptr);
+    total += span.bytes;
+    if (z.count && z.ptr[z.count - 1] + z.bytes[z.count - 1] == p) {  // follows the span before
+      z.bytes[z.count - 1] += span.bytes;
       continue;
     }
-    if (bytes) PE_CUDA(cudaMemsetAsync(begin, 0, (size_t)bytes, stream));
-    begin = static_cast<char*>(span.ptr);
-    bytes = span.bytes;
+    if (z.count == kZeroSpans) {
+      total -= span.bytes;
+      const int status = launch();
+      if (status != kOk) return status;
+      total = span.bytes;
+    }
+    z.ptr[z.count] = p;
+    z.bytes[z.count++] = span.bytes;
   }
-  if (bytes) PE_CUDA(cudaMemsetAsync(begin, 0, (size_t)bytes, stream));
-  return kOk;
+  return launch();
 }
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
@@ -66,6 +107,12 @@ PE_API const char* pe_last_error(void) { return pe::g_message; }
 // Number of kernels this library has launched since load (or the last reset).
 PE_API long long pe_launch_count(void) { return pe::g_launches.load(); }
 PE_API void pe_reset_launch_count(void) { pe::g_launches.store(0); }
+
+// Zeroes `bytes` bytes at `ptr` on the stream.
+PE_API int pe_zero(void* ptr, int64_t bytes, cudaStream_t stream) {
+  PE_REQUIRE(bytes >= 0 && (ptr || !bytes), "invalid span");
+  return pe::zero_spans({{ptr, bytes}}, stream);
+}
 
 // ABI version: bump on any signature change.
 PE_API int pe_abi_version(void) { return 2; }

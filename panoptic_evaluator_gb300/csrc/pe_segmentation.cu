@@ -893,9 +893,8 @@ PE_API int pe_inst_overlap(const int64_t* descs, int64_t B, int64_t total_chunks
                            int64_t inter_len, uint64_t* pa, int64_t pa_len, uint64_t* ga, int64_t ga_len,
                            cudaStream_t stream) {
   PE_REQUIRE(B >= 0 && total_chunks >= 0, "invalid batch");
-  if (inter_len) PE_CUDA(cudaMemsetAsync(inter, 0, sizeof(uint32_t) * inter_len, stream));
-  if (pa_len) PE_CUDA(cudaMemsetAsync(pa, 0, sizeof(uint64_t) * pa_len, stream));
-  if (ga_len) PE_CUDA(cudaMemsetAsync(ga, 0, sizeof(uint64_t) * ga_len, stream));
+  const int zeroed = zero_spans({{inter, 4 * inter_len}, {pa, 8 * pa_len}, {ga, 8 * ga_len}}, stream);
+  if (zeroed != kOk) return zeroed;
   if (B == 0 || total_chunks == 0) return kOk;
   const size_t smem = (size_t)std::max<int64_t>(max_rows, 1) * (kOvWords * sizeof(uint32_t) + sizeof(int2));
   PE_REQUIRE(smem <= 220 * 1024, "too many masks per image for the overlap kernel (%lld)", (long long)max_rows);

@@ -122,3 +122,14 @@ def test_detection_areas_beside_the_scoring(images, validate):
     joint = pe.SegmentationEvaluator(133, isthing=isthing, validate=validate)
     joint.update_images(SegmentationImages(*([getattr(i, f) for i in batch] for f in fields)))
     assert_tree(joint.compute(), oracle.compute())
+
+
+@pytest.mark.parametrize("offset", (0, 1, 4, 15))
+@pytest.mark.parametrize("size", (0, 1, 3, 15, 16, 17, 31, 4096, 1_000_003))
+def test_zeroing_clears_the_span_and_nothing_beside_it(offset, size):
+    from panoptic_evaluator_gb300 import _native as N
+    data = torch.full((size + 64,), 7, dtype=torch.uint8, device="cuda")
+    N.call("pe_zero", data.data_ptr() + offset, size, N.stream_handle(data.device))
+    want = torch.full_like(data, 7)
+    want[offset:offset + size] = 0
+    assert torch.equal(data, want)
