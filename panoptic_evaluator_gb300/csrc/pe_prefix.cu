@@ -2,7 +2,7 @@
 //
 // The reference draws masks one launch at a time and scores each step with a
 // single CTA (prefix_kernel.cu:142-199: 2N+1 launches per image). Here every
-// batch is six launches, whatever the number of images or masks:
+// batch is five launches, whatever the number of images or masks:
 //   1. prefix_pass   one read of the target map and of every mask byte. Each
 //                    lane tracks the visible owner of its 16 pixels (the last
 //                    mask drawn over them) and, at every requested checkpoint,
@@ -12,14 +12,13 @@
 //                    intersections used by instance matching.
 //   2. prefix_scan   running sums over checkpoints turn deltas into the canvas
 //                    pair histograms (column 0 starts with the target areas).
-//   3. prefix_score  one CTA per (image, checkpoint): canvas PQ / confusion with
+//   3. prefix_rows   one CTA per (image, checkpoint): canvas PQ / confusion with
 //                    active labels (segments with visible pixels), shared with
-//                    the panoptic evaluator's scoring code.
-//   4. prefix_match  one CTA per image, one warp per IoU threshold: greedy
-//                    generation-order matching (prefix.py:106-118), snapshots
-//                    of TP/FP/FN at the checkpoints; prefix_ratio then turns
-//                    them into precision / recall over the whole grid.
-//   5. pe_compute    per-checkpoint PQ/SQ/RQ/IoU summaries.
+//                    the panoptic evaluator's scoring code; beside them one CTA
+//                    or more per image: greedy generation-order matching
+//                    (prefix.py:106-118), a chain per (threshold, class), its
+//                    counts, precision and recall at the checkpoints.
+//   4. pe_compute    per-checkpoint PQ/SQ/RQ/IoU summaries.
 #include "pe_common.cuh"
 #include "pe_fields.h"
 #include "pe_score.cuh"
@@ -543,15 +542,10 @@ __host__ __device__ inline size_t label_bytes(int64_t P) { return ((size_t)P * s
 
 // Canvas PQ of one (image, checkpoint) row, scored in one pass (pe_score.cuh). smem: dynamic shared memory of
 // the launch (labels, then tables and entry list); rows whose tables do not fit it are scored in place.
-constexpr int kPrefixScoreThreads = 512;
-__global__ void __launch_bounds__(kPrefixScoreThreads)
-prefix_score_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __restrict__ pairs,
-                    const int* __restrict__ classes, const int* __restrict__ gc, const uint8_t* __restrict__ crowd,
-                    int C, int64_t* __restrict__ tp, int64_t* __restrict__ fp, int64_t* __restrict__ fn,
-                    double* __restrict__ sums, int64_t* __restrict__ confusion, int smem) {
-  wait_for_earlier_kernels();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int64_t row = blockIdx.x;
+__device__ __forceinline__ void score_row(const int64_t* descs, int64_t B, int64_t row, const int* pairs,
+                                          const int* classes, const int* gc, const uint8_t* crowd, int C, int64_t* tp,
+                                          int64_t* fp, int64_t* fn, double* sums, int64_t* confusion,
+                                          unsigned char* smem_raw, int smem) {
   const int64_t b = find_image(descs, B, kPrefixQBegin, row);
   const int64_t* d = pdesc(descs, b);
   const int N = (int)d[kPrefixN], G = (int)d[kPrefixG], P = N + 1;
@@ -585,256 +579,297 @@ prefix_score_kernel(const int64_t* __restrict__ descs, int64_t B, const int* __r
   score_accumulate<u32, false>(pq, gc, labels, crowd, areas, matched, G, P, C, out, staging);
 }
 
-// Greedy generation-order matching (prefix.py:106-118) and the validation of one image's metadata: one
-// CTA per image. Phase 1 (all threads): each mask's area on valid slots and, for thing masks, its IoU
-// with every target slot of its class, staged in shared memory (kStaged) or left to phase 2. Phase 2:
-// one warp per IoU threshold walks the masks in generation order; its lanes split the candidate slots
-// and a warp arg-max (largest IoU, first slot on ties) picks the match, so the chain has no block
-// barrier; at every checkpoint the warp writes its threshold's snapshot. Error bits: 2 empty prediction
-// mask, 4 bad target class / slot 0 not void, 8 target areas vs metadata, 16 bad prediction class.
-constexpr int kPrefixMatchThreads = 512;  // 16 warps: every IoU threshold's chain has its own warp
-constexpr int kSerialCandidates = 8;      // candidate slots a single lane scans in the chain
-template <bool kStaged>
-__global__ void __launch_bounds__(kPrefixMatchThreads)
-prefix_match_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ ga, const u32* __restrict__ raw,
-                    const int* __restrict__ classes, const int* __restrict__ gc, const uint8_t* __restrict__ crowd,
-                    const uint8_t* __restrict__ isthing, const double* __restrict__ thresholds, int T, int C,
-                    const int* __restrict__ step_q, int64_t* __restrict__ itp, int64_t* __restrict__ ifp,
-                    int64_t* __restrict__ ifn, double* __restrict__ precision, double* __restrict__ recall,
-                    int validate, int* __restrict__ error) {
-  wait_for_earlier_kernels();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int64_t* d = pdesc(descs, blockIdx.x);
-  const int N = (int)d[kPrefixN], G = (int)d[kPrefixG];
-  const int64_t qb = d[kPrefixQBegin];
-  const int* steps = step_q + d[kPrefixStepBegin];
-  ga += d[kPrefixSlotBegin];
-  gc += d[kPrefixSlotBegin];
-  crowd += d[kPrefixSlotBegin];
-  classes += d[kPrefixDetBegin];
-  raw += d[kPrefixRawBegin];
+// Greedy generation-order matching (prefix.py:106-118) and the validation of an image's metadata. Only masks and
+// targets of one class meet, so every (IoU threshold, class) is a chain of its own: the masks of the class in
+// generation order, each taking the free target of the largest IoU (the first slot on ties), the counts written at
+// every checkpoint. `splits` CTAs share an image's classes. A CTA groups its classes' slots and masks, takes the
+// IoU of every pair once into shared memory (where `smem` has room for them) and then walks one chain per thread.
+// Error bits: 2 empty prediction mask, 4 bad target class / slot 0 not void, 8 target areas vs metadata, 16 bad
+// prediction class.
+//
+// The chains are latency: one warp per threshold walking all masks of an image took 40.8 us for 16 images of 64
+// masks, 101 slots and 133 classes on 16 SMs, and 6.0 us more for the ratios in a launch of their own.
+constexpr int kSerialSlots = 8;      // a thread alone walks chains of up to 8 slots a class ...
+constexpr int kSerialPairs = 128;    // ... or 128 pairs in all (a warp step costs about as much as 8 slots)
+constexpr int kMatchClasses = 16;    // classes per CTA, at least, while an image's classes are shared
+
+__host__ __device__ inline size_t prefix_match_bytes(int64_t N, int64_t G, int64_t T, int64_t C) {
+  const int64_t ints = 3 * N + 1 + 2 * G + 4 * C + 3 + T * ((G + 31) / 32);
+  return sizeof(u64) * N + sizeof(int) * ints + G + 16;
+}
+
+struct PrefixMatch {
+  const int64_t* descs;
+  const u32* ga;
+  const u32* raw;
+  const int* classes;
+  const int* gc;
+  const uint8_t* crowd;
+  const uint8_t* isthing;
+  const double* thresholds;
+  int T, C;
+  const int* step_q;
+  int64_t *itp, *ifp, *ifn;
+  double *precision, *recall;
+  int validate;
+  int* error;
+};
+
+__device__ __forceinline__ int warp_exclusive_sum(int v, int lane, int* total) {
+  int sum = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, sum, off);
+    if (lane >= off) sum += u;
+  }
+  *total = __shfl_sync(0xffffffffu, sum, 31);
+  return sum - v;
+}
+
+__device__ __forceinline__ void match_classes(const PrefixMatch& a, int64_t image, int split, int splits,
+                                              unsigned char* smem_raw, int smem) {
+  const int64_t* d = pdesc(a.descs, image);
+  const int N = (int)d[kPrefixN], G = (int)d[kPrefixG], T = a.T, C = a.C;
+  const int64_t first_row = d[kPrefixQBegin];
+  const int* steps = a.step_q + d[kPrefixStepBegin];
+  const u32* ga = a.ga + d[kPrefixSlotBegin];
+  const int* gc = a.gc + d[kPrefixSlotBegin];
+  const uint8_t* crowd = a.crowd + d[kPrefixSlotBegin];
+  const int* classes = a.classes + d[kPrefixDetBegin];
+  const u32* raw = a.raw + d[kPrefixRawBegin];
+  const int per = (C + splits - 1) / splits;
+  const int c0 = min(C, split * per), nc = min(C, c0 + per) - c0;  // this CTA's classes: c0 and the nc - 1 after it
   const int words = (G + 31) / 32;
-  u64* areas = reinterpret_cast<u64*>(smem_raw);                   // N mask areas on valid slots
-  long long* iou_all = reinterpret_cast<long long*>(areas + N);    // candidate IoU bit patterns (kStaged)
-  int* ints = reinterpret_cast<int*>(iou_all + (kStaged ? (int64_t)N * G : 0));
-  int* positives = ints;                                           // C
-  int* by_class = positives + C;                                   // G slots ordered by class
-  int* class_start = by_class + G;                                 // C + 1
-  int* cand_off = class_start + C + 1;                             // N + 1
-  int* tp_s = cand_off + N + 1;                                    // T x C
-  int* fp_s = tp_s + T * C;                                        // T x C
-  int* thing_class = fp_s + T * C;                                 // N: the mask's class if a thing, else -1
-  int* step_s = thing_class + N;                                   // N + 1: checkpoint index of prefix k or -1
-  u32* used = reinterpret_cast<u32*>(step_s + N + 1);              // T x words
-  int* gc_s = reinterpret_cast<int*>(used + T * words);            // G: slot classes
-  uint8_t* crowd_s = reinterpret_cast<uint8_t*>(gc_s + G);         // G
-  __shared__ int s_err;
+
+  u64* areas = reinterpret_cast<u64*>(smem_raw);             // N: mask areas on valid slots
+  u32* checks = reinterpret_cast<u32*>(areas + N);           // N + 1: checkpoints by prefix, prefix << 16 | row
+  int* mask_class = reinterpret_cast<int*>(checks + N + 1);  // N: the mask's class here if a thing, else -1
+  int* by_mask = mask_class + N;                             // N: masks by class, in generation order
+  int* slot_class = by_mask + N;                             // G
+  int* by_slot = slot_class + G;                             // G: slots by class, in slot order
+  int* slot_start = by_slot + G;                             // nc + 1
+  int* mask_start = slot_start + nc + 1;                     // nc + 1
+  int* pair_start = mask_start + nc + 1;                     // nc + 1
+  int* positives = pair_start + nc + 1;                      // nc
+  u32* used = reinterpret_cast<u32*>(positives + nc);        // T x words: targets taken, by position in by_slot
+  uint8_t* crowd_s = reinterpret_cast<uint8_t*>(used + T * words);
+  const size_t at = (prefix_match_bytes(N, G, T, C) + 7) & ~size_t{7};
+  long long* ious = reinterpret_cast<long long*>(smem_raw + at);  // IoU bit patterns: per class, mask major
+  const int room = (size_t)smem > at ? (int)(((size_t)smem - at) / sizeof(long long)) : 0;
+  __shared__ int s_err, s_checks;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = (int)(blockDim.x >> 5);
+
   if (tid == 0) s_err = 0;
-  for (int c = tid; c < C; c += blockDim.x) positives[c] = 0;
-  for (int k = tid; k <= C; k += blockDim.x) class_start[k] = 0;
-  for (int k = tid; k < T * C; k += blockDim.x) tp_s[k] = fp_s[k] = 0;
+  for (int k = tid; k <= nc; k += blockDim.x) slot_start[k] = mask_start[k] = 0;
+  for (int k = tid; k < nc; k += blockDim.x) positives[k] = 0;
   for (int k = tid; k < T * words; k += blockDim.x) used[k] = 0;
-  // Everything the sequential chain reads per mask or slot is staged here, off its critical path.
-  for (int k = tid; k <= N; k += blockDim.x) step_s[k] = steps[k];
-  for (int g = tid; g < G; g += blockDim.x) {
-    crowd_s[g] = crowd[g];
-    gc_s[g] = gc[g];
-  }
-  for (int i = tid; i < N; i += blockDim.x) {
-    const int c = classes[i];
-    thing_class[i] = (c >= 0 && c < C && isthing[c]) ? c : -1;
-  }
   __syncthreads();
   int err = 0;
   for (int g = tid; g < G; g += blockDim.x) {
     const int c = gc[g];
-    if (c >= 0 && c < C) {
-      atomicAdd(class_start + c + 1, 1);
-      if (isthing[c] && !crowd[g]) atomicAdd(positives + c, 1);
+    const bool ignored = crowd[g];
+    const bool here = c >= c0 && c < c0 + nc && a.isthing[c];
+    crowd_s[g] = ignored;
+    slot_class[g] = here ? c - c0 : -1;
+    if (here) {
+      atomicAdd(slot_start + c - c0, 1);
+      if (!ignored) atomicAdd(positives + c - c0, 1);
     }
-    if (validate) {
-      if (c < -1 || c >= C || (g == 0 && (c != -1 || crowd[g]))) err |= 4;
+    if (a.validate && split == 0) {
+      if (c < -1 || c >= C || (g == 0 && (c != -1 || ignored))) err |= 4;
       if (g > 0 && ((ga[g] > 0) != (c >= 0))) err |= 8;
     }
   }
-  // Mask areas (one warp per mask).
+  for (int i = tid; i < N; i += blockDim.x) {
+    const int c = classes[i];
+    const bool here = c >= c0 && c < c0 + nc && a.isthing[c];
+    mask_class[i] = here ? c - c0 : -1;
+    if (here) atomicAdd(mask_start + c - c0, 1);
+    if (a.validate && split == 0 && (c < 0 || c >= C)) err |= 16;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    // Starts of every class's slots, masks and pairs.
+    int slots = 0, masks = 0, pairs = 0;
+    for (int base = 0; base < nc; base += 32) {
+      const int k = base + lane;
+      const int s = k < nc ? slot_start[k] : 0, m = k < nc ? mask_start[k] : 0;
+      int total_s, total_m, total_p;
+      const int ss = warp_exclusive_sum(s, lane, &total_s), ms = warp_exclusive_sum(m, lane, &total_m);
+      const int ps = warp_exclusive_sum(s * m, lane, &total_p);
+      if (k < nc) {
+        slot_start[k] = slots + ss;
+        mask_start[k] = masks + ms;
+        pair_start[k] = pairs + ps;
+      }
+      slots += total_s, masks += total_m, pairs += total_p;
+    }
+    if (lane == 0) slot_start[nc] = slots, mask_start[nc] = masks, pair_start[nc] = pairs;
+  } else if (warp == 1) {
+    int n = 0;
+    for (int base = 0; base <= N; base += 32) {
+      const int k = base + lane, q = k <= N ? steps[k] : -1;
+      const u32 some = __ballot_sync(0xffffffffu, q >= 0);
+      if (q >= 0) checks[n + __popc(some & ((1u << lane) - 1u))] = (u32)k << 16 | (u32)q;
+      n += __popc(some);
+    }
+    if (lane == 0) s_checks = n;
+  }
+  // Areas of the masks matched here, and, when they are checked, of this CTA's share of all masks.
   for (int i = warp; i < N; i += warps) {
+    const bool checked = a.validate && i % splits == split;
+    if (mask_class[i] < 0 && !checked) continue;
     u64 area = 0;
     for (int g = lane; g < G; g += 32) area += raw[(int64_t)i * G + g];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) area += __shfl_xor_sync(0xffffffffu, area, off);
     if (lane == 0) {
       areas[i] = area;
-      const int c = classes[i];
-      if (validate && (c < 0 || c >= C)) err |= 16;
-      if (validate && area == 0) err |= 2;
+      if (checked && area == 0) err |= 2;
     }
   }
   if (err) atomicOr(&s_err, err);
   __syncthreads();
-  if (warp == 0) {
-    // Exclusive scan of the class sizes (C + 1 entries; entry c + 1 holds class c's size), then of the
-    // thing masks' candidate counts.
-    int carry = 0;
-    for (int base = 0; base <= C; base += 32) {
-      const int k = base + lane;
-      int v = k <= C ? class_start[k] : 0;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, off);
-        if (lane >= off) v += u;
-      }
-      if (k <= C) class_start[k] = v + carry;
-      carry += __shfl_sync(0xffffffffu, v, 31);
-    }
-    __syncwarp();
-    carry = 0;
-    for (int base = 0; base < N; base += 32) {
-      const int i = base + lane;
-      const int c = i < N ? classes[i] : -1;
-      const int n = (c >= 0 && c < C && isthing[c]) ? class_start[c + 1] - class_start[c] : 0;
-      int v = n;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, off);
-        if (lane >= off) v += u;
-      }
-      if (i < N) cand_off[i] = carry + v - n;
-      carry += __shfl_sync(0xffffffffu, v, 31);
-    }
-  }
-  __syncthreads();
-  // Slots grouped by class, in slot order within a class (stable).
-  for (int g = tid; g < G; g += blockDim.x) {
-    const int c = gc[g];
-    if (c < 0 || c >= C) continue;
-    int rank = 0;
-    for (int h = 0; h < g; ++h) rank += gc_s[h] == c;
-    by_class[class_start[c] + rank] = g;
-  }
-  __syncthreads();
-  // Same-class IoUs of every thing mask: inter / union, crowd slots against the mask area.
+  // Slots and masks grouped by class, in their own order within it; then the class's IoUs: inter / union, crowd
+  // slots against the mask's area. A warp packs its class's pairs into full FP64 operations.
+  const bool staged = pair_start[nc] <= room;
   auto iou_of = [&](int i, int g) -> long long {
     const u64 inter = raw[(int64_t)i * G + g];
     const u64 uni = crowd_s[g] ? areas[i] : areas[i] + ga[g] - inter;
-    return __double_as_longlong((double)inter / (double)(uni > 1 ? uni : 1));
+    return inter ? __double_as_longlong((double)inter / (double)(uni > 1 ? uni : 1)) : 0;
   };
-  if constexpr (kStaged) {
-    for (int i = warp; i < N; i += warps) {
-      const int c = classes[i];
-      if (c < 0 || c >= C || !isthing[c]) continue;
-      const int s0 = class_start[c], s1 = class_start[c + 1];
-      for (int k = s0 + lane; k < s1; k += 32) iou_all[cand_off[i] + k - s0] = iou_of(i, by_class[k]);
-    }
-    __syncthreads();
-  }
-  // Phase 2: one warp per threshold.
-  for (int t = warp; t < T; t += warps) {
-    const long long thr = __double_as_longlong(thresholds[t]);
-    int* tpc = tp_s + t * C;
-    int* fpc = fp_s + t * C;
-    u32* taken = used + t * words;
-    // Counts only: precision and recall of every row are computed afterwards by prefix_ratio_kernel over
-    // the whole grid, so no FP64 division sits in this sequential chain.
-    auto snapshot = [&](int q) {
-      __syncwarp();
-      const int64_t row = qb + q;
-      for (int c = lane; c < C; c += 32) {
-        const int64_t a = tpc[c], f = fpc[c], n = positives[c];
-        const int64_t o = (row * T + t) * C + c;
-        itp[o] = a;
-        ifp[o] = f;
-        ifn[o] = n - a;
+  for (int c = warp; c < nc; c += warps) {
+    const int s0 = slot_start[c], ns = slot_start[c + 1] - s0, m0 = mask_start[c], nm = mask_start[c + 1] - m0;
+    if (ns == 0 && nm == 0) continue;
+    auto place = [&](const int* of, int n, int* out) {
+      for (int base = 0; base < n; base += 32) {
+        const int k = base + lane;
+        const u32 mine = __ballot_sync(0xffffffffu, k < n && of[k] == c);
+        if ((mine >> lane) & 1u) out[__popc(mine & ((1u << lane) - 1u))] = k;
+        out += __popc(mine);
       }
     };
-    if (step_s[0] >= 0) snapshot(step_s[0]);
-    for (int i = 0; i < N; ++i) {
-      const int c = thing_class[i];
-      if (c >= 0 && class_start[c + 1] - class_start[c] <= kSerialCandidates) {
-        // Few candidate slots (the usual case): lane 0 scans them in slot order, keeping the first of the
-        // largest IoUs, the same pick as the warp arg-max below without its shuffles.
-        if (lane == 0) {
-          const int s0 = class_start[c], s1 = class_start[c + 1];
-          long long best_iou = -1;
-          int best_k = INT_MAX;
+    place(slot_class, G, by_slot + s0);
+    place(mask_class, N, by_mask + m0);
+    __syncwarp();
+    for (int k = lane; staged && k < ns * nm; k += 32)
+      ious[pair_start[c] + k] = iou_of(by_mask[m0 + k / ns], by_slot[s0 + k % ns]);
+  }
+  __syncthreads();
+  // Chains: item t * nc + c. A warp takes 32 of them, a lane each, then together those of many slots.
+  const int checkpoints = s_checks;
+  const int items = T * nc;  // the shared memory for it bounds T and C
+  for (int base = warp * 32; base < items; base += warps * 32) {
+    const int item = base + lane;
+    const int t = item < items ? item / nc : 0, c = item < items ? item % nc : 0;
+    const int slots = slot_start[c + 1] - slot_start[c], masks = mask_start[c + 1] - mask_start[c];
+    const bool alone = item < items && (slots <= kSerialSlots || (slots <= 32 && slots * masks <= kSerialPairs));
+    auto write = [&](int t_, int c_, u32 check, int tp, int fp) {
+      const int64_t o = ((first_row + (check & 0xffffu)) * T + t_) * C + c0 + c_;
+      const int n = positives[c_];
+      a.itp[o] = tp;
+      a.ifp[o] = fp;
+      a.ifn[o] = n - tp;
+      // tp / max(tp + fp, 1) and tp / max(positives, 1) (prefix.py:106-118)
+      a.precision[o] = tp ? (double)tp / (double)(tp + fp) : 0.0;
+      a.recall[o] = tp ? (double)tp / (double)(n > 1 ? n : 1) : 0.0;
+    };
+    if (alone) {
+      const long long thr = __double_as_longlong(a.thresholds[t]);
+      const int s0 = slot_start[c], m0 = mask_start[c];
+      const long long* iou_c = ious + pair_start[c];
+      int tp = 0, fp = 0, m = 0;
+      u32 taken = 0;
+      for (int e = 0; e < checkpoints; ++e) {
+        const u32 check = checks[e];
+        for (; m < masks && by_mask[m0 + m] < (int)(check >> 16); ++m) {
+          long long best = -1;
+          int best_k = -1;
           bool ignored = false;
-          for (int k = s0; k < s1; ++k) {
-            const int g = by_class[k];
-            const long long iou = kStaged ? iou_all[cand_off[i] + k - s0] : iou_of(i, g);
+          for (int k = 0; k < slots; ++k) {
+            const int g = by_slot[s0 + k];
+            const long long iou = staged ? iou_c[m * slots + k] : iou_of(by_mask[m0 + m], g);
             if (iou < thr) continue;
             if (crowd_s[g]) {
               ignored = true;
-            } else if (!((taken[g >> 5] >> (g & 31)) & 1u) && iou > best_iou) {
-              best_iou = iou;
+            } else if (!((taken >> k) & 1u) && iou > best) {
+              best = iou;
               best_k = k;
             }
           }
-          if (best_k != INT_MAX) {
-            const int g = by_class[best_k];
-            taken[g >> 5] |= 1u << (g & 31);
-            ++tpc[c];
+          if (best_k >= 0) {
+            taken |= 1u << best_k;
+            ++tp;
           } else if (!ignored) {
-            ++fpc[c];
+            ++fp;
           }
         }
-        __syncwarp();
-      } else if (c >= 0) {
-        const int s0 = class_start[c], s1 = class_start[c + 1];
-        long long best_iou = -1;
-        int best_k = INT_MAX;
-        bool ignored = false;
-        for (int k = s0 + lane; k < s1; k += 32) {
-          const int g = by_class[k];
-          const long long iou = kStaged ? iou_all[cand_off[i] + k - s0] : iou_of(i, g);
-          if (iou < thr) continue;
-          if (crowd_s[g]) {
-            ignored = true;
-          } else if (!((taken[g >> 5] >> (g & 31)) & 1u) && iou > best_iou) {
-            best_iou = iou;  // each lane scans increasing k: strictly greater keeps the first slot
-            best_k = k;
-          }
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          const long long other_iou = __shfl_xor_sync(0xffffffffu, best_iou, off);
-          const int other_k = __shfl_xor_sync(0xffffffffu, best_k, off);
-          if (other_iou > best_iou || (other_iou == best_iou && other_k < best_k)) {
-            best_iou = other_iou;
-            best_k = other_k;
-          }
-        }
-        ignored = __any_sync(0xffffffffu, ignored);
-        if (lane == 0) {
-          if (best_k != INT_MAX) {
-            const int g = by_class[best_k];
-            taken[g >> 5] |= 1u << (g & 31);
-            ++tpc[c];
-          } else if (!ignored) {
-            ++fpc[c];
-          }
-        }
-        __syncwarp();
+        write(t, c, check, tp, fp);
       }
-      const int q = step_s[i + 1];
-      if (q >= 0) snapshot(q);
+    }
+    for (u32 rest = __ballot_sync(0xffffffffu, item < items && !alone); rest; rest &= rest - 1) {
+      const int together = base + __ffs(rest) - 1;
+      const int tt = together / nc, cc = together % nc;
+      const long long thr = __double_as_longlong(a.thresholds[tt]);
+      const int s0 = slot_start[cc], ns = slot_start[cc + 1] - s0, m0 = mask_start[cc];
+      const int nm = mask_start[cc + 1] - m0;
+      const long long* iou_c = ious + pair_start[cc];
+      u32* taken = used + tt * words;
+      int tp = 0, fp = 0, m = 0;
+      for (int e = 0; e < checkpoints; ++e) {
+        const u32 check = checks[e];
+        for (; m < nm && by_mask[m0 + m] < (int)(check >> 16); ++m) {
+          long long best = -1;
+          int best_k = INT_MAX;
+          bool ignored = false;
+          for (int k = lane; k < ns; k += 32) {
+            const int g = by_slot[s0 + k];
+            const long long iou = staged ? iou_c[m * ns + k] : iou_of(by_mask[m0 + m], g);
+            if (iou < thr) continue;
+            if (crowd_s[g]) {
+              ignored = true;
+            } else if (!((taken[(s0 + k) >> 5] >> ((s0 + k) & 31)) & 1u) && iou > best) {
+              best = iou;  // a lane scans increasing k: strictly greater keeps the first slot
+              best_k = k;
+            }
+          }
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) {
+            const long long other = __shfl_xor_sync(0xffffffffu, best, off);
+            const int other_k = __shfl_xor_sync(0xffffffffu, best_k, off);
+            if (other > best || (other == best && other_k < best_k)) best = other, best_k = other_k;
+          }
+          if (best_k != INT_MAX) {
+            // Classes of another warp share words at their ends.
+            if (lane == 0) atomicOr(taken + ((s0 + best_k) >> 5), 1u << ((s0 + best_k) & 31));
+            ++tp;
+          } else if (!__any_sync(0xffffffffu, ignored)) {
+            ++fp;
+          }
+          __syncwarp();
+        }
+        if (lane == 0) write(tt, cc, check, tp, fp);
+      }
     }
   }
-  __syncthreads();
-  if (tid == 0 && s_err) atomicOr(error, s_err);
+  if (tid == 0 && s_err) atomicOr(a.error, s_err);
 }
 
-// Precision tp / max(tp + fp, 1) and recall tp / max(positives, 1) of every (row, threshold, class) from
-// the matching counts (positives = tp + fn), grid-stride over all rows of the batch (prefix.py:106-118).
-__global__ void prefix_ratio_kernel(const int64_t* __restrict__ itp, const int64_t* __restrict__ ifp,
-                                    const int64_t* __restrict__ ifn, int64_t entries, double* __restrict__ precision,
-                                    double* __restrict__ recall) {
+// Both roles in one launch: matching first (`match_blocks` CTAs, the longer ones), then a CTA per checkpoint row.
+// Neither reads what the other writes.
+constexpr int kPrefixScoreThreads = 512;
+__global__ void __launch_bounds__(kPrefixScoreThreads)
+prefix_rows_kernel(PrefixMatch match, int splits, int match_blocks, int64_t B, const int* __restrict__ pairs,
+                   int64_t* __restrict__ tp, int64_t* __restrict__ fp, int64_t* __restrict__ fn,
+                   double* __restrict__ sums, int64_t* __restrict__ confusion, int smem) {
   wait_for_earlier_kernels();
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < entries; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t a = itp[e], f = ifp[e], n = a + ifn[e];
-    precision[e] = (double)a / (double)(a + f > 1 ? a + f : 1);
-    recall[e] = (double)a / (double)(n > 1 ? n : 1);
-  }
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int block = blockIdx.x;
+  if (block < match_blocks)
+    match_classes(match, block / splits, block % splits, splits, smem_raw, smem);
+  else
+    score_row(match.descs, B, block - match_blocks, pairs, match.classes, match.gc, match.crowd, match.C, tp, fp, fn,
+              sums, confusion, smem_raw, smem);
 }
 
 }  // namespace
@@ -897,44 +932,28 @@ PE_API int pe_prefix(const int64_t* descs, int64_t B, int64_t total_chunks, int6
     PE_LAUNCHED("prefix_scan");
     count_launch();
   }
-  if (total_rows) {
+  {
     const size_t in_place = label_bytes(max_p) + sizeof(u64) * (max_g + max_p) + sizeof(int) * max_g +
                             score_staging_bytes(max_p) + 32;
-    PE_REQUIRE(in_place <= 200 * 1024, "prefix histogram too large for scoring (G=%lld, N+1=%lld)", (long long)max_g,
-               (long long)max_p);
-    // Two CTAs per SM.
-    const size_t want = label_bytes(max_p) + score_bytes(max_g, max_p, C, max_g * max_p);
-    const size_t smem = std::max(in_place, std::min<size_t>(want, 110 * 1024));
-    if (smem > 48 * 1024)
-      PE_CUDA(cudaFuncSetAttribute(prefix_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_kernel(prefix_score_kernel, (unsigned)total_rows, kPrefixScoreThreads, smem, stream, descs, B, pairs,
-        classes, gc, crowd, (int)C, tp, fp, fn, sums, confusion, (int)smem);
-    PE_LAUNCHED("prefix_score");
-    count_launch();
-  }
-  {
-    const int64_t words = ceil_div(std::max<int64_t>(max_g, 1), 32);
-    const int64_t n = max_p - 1;  // masks per image at most
-    const size_t base = sizeof(u64) * n + sizeof(int) * (C + max_g + C + 1 + n + 1 + 2 * T * C + n + n + 1) +
-                        sizeof(u32) * T * words + sizeof(int) * max_g + max_g + 16;
-    const size_t staged = sizeof(long long) * n * std::max<int64_t>(max_g, 1);
-    // Same-class IoUs staged in shared memory when every mask x slot pair fits, else computed in the chain.
-    const bool stage = base + staged <= 160 * 1024;
-    const size_t smem = base + (stage ? staged : 0);
-    PE_REQUIRE(smem <= 200 * 1024, "prefix matching state too large (G=%lld, T=%lld, C=%lld)", (long long)max_g,
+    PE_REQUIRE(!total_rows || in_place <= 200 * 1024, "prefix histogram too large for scoring (G=%lld, N+1=%lld)",
+               (long long)max_g, (long long)max_p);
+    const size_t state = prefix_match_bytes(max_p - 1, max_g, T, C) + 8;
+    PE_REQUIRE(state <= 200 * 1024, "prefix matching state too large (G=%lld, T=%lld, C=%lld)", (long long)max_g,
                (long long)T, (long long)C);
-    auto kernel = stage ? prefix_match_kernel<true> : prefix_match_kernel<false>;
-    if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_kernel(kernel, (unsigned)B, kPrefixMatchThreads, smem, stream, descs, ga, raw, classes, gc, crowd, isthing,
-        thresholds, (int)T, (int)C, step_q, itp, ifp, ifn, precision, recall, validate, error);
-    PE_LAUNCHED("prefix_match");
-    count_launch();
-  }
-  if (total_rows) {
-    const int64_t entries = total_rows * T * C;
-    const int64_t blocks = std::min<int64_t>(ceil_div(entries, 256), (int64_t)sm_count() * 4);
-    launch_kernel(prefix_ratio_kernel, (unsigned)blocks, 256, 0, stream, itp, ifp, ifn, entries, precision, recall);
-    PE_LAUNCHED("prefix_ratio");
+    // Two CTAs per SM, where the tables of a row and the IoUs of a CTA's classes have use for less.
+    const size_t row = label_bytes(max_p) + score_bytes(max_g, max_p, C, max_g * max_p);
+    const size_t ious = state + sizeof(long long) * (max_p - 1) * max_g;
+    const size_t want = std::min<size_t>(std::max(row, ious), 110 * 1024);
+    const size_t smem = std::max({want, state, total_rows ? in_place : 0});
+    if (smem > 48 * 1024)
+      PE_CUDA(cudaFuncSetAttribute(prefix_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // An image's classes on as many CTAs as there are SMs for the batch.
+    const int64_t splits = std::max<int64_t>(1, std::min<int64_t>(ceil_div(C, kMatchClasses), sm_count() / B));
+    const PrefixMatch match{descs, ga, raw, classes, gc, crowd, isthing, thresholds, (int)T, (int)C, step_q, itp, ifp,
+                            ifn, precision, recall, validate, error};
+    launch_kernel(prefix_rows_kernel, (unsigned)(B * splits + total_rows), kPrefixScoreThreads, smem, stream, match,
+        (int)splits, (int)(B * splits), B, pairs, tp, fp, fn, sums, confusion, (int)smem);
+    PE_LAUNCHED("prefix_rows");
     count_launch();
   }
   if (total_rows) {
