@@ -182,7 +182,9 @@ seg_pass_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chun
 // into a ring of kRing shared-memory slots with cp.async.bulk, completing on
 // per-slot "full" mbarriers. Halves come from a global counter (`schedule`,
 // one atomicAdd per `grab` of them), so CTAs that run faster take more of them,
-// or, without a counter, from a contiguous range of chunks per CTA. Warps 0-7 consume: they
+// or, without a counter, from a contiguous range of chunks per CTA. The counter's last halves
+// are taken in parts, a range of the detections each: whole halves would leave most CTAs waiting
+// for the few with one half more (see pe_seg_pass). Warps 0-7 consume: they
 // take the next half from the queue, read the target/prediction slots of their
 // 16 pixels with plain loads (kept in registers), then take each mask segment
 // from the ring, bin it exactly as the register path does and release the slot
@@ -196,6 +198,7 @@ constexpr int kHalf = kBulkConsumers * kPassPixels;  // 4096 pixels per step
 constexpr int kStageMasks = 4;  // mask-row segments per ring stage (one barrier each)
 constexpr int kRing = 6;        // stages in flight per CTA (two CTAs hold 197 KB; 4 stages: 310 us where 6 take 293)
 constexpr int kHalfRing = 4;    // published halves in flight per CTA
+constexpr int kPartRows = 16;   // detections of a part, at least: its maps are read again, from L2
 constexpr long long kWaitLimit = 4000000000ll;  // about two seconds of SM clock
 constexpr int kTimeoutBit = 1 << 30;
 
@@ -204,6 +207,7 @@ struct BulkShared {
   unsigned char shift[kRing][kStageMasks];             // each row's start offset mod 16
   int64_t half_x0[kHalfRing];     // first pixel of the half
   int64_t half_image[kHalfRing];  // image index; -1 ends the CTA's work
+  int half_rows[kHalfRing][2];    // detections [first, end); the first part counts the maps' pairs too
   uint64_t full[kRing];
   uint64_t empty[kRing];
   uint64_t half_full[kHalfRing];
@@ -215,6 +219,7 @@ template <bool ANY_ALIGN>
 __global__ void __launch_bounds__(kBulkThreads, 2)
 seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chunks, int64_t chunks_per_cta,
                      const int64_t* __restrict__ bounds, unsigned long long* __restrict__ schedule, int grab,
+                     int64_t whole, int parts,
                      const int64_t* __restrict__ order, u32* __restrict__ pairs, u32* __restrict__ dpairs,
                      int* __restrict__ error) {
   wait_for_earlier_kernels();
@@ -243,31 +248,43 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
     // ---- producer --------------------------------------------------------
     if (threadIdx.x != kBulkConsumers) return;
     int64_t seq = 0, halves = 0, next = 2 * c_begin;  // work is taken in halves, two per chunk
-    int64_t grabbed = 0, grab_end = 0;  // with a counter: the current grab of `grab` consecutive halves
+    // With a counter: the current grab of `grab` consecutive units, the first `whole` of them halves, then
+    // the other halves' first parts, their second parts, and so on.
+    int64_t grabbed = 0, grab_end = 0;
+    const int64_t split = 2 * total_chunks - whole, units = whole + split * parts;
     bool ok = true;
     // Publish the next half (image -1: no more work); false when the wait for a free entry fails.
-    auto publish = [&](int64_t image, int64_t x0) {
+    auto publish = [&](int64_t image, int64_t x0, int first_row, int end_row) {
       const int h = (int)(halves % kHalfRing);
       const int64_t use = halves / kHalfRing;
       if ((use > 0 && !mbar_wait(&sm.half_empty[h], (uint32_t)((use - 1) & 1), kWaitLimit)) || *abort) return false;
       sm.half_x0[h] = x0;
       sm.half_image[h] = image;
+      sm.half_rows[h][0] = first_row;
+      sm.half_rows[h][1] = end_row;
       mbar_arrive(&sm.half_full[h]);  // release: the entry is visible to consumers that see the phase
       ++halves;
       return true;
     };
     while (ok) {
       int64_t unit;
+      int part = 0, of = 1;
       if (schedule) {
         if (grabbed == grab_end) {
           grabbed = (int64_t)atomicAdd(schedule, (unsigned long long)grab);
-          grab_end = min(grabbed + grab, 2 * total_chunks);
+          grab_end = min(grabbed + grab, units);
         }
-        unit = grabbed < grab_end ? grabbed++ : 2 * total_chunks;
+        if (grabbed >= grab_end) break;
+        unit = grabbed++;
+        if (unit >= whole) {
+          of = parts;
+          part = (int)((unit - whole) / split);
+          unit = whole + (unit - whole) % split;
+        }
       } else {
-        unit = next < 2 * c_end ? next++ : 2 * total_chunks;
+        if (next >= 2 * c_end) break;
+        unit = next++;
       }
-      if (unit >= 2 * total_chunks) break;
       const int64_t chunk = unit >> 1;
       const int64_t b = image_of_chunk(descs, B, chunk);
       const int64_t* d = desc_of(descs, b);
@@ -275,13 +292,16 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
       const int64_t x0 = (chunk - d[kChunkBegin]) * kChunk + (unit & 1) * kHalf;
       if (x0 >= pixels) continue;  // the second half of an image's last chunk
       const int D = (int)d[kD];
+      const int each = of == 1 ? D : max(kPartRows, (D + of - 1) / of);
+      const int first_row = part * each, end_row = min(D, first_row + each);
+      if (part > 0 && first_row >= D) continue;
       const int* target = reinterpret_cast<const int*>(d[kTarget]);
       const int* pred = reinterpret_cast<const int*>(d[kPred]);
       const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kMasks]);
       const int64_t stride = d[kMaskStride];
       const int64_t* ord = order + d[kDetBegin];
       const bool vec_maps = d[kFlags] & 1;
-      if (!publish(b, x0)) {
+      if (!publish(b, x0, first_row, end_row)) {
         ok = false;
         break;
       }
@@ -289,16 +309,16 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
       const uint32_t map_bytes = (uint32_t)((len * 4) & ~15ll);
       if (vec_maps && map_bytes) {
         bulk_prefetch_l2(target + x0, map_bytes);
-        if (pred) bulk_prefetch_l2(pred + x0, map_bytes);
+        if (pred && part == 0) bulk_prefetch_l2(pred + x0, map_bytes);
       }
-      for (int r0 = 0; r0 < D; r0 += kStageMasks) {
+      for (int r0 = first_row; r0 < end_row; r0 += kStageMasks) {
         const int slot = (int)(seq % kRing);
         const int64_t use = seq / kRing;
         if ((use > 0 && !mbar_wait(&sm.empty[slot], (uint32_t)((use - 1) & 1), kWaitLimit)) || *abort) {
           ok = false;
           break;
         }
-        const int n = min(kStageMasks, D - r0);
+        const int n = min(kStageMasks, end_row - r0);
         // Rows may start at any byte: copy the aligned words from the one holding pixel x0 to the
         // one holding the segment's last byte; the consumers re-align by the row's offset.
         if constexpr (ANY_ALIGN) {
@@ -324,7 +344,7 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
         ++seq;
       }
     }
-    if (ok) ok = publish(-1, 0);
+    if (ok) ok = publish(-1, 0, 0, 0);
     if (!ok) {
       *abort = 1;
       atomicOr(error, kTimeoutBit);
@@ -347,15 +367,16 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
       break;
     }
     const int64_t b = sm.half_image[h], x0 = sm.half_x0[h];
+    const int first_row = sm.half_rows[h][0], end_row = sm.half_rows[h][1];
     __syncwarp();
     if (lane == 0) mbar_arrive(&sm.half_empty[h]);
     ++halves;
     if (b < 0) break;
     const int64_t* d = desc_of(descs, b);
     const int64_t pixels = d[kPixels];
-    const int G = (int)d[kG], P = (int)d[kP], D = (int)d[kD];
+    const int G = (int)d[kG], P = (int)d[kP];
     const int* target = reinterpret_cast<const int*>(d[kTarget]);
-    const int* pred = reinterpret_cast<const int*>(d[kPred]);
+    const int* pred = first_row ? nullptr : reinterpret_cast<const int*>(d[kPred]);
     const bool vec_maps = d[kFlags] & 1;
     u32* image_pairs = pairs + d[kPairBegin];
     u32* image_dpairs = dpairs + d[kDPairBegin];
@@ -372,7 +393,7 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
     }
     const bool in_range = x < x0 + len;
     const LaneSlots ls = lane_slots(t, x, pixels, G, bad);
-    for (int r0 = 0; r0 < D; r0 += kStageMasks) {
+    for (int r0 = first_row; r0 < end_row; r0 += kStageMasks) {
       const int slot = (int)(seq % kRing);
       const bool got = mbar_wait(&sm.full[slot], (uint32_t)((seq / kRing) & 1), kWaitLimit);
       if (!__all_sync(0xffffffffu, got && !*abort)) {  // warp-uniform decision
@@ -395,7 +416,7 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
         }
         hit |= (u32)(any != 0) << k;
       }
-      hit = __reduce_or_sync(0xffffffffu, in_range ? hit : 0u) & ((1u << min(kStageMasks, D - r0)) - 1u);
+      hit = __reduce_or_sync(0xffffffffu, in_range ? hit : 0u) & ((1u << min(kStageMasks, end_row - r0)) - 1u);
 #pragma unroll 1
       for (; hit; hit &= hit - 1) {
         const int k = __ffs(hit) - 1;
@@ -789,20 +810,28 @@ PE_API int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, co
     int64_t grid = cta_bounds ? ctas : ceil_div(total_chunks, per_cta);
     // Chunks taken from the counter, `grab` at a time, by the chosen CTAs per SM; half a chunk at a time
     // while the halves are fewer than kFewHalves per CTA, where a CTA left with one chunk more than the
-    // others is a large part of the launch (384 chunks on 304 CTAs: 207 us by chunks, 161 by halves).
-    int grab = 2 * choice.grab;
+    // others is a large part of the launch (384 chunks on 304 CTAs: 207 us by chunks, 161 by halves). There
+    // the halves beyond the last full round go in kParts parts (149 us, and 1.02 for one image of 640 x 480);
+    // with more rounds it measured the same either way.
+    int grab = 2 * choice.grab, parts = 1;
+    int64_t whole = 2 * total_chunks;
     if (schedule) {
       constexpr int64_t kFewHalves = 16;
+      constexpr int kParts = 8;
       const int64_t all = (int64_t)sm_count() * choice.per_sm;
-      if (2 * total_chunks < kFewHalves * all) grab = 1;
-      grid = std::min(ceil_div(2 * total_chunks, grab), all);
+      if (whole < kFewHalves * all) {
+        grab = 1;
+        parts = kParts;
+        whole = whole / all * all;
+      }
+      grid = std::min(ceil_div(whole + (2 * total_chunks - whole) * parts, grab), all);
       cta_bounds = nullptr;
     }
     const size_t smem = sizeof(BulkShared) + 128;
     auto kernel = bulk == 2 ? seg_pass_bulk_kernel<true> : seg_pass_bulk_kernel<false>;
     PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     launch_kernel(kernel, (unsigned)grid, kBulkThreads, smem, stream, descs, B, total_chunks, per_cta, cta_bounds,
-        reinterpret_cast<unsigned long long*>(schedule), grab, order, pairs, dpairs, error);
+        reinterpret_cast<unsigned long long*>(schedule), grab, whole, parts, order, pairs, dpairs, error);
     PE_LAUNCHED("seg_pass_bulk");
     count_launch();
     return kOk;

@@ -133,3 +133,22 @@ def test_zeroing_clears_the_span_and_nothing_beside_it(offset, size):
     want = torch.full_like(data, 7)
     want[offset:offset + size] = 0
     assert torch.equal(data, want)
+
+
+@pytest.mark.parametrize("dets", (0, 1, 16, 17, 33, 130))
+def test_the_last_halves_of_the_pass_in_parts(dets):
+    """More halves of 4096 pixels than two CTAs per SM: whole ones, then parts of 16 detections and more."""
+    import panoptic_evaluator_gb300 as pe
+    from oracle import combined as ocomb
+    from panoptic_evaluator_gb300 import synthetic
+    from panoptic_evaluator_gb300.ragged import SegmentationImages
+    batch = synthetic.segmentation_batch(seed=dets, images=2, fixed_hw=(1009, 701), slots=(20, 40), dets=(dets, dets))
+    isthing = list(np.arange(133) < 80)
+    oracle = ocomb.SegmentationOracle(133, isthing)
+    fields = ("target", "target_classes", "crowd", "pred", "pred_classes", "det_masks", "det_classes", "scores")
+    for i in batch:
+        oracle.update(i.pred[None], i.pred_classes[None], [i.det_masks], [i.det_classes], [i.scores], i.target[None],
+                      i.target_classes[None], i.crowd[None])
+    joint = pe.SegmentationEvaluator(133, isthing=isthing)
+    joint.update_images(SegmentationImages(*([getattr(i, f) for i in batch] for f in fields)))
+    assert_tree(joint.compute(), oracle.compute())
