@@ -160,6 +160,44 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
+// A position in a ring of N slots with a full and an empty barrier each. A consumer waits for the full barrier's
+// `phase`, a producer for the empty barrier's `phase ^ 1` (which a fresh barrier passes).
+template <int N>
+struct RingSlot {
+  int at = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++at == N) {
+      at = 0;
+      phase ^= 1u;
+    }
+  }
+};
+
+// The last of B table rows (kFields words each) whose `field` is at most `value`, the first row's being so; `field`
+// does not fall. By a whole warp, 128 rows in one round trip: one thread's binary search takes a round trip a step.
+template <int kFields>
+__device__ __forceinline__ int64_t find_row(const int64_t* table, int64_t B, int field, int64_t value) {
+  constexpr int kLoads = 4;
+  const int lane = threadIdx.x & 31;
+  int64_t lo = 0, hi = B;
+  while (hi - lo > 1) {
+    const int64_t step = (hi - lo + 32 * kLoads - 1) / (32 * kLoads);
+    bool reached[kLoads];
+#pragma unroll
+    for (int j = 0; j < kLoads; ++j) {
+      const int64_t row = lo + step * (lane + 32 * j);
+      reached[j] = row < hi && __ldg(table + row * kFields + field) <= value;
+    }
+    int n = 0;
+#pragma unroll
+    for (int j = 0; j < kLoads; ++j) n += __popc(__ballot_sync(0xffffffffu, reached[j]));
+    lo += step * (n - 1);
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
 // Barrier among the first `threads` threads of the CTA (named barrier `id`).
 __device__ __forceinline__ void named_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");

@@ -176,11 +176,17 @@ seg_pass_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total_chun
 // row starts on a 16-byte boundary (e.g. a ragged.SegmentationImages arena);
 // true: rows at any byte offset, the producer copies the aligned 16-byte words
 // covering each row segment and the consumers re-align them by the row's offset.
-// Warp 8 is the producer: one lane takes 4096-pixel halves of 8192-pixel chunks,
-// publishes each (image, first pixel) in a small queue of kHalfRing entries,
-// prefetches its slot maps into L2 and streams its 4096-byte mask-row segments
-// into a ring of kRing shared-memory slots with cp.async.bulk, completing on
-// per-slot "full" mbarriers. Halves come from a global counter (`schedule`,
+// Warp 8 is the producer: it takes 4096-pixel halves of 8192-pixel chunks,
+// publishes each with its image's descriptor in a small queue of kHalfRing
+// entries, prefetches its slot maps into L2 and streams its 4096-byte mask-row
+// segments into a ring of kRing shared-memory slots with cp.async.bulk,
+// completing on per-slot "full" mbarriers. What the producer waits for bounds the
+// launch (by one lane, a stage took it 1800 cycles, 250 of them for a free slot: a
+// load of each row's place in the score order, and a search for the image per
+// half), so the whole warp produces: 32 places are loaded at once, one stage block
+// ahead, a lane copies a row, the image is found in one round trip and the next
+// half is claimed before this one's last rows: 8 images of 512 x 768 with 256
+// detections 149 -> 124 us, 64 uneven images 322 -> 278 (6.3 TB/s). Halves come from a global counter (`schedule`,
 // one atomicAdd per `grab` of them), so CTAs that run faster take more of them,
 // or, without a counter, from a contiguous range of chunks per CTA. The counter's last halves
 // are taken in parts, a range of the detections each: whole halves would leave most CTAs waiting
@@ -205,8 +211,8 @@ constexpr int kTimeoutBit = 1 << 30;
 struct BulkShared {
   unsigned char ring[kRing][kStageMasks][kHalf + 16];  // the aligned words covering each row segment
   unsigned char shift[kRing][kStageMasks];             // each row's start offset mod 16
-  int64_t half_x0[kHalfRing];     // first pixel of the half
-  int64_t half_image[kHalfRing];  // image index; -1 ends the CTA's work
+  int64_t half_desc[kHalfRing][kDescFields];  // the image's descriptor
+  int64_t half_x0[kHalfRing];     // first pixel of the half; -1 ends the CTA's work
   int half_rows[kHalfRing][2];    // detections [first, end); the first part counts the maps' pairs too
   uint64_t full[kRing];
   uint64_t empty[kRing];
@@ -246,36 +252,49 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
 
   if (threadIdx.x >= kBulkConsumers) {
     // ---- producer --------------------------------------------------------
-    if (threadIdx.x != kBulkConsumers) return;
-    int64_t seq = 0, halves = 0, next = 2 * c_begin;  // work is taken in halves, two per chunk
-    // With a counter: the current grab of `grab` consecutive units, the first `whole` of them halves, then
+    const int lane = threadIdx.x & 31;
+    RingSlot<kRing> stage;
+    RingSlot<kHalfRing> half;
+    int64_t sent = 0, next = 2 * c_begin;  // stages; work is taken in halves, two per chunk
+    // With a counter: the current claim of `grab` consecutive units, the first `whole` of them halves, then
     // the other halves' first parts, their second parts, and so on.
-    int64_t grabbed = 0, grab_end = 0;
+    int64_t claimed = 0, claim_end = 0;
+    unsigned long long claim = 0;
+    bool ok = true, asked = false;
     const int64_t split = 2 * total_chunks - whole, units = whole + split * parts;
-    bool ok = true;
-    // Publish the next half (image -1: no more work); false when the wait for a free entry fails.
-    auto publish = [&](int64_t image, int64_t x0, int first_row, int end_row) {
-      const int h = (int)(halves % kHalfRing);
-      const int64_t use = halves / kHalfRing;
-      if ((use > 0 && !mbar_wait(&sm.half_empty[h], (uint32_t)((use - 1) & 1), kWaitLimit)) || *abort) return false;
-      sm.half_x0[h] = x0;
-      sm.half_image[h] = image;
-      sm.half_rows[h][0] = first_row;
-      sm.half_rows[h][1] = end_row;
-      mbar_arrive(&sm.half_full[h]);  // release: the entry is visible to consumers that see the phase
-      ++halves;
+    auto ask = [&] {
+      if (lane == 0) claim = atomicAdd(schedule, (unsigned long long)grab);
+      asked = true;
+    };
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, kWaitLimit) && !*abort) != 0;
+    };
+    // Publish the next half (x0 -1: no more work); false when the wait for a free entry fails.
+    auto publish = [&](int64_t word, int64_t x0, int first_row, int end_row) {
+      if (!wait(&sm.half_empty[half.at], half.phase ^ 1u)) return false;
+      if (lane < kDescFields) sm.half_desc[half.at][lane] = word;
+      if (lane == 0) {
+        sm.half_x0[half.at] = x0;
+        sm.half_rows[half.at][0] = first_row;
+        sm.half_rows[half.at][1] = end_row;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.half_full[half.at]);  // release: the entry is visible with the phase
+      half.next();
       return true;
     };
     while (ok) {
       int64_t unit;
       int part = 0, of = 1;
       if (schedule) {
-        if (grabbed == grab_end) {
-          grabbed = (int64_t)atomicAdd(schedule, (unsigned long long)grab);
-          grab_end = min(grabbed + grab, units);
+        if (claimed == claim_end) {
+          if (!asked) ask();
+          claimed = (int64_t)__shfl_sync(0xffffffffu, claim, 0);
+          claim_end = min(claimed + grab, units);
+          asked = false;
         }
-        if (grabbed >= grab_end) break;
-        unit = grabbed++;
+        if (claimed >= claim_end) break;
+        unit = claimed++;
         if (unit >= whole) {
           of = parts;
           part = (int)((unit - whole) / split);
@@ -286,93 +305,84 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
         unit = next++;
       }
       const int64_t chunk = unit >> 1;
-      const int64_t b = image_of_chunk(descs, B, chunk);
-      const int64_t* d = desc_of(descs, b);
-      const int64_t pixels = d[kPixels];
-      const int64_t x0 = (chunk - d[kChunkBegin]) * kChunk + (unit & 1) * kHalf;
+      const int64_t b = find_row<kDescFields>(descs, B, kChunkBegin, chunk);
+      const int64_t word = lane < kDescFields ? desc_of(descs, b)[lane] : 0;
+      auto field = [&](int f) { return __shfl_sync(0xffffffffu, word, f); };
+      const int64_t pixels = field(kPixels);
+      const int64_t x0 = (chunk - field(kChunkBegin)) * kChunk + (unit & 1) * kHalf;
       if (x0 >= pixels) continue;  // the second half of an image's last chunk
-      const int D = (int)d[kD];
+      const int D = (int)field(kD);
       const int each = of == 1 ? D : max(kPartRows, (D + of - 1) / of);
       const int first_row = part * each, end_row = min(D, first_row + each);
       if (part > 0 && first_row >= D) continue;
-      const int* target = reinterpret_cast<const int*>(d[kTarget]);
-      const int* pred = reinterpret_cast<const int*>(d[kPred]);
-      const uint8_t* masks = reinterpret_cast<const uint8_t*>(d[kMasks]);
-      const int64_t stride = d[kMaskStride];
-      const int64_t* ord = order + d[kDetBegin];
-      const bool vec_maps = d[kFlags] & 1;
-      if (!publish(b, x0, first_row, end_row)) {
+      const int64_t stride = field(kMaskStride);
+      const uint8_t* masks = reinterpret_cast<const uint8_t*>(field(kMasks)) + x0;
+      const int64_t* ord = order + field(kDetBegin);
+      int64_t place = first_row + lane < end_row ? ord[first_row + lane] : 0;
+      if (!publish(word, x0, first_row, end_row)) {
         ok = false;
         break;
       }
       const int64_t len = min((int64_t)kHalf, pixels - x0);
       const uint32_t map_bytes = (uint32_t)((len * 4) & ~15ll);
-      if (vec_maps && map_bytes) {
-        bulk_prefetch_l2(target + x0, map_bytes);
-        if (pred && part == 0) bulk_prefetch_l2(pred + x0, map_bytes);
+      if ((field(kFlags) & 1) && map_bytes) {  // lane 0: the target map, lane 1: the prediction
+        const int64_t map = field(lane == 1 ? kPred : kTarget);
+        if (lane < (part == 0 ? 2 : 1) && map) bulk_prefetch_l2(reinterpret_cast<const int*>(map) + x0, map_bytes);
       }
-      for (int r0 = first_row; r0 < end_row; r0 += kStageMasks) {
-        const int slot = (int)(seq % kRing);
-        const int64_t use = seq / kRing;
-        if ((use > 0 && !mbar_wait(&sm.empty[slot], (uint32_t)((use - 1) & 1), kWaitLimit)) || *abort) {
-          ok = false;
-          break;
-        }
-        const int n = min(kStageMasks, end_row - r0);
-        // Rows may start at any byte: copy the aligned words from the one holding pixel x0 to the
-        // one holding the segment's last byte; the consumers re-align by the row's offset.
-        if constexpr (ANY_ALIGN) {
-          const uint8_t* rows[kStageMasks];
-          uint32_t total = 0;
-          for (int k = 0; k < n; ++k) {
-            rows[k] = masks + ord[r0 + k] * stride + x0;
-            const int o = (int)(reinterpret_cast<uintptr_t>(rows[k]) & 15);
-            sm.shift[slot][k] = (unsigned char)o;
-            total += (uint32_t)round_up(len + o, 16);
+      for (int r32 = first_row; ok && r32 < end_row; r32 += 32) {
+        const uint8_t* row = masks + place * stride;  // lane l: row r32 + l
+        if (r32 + 32 + lane < end_row) place = ord[r32 + 32 + lane];
+        for (int r0 = r32; r0 < min(r32 + 32, end_row); r0 += kStageMasks) {
+          if (!wait(&sm.empty[stage.at], stage.phase ^ 1u)) {
+            ok = false;
+            break;
           }
-          mbar_arrive_expect_tx(&sm.full[slot], total);  // release: the offsets are visible with the phase
-          for (int k = 0; k < n; ++k) {
-            const int o = sm.shift[slot][k];
-            bulk_copy_g2s(sm.ring[slot][k], rows[k] - o, (uint32_t)round_up(len + o, 16), &sm.full[slot]);
-          }
-        } else {  // every row starts on a 16-byte boundary
-          const uint32_t bytes = (uint32_t)round_up(len, 16);
-          mbar_arrive_expect_tx(&sm.full[slot], bytes * (uint32_t)n);
-          for (int k = 0; k < n; ++k)
-            bulk_copy_g2s(sm.ring[slot][k], masks + ord[r0 + k] * stride + x0, bytes, &sm.full[slot]);
+          const int n = min(kStageMasks, end_row - r0);
+          // Rows may start at any byte: copy the aligned words from the one holding pixel x0 to the
+          // one holding the segment's last byte; the consumers re-align by the row's offset.
+          const uint64_t from = __shfl_sync(0xffffffffu, reinterpret_cast<uint64_t>(row), (r0 - r32 + lane) & 31);
+          const int o = ANY_ALIGN ? (int)(from & 15) : 0;
+          const uint32_t bytes = lane < n ? (uint32_t)round_up(len + o, 16) : 0u;
+          if (ANY_ALIGN && lane < n) sm.shift[stage.at][lane] = (unsigned char)o;
+          const uint32_t total = __reduce_add_sync(0xffffffffu, bytes);
+          __syncwarp();
+          if (lane == 0) mbar_arrive_expect_tx(&sm.full[stage.at], total);  // release: the offsets too
+          __syncwarp();
+          if (lane < n)
+            bulk_copy_g2s(sm.ring[stage.at][lane], reinterpret_cast<const uint8_t*>(from) - o, bytes,
+                          &sm.full[stage.at]);
+          stage.next();
+          ++sent;
+          if (schedule && claimed == claim_end && !asked && r0 + 2 * kStageMasks >= end_row) ask();
         }
-        ++seq;
       }
     }
-    if (ok) ok = publish(-1, 0, 0, 0);
+    if (ok) ok = publish(0, -1, 0, 0);
     if (!ok) {
       *abort = 1;
-      atomicOr(error, kTimeoutBit);
+      if (lane == 0) atomicOr(error, kTimeoutBit);
     }
     // Wait for the copies still in flight into this CTA's shared memory.
-    for (int64_t q = seq > kRing ? seq - kRing : 0; q < seq; ++q)
+    for (int64_t q = sent > kRing ? sent - kRing : 0; q < sent; ++q)
       mbar_wait(&sm.full[q % kRing], (uint32_t)((q / kRing) & 1), kWaitLimit);
     return;
   }
 
   // ---- consumers ---------------------------------------------------------
   const int ctid = threadIdx.x, lane = ctid & 31;
-  int64_t seq = 0, halves = 0;
+  RingSlot<kRing> stage;
+  RingSlot<kHalfRing> half;
   bool ok = true, bad = false;
   while (ok) {
-    const int h = (int)(halves % kHalfRing);
-    const bool ready = mbar_wait(&sm.half_full[h], (uint32_t)((halves / kHalfRing) & 1), kWaitLimit);
+    const bool ready = mbar_wait(&sm.half_full[half.at], half.phase, kWaitLimit);
     if (!__all_sync(0xffffffffu, ready && !*abort)) {
       ok = false;
       break;
     }
-    const int64_t b = sm.half_image[h], x0 = sm.half_x0[h];
-    const int first_row = sm.half_rows[h][0], end_row = sm.half_rows[h][1];
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.half_empty[h]);
-    ++halves;
-    if (b < 0) break;
-    const int64_t* d = desc_of(descs, b);
+    const int64_t x0 = sm.half_x0[half.at];
+    const int first_row = sm.half_rows[half.at][0], end_row = sm.half_rows[half.at][1];
+    const int64_t* d = sm.half_desc[half.at];
+    if (x0 < 0) break;
     const int64_t pixels = d[kPixels];
     const int G = (int)d[kG], P = (int)d[kP];
     const int* target = reinterpret_cast<const int*>(d[kTarget]);
@@ -380,6 +390,9 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
     const bool vec_maps = d[kFlags] & 1;
     u32* image_pairs = pairs + d[kPairBegin];
     u32* image_dpairs = dpairs + d[kDPairBegin];
+    __syncwarp();  // the entry is in registers
+    if (lane == 0) mbar_arrive(&sm.half_empty[half.at]);
+    half.next();
     const int64_t len = min((int64_t)kHalf, pixels - x0);
     const int64_t x = x0 + (int64_t)ctid * kPassPixels;
     int t[16];
@@ -394,8 +407,7 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
     const bool in_range = x < x0 + len;
     const LaneSlots ls = lane_slots(t, x, pixels, G, bad);
     for (int r0 = first_row; r0 < end_row; r0 += kStageMasks) {
-      const int slot = (int)(seq % kRing);
-      const bool got = mbar_wait(&sm.full[slot], (uint32_t)((seq / kRing) & 1), kWaitLimit);
+      const bool got = mbar_wait(&sm.full[stage.at], stage.phase, kWaitLimit);
       if (!__all_sync(0xffffffffu, got && !*abort)) {  // warp-uniform decision
         ok = false;
         break;
@@ -403,14 +415,14 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
       // One warp-wide OR tells which masks of the stage have a pixel here (a superset for rows at any
       // offset: the staged words as they lie); only those are re-aligned and counted, by one copy of the
       // counting code.
-      const unsigned char* staged = &sm.ring[slot][0][ctid * kPassPixels];
+      const unsigned char* staged = &sm.ring[stage.at][0][ctid * kPassPixels];
       constexpr int kRowBytes = kHalf + 16;
       u32 hit = 0;
 #pragma unroll
       for (int k = 0; k < kStageMasks; ++k) {
         const uint4 a = *reinterpret_cast<const uint4*>(staged + k * kRowBytes);
         u32 any = a.x | a.y | a.z | a.w;
-        if (ANY_ALIGN && lane == 31 && sm.shift[slot][k]) {  // the warp's pixels end in the next word
+        if (ANY_ALIGN && lane == 31 && sm.shift[stage.at][k]) {  // the warp's pixels end in the next word
           const uint4 c = *reinterpret_cast<const uint4*>(staged + k * kRowBytes + 16);
           any |= c.x | c.y | c.z | c.w;
         }
@@ -422,14 +434,14 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
         const int k = __ffs(hit) - 1;
         uint4 w = *reinterpret_cast<const uint4*>(staged + k * kRowBytes);
         if constexpr (ANY_ALIGN) {
-          const int o = sm.shift[slot][k];  // the same for the whole warp
+          const int o = sm.shift[stage.at][k];  // the same for the whole warp
           if (o) w = realign16(w, *reinterpret_cast<const uint4*>(staged + k * kRowBytes + 16), o);
         }
         add_slots(t, ls, pack16(w), image_dpairs + (int64_t)(r0 + k) * G);
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.empty[slot]);
-      ++seq;
+      if (lane == 0) mbar_arrive(&sm.empty[stage.at]);
+      stage.next();
     }
   }
   if (!ok) {
@@ -811,7 +823,7 @@ PE_API int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, co
     // Chunks taken from the counter, `grab` at a time, by the chosen CTAs per SM; half a chunk at a time
     // while the halves are fewer than kFewHalves per CTA, where a CTA left with one chunk more than the
     // others is a large part of the launch (384 chunks on 304 CTAs: 207 us by chunks, 161 by halves). There
-    // the halves beyond the last full round go in kParts parts (149 us, and 1.02 for one image of 640 x 480);
+    // the halves beyond the last full round go in kParts parts (149 us by the one-lane producer, 124 now);
     // with more rounds it measured the same either way.
     int grab = 2 * choice.grab, parts = 1;
     int64_t whole = 2 * total_chunks;
