@@ -22,7 +22,7 @@ namespace {
 
 constexpr int kChains = 40;
 constexpr int kMaxDets = 100;
-constexpr int kMatchThreads = 128;
+constexpr int kMatchThreads = 256;  // threads of a matching CTA, half of them where CTAs are many
 
 __device__ __forceinline__ void area_range(int a, double& lo, double& hi) {
   lo = a == 2 ? 1024.0 : (a == 3 ? 9216.0 : 0.0);
@@ -39,12 +39,19 @@ __device__ __forceinline__ double iou_threshold(int t) {
 constexpr int kMatchList = 512;
 __host__ __device__ inline int match_entries(int g_max) { return g_max > kMatchList ? g_max : kMatchList; }
 
-// Shared memory of one matching CTA for up to g_max targets per image: candidate IoUs and targets, the
-// detections' list ranges, 40 chains' taken bits, the class's detections and targets.
+// A detection of the class: its entries [first, first + length), its index in the image, bit a: its area is inside
+// range a.
+struct __align__(16) MatchRecord {
+  int first, length, det;
+  u32 ranges;
+};
+
+// Shared memory of one matching CTA for up to g_max targets per image: the class's detections, candidate IoUs and
+// targets, 40 chains' taken bits, the class's targets.
 __host__ __device__ inline size_t match_bytes(int g_max) {
   const int words = (g_max + 31) / 32;
-  return (sizeof(long long) + sizeof(uint32_t)) * (size_t)match_entries(g_max) + sizeof(int) * 3 * kMaxDets +
-         sizeof(uint32_t) * kChains * (size_t)words + sizeof(uint16_t) * (size_t)g_max + (size_t)g_max + kMaxDets + 16;
+  return sizeof(MatchRecord) * kMaxDets + (sizeof(long long) + sizeof(uint32_t)) * (size_t)match_entries(g_max) +
+         sizeof(uint32_t) * kChains * (size_t)words + sizeof(uint16_t) * (size_t)g_max + (size_t)g_max + 16;
 }
 
 struct FlagLayout {
@@ -88,7 +95,11 @@ __device__ __forceinline__ int nth_present_class(const u32* __restrict__ row, in
 // with its crowd and area-ignored bits. A chain's step is then a walk to the
 // first usable entry, usually one or two shared reads. 32 COCO-like images of
 // 100 detections: 21.8 us against 50.7 with one warp per class that divided and
-// balloted inside the chain; 8 images of 256 detections 27.4 against 153.
+// balloted inside the chain; 8 images of 256 detections 27.4 against 153. The
+// longest class sets the time, so a warp lists as many detections at a time as
+// it has lanes for their targets, eight warps list, and a chain's records and
+// first entries are read ahead of it: 16 images on a canvas 24.0 -> 14.1 us, 32
+// COCO-like ones 21.9 -> 17.7, 8 of 256 detections 31.4 -> 25.6.
 template <typename Count>
 __global__ void __launch_bounds__(kMatchThreads)
 match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_off,
@@ -106,7 +117,7 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
   // class of image b: of all classes, or with per-image class bits of those present in it (about a third
   // in COCO-like batches), so that the CTAs left without a class come last.
   const int b = (int)blockIdx.x, entry = (int)(blockIdx.y + gridDim.y * blockIdx.z);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = kMatchThreads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (int)(blockDim.x >> 5);
   const int bit_words = (C + 31) / 32;
   const int c = class_bits ? nth_present_class(class_bits + (int64_t)b * bit_words, bit_words, entry, lane) : entry;
   if (c < 0 || c >= C) return;
@@ -120,15 +131,12 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
   const int words = (g_max + 31) / 32, capacity = match_entries(g_max);
   // IoUs as IEEE bit patterns: for non-negative doubles the int64 order is the
   // numeric order, so lists and chains compare integers only.
-  long long* iou_s = reinterpret_cast<long long*>(smem_raw);
+  MatchRecord* recs = reinterpret_cast<MatchRecord*>(smem_raw);
+  long long* iou_s = reinterpret_cast<long long*>(recs + kMaxDets);
   u32* cand = reinterpret_cast<u32*>(iou_s + capacity);  // target j | ignored-in-range bits << 16 | crowd << 20
-  int* dets = reinterpret_cast<int*>(cand + capacity);
-  int* first = dets + kMaxDets;                          // a detection's entries: [first, first + length)
-  int* length = first + kMaxDets;
-  u32* used = reinterpret_cast<u32*>(length + kMaxDets);
+  u32* used = cand + capacity;
   uint16_t* gts = reinterpret_cast<uint16_t*>(used + kChains * words);
   uint8_t* target_bits = reinterpret_cast<uint8_t*>(gts + g_max);  // bits 0-3: ignored in range a, bit 4: crowd
-  uint8_t* range_s = target_bits + g_max;                          // bit a: detection area inside range a
   __shared__ int s_nd, s_ng, s_total;
   const u32 below = (1u << lane) - 1;
   constexpr int kScanBlocks = 4;  // blocks of 32 whose loads a lane issues before the ballots use them
@@ -152,7 +160,7 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
         if (sel) {
           const int rank = nd + __popc(ballot & below);
           if (rank < kMaxDets) {
-            dets[rank] = d;
+            recs[rank].det = d;
             ranks[d] = rank + 1;
           } else {
             unranked = true;
@@ -208,14 +216,14 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
     }
     if (lane == 0) s_ng = ng;
   } else {
-    for (int k = threadIdx.x - 64; k < kChains * words; k += kMatchThreads - 64) used[k] = 0;
+    for (int k = threadIdx.x - 64; k < kChains * words; k += blockDim.x - 64) used[k] = 0;
     if (threadIdx.x == 64) s_total = 0;
   }
   __syncthreads();
   const int nd = s_nd, ng = s_ng;
   if (nd == 0) return;
-  for (int i = threadIdx.x; i < nd; i += kMatchThreads) {
-    const double dpa = pa[dets[i]];
+  for (int i = threadIdx.x; i < nd; i += blockDim.x) {
+    const double dpa = pa[recs[i].det];
     u32 bits = 0;
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
@@ -223,24 +231,22 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
       area_range(a, lo, hi);
       bits |= (u32)(lo <= dpa && dpa <= hi) << a;
     }
-    range_s[i] = (uint8_t)bits;
+    recs[i].ranges = bits;
   }
   // Candidates of detection i into entries [at, at + n), sorted; `at` from the shared counter, or 0 for
   // one detection at a time. Entries past the capacity are counted, not stored. One warp.
+  const long long lowest = __double_as_longlong(0.5);
+  auto iou_between = [&](int d, int j) -> long long {
+    const int g = gts[j];
+    const double inter = (double)P[(int64_t)d * G + g], pa_d = pa[d], ga_g = ga[g];
+    if (!(inter > 0.0)) return -1;
+    const double uni = fmax((target_bits[j] & 16) ? pa_d : (pa_d + ga_g) - inter, 1.0);
+    if (inter * 2.001 < uni) return -1;  // clearly under the lowest threshold: no division
+    return __double_as_longlong(inter / uni);
+  };
   auto list_candidates = [&](int i, bool alone) {
-    const int d = dets[i];
-    const double pa_d = pa[d];
-    const Count* row = P + (int64_t)d * G;
-    auto iou_of = [&](int j) -> long long {
-      if (j >= ng) return -1;
-      const int g = gts[j];
-      const double inter = (double)row[g];
-      if (!(inter > 0.0)) return -1;
-      const double uni = fmax((target_bits[j] & 16) ? pa_d : (pa_d + ga[g]) - inter, 1.0);
-      if (inter * 2.001 < uni) return -1;  // clearly under the lowest threshold: no division
-      return __double_as_longlong(inter / uni);
-    };
-    const long long lowest = __double_as_longlong(0.5);
+    const int d = recs[i].det;
+    auto iou_of = [&](int j) -> long long { return j < ng ? iou_between(d, j) : -1; };
     const long long own = iou_of(lane);  // up to 32 targets: one evaluation serves both passes
     int n = __popc(__ballot_sync(0xffffffffu, own >= lowest)), at = 0;
     for (int j0 = 32; j0 < ng; j0 += 32) n += __popc(__ballot_sync(0xffffffffu, iou_of(j0 + lane) >= lowest));
@@ -259,8 +265,8 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
       k += __popc(ballot);
     }
     if (lane == 0) {
-      first[i] = at;
-      length[i] = n;
+      recs[i].first = at;
+      recs[i].length = n;
     }
     __syncwarp();
     if (n < 2 || at + n > capacity) return;
@@ -293,41 +299,99 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
     }
     __syncwarp();
   };
+  // The same for up to 32 targets: 32 / width detections i0, i0 + 1, ... at a time, `width` lanes each.
+  const int width = ng <= 1 ? 1 : 1 << (32 - __clz(ng - 1));
+  auto list_some = [&](int i0) {
+    const int j = lane & (width - 1), group = lane - j, i = i0 + group / width;
+    const bool valid = i < nd && j < ng;
+    const long long iou = valid ? iou_between(recs[i].det, j) : -1;
+    const u32 all = __ballot_sync(0xffffffffu, iou >= lowest);
+    const u32 mine = (all >> group) & (width < 32 ? (1u << width) - 1u : 0xffffffffu);
+    int at = 0;
+    if (lane == 0 && all) at = atomicAdd(&s_total, __popc(all));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(all & ((1u << group) - 1u));
+    const int n = __popc(mine), own = __popc(mine & ((1u << j) - 1u));
+    const bool listed = iou >= lowest && at + n <= capacity;
+    if (listed) iou_s[at + own] = iou;
+    __syncwarp();
+    int rank = 0;  // falling IoU, later targets first on ties
+    for (int k = 0; listed && k < n; ++k) {
+      const long long o = iou_s[at + k];
+      rank += o > iou || (o == iou && k > own);
+    }
+    __syncwarp();
+    if (listed) {
+      iou_s[at + rank] = iou;
+      cand[at + rank] = (u32)j | (u32)target_bits[j] << 16;
+    }
+    if (j == 0 && i < nd) {
+      recs[i].first = at;
+      recs[i].length = n;
+    }
+  };
   // One detection of one chain: eligible targets before ignored ones, the largest IoU, the later target
-  // on ties (a taken target is skipped unless it is a crowd).
+  // on ties (a taken target is skipped unless it is a crowd). `iou` and `w` are the detection's first entry,
+  // `bits` the targets taken where they fit a word.
   const int chain = threadIdx.x, a = chain / 10;
   const long long thr = chain < kChains ? __double_as_longlong(iou_threshold(chain % 10)) : 0;
   u32* taken = used + chain * words;
-  auto step = [&](int i) {
+  const bool in_word = ng <= 32;
+  u32 bits = 0;
+  auto step = [&](const MatchRecord& r, long long iou, u32 w) {
     int best = -1, ignored = -1;
-    for (int e = first[i], end = e + length[i]; e < end; ++e) {
-      if (iou_s[e] < thr) break;
-      const u32 w = cand[e];
+    for (int e = r.first, end = r.first + r.length; e < end;) {
+      if (iou < thr) break;
       const int j = (int)(w & 0xffffu);
-      if (!((w >> 20) & 1u) && ((taken[j >> 5] >> (j & 31)) & 1u)) continue;
-      if (!((w >> (16 + a)) & 1u)) {
-        best = j;
-        break;
+      const u32 word = in_word ? bits : taken[j >> 5];
+      if (((w >> 20) & 1u) || !((word >> (j & 31)) & 1u)) {
+        if (!((w >> (16 + a)) & 1u)) {
+          best = j;
+          break;
+        }
+        if (ignored < 0) ignored = j;
       }
-      if (ignored < 0) ignored = j;
+      if (++e < end) {
+        iou = iou_s[e];
+        w = cand[e];
+      }
     }
     int8_t flag = best >= 0 ? 1 : -1;
     if (best < 0) best = ignored;
-    if (best >= 0) taken[best >> 5] |= 1u << (best & 31);
-    else if ((range_s[i] >> a) & 1) flag = 0;
-    fbase[chain * flags.chain_stride + (int64_t)dets[i] * flags.det_stride] = flag;
+    if (best >= 0) {
+      if (in_word) bits |= 1u << best;
+      else taken[best >> 5] |= 1u << (best & 31);
+    } else if ((r.ranges >> a) & 1) {
+      flag = 0;
+    }
+    fbase[chain * flags.chain_stride + (int64_t)r.det * flags.det_stride] = flag;
   };
-  for (int i = warp; i < nd; i += warps) list_candidates(i, false);
+  if (ng <= 32)
+    for (int i = warp * (32 / width); i < nd; i += warps * (32 / width)) list_some(i);
+  else
+    for (int i = warp; i < nd; i += warps) list_candidates(i, false);
   __syncthreads();
   if (s_total <= capacity) {
-    if (chain < kChains)
-      for (int i = 0; i < nd; ++i) step(i);
+    if (chain >= kChains) return;
+    // Two records and one first entry ahead of the chain. The last detections read the last one's again.
+    MatchRecord now = recs[0], next = recs[min(1, nd - 1)];
+    long long iou = iou_s[now.first];
+    u32 w = cand[now.first];
+    for (int i = 0; i < nd; ++i) {
+      const MatchRecord after = recs[min(i + 2, nd - 1)];
+      const long long iou_next = iou_s[next.first];
+      const u32 w_next = cand[next.first];
+      step(now, iou, w);
+      now = next;
+      next = after;
+      iou = iou_next;
+      w = w_next;
+    }
     return;
   }
   for (int i = 0; i < nd; ++i) {  // more candidates than the list holds: one detection at a time
     if (warp == 0) list_candidates(i, true);
     __syncthreads();
-    if (chain < kChains) step(i);
+    if (chain < kChains) step(recs[i], iou_s[recs[i].first], cand[recs[i].first]);
     __syncthreads();
   }
 }
@@ -1000,15 +1064,18 @@ int launch_match(const void* pairs, bool pairs_u32, const int64_t* pair_off, con
   const unsigned rows = (unsigned)std::min(C, 65535);
   const dim3 grid((unsigned)B, rows, (unsigned)ceil_div(C, rows));
   FlagLayout layout{flags, chain_stride, det_stride};
+  // Many CTAs are bounded by how many an SM holds at a time (64 images of 133 classes: 30 us with 256 threads, 18.7
+  // with 128), few by the longest class (32 images of 80: 17.7 us, 21.8 with 128 threads).
+  const unsigned threads = B * C > 4096 ? kMatchThreads / 2 : kMatchThreads;
   if (pairs_u32) {
     auto kernel = match_kernel<u32>;
     if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_kernel(kernel, grid, kMatchThreads, smem, stream, static_cast<const u32*>(pairs), pair_off, d_off, g_off,
+    launch_kernel(kernel, grid, threads, smem, stream, static_cast<const u32*>(pairs), pair_off, d_off, g_off,
         single_d, single_g, pc, pa, gc, ga, crowd, areas, C, g_max, layout, ranks, counts, gate, class_bits);
   } else {
     auto kernel = match_kernel<int64_t>;
     if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_kernel(kernel, grid, kMatchThreads, smem, stream, static_cast<const int64_t*>(pairs), pair_off, d_off, g_off,
+    launch_kernel(kernel, grid, threads, smem, stream, static_cast<const int64_t*>(pairs), pair_off, d_off, g_off,
         single_d, single_g, pc, pa, gc, ga, crowd, areas, C, g_max, layout, ranks, counts, gate, class_bits);
   }
   PE_LAUNCHED("match");
