@@ -295,6 +295,22 @@ int pe_inst_intersect(const int64_t* descs, int64_t B, int64_t pair_chunks, cons
                       uint32_t* inter, int64_t inter_len, uint64_t* pa, int64_t pa_len, uint64_t* ga, int64_t ga_len,
                       const void* maps, int64_t limit, uint64_t* work, int32_t* error, cudaStream_t stream);
 /*
+ * An update's first launch and its counts. pe_inst_begin: pe_inst_gather, then
+ * pe_seg_sort of what it gathered; clears inter, pa and ga and, with limit > 0
+ * (pe_stream_limit), samples the masks into work (8 B + 1 u64, device scratch).
+ * pe_inst_counts: pe_inst_contract's counts into the cleared outputs, streamed
+ * where the sample stays within limit.
+ */
+int pe_inst_begin(const int64_t* descs, const int64_t* fields, int64_t B, int32_t* pc, double* scores, int32_t* gc,
+                  uint8_t* crowd, double* areas, int64_t total_detections, int64_t* order, double* sorted_scores,
+                  int32_t* sorted_classes, void* workspace, int64_t workspace_bytes, uint32_t* inter,
+                  int64_t inter_len, uint64_t* pa, int64_t pa_len, uint64_t* ga, int64_t ga_len, int64_t limit,
+                  uint64_t* work, cudaStream_t stream);
+int pe_inst_counts(const int64_t* descs, int64_t B, int64_t pair_chunks, const int64_t* blocks, int64_t n_blocks,
+                   int64_t total_chunks, const int64_t* cta_bounds, int64_t ctas, const int64_t* order, uint32_t* inter,
+                   uint64_t* pa, uint64_t* ga, const void* maps, int64_t limit, uint64_t* work, int32_t* error,
+                   cudaStream_t stream);
+/*
  * Host-side companion of pe_inst_contract (no GPU work): for each image of the
  * HOST descriptor table whose mask rows start on 16-byte boundaries (flags
  * bit 1), with detections and targets, encodes two CUtensorMap (detection

@@ -38,8 +38,8 @@ using namespace pe;
 
 #define PE_HOST_API(X)                                                                              \
   X(pe_update) X(pe_zero) X(pe_compute) X(pe_reward_pq) X(pe_pack) X(pe_pack_rgb) X(pe_contract_maps)          \
-  X(pe_contract_blocks) X(pe_inst_gather) X(pe_seg_sort) X(pe_seg_sort_workspace)                   \
-  X(pe_inst_contract) X(pe_inst_intersect) X(pe_stream_limit) X(pe_inst_prepare) X(pe_seg_match) X(pe_instance_accumulate)                  \
+  X(pe_contract_blocks) X(pe_inst_begin) X(pe_seg_sort) X(pe_seg_sort_workspace)                   \
+  X(pe_inst_counts) X(pe_stream_limit) X(pe_inst_prepare) X(pe_seg_match) X(pe_instance_accumulate)                  \
   X(pe_instance_accumulate_workspace) X(pe_seg_pass) X(pe_seg_score) X(pe_prefix)
 
 struct Api {
@@ -798,20 +798,16 @@ PyObject* instance_update(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   int code = 0;
   {
     ReleaseGil released;
-    code = api.pe_inst_gather(descs, descs + p.rows_at, B, pc, scores, gc, crowd, ann_in, stream);
-    if (!code)
-      code = api.pe_seg_sort(descs, B, scores, pc, D, order, tail.scores, tail.classes, at_address<void>(base + sort_at),
-                             sort_bytes, stream);
+    uint64_t* sample = at_address<uint64_t>(base + stream_at);
+    code = api.pe_inst_begin(descs, descs + p.rows_at, B, pc, scores, gc, crowd, ann_in, D, order, tail.scores,
+                             tail.classes, at_address<void>(base + sort_at), sort_bytes, inter, inter_len, pa, D,
+                             pa + D, G, p.stream_limit, sample, stream);
     const int64_t* blocks = p.total_chunks ? descs + p.blocks_at : nullptr;
     const int64_t* bounds = p.total_chunks ? descs + p.bounds_at : nullptr;
     const int64_t* maps = p.maps_at >= 0 && p.total_chunks ? descs + p.maps_at : nullptr;
-    if (!code && p.stream_limit > 0)  // sparse masks may be counted faster by streaming them
-      code = api.pe_inst_intersect(descs, B, p.chunks, blocks, p.n_blocks, p.total_chunks, bounds, p.ranges, order, inter,
-                                   inter_len, pa, D, pa + D, G, maps, p.stream_limit,
-                                   at_address<uint64_t>(base + stream_at), error, stream);
-    else if (!code)
-      code = api.pe_inst_contract(descs, blocks, p.n_blocks, p.total_chunks, bounds, p.ranges, order, inter, inter_len,
-                                  pa, D, pa + D, G, maps, error, stream);
+    if (!code)
+      code = api.pe_inst_counts(descs, B, p.chunks, blocks, p.n_blocks, p.total_chunks, bounds, p.ranges, order, inter,
+                                pa, pa + D, maps, p.stream_limit, sample, error, stream);
     if (!code)
       code = api.pe_inst_prepare(descs, B, pa, pa + D, pa_d, ga_d, tail.classes, gc, tail.scores, ann_in, ann, *C, check,
                                  bits, error, stream);
@@ -921,6 +917,12 @@ struct SegInputs {
   const int32_t* det_classes = nullptr;
   const double* det_scores = nullptr;
   const double* areas = nullptr;
+  // With fields still to gather (pe_inst_gather's rows): the arrays they go to.
+  const int64_t* rows = nullptr;
+  int32_t* rows_classes = nullptr;
+  double* rows_scores = nullptr;
+  int32_t* rows_gc = nullptr;
+  uint8_t* rows_crowd = nullptr;
 };
 
 struct SegEvaluator {
@@ -984,8 +986,12 @@ int launch_seg(const SegSizes& z, const SegInputs& in, const SegScratch& w, SegE
   double* ann = at_address<double>(base + w.ann);
   int32_t* slot_class = at_address<int32_t>(base + w.slot_class);
   uint32_t* bits = at_address<uint32_t>(base + w.bits);
-  int code = api.pe_seg_sort(in.descs, z.B, in.det_scores, in.det_classes, z.D, order, ev.tail.scores, ev.tail.classes,
-                             at_address<void>(base + w.sort), w.sort_bytes, stream);
+  void* sort = at_address<void>(base + w.sort);
+  int code = in.rows ? api.pe_inst_begin(in.descs, in.rows, z.B, in.rows_classes, in.rows_scores, in.rows_gc,
+                                         in.rows_crowd, nullptr, z.D, order, ev.tail.scores, ev.tail.classes, sort,
+                                         w.sort_bytes, nullptr, 0, nullptr, 0, nullptr, 0, 0, nullptr, stream)
+                     : api.pe_seg_sort(in.descs, z.B, in.det_scores, in.det_classes, z.D, order, ev.tail.scores,
+                                       ev.tail.classes, sort, w.sort_bytes, stream);
   if (!code)
     code = api.pe_seg_pass(in.descs, z.B, in.total_chunks, order, pairs, z.pairs, dpairs, w.dpairs_len, z.pan_cap,
                            z.det_cap, z.rows16 ? 1 : 2, nullptr, 0, reinterpret_cast<uint64_t*>(dpairs + w.dpairs_len),
@@ -1111,19 +1117,17 @@ PyObject* combined_update(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   in.gc = data<int32_t>(p.gt.classes);
   in.pc = data<int32_t>(p.pred.classes);
   in.crowd = data<uint8_t>(p.crowd);
-  int32_t* classes = at_address<int32_t>(base + classes_at);
-  double* scores = at_address<double>(base + scores_at);
-  in.det_classes = classes;
-  in.det_scores = scores;
+  if (p.sizes.D) in.rows = in.descs + p.rows_at;
+  in.det_classes = in.rows_classes = at_address<int32_t>(base + classes_at);
+  in.det_scores = in.rows_scores = at_address<double>(base + scores_at);
+  in.rows_gc = at_address<int32_t>(base + gc_at);
+  in.rows_crowd = at_address<uint8_t>(base + crowd_at);
   const cudaStream_t stream = current_stream(index);
   int32_t* error = nullptr;
   int code = 0;
   {
     ReleaseGil released;
-    if (p.sizes.D)
-      code = api.pe_inst_gather(in.descs, in.descs + p.rows_at, B, classes, scores, at_address<int32_t>(base + gc_at),
-                                at_address<uint8_t>(base + crowd_at), nullptr, stream);
-    if (!code) code = launch_seg(p.sizes, in, w, ev, base, error, stream);
+    code = launch_seg(p.sizes, in, w, ev, base, error, stream);
   }
   return finish_seg(ev, p.sizes, code, error, stream);
   END_HANDLE_TH_ERRORS

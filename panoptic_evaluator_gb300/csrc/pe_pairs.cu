@@ -14,20 +14,19 @@
 // that are present, by AND and popcount.
 //
 // The contraction (pe_contract.cu) multiplies every pair whatever it holds: its
-// time does not depend on the masks. Rows on 16-byte boundaries reach it by TMA
-// at 6.1 TB/s and stay there; rows at any byte offset move through shared memory
-// four times (4.3 TB/s), and more than 127 detections or 63 targets are read again
-// for every tile. There streaming is faster while masks are sparse (us, rectangles
-// of 1, 3, 5 and 20 % of the image; 641 x 639): 16 images of 100 x 50 masks 184,
-// 209, 247, 516 against 223 by contraction; 32 of 100 x 8: 264, 269, 293, 520
-// against 350; 6 of 300 x 100: 290, 394, 491, 1284 against 590. 32 COCO-like images:
-// 226 against 303, 5.4 TB/s. Which of the two a batch gets is decided on the device,
-// from a sample of its masks (inst_sample_kernel): both are launched, the other one
-// returns at once. The sample and the empty launch take 9 to 13 us.
+// time does not depend on the masks, rows reach it at 5.0 TB/s by TMA and staged,
+// and more than 127 detections or 63 targets are read again for every tile.
+// Streaming reads at 6.3 TB/s while masks are sparse (us, 16 images of 640 x 640
+// with 100 x 50 masks of 0.8 %: 129 against 163). With rectangles of 1, 3, 5 and
+// 20 % of 641 x 639, and one lane producing as it did (5.4 TB/s): 16 images of
+// 100 x 50 masks 184, 209, 247, 516 against 223 by contraction; 32 of 100 x 8:
+// 264, 269, 293, 520 against 350; 6 of 300 x 100: 290, 394, 491, 1284 against 590.
+// Which of the two a batch gets is decided on the device, from a sample of its
+// masks (sample_image): both are launched, the other one returns at once.
 #include "pe_bins.cuh"
 #include "pe_common.cuh"
 #include "pe_contract.cuh"
-#include "pe_desc.cuh"
+#include "pe_order.cuh"
 
 namespace pe {
 namespace {
@@ -66,24 +65,31 @@ constexpr int kZeroBlocks = 32;
 // Picoseconds of the whole device per row of a warp's 512 pixels, per row with a pixel there, and per pair of them.
 constexpr u64 kRowCost = 42, kHitCost = 280, kPairCost = 15;
 
+struct PairSample {
+  u64* costs;  // null: no estimate wanted
+  u32* inter;
+  int64_t inter_len;
+  u64* pa;
+  int64_t pa_len;
+  u64* ga;
+  int64_t ga_len;
+  unsigned long long* schedule;
+};
+
 // Estimates what streaming the image would take where the masks' content decides: costs[kSampleParts * image + part],
-// from the rows with pixels in a part's windows. The blocks behind clear the outputs and the chunk counter
-// (a memset before).
-__global__ void __launch_bounds__(kSampleThreads)
-inst_sample_kernel(const int64_t* __restrict__ descs, int64_t B, u64* __restrict__ costs, u32* __restrict__ inter,
-                   int64_t inter_len, u64* __restrict__ pa, int64_t pa_len, u64* __restrict__ ga, int64_t ga_len,
-                   unsigned long long* __restrict__ schedule) {
-  wait_for_earlier_kernels();
-  const int64_t image = blockIdx.x / kSampleParts;
-  if (image >= B) {
-    const int64_t first = (blockIdx.x - B * kSampleParts) * kSampleThreads + threadIdx.x;
+// from the rows with pixels in a part's windows. The blocks behind those of the images clear the outputs and the
+// chunk counter (a memset before).
+__device__ __forceinline__ void sample_image(const int64_t* descs, int64_t samples, int64_t block, const PairSample& a) {
+  if (block >= samples) {
+    const int64_t first = (block - samples) * kSampleThreads + threadIdx.x;
     constexpr int64_t kStep = kZeroBlocks * kSampleThreads;
-    for (int64_t i = first; i < inter_len; i += kStep) inter[i] = 0;
-    for (int64_t i = first; i < pa_len; i += kStep) pa[i] = 0;
-    for (int64_t i = first; i < ga_len; i += kStep) ga[i] = 0;
-    if (first == 0) *schedule = 0;
+    for (int64_t i = first; i < a.inter_len; i += kStep) a.inter[i] = 0;
+    for (int64_t i = first; i < a.pa_len; i += kStep) a.pa[i] = 0;
+    for (int64_t i = first; i < a.ga_len; i += kStep) a.ga[i] = 0;
+    if (first == 0 && a.schedule) *a.schedule = 0;
     return;
   }
+  const int64_t image = block / kSampleParts;
   __shared__ int present[2][kPartWindows];  // targets, detections with a pixel in the window
   if (threadIdx.x < 2 * kPartWindows) present[threadIdx.x / kPartWindows][threadIdx.x % kPartWindows] = 0;
   __syncthreads();
@@ -91,7 +97,7 @@ inst_sample_kernel(const int64_t* __restrict__ descs, int64_t B, u64* __restrict
   const int64_t pixels = d[kPixels], stride = d[kMaskStride], G = d[kG], D = d[kD];
   if (pixels > 0) {
     const int mine = threadIdx.x % kPartWindows;
-    const int64_t window = blockIdx.x % kSampleParts * kPartWindows + mine;
+    const int64_t window = block % kSampleParts * kPartWindows + mine;
     // One window in each sixteenth of the image, at changing columns.
     const int64_t x0 = pixels * (16 * window + 5 * window % 16) / (16 * kSampleWindows);
 #pragma unroll 2
@@ -116,8 +122,33 @@ inst_sample_kernel(const int64_t* __restrict__ descs, int64_t B, u64* __restrict
       const u64 g = (u64)present[0][w], dets = (u64)present[1][w];
       sum += kRowCost * (u64)(G + D * passes) + kHitCost * (g + dets * passes) + kPairCost * g * dets;
     }
-    costs[blockIdx.x] = sum * (u64)ceil_div(pixels, 512) / kSampleWindows;
+    a.costs[block] = sum * (u64)ceil_div(pixels, 512) / kSampleWindows;
   }
+}
+
+__global__ void __launch_bounds__(kSampleThreads)
+inst_sample_kernel(const int64_t* __restrict__ descs, int64_t samples, PairSample sample) {
+  wait_for_earlier_kernels();
+  sample_image(descs, samples, blockIdx.x, sample);
+}
+
+// All that comes before the masks are counted, in one launch: the first B blocks gather and sort an image's
+// metadata, the others sample and clear. As kernels of their own these took 4.7, 6.4 and 11.2 us one after another
+// for 32 images of 100 detections; together 15.6 (16 images 10.3, one 7.9 for 10.6).
+static_assert(kSampleThreads == kSortThreads, "one block size for both kinds of work");
+__global__ void __launch_bounds__(kSampleThreads)
+inst_begin_kernel(const int64_t* __restrict__ descs, int64_t B, FieldGather fields, ScoreOrder order, int64_t samples,
+                  PairSample sample) {
+  wait_for_earlier_kernels();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (blockIdx.x >= B) {
+    sample_image(descs, samples, blockIdx.x - B, sample);
+    return;
+  }
+  const int64_t* d = desc_of(descs, blockIdx.x);
+  gather_image(d, blockIdx.x, fields);
+  __syncthreads();
+  sort_image(d, order, smem_raw);
 }
 
 __global__ void __launch_bounds__(kPairThreads, 2)
@@ -331,17 +362,19 @@ using namespace pe;
 
 // How long streaming a batch may take, in picoseconds by inst_sample_kernel's estimate, to be faster than its
 // contraction; 0: contract whatever the masks hold. Image b has dets[b] detection masks, gts[b] target masks and
-// pixels[b] pixels; tma (optional) marks the images that the contraction loads by TMA; sms: the device's SMs.
-// Host side, no GPU work.
+// pixels[b] pixels; tma (optional) marks the images that the contraction loads by TMA (as fast as the others);
+// sms: the device's SMs. Host side, no GPU work.
 //
-// Times, from 640 x 640 and 641 x 639 images with 100 x 8 to 300 x 100 masks: the contraction reads the rows of
-// its tiles, with sixteen rows' worth of fixed work, at 4.75 TB/s staged and 6.6 TB/s by TMA; streaming reads the
-// targets once and the detections once per 63 targets at 5.4 TB/s, or takes the estimate if that is longer. The
-// sample and the second launch take 12 us.
-PE_API int64_t pe_stream_limit(const int64_t* dets, const int64_t* gts, const int64_t* pixels, const uint8_t* tma,
-                               int64_t B, int64_t sms) {
+// Times, from 640 x 640 and 637 x 640 images with 100 x 8 and 100 x 50 masks of 0.8 % of the image: the contraction
+// reads the rows of its tiles, with sixteen rows' worth of fixed work, at 5.6 TB/s, by TMA and staged; streaming reads
+// the targets once and the detections once per 63 targets at 6.8 TB/s, or takes the estimate if that is longer, and
+// its last chunks, the sample and the second launch take 14 us. Updates of 16 images 222 us contracted and 198
+// streamed, of 8 135 and 130 (100 x 8) or 136 and 139 (100 x 50), of 4 92 and 98, with 7 us of them for the sample
+// that no longer show (inst_begin_kernel).
+PE_API int64_t pe_stream_limit(const int64_t* dets, const int64_t* gts, const int64_t* pixels,
+                               const uint8_t* /*tma*/, int64_t B, int64_t sms) {
   PE_REQUIRE(B >= 0 && (B == 0 || (dets && gts && pixels)) && sms > 0, "invalid arguments");
-  constexpr double kStaged = 4.75, kTma = 6.6, kStreamed = 5.4, kFixed = 12e6;  // bytes per ps; ps
+  constexpr double kContracted = 5.6, kStreamed = 6.8, kFixed = 14e6;  // bytes per ps; ps
   constexpr int64_t kTileRows = 127, kTileCols = 63, kTileWork = 16;
   double contraction = 0.0, streamed = 0.0, chunks = 0.0;
   for (int64_t b = 0; b < B; ++b) {
@@ -350,14 +383,89 @@ PE_API int64_t pe_stream_limit(const int64_t* dets, const int64_t* gts, const in
     const double n = (double)std::max<int64_t>(ceil_div(gts[b], kTileCols), 1);
     const double D = (double)dets[b], G = (double)gts[b], P = (double)pixels[b];
     if (D + G == 0.0) continue;
-    contraction += (D * n + G * m + kTileWork * m * n) * P / (tma && tma[b] ? kTma : kStaged);
+    contraction += (D * n + G * m + kTileWork * m * n) * P / kContracted;
     streamed += (D * n + G) * P / kStreamed;
     chunks += std::ceil(P / kPairChunk);
   }
-  const double slots = 2.0 * (double)sms;  // chunks in flight: a last wave that is nearly empty costs a whole one
-  if (chunks > 0.0) streamed *= std::ceil(chunks / slots) * slots / chunks;
+  // Fewer chunks than CTAs leave SMs without one.
+  if (chunks > 0.0) streamed *= std::max(1.0, 2.0 * (double)sms / chunks);
   const double limit = contraction - kFixed;
   return streamed < limit ? (int64_t)std::min(limit, 9e18) : 0;
+}
+
+namespace {
+
+bool valid_sample(int64_t B, int64_t inter_len, int64_t pa_len, int64_t ga_len) {
+  return B >= 0 && B <= INT_MAX / (kSampleParts + 1) - kZeroBlocks && inter_len >= 0 && pa_len >= 0 && ga_len >= 0;
+}
+
+// `costs` and the chunk counter behind them: 8 B + 1 words.
+PairSample pair_sample(uint64_t* work, int64_t B, uint32_t* inter, int64_t inter_len, uint64_t* pa, int64_t pa_len,
+                       uint64_t* ga, int64_t ga_len) {
+  return PairSample{reinterpret_cast<u64*>(work), inter, inter_len, reinterpret_cast<u64*>(pa), pa_len,
+                    reinterpret_cast<u64*>(ga), ga_len,
+                    work ? reinterpret_cast<unsigned long long*>(work + B * kSampleParts) : nullptr};
+}
+
+// Both ways, of which one works.
+int launch_counts(const int64_t* descs, int64_t B, int64_t pair_chunks, const int64_t* blocks, int64_t n_blocks,
+                  int64_t total_chunks, const int64_t* cta_bounds, int64_t ctas, const int64_t* order, uint32_t* inter,
+                  uint64_t* pa, uint64_t* ga, const void* maps, int64_t limit, uint64_t* work, int32_t* error,
+                  cudaStream_t stream) {
+  const Choice choice{reinterpret_cast<const u64*>(work), B * kSampleParts, limit};
+  const size_t smem = sizeof(PairShared);
+  PE_CUDA(cudaFuncSetAttribute(inst_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int64_t grid = std::min(pair_chunks, (int64_t)sm_count() * 2);
+  launch_kernel(inst_pairs_kernel, (unsigned)grid, kPairThreads, smem, stream, descs, B, pair_chunks, choice,
+      reinterpret_cast<unsigned long long*>(work + B * kSampleParts), order, reinterpret_cast<u32*>(inter),
+      reinterpret_cast<u64*>(pa), reinterpret_cast<u64*>(ga), error);
+  PE_LAUNCHED("inst_pairs");
+  count_launch();
+  return launch_contract(descs, blocks, n_blocks, total_chunks, cta_bounds, ctas, order, inter, pa, ga, maps, choice,
+                         error, stream);
+}
+
+}  // namespace
+
+// pe_inst_gather and pe_seg_sort in one launch, which also clears the outputs of pe_inst_counts and, with a limit
+// above 0, samples the masks for it (work: 8 B + 1 u64 of device scratch).
+PE_API int pe_inst_begin(const int64_t* descs, const int64_t* fields, int64_t B, int32_t* pc, double* scores,
+                         int32_t* gc, uint8_t* crowd, double* areas, int64_t total_detections, int64_t* order,
+                         double* sorted_scores, int32_t* sorted_classes, void* workspace, int64_t workspace_bytes,
+                         uint32_t* inter, int64_t inter_len, uint64_t* pa, int64_t pa_len, uint64_t* ga,
+                         int64_t ga_len, int64_t limit, uint64_t* work, cudaStream_t stream) {
+  PE_REQUIRE(valid_sample(B, inter_len, pa_len, ga_len) && total_detections >= 0, "invalid batch");
+  PE_REQUIRE(workspace_bytes >= pe_seg_sort_workspace(total_detections), "sort workspace too small");
+  PE_REQUIRE(limit <= 0 || work, "a sample needs its scratch");
+  const int64_t samples = limit > 0 ? B * kSampleParts : 0;
+  const int64_t clearing = inter_len + pa_len + ga_len > 0 || samples ? kZeroBlocks : 0;
+  if (B + clearing == 0) return kOk;
+  const ScoreOrder out =
+      score_order(scores, pc, total_detections, order, sorted_scores, sorted_classes, workspace);
+  PE_CUDA(cudaFuncSetAttribute(inst_begin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sort_bytes(kOrderCap)));
+  launch_kernel(inst_begin_kernel, (unsigned)(B + samples + clearing), kSampleThreads, sort_bytes(out.cap), stream,
+      descs, B, FieldGather{fields, pc, scores, gc, crowd, areas}, out, samples,
+      pair_sample(samples ? work : nullptr, B, inter, inter_len, pa, pa_len, ga, ga_len));
+  PE_LAUNCHED("inst_begin");
+  count_launch();
+  return kOk;
+}
+
+// The counts of pe_inst_contract into outputs that pe_inst_begin cleared, streamed where its sample stays within
+// `limit` (0: contracted).
+PE_API int pe_inst_counts(const int64_t* descs, int64_t B, int64_t pair_chunks, const int64_t* blocks,
+                          int64_t n_blocks, int64_t total_chunks, const int64_t* cta_bounds, int64_t ctas,
+                          const int64_t* order, uint32_t* inter, uint64_t* pa, uint64_t* ga, const void* maps,
+                          int64_t limit, uint64_t* work, int32_t* error, cudaStream_t stream) {
+  PE_REQUIRE(B >= 0 && pair_chunks >= 0 && n_blocks >= 0 && total_chunks >= 0 && (limit <= 0 || work), "invalid batch");
+  PE_REQUIRE(n_blocks > 0 || total_chunks == 0, "chunks without blocks");
+  PE_REQUIRE((reinterpret_cast<uintptr_t>(maps) & 63) == 0, "tensor maps must be 64-byte aligned");
+  if (limit <= 0 || B == 0 || pair_chunks == 0)
+    return launch_contract(descs, blocks, n_blocks, total_chunks, cta_bounds, ctas, order, inter, pa, ga, maps,
+                           Choice{nullptr, 0, 0}, error, stream);
+  return launch_counts(descs, B, pair_chunks, blocks, n_blocks, total_chunks, cta_bounds, ctas, order, inter, pa, ga,
+                       maps, limit, work, error, stream);
 }
 
 // pe_inst_contract for a batch whose masks may be sparse: the same inputs, outputs and counts, streamed where
@@ -369,24 +477,13 @@ PE_API int pe_inst_intersect(const int64_t* descs, int64_t B, int64_t pair_chunk
                              const int64_t* order, uint32_t* inter, int64_t inter_len, uint64_t* pa, int64_t pa_len,
                              uint64_t* ga, int64_t ga_len, const void* maps, int64_t limit, uint64_t* work,
                              int32_t* error, cudaStream_t stream) {
-  PE_REQUIRE(B >= 0 && B <= INT_MAX / kSampleParts - kZeroBlocks && pair_chunks >= 0 && work, "invalid batch");
-  PE_REQUIRE(inter_len >= 0 && pa_len >= 0 && ga_len >= 0, "invalid batch");
-  u64* costs = reinterpret_cast<u64*>(work);
-  unsigned long long* schedule = reinterpret_cast<unsigned long long*>(work + B * kSampleParts);
-  launch_kernel(inst_sample_kernel, (unsigned)(B * kSampleParts + kZeroBlocks), kSampleThreads, 0, stream, descs, B,
-      costs, reinterpret_cast<u32*>(inter), inter_len, reinterpret_cast<u64*>(pa), pa_len, reinterpret_cast<u64*>(ga),
-      ga_len, schedule);
+  PE_REQUIRE(valid_sample(B, inter_len, pa_len, ga_len) && pair_chunks >= 0 && work, "invalid batch");
+  const int64_t samples = B * kSampleParts;
+  launch_kernel(inst_sample_kernel, (unsigned)(samples + kZeroBlocks), kSampleThreads, 0, stream, descs, samples,
+      pair_sample(work, B, inter, inter_len, pa, pa_len, ga, ga_len));
   PE_LAUNCHED("inst_sample");
   count_launch();
   if (B == 0 || pair_chunks == 0) return kOk;
-  const Choice choice{costs, B * kSampleParts, limit};
-  const size_t smem = sizeof(PairShared);
-  PE_CUDA(cudaFuncSetAttribute(inst_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int64_t grid = std::min(pair_chunks, (int64_t)sm_count() * 2);
-  launch_kernel(inst_pairs_kernel, (unsigned)grid, kPairThreads, smem, stream, descs, B, pair_chunks, choice, schedule,
-      order, reinterpret_cast<u32*>(inter), reinterpret_cast<u64*>(pa), reinterpret_cast<u64*>(ga), error);
-  PE_LAUNCHED("inst_pairs");
-  count_launch();
-  return launch_contract(descs, blocks, n_blocks, total_chunks, cta_bounds, ctas, order, inter, pa, ga, maps, choice,
-                         error, stream);
+  return launch_counts(descs, B, pair_chunks, blocks, n_blocks, total_chunks, cta_bounds, ctas, order, inter, pa, ga,
+                       maps, limit, work, error, stream);
 }

@@ -22,7 +22,7 @@
 #include "pe_score.cuh"
 #include "pe_bins.cuh"
 #include "pe_desc.cuh"
-#include "pe_sort.cuh"
+#include "pe_order.cuh"
 
 #include <cfloat>
 #include <map>
@@ -41,42 +41,13 @@ namespace {
 constexpr int kPassThreads = 512;
 constexpr int kPassPixels = 16;
 constexpr int kChunk = kPassThreads * kPassPixels;  // 8192 pixels
-constexpr int kSortCap = 4096;
 constexpr int kScoreThreads = 1024;  // half of them when images outnumber the SMs
 constexpr size_t kScoreSmemAlone = 200 * 1024, kScoreSmemShared = 110 * 1024;
 
-// 1. Per-image stable descending score order (NaN scores last). Latency bounds it: 32 images of 100
-// detections took 10.6 us, 8 of 256 15.8, with a bitonic network over FP64 keys; 4.5 and 8.5 now.
-constexpr int kSortThreads = 256;
-__global__ void __launch_bounds__(kSortThreads)
-seg_sort_kernel(const int64_t* __restrict__ descs, const double* __restrict__ scores, const int* __restrict__ classes,
-                int64_t* __restrict__ order, double* __restrict__ sorted_scores, int* __restrict__ sorted_classes,
-                u64* __restrict__ ws_key, int* __restrict__ ws_idx) {
+__global__ void __launch_bounds__(kSortThreads) seg_sort_kernel(const int64_t* __restrict__ descs, ScoreOrder order) {
   wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int64_t* d = desc_of(descs, blockIdx.x);
-  const int D = (int)d[kD];
-  const int64_t base = d[kDetBegin];
-  if (D == 0) return;
-  int padded = 1;
-  while (padded < D) padded <<= 1;
-  const bool in_smem = padded <= kSortCap;
-  u64* key = in_smem ? reinterpret_cast<u64*>(smem_raw) : ws_key + 2 * base;
-  int* idx = in_smem ? reinterpret_cast<int*>(smem_raw + sizeof(u64) * kSortCap) : ws_idx + 2 * base;
-  for (int i = threadIdx.x; i < D; i += blockDim.x) {
-    key[i] = score_key(scores[base + i]);
-    idx[i] = i;
-  }
-  __syncthreads();
-  if (D <= kSortThreads) rank_sort(key, idx, D);
-  else if (in_smem) bitonic_sort<false>(key, idx, D, padded);
-  else bitonic_sort<true>(key, idx, D, padded);
-  for (int r = threadIdx.x; r < D; r += blockDim.x) {
-    const int i = idx[r];
-    order[base + r] = i;
-    sorted_scores[base + r] = scores[base + i];
-    sorted_classes[base + r] = classes[base + i];
-  }
+  sort_image(desc_of(descs, blockIdx.x), order, smem_raw);
 }
 
 // Tunables of the fused pass (compile-time): masks per look-ahead group, and
@@ -643,37 +614,12 @@ inst_overlap_kernel(const int64_t* __restrict__ descs, int64_t B, const int64_t*
   }
 }
 
-// Instance prep: pixel areas to double, validation of classes/scores/areas.
-// Per-image metadata of an instance update gathered into flat arrays at each image's detection / slot
-// offsets (one launch instead of a host-side concatenation per field). fields: one row of
-// kGatherFields int64 per image: device pointers of its prediction classes, scores, target classes,
-// crowd flags and annotation areas (0: absent), then element sizes (bit 0: prediction classes int64,
-// bit 1: scores float64, bit 2: target classes int64, bit 4: areas float64; else int32 / float32).
-constexpr int kGatherFields = 6;
-
-__global__ void __launch_bounds__(128)
-inst_gather_kernel(const int64_t* __restrict__ descs, const int64_t* __restrict__ fields, int* __restrict__ pc,
-                   double* __restrict__ scores, int* __restrict__ gc, uint8_t* __restrict__ crowd,
-                   double* __restrict__ areas) {
+__global__ void __launch_bounds__(128) inst_gather_kernel(const int64_t* __restrict__ descs, FieldGather fields) {
   wait_for_earlier_kernels();
-  const int64_t* d = desc_of(descs, blockIdx.x);
-  const int64_t* f = fields + (int64_t)blockIdx.x * kGatherFields;
-  const int D = (int)d[kD], G = (int)d[kG];
-  const int64_t db = d[kDetBegin], sb = d[kSlotBegin], bits = f[5];
-  for (int i = threadIdx.x; i < D; i += blockDim.x) {
-    pc[db + i] = (bits & 1) ? (int)reinterpret_cast<const int64_t*>(f[0])[i] : reinterpret_cast<const int*>(f[0])[i];
-    scores[db + i] = (bits & 2) ? reinterpret_cast<const double*>(f[1])[i]
-                                : (double)reinterpret_cast<const float*>(f[1])[i];
-  }
-  for (int g = threadIdx.x; g < G; g += blockDim.x) {
-    gc[sb + g] = (bits & 4) ? (int)reinterpret_cast<const int64_t*>(f[2])[g] : reinterpret_cast<const int*>(f[2])[g];
-    crowd[sb + g] = f[3] ? reinterpret_cast<const uint8_t*>(f[3])[g] : 0;
-    if (areas && f[4])
-      areas[sb + g] = (bits & 16) ? reinterpret_cast<const double*>(f[4])[g]
-                                  : (double)reinterpret_cast<const float*>(f[4])[g];
-  }
+  gather_image(desc_of(descs, blockIdx.x), blockIdx.x, fields);
 }
 
+// Instance prep: pixel areas to double, validation of classes/scores/areas.
 __global__ void inst_prepare_kernel(const int64_t* __restrict__ descs, const u64* __restrict__ pa_count,
                                     const u64* __restrict__ ga_count, double* __restrict__ pa, double* __restrict__ ga,
                                     const int* __restrict__ pc, const int* __restrict__ gc,
@@ -747,13 +693,9 @@ PE_API int pe_seg_sort(const int64_t* descs, int64_t B, const double* scores, co
   PE_REQUIRE(B >= 0 && total_detections >= 0, "invalid batch");
   PE_REQUIRE(workspace_bytes >= pe_seg_sort_workspace(total_detections), "sort workspace too small");
   if (B == 0 || total_detections == 0) return kOk;
-  const int64_t entries = 2 * round_up(total_detections + 1, 64);
-  auto* ws_key = static_cast<u64*>(workspace);
-  int* ws_idx = reinterpret_cast<int*>(ws_key + entries);
-  const size_t smem = (sizeof(u64) + sizeof(int)) * kSortCap;
-  PE_CUDA(cudaFuncSetAttribute(seg_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_kernel(seg_sort_kernel, (unsigned)B, kSortThreads, smem, stream, descs, scores, classes, order, sorted_scores,
-      sorted_classes, ws_key, ws_idx);
+  const ScoreOrder out = score_order(scores, classes, total_detections, order, sorted_scores, sorted_classes, workspace);
+  PE_CUDA(cudaFuncSetAttribute(seg_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_bytes(out.cap)));
+  launch_kernel(seg_sort_kernel, (unsigned)B, kSortThreads, sort_bytes(out.cap), stream, descs, out);
   PE_LAUNCHED("seg_sort");
   count_launch();
   return kOk;
@@ -956,7 +898,8 @@ PE_API int pe_inst_gather(const int64_t* descs, const int64_t* fields, int64_t B
                           int32_t* gc, uint8_t* crowd, double* areas, cudaStream_t stream) {
   PE_REQUIRE(B >= 0 && B <= INT_MAX, "invalid batch");
   if (B == 0) return kOk;
-  launch_kernel(inst_gather_kernel, (unsigned)B, 128, 0, stream, descs, fields, pc, scores, gc, crowd, areas);
+  launch_kernel(inst_gather_kernel, (unsigned)B, 128, 0, stream, descs,
+      FieldGather{fields, pc, scores, gc, crowd, areas});
   PE_LAUNCHED("inst_gather");
   count_launch();
   return kOk;
