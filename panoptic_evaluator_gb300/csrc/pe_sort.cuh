@@ -47,20 +47,33 @@ __device__ void bitonic_sort(u64* key, int* idx, int n, int padded) {
   }
 }
 
-// Up to one record per thread: each record's place is the number of records before it, one pass over
+// Up to kEach records per thread: each record's place is the number of records before it, one pass over
 // the others instead of a barrier per stage of the network (100 records: 1 pass, against 28 barriers).
 // idx is left in order, the keys as they were. Synchronises the block.
+template <int kEach = 1>
 __device__ __forceinline__ void rank_sort(const u64* key, int* idx, int n) {
-  int place = -1, mine = 0;
+  int place[kEach], mine[kEach];
+  u64 own[kEach];
+#pragma unroll
+  for (int e = 0; e < kEach; ++e) {
+    const int i = threadIdx.x + e * blockDim.x;
+    own[e] = i < n ? key[i] : 0;
+    mine[e] = i < n ? idx[i] : 0;
+    place[e] = 0;
+  }
   if ((int)threadIdx.x < n) {
-    const u64 k = key[threadIdx.x];
-    mine = idx[threadIdx.x];
-    place = 0;
 #pragma unroll 4
-    for (int j = 0; j < n; ++j) place += before_in_order(key[j], idx[j], k, mine);
+    for (int j = 0; j < n; ++j) {
+      const u64 k = key[j];
+      const int i = idx[j];
+#pragma unroll
+      for (int e = 0; e < kEach; ++e) place[e] += before_in_order(k, i, own[e], mine[e]);
+    }
   }
   __syncthreads();
-  if (place >= 0) idx[place] = mine;
+#pragma unroll
+  for (int e = 0; e < kEach; ++e)
+    if ((int)(threadIdx.x + e * blockDim.x) < n) idx[place[e]] = mine[e];
   __syncthreads();
 }
 
