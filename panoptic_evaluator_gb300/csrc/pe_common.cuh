@@ -234,19 +234,29 @@ inline cudaLaunchAttribute early_launch() {
   return attribute;
 }
 
-// kernel<<<grid, block, smem, stream>>>(args...), launched ahead. Errors are left to PE_LAUNCHED.
+// kernel<<<grid, block, smem, stream>>>(args...), launched ahead, in clusters of cluster_y CTAs along y. Errors are
+// left to PE_LAUNCHED.
 template <typename... Params, typename... Args>
-void launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+void launch_clusters(void (*kernel)(Params...), dim3 grid, unsigned cluster_y, dim3 block, size_t smem,
+                     cudaStream_t stream, Args... args) {
   static_assert(sizeof...(Params) == sizeof...(Args), "one argument per kernel parameter");
-  cudaLaunchAttribute attribute = early_launch();
+  cudaLaunchAttribute attributes[2] = {early_launch(), {}};
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = attributes[1].val.clusterDim.z = 1;
+  attributes[1].val.clusterDim.y = cluster_y;
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
+  config.attrs = attributes;
+  config.numAttrs = cluster_y > 1 ? 2 : 1;
   cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+void launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  launch_clusters(kernel, grid, 1, block, smem, stream, args...);
 }
 
 }  // namespace pe

@@ -295,8 +295,8 @@ slot_histogram(const int* __restrict__ gt, const int* __restrict__ pred, int64_t
   if (bad && error) atomicOr(error, 1);
 }
 
-// flags: 1 = areas, 2 = validate (needs areas), 4 = accumulate, 8 = gate on *error. One CTA per image,
-// scored in one pass (pe_score.cuh); smem: dynamic shared memory of the launch.
+// flags: 1 = areas, 2 = validate (needs areas), 4 = accumulate, 8 = gate on *error. One CTA per image, or a cluster of
+// gridDim.y of them, scored in one pass (pe_score.cuh); smem: dynamic shared memory of the launch.
 template <bool REWARD>
 __global__ void __launch_bounds__(1024)
 score_blocks(const u64* __restrict__ pairs, const int* __restrict__ gc, const int* __restrict__ pc,
@@ -313,7 +313,8 @@ score_blocks(const u64* __restrict__ pairs, const int* __restrict__ gc, const in
   crowd += b * G;
   const int64_t o = REWARD ? b * C : 0;
   const ScoreTables t = ScoreTables::at(smem_raw, G, P, C, smem);
-  score_totals(pairs, t, gc, crowd, G, P, C);
+  score_totals(pairs, t, gc, crowd, G, P, C, blockIdx.y, gridDim.y);
+  if (blockIdx.y) return;
   if (flags & 1) {
     areas += b * (int64_t)(G + P);
     for (int k = threadIdx.x; k < G; k += blockDim.x) areas[k] = t.row[k];
@@ -764,9 +765,10 @@ PE_API int pe_update(const void* gt, int gt_is_int64, const void* pred, int pred
     PE_CUDA(cudaFuncSetAttribute(blocks ? reinterpret_cast<const void*>(by_blocks)
                                         : reinterpret_cast<const void*>(in_place),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const unsigned parts = G * P > kSharedScore ? score_parts(B, sm_count()) : 1;
   auto launch = [&](int flags, int* word) {
     if (blocks)
-      launch_kernel(by_blocks, (unsigned)B, score_threads, smem, stream, upairs, gc, pc, crowd, ua, matched, utp, ufp,
+      launch_clusters(by_blocks, dim3((unsigned)B, parts), parts, score_threads, smem, stream, upairs, gc, pc, crowd, ua, matched, utp, ufp,
           ufn, iou_sum, uconf, (int)G, (int)P, (int)C, flags, (int)smem, word);
     else
       launch_kernel(in_place, (unsigned)B, score_threads, smem, stream, upairs, gc, pc, crowd, ua, matched, utp, ufp,

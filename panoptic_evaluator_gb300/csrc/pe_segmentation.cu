@@ -443,6 +443,7 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
   const u32* pan = pairs + d[kPairBegin];
   const bool blocks = P > 0 && ScoreTables::base_bytes(G, P, C) <= (size_t)smem;
   const ScoreTables t = ScoreTables::at(smem_raw, G, P, C, blocks ? smem : ScoreTables::base_bytes(G, P, C));
+  const int shares = (int64_t)G * P > kSharedScore ? (int)gridDim.y : 1;  // CTAs that count the image's pairs
   const u32* det = dpairs + d[kDPairBegin];
   // Detection areas (full mask area: every slot, including void and stuff) and checks, by `parts` blocks: a warp
   // sums the rows of kAreaRows detections at once with coalesced loads, so their L2 round trips overlap.
@@ -481,7 +482,9 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
     }
     return err;
   };
-  if (blockIdx.y) {  // blocks beside the image's scoring
+  if (blockIdx.y) {  // blocks beside the image's scoring: their share of the counts, then the detections
+    if (blocks && shares > 1) score_totals(pan, t, gc + sb, crowd + sb, G, P, C, blockIdx.y, shares);
+    if (!(mode & 1)) return;
     const int err = detection_areas(blockIdx.y - 1, gridDim.y - 1);
     if (err) atomicOr(error, err);
     return;
@@ -489,7 +492,7 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
   gc += sb; crowd += sb; matched += sb;
   pc += pb;
   u64* ar = areas + sb + pb;  // per image G + P entries at offset (slot_begin + pslot_begin)
-  if (blocks) score_totals(pan, t, gc, crowd, G, P, C);
+  if (blocks) score_totals(pan, t, gc, crowd, G, P, C, 0, shares);
   if (mode & 1) {
     int err = 0;
     if (blocks) {
@@ -825,27 +828,28 @@ PE_API int pe_seg_score(const int64_t* descs, int64_t B, int64_t max_p, int64_t 
   const size_t want = score_bytes(kScoreSlots, max_p, C, max_pairs);
   const size_t smem = std::max(in_place, std::min(want, alone ? kScoreSmemAlone : kScoreSmemShared));
   const int threads = alone ? kScoreThreads : kScoreThreads / 2;
-  // SMs without an image sum detection areas meanwhile: 8 images of 257 x 277 slots and 256 detections took 41 us
-  // with them in the image's block and one list atomic per row, 32 us now.
-  const dim3 areas_grid((unsigned)B, 1 + (unsigned)std::min<int64_t>(alone ? sm_count() / B - 1 : 0, 7));
+  // SMs without an image take a share of its counts and sum its detections' areas: 8 images of 257 x 277 slots and 256
+  // detections took 41 us with both in the image's block and one list atomic per row, 21.9 now.
+  const unsigned parts = score_parts(B, sm_count());
+  const dim3 grid((unsigned)B, parts);
   if (smem > 48 * 1024)
     PE_CUDA(cudaFuncSetAttribute(seg_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   ScoreOut out{reinterpret_cast<u64*>(tp), reinterpret_cast<u64*>(fp), reinterpret_cast<u64*>(fn), iou_sum,
                reinterpret_cast<u64*>(confusion)};
   auto* ua = reinterpret_cast<u64*>(areas);
   if (validate) {
-    launch_kernel(seg_score_kernel, areas_grid, threads, smem, stream, descs, pairs, dpairs, gc, pc, crowd, ua, matched,
+    launch_clusters(seg_score_kernel, grid, parts, threads, smem, stream, descs, pairs, dpairs, gc, pc, crowd, ua, matched,
         out, (int)C, isthing, det_classes, det_scores, det_pa, slot_ga, slot_class, ann_in, ann_out, 1, 1, reward,
         (int)smem, nullptr, error);
     PE_LAUNCHED("seg_score(areas)");
-    launch_kernel(seg_score_kernel, (unsigned)B, threads, smem, stream, descs, pairs, dpairs, gc, pc, crowd, ua,
+    launch_clusters(seg_score_kernel, grid, parts, threads, smem, stream, descs, pairs, dpairs, gc, pc, crowd, ua,
         matched, out, (int)C, isthing, det_classes, det_scores, det_pa, slot_ga, slot_class, ann_in, ann_out, 2 | 4, 1,
         reward, (int)smem, bits, error);
     PE_LAUNCHED("seg_score(accumulate)");
     count_launch(2);
     return kOk;
   }
-  launch_kernel(seg_score_kernel, areas_grid, threads, smem, stream, descs, pairs, dpairs, gc, pc, crowd, ua, matched,
+  launch_clusters(seg_score_kernel, grid, parts, threads, smem, stream, descs, pairs, dpairs, gc, pc, crowd, ua, matched,
       out, (int)C, isthing, det_classes, det_scores, det_pa, slot_ga, slot_class, ann_in, ann_out, 1 | 2, 0, reward,
       (int)smem, bits, error);
   PE_LAUNCHED("seg_score");

@@ -152,3 +152,25 @@ def test_the_last_halves_of_the_pass_in_parts(dets):
     joint = pe.SegmentationEvaluator(133, isthing=isthing)
     joint.update_images(SegmentationImages(*([getattr(i, f) for i in batch] for f in fields)))
     assert_tree(joint.compute(), oracle.compute())
+
+
+@pytest.mark.parametrize("shape", [
+    (1, 150, 150, 150, 120, 20, 0.6),   # eight CTAs an image, a list that overflows
+    (3, 127, 129, 6000, 3, 7, 0.9),     # hardly any columns
+    (2, 64, 129, 3, 6000, 5, 0.9),      # fewer rows than CTAs: row 0 with the first
+    (2, 64, 65, 5, 4000, 5, 0.9),
+    (20, 61, 67, 140, 130, 33, 0.9),    # four CTAs an image
+    (60, 41, 43, 135, 145, 15, 0.9),    # two
+    (90, 41, 43, 135, 145, 15, 0.9),    # more images than pairs of SMs
+])
+def test_counts_shared_by_a_cluster(shape):
+    import panoptic_evaluator_gb300 as pe
+    C = shape[5]
+    gt, gc, crowd, pred, pc = _arrays(13, *shape, consistent=False)
+    isthing = np.arange(C) < (C + 1) // 2
+    oracle = opan.PanopticOracle(C, isthing, validate=False)
+    oracle.update(pred, pc, gt, gc, crowd)
+    ev = pe.PanopticEvaluator(C, isthing=isthing, validate=False)
+    dev = lambda x: torch.from_numpy(x).cuda()  # noqa: E731
+    ev.update(pe.PanopticBatch(dev(pred), dev(pc)), pe.PanopticBatch(dev(gt), dev(gc), dev(crowd)))
+    assert_tree(ev.compute(), oracle.compute())
