@@ -8,7 +8,7 @@
 // (area range x IoU threshold) chain and walks the detections through their
 // candidate lists.
 //
-// Accumulation runs kAccParts CTAs per class, each with two of the ten IoU
+// Accumulation runs five or ten CTAs per class, each with two or one of the ten IoU
 // thresholds: it gathers the class's records, sorts them by descending score,
 // and one warp at a time builds a (threshold, area, maxDets) chain's precision
 // envelope with integer comparisons only.
@@ -401,9 +401,9 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
 constexpr int kAccThreads = 256;
 constexpr int kSortCap = 1024;  // records of one class sorted and staged in shared memory, at most
 constexpr int kSmallCap = 512;  // classes up to this many records: a smaller stage, more CTAs per SM
-constexpr int kAccT = 2;        // IoU thresholds of one CTA
-constexpr int kAccParts = 10 / kAccT;
-constexpr int kAccChains = 12 * kAccT;  // (threshold, area, maxDets) chains of one CTA
+// IoU thresholds of one CTA: two, or one while that leaves SMs without a CTA. A CTA has twelve (threshold, area,
+// maxDets) chains of each.
+constexpr int kAccT = 2;
 // Records up to which every CTA scans the class array itself; above, three kernels group the records by
 // class first (at 3200 records and 80 classes they and their memset took 8 us of the stream).
 constexpr int64_t kScanRecords = 8192;
@@ -484,7 +484,7 @@ __device__ __forceinline__ int64_t recall_reached_at(int64_t np, int r) {
   return t + (t * 100 == scaled && !exact_ok ? 1 : 0);
 }
 
-// kAccParts CTAs per class. `scores` == nullptr means the records are already in
+// 10 / kT CTAs per class. `scores` == nullptr means the records are already in
 // global descending-score order. Records: classes[n], ranks[n] and flags at
 // flags[chain * chain_stride + record * det_stride]; list / cursor / hist: the
 // records grouped by class, or list == nullptr and every CTA scans `classes`.
@@ -508,38 +508,42 @@ __device__ __forceinline__ int64_t recall_reached_at(int64_t np, int r) {
 // summaries. 3200 records of 80 classes: 17.9 us (43.2, after 8 us of grouping
 // kernels, with all 120 chains walked by four CTAs and FP64 recall thresholds);
 // 100 records 10.5 (26.9).
-template <int kCap>
+template <int kCap, int kT>
 struct AccShared {
+  static constexpr int kChainsHere = 12 * kT;
   unsigned long long key[kCap];
   int idx[kCap];
   int rank[kCap];
-  int8_t flags[kCap][4 * kAccT];  // the staged records' flags of this CTA's thresholds, [t][area]
-  long long seg[kAccChains][101];   // packed (tp, fp) of a segment, then its value
-  unsigned char seg_lo[kAccChains][101 + 3];
+  int8_t flags[kCap][4 * kT];  // the staged records' flags of this CTA's thresholds, [t][area]
+  long long seg[kChainsHere][101];   // packed (tp, fp) of a segment, then its value
+  unsigned char seg_lo[kChainsHere][101 + 3];
   unsigned short env[kAccThreads / 32][2][kCap + 1];
   int tp_min[4][101];
-  int nseg[kAccChains], hi[kAccChains], tp[kAccChains], off[kAccChains + 1];
+  int nseg[kChainsHere], hi[kChainsHere], tp[kChainsHere], off[kChainsHere + 1];
   int64_t npos[4];
   int count, before;
 };
 
-template <int kCap>
+template <int kCap, int kT>
 __global__ void __launch_bounds__(kAccThreads)
 accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restrict__ list,
-                  const int* __restrict__ cursor, const int* __restrict__ hist, const int* __restrict__ ranks,
+                  const int* __restrict__ cursor, int* __restrict__ hist, const int* __restrict__ ranks,
                   const int8_t* __restrict__ flags, int64_t chain_stride, int64_t det_stride,
                   const double* __restrict__ scores, const int64_t* __restrict__ positives,
                   unsigned long long* __restrict__ ws_key, int* __restrict__ ws_idx,
                   int C, int* __restrict__ env_ws, double* __restrict__ precision,
                   double* __restrict__ recall, double* __restrict__ chain_stats, int above) {
   wait_for_earlier_kernels();
+  constexpr int kParts = 10 / kT, kChainsHere = 12 * kT;
   // The bitonic sort pads a class's records to the next power of two inside the kCap-entry stage.
   static_assert(kCap > 0 && (kCap & (kCap - 1)) == 0, "a stage cap must be a power of two");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  AccShared<kCap>& sm = *reinterpret_cast<AccShared<kCap>*>(smem_raw);
-  const int c = blockIdx.x / kAccParts, part = blockIdx.x % kAccParts;
+  AccShared<kCap, kT>& sm = *reinterpret_cast<AccShared<kCap, kT>*>(smem_raw);
+  const int c = blockIdx.x / kParts, part = blockIdx.x % kParts;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = kAccThreads / 32;
   const unsigned below = (1u << lane) - 1u;
+  // The second launch reads the count that the first one found: usually it has nothing to do (5.3 -> 3.0 us).
+  if (above >= 0 && hist[c] <= above) return;
   if (threadIdx.x < 4) sm.npos[threadIdx.x] = positives[c * 4 + threadIdx.x];
   // Records of this class, and of the classes before it (where its workspace regions start).
   int count, before;
@@ -567,11 +571,12 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
     __syncthreads();
     count = sm.count;
     before = sm.before;
+    if (above < 0 && part == 0 && threadIdx.x == 0) hist[c] = count;
   }
   // Classes of up to kCap records (more than `above`) are this launch's: the other launch takes the rest.
   if (count <= above || (kCap < kSortCap && count > kCap)) return;
   const bool staged = count <= kCap;
-  const int parts = staged ? kAccParts : 1;
+  const int parts = staged ? kParts : 1;
   if (part >= parts) return;
   int padded = 1;
   while (padded < max(count, 1)) padded <<= 1;
@@ -619,18 +624,18 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
     const int64_t lhs = (int64_t)ct * ((int64_t)bt + bf), rhs = (int64_t)bt * ((int64_t)ct + cf);
     return lhs > rhs || (lhs == rhs && bt + bf == 1 && ct + cf >= 2);
   };
-  for (int group = part; group < kAccParts; group += parts) {
-    const int t_base = group * kAccT;
+  for (int group = part; group < kParts; group += parts) {
+    const int t_base = group * kT;
     if (staged) {  // ranks and this group's flags of every record, in walk order
       for (int k = threadIdx.x; k < count; k += kAccThreads) sm.rank[k] = ranks[idx[k]];
-      for (int e = threadIdx.x; e < count * 4 * kAccT; e += kAccThreads) {
-        const int k = e / (4 * kAccT), f = e % (4 * kAccT), a = f % 4, t = f / 4;
+      for (int e = threadIdx.x; e < count * 4 * kT; e += kAccThreads) {
+        const int k = e / (4 * kT), f = e % (4 * kT), a = f % 4, t = f / 4;
         sm.flags[k][f] = flags[(a * 10 + t_base + t) * chain_stride + (int64_t)idx[k] * det_stride];
       }
       __syncthreads();
     }
     // Phase A (integers only): one warp per chain builds the chain's envelope segments.
-    for (int ch = warp; ch < kAccChains; ch += warps) {
+    for (int ch = warp; ch < kChainsHere; ch += warps) {
       const int m = ch % 3, a = (ch / 3) % 4, t = ch / 12;
       int nseg = 0, hi = 0;
       unsigned tp = 0;
@@ -713,21 +718,21 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
     }
     __syncthreads();
     if (warp == 0) {  // segment offsets (exclusive scan over the chains)
-      static_assert(kAccChains <= 32, "one lane per chain");
-      const int v0 = lane < kAccChains ? sm.nseg[lane] : 0;
+      static_assert(kChainsHere <= 32, "one lane per chain");
+      const int v0 = lane < kChainsHere ? sm.nseg[lane] : 0;
       int v = v0;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
         const int u = __shfl_up_sync(0xffffffffu, v, off);
         if (lane >= off) v += u;
       }
-      if (lane < kAccChains) sm.off[lane] = v - v0;
-      if (lane == 31) sm.off[kAccChains] = v;
+      if (lane < kChainsHere) sm.off[lane] = v - v0;
+      if (lane == 31) sm.off[kChainsHere] = v;
     }
     __syncthreads();
     // Phase B: every segment's value, fl(tp / ((tp + fp) + eps)), the segments spread over all threads.
-    for (int e = threadIdx.x; e < sm.off[kAccChains]; e += kAccThreads) {
-      int lo = 0, hi = kAccChains - 1;  // chain holding flat segment e
+    for (int e = threadIdx.x; e < sm.off[kChainsHere]; e += kAccThreads) {
+      int lo = 0, hi = kChainsHere - 1;  // chain holding flat segment e
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (sm.off[mid] <= e) lo = mid; else hi = mid - 1;
@@ -741,7 +746,7 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
     // Phase C: precision values (segment s covers [lo_s, lo_{s+1}), the last up to hi), twelve chains of a
     // (threshold, recall) next to one another; the last warp writes recalls and the chains' sums.
     if (warp == warps - 1) {
-      if (lane < kAccChains) {
+      if (lane < kChainsHere) {
         const int a = (lane / 3) % 4, t = t_base + lane / 12;
         const int64_t np = sm.npos[a];
         const double rc = np ? (double)sm.tp[lane] / (double)np : -1.0;
@@ -759,7 +764,7 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
         }
       }
     } else {
-      for (int e = threadIdx.x; e < kAccChains * 101; e += kAccThreads - 32) {
+      for (int e = threadIdx.x; e < kChainsHere * 101; e += kAccThreads - 32) {
         const int k = e % 12, r = (e / 12) % 101, t = e / (12 * 101), ch = t * 12 + k;
         double v = sm.npos[k / 3] ? 0.0 : -1.0;
         if (r < sm.hi[ch]) {
@@ -773,7 +778,7 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
         precision[(((int64_t)(t_base + t) * 101 + r) * C + c) * 12 + k] = v;
       }
     }
-    if (group + parts < kAccParts) __syncthreads();  // the next group rewrites the tables
+    if (group + parts < kParts) __syncthreads();  // the next group rewrites the tables
   }
 }
 
@@ -1097,16 +1102,16 @@ int64_t accumulate_workspace_bytes(int64_t n, int64_t C) {
          2 * (kAccThreads / 32) * (n + C) * (int64_t)sizeof(int);
 }
 
-template <int kCap>
-int launch_accumulate_cap(const int* classes, int64_t n, const int* list, const int* cursor, const int* hist,
+template <int kCap, int kT>
+int launch_accumulate_cap(const int* classes, int64_t n, const int* list, const int* cursor, int* hist,
                           const int* ranks, const int8_t* flags, int64_t chain_stride, int64_t det_stride,
                           const double* scores, const int64_t* positives, unsigned long long* ws_key, int* ws_idx,
                           int C, int* env_ws, double* precision, double* recall, double* chain_stats, int above,
                           cudaStream_t stream) {
-  auto kernel = accumulate_kernel<kCap>;
-  const size_t smem = sizeof(AccShared<kCap>);
+  auto kernel = accumulate_kernel<kCap, kT>;
+  const size_t smem = sizeof(AccShared<kCap, kT>);
   PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_kernel(kernel, (unsigned)(C * kAccParts), kAccThreads, smem, stream, classes, n, list, cursor, hist, ranks,
+  launch_kernel(kernel, (unsigned)(C * (10 / kT)), kAccThreads, smem, stream, classes, n, list, cursor, hist, ranks,
       flags, chain_stride, det_stride, scores, positives, ws_key, ws_idx, C, env_ws, precision, recall, chain_stats,
       above);
   PE_LAUNCHED("accumulate");
@@ -1144,13 +1149,14 @@ int launch_accumulate(const int* classes, const int* ranks, const int8_t* flags,
   }
   // Classes of up to kSmallCap records in a smaller stage; when some class can be larger, a second launch
   // takes those (staged up to kSortCap, else in the workspace).
-  int status = launch_accumulate_cap<kSmallCap>(classes, n, list, cursor, hist, ranks, flags, chain_stride, det_stride,
-                                                scores, positives, ws_key, ws_idx, C, env_ws, precision, recall,
-                                                chain_stats, -1, stream);
+  const bool few = C * (10 / kAccT) <= sm_count();  // 15 classes of 230 records: 23.4 us, 20.1 with a threshold per CTA
+  auto small = few ? launch_accumulate_cap<kSmallCap, 1> : launch_accumulate_cap<kSmallCap, kAccT>;
+  auto large = few ? launch_accumulate_cap<kSortCap, 1> : launch_accumulate_cap<kSortCap, kAccT>;
+  int status = small(classes, n, list, cursor, hist, ranks, flags, chain_stride, det_stride, scores, positives, ws_key,
+                     ws_idx, C, env_ws, precision, recall, chain_stats, -1, stream);
   if (status == kOk && n > kSmallCap)
-    status = launch_accumulate_cap<kSortCap>(classes, n, list, cursor, hist, ranks, flags, chain_stride, det_stride,
-                                             scores, positives, ws_key, ws_idx, C, env_ws, precision, recall,
-                                             chain_stats, kSmallCap, stream);
+    status = large(classes, n, list, cursor, hist, ranks, flags, chain_stride, det_stride, scores, positives, ws_key,
+                   ws_idx, C, env_ws, precision, recall, chain_stats, kSmallCap, stream);
   if (status != kOk) return status;
   if (summary) {
     launch_kernel(summarize_chains_kernel, 12, kSummarizeThreads, 0, stream, chain_stats, C, summary);
