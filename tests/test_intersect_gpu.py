@@ -85,3 +85,16 @@ def test_the_masks_decide(density, streamed, monkeypatch):
     for other in (-1, 2**62):
         for x, y in zip(chosen, _count(pm, gm, other, monkeypatch)):
             assert all(torch.equal(i, j) for i, j in zip(x, y))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pixels", [(700, 500), (1117, 1201)])
+@pytest.mark.parametrize("dets, gts", [(0, 3), (1, 1), (16, 2), (17, 64), (130, 5)])
+def test_the_last_chunks_in_parts(pixels, dets, gts, monkeypatch):
+    """Fewer chunks of 4096 pixels than two CTAs per SM, and a few more: parts of 16 detections and more."""
+    generator = torch.Generator("cuda").manual_seed(dets)
+    pm, gm = [_masks(dets, *pixels, 0.01, generator)], [_masks(gts, *pixels, 0.01, generator)]
+    (inter, pa, ga), = _count(pm, gm, 2**62, monkeypatch)
+    a, b = pm[0].flatten(1).double(), gm[0].flatten(1).double()
+    assert torch.equal(inter, (a @ b.T).long())
+    assert torch.equal(pa, a.sum(1).long()) and torch.equal(ga, b.sum(1).long())
