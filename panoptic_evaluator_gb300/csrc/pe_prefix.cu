@@ -938,7 +938,7 @@ PE_API int pe_prefix(const int64_t* descs, int64_t B, int64_t total_chunks, int6
     PE_REQUIRE(!total_rows || in_place <= 200 * 1024, "prefix histogram too large for scoring (G=%lld, N+1=%lld)",
                (long long)max_g, (long long)max_p);
     const size_t state = prefix_match_bytes(max_p - 1, max_g, T, C) + 8;
-    PE_REQUIRE(state <= 200 * 1024, "prefix matching state too large (G=%lld, T=%lld, C=%lld)", (long long)max_g,
+    PE_REQUIRE(state <= 201 * 1024, "prefix matching state too large (G=%lld, T=%lld, C=%lld)", (long long)max_g,
                (long long)T, (long long)C);
     // Two CTAs per SM, where the tables of a row and the IoUs of a CTA's classes have use for less.
     const size_t row = label_bytes(max_p) + score_bytes(max_g, max_p, C, max_g * max_p);
