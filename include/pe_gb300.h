@@ -299,13 +299,21 @@ int pe_inst_intersect(const int64_t* descs, int64_t B, int64_t pair_chunks, cons
  * pe_seg_sort of what it gathered; clears inter, pa and ga and, with limit > 0
  * (pe_stream_limit), samples the masks into work (8 B + 1 u64, device scratch).
  * pe_inst_counts: pe_inst_contract's counts into the cleared outputs, streamed
- * where the sample stays within limit.
+ * where the sample stays within limit. class_bits (optional): as of
+ * pe_inst_prepare. pe_inst_match: pe_seg_match from the pixel counts, where
+ * nothing is to be checked; areas (optional): annotation areas, else the
+ * targets' pixels.
  */
 int pe_inst_begin(const int64_t* descs, const int64_t* fields, int64_t B, int32_t* pc, double* scores, int32_t* gc,
                   uint8_t* crowd, double* areas, int64_t total_detections, int64_t* order, double* sorted_scores,
                   int32_t* sorted_classes, void* workspace, int64_t workspace_bytes, uint32_t* inter,
                   int64_t inter_len, uint64_t* pa, int64_t pa_len, uint64_t* ga, int64_t ga_len, int64_t limit,
-                  uint64_t* work, cudaStream_t stream);
+                  uint64_t* work, int64_t C, uint32_t* class_bits, cudaStream_t stream);
+int pe_inst_match(const uint32_t* pairs, const int64_t* pair_off, const int64_t* d_off, const int64_t* g_off, int64_t B,
+                  const int32_t* pc, const uint64_t* pa, const int32_t* gc, const uint64_t* ga, const uint8_t* crowd,
+                  const double* areas, int64_t C, int64_t g_max, int8_t* flags, int64_t chain_stride,
+                  int64_t det_stride, int32_t* ranks, int64_t* counts, const int32_t* gate, const uint32_t* class_bits,
+                  cudaStream_t stream);
 int pe_inst_counts(const int64_t* descs, int64_t B, int64_t pair_chunks, const int64_t* blocks, int64_t n_blocks,
                    int64_t total_chunks, const int64_t* cta_bounds, int64_t ctas, const int64_t* order, uint32_t* inter,
                    uint64_t* pa, uint64_t* ga, const void* maps, int64_t limit, uint64_t* work, int32_t* error,

@@ -53,7 +53,8 @@ SIGNATURES = {
     "pe_pack_rgb": [P, I64, I64, P, P, I64, P, P, P],
     "pe_inst_contract": [P, P, I64, I64, P, I64, P, P, I64, P, I64, P, I64, P, P, P],
     "pe_inst_intersect": [P, I64, I64, P, I64, I64, P, I64, P, P, I64, P, I64, P, I64, P, I64, P, P, P],
-    "pe_inst_begin": [P, P, I64, P, P, P, P, P, I64, P, P, P, P, I64, P, I64, P, I64, P, I64, I64, P, P],
+    "pe_inst_begin": [P, P, I64, P, P, P, P, P, I64, P, P, P, P, I64, P, I64, P, I64, P, I64, I64, P, I64, P, P],
+    "pe_inst_match": [P, P, P, P, I64, P, P, P, P, P, P, I64, I64, P, I64, I64, P, P, P, P, P],
     "pe_inst_counts": [P, I64, I64, P, I64, I64, P, I64, P, P, P, P, P, I64, P, P, P],
     "pe_stream_limit": [P, P, P, P, I64, I64],
     "pe_contract_maps": [P, I64, P],

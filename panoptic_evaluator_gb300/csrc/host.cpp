@@ -39,7 +39,7 @@ using namespace pe;
 #define PE_HOST_API(X)                                                                              \
   X(pe_update) X(pe_zero) X(pe_compute) X(pe_reward_pq) X(pe_pack) X(pe_pack_rgb) X(pe_contract_maps)          \
   X(pe_contract_blocks) X(pe_inst_begin) X(pe_seg_sort) X(pe_seg_sort_workspace)                   \
-  X(pe_inst_counts) X(pe_stream_limit) X(pe_inst_prepare) X(pe_seg_match) X(pe_instance_accumulate)                  \
+  X(pe_inst_counts) X(pe_inst_match) X(pe_stream_limit) X(pe_inst_prepare) X(pe_seg_match) X(pe_instance_accumulate)                  \
   X(pe_instance_accumulate_workspace) X(pe_seg_pass) X(pe_seg_score) X(pe_prefix)
 
 struct Api {
@@ -801,20 +801,25 @@ PyObject* instance_update(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     uint64_t* sample = at_address<uint64_t>(base + stream_at);
     code = api.pe_inst_begin(descs, descs + p.rows_at, B, pc, scores, gc, crowd, ann_in, D, order, tail.scores,
                              tail.classes, at_address<void>(base + sort_at), sort_bytes, inter, inter_len, pa, D,
-                             pa + D, G, p.stream_limit, sample, stream);
+                             pa + D, G, p.stream_limit, sample, *C, check ? nullptr : bits, stream);
     const int64_t* blocks = p.total_chunks ? descs + p.blocks_at : nullptr;
     const int64_t* bounds = p.total_chunks ? descs + p.bounds_at : nullptr;
     const int64_t* maps = p.maps_at >= 0 && p.total_chunks ? descs + p.maps_at : nullptr;
     if (!code)
       code = api.pe_inst_counts(descs, B, p.chunks, blocks, p.n_blocks, p.total_chunks, bounds, p.ranges, order, inter,
                                 pa, pa + D, maps, p.stream_limit, sample, error, stream);
-    if (!code)
+    if (!code && check) {
       code = api.pe_inst_prepare(descs, B, pa, pa + D, pa_d, ga_d, tail.classes, gc, tail.scores, ann_in, ann, *C, check,
                                  bits, error, stream);
-    if (!code)
-      code = api.pe_seg_match(inter, d_off + 2 * B + 2, d_off, d_off + B + 1, B, tail.classes, pa_d, gc, ga_d, crowd,
-                              ann, *C, p.max_g, tail.flags, 1, kChains, tail.ranks, data<int64_t>(*counts), error, bits,
-                              stream);
+      if (!code)
+        code = api.pe_seg_match(inter, d_off + 2 * B + 2, d_off, d_off + B + 1, B, tail.classes, pa_d, gc, ga_d, crowd,
+                                ann, *C, p.max_g, tail.flags, 1, kChains, tail.ranks, data<int64_t>(*counts), error,
+                                bits, stream);
+    } else if (!code) {
+      code = api.pe_inst_match(inter, d_off + 2 * B + 2, d_off, d_off + B + 1, B, tail.classes, pa, gc, pa + D, crowd,
+                               ann_in, *C, p.max_g, tail.flags, 1, kChains, tail.ranks, data<int64_t>(*counts), error,
+                               bits, stream);
+    }
   }
   if (!code && check) code = read_error(error, stream);
   if (!code && !store_count(store.p, tail.n + D)) return nullptr;
@@ -989,7 +994,7 @@ int launch_seg(const SegSizes& z, const SegInputs& in, const SegScratch& w, SegE
   void* sort = at_address<void>(base + w.sort);
   int code = in.rows ? api.pe_inst_begin(in.descs, in.rows, z.B, in.rows_classes, in.rows_scores, in.rows_gc,
                                          in.rows_crowd, nullptr, z.D, order, ev.tail.scores, ev.tail.classes, sort,
-                                         w.sort_bytes, nullptr, 0, nullptr, 0, nullptr, 0, 0, nullptr, stream)
+                                         w.sort_bytes, nullptr, 0, nullptr, 0, nullptr, 0, 0, nullptr, 0, nullptr, stream)
                      : api.pe_seg_sort(in.descs, z.B, in.det_scores, in.det_classes, z.D, order, ev.tail.scores,
                                        ev.tail.classes, sort, w.sort_bytes, stream);
   if (!code)

@@ -100,12 +100,13 @@ __device__ __forceinline__ int nth_present_class(const u32* __restrict__ row, in
 // it has lanes for their targets, eight warps list, and a chain's records and
 // first entries are read ahead of it: 16 images on a canvas 24.0 -> 14.1 us, 32
 // COCO-like ones 21.9 -> 17.7, 8 of 256 detections 31.4 -> 25.6.
-template <typename Count>
+// Area: double, or the pixel counts themselves; areas == nullptr: the targets' own.
+template <typename Count, typename Area>
 __global__ void __launch_bounds__(kMatchThreads)
 match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_off,
              const int64_t* __restrict__ d_off, const int64_t* __restrict__ g_off, int single_d, int single_g,
-             const int* __restrict__ pc, const double* __restrict__ pa,
-             const int* __restrict__ gc, const double* __restrict__ ga, const uint8_t* __restrict__ crowd,
+             const int* __restrict__ pc, const Area* __restrict__ pa,
+             const int* __restrict__ gc, const Area* __restrict__ ga, const uint8_t* __restrict__ crowd,
              const double* __restrict__ areas, int C, int g_max, FlagLayout flags, int* __restrict__ ranks,
              int64_t* __restrict__ counts, const int* __restrict__ gate,
              const u32* __restrict__ class_bits) {
@@ -126,7 +127,8 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
   const int G = g_off ? (int)(g_off[b + 1] - g0) : single_g;
   const Count* P = pairs + (pair_off ? pair_off[b] : 0);
   pc += d0; pa += d0; ranks += d0;
-  gc += g0; ga += g0; crowd += g0; areas += g0;
+  gc += g0; ga += g0; crowd += g0;
+  if (areas) areas += g0;
   int8_t* fbase = flags.base + d0 * flags.det_stride;
   const int words = (g_max + 31) / 32, capacity = match_entries(g_max);
   // IoUs as IEEE bit patterns: for non-negative doubles the int64 order is the
@@ -193,7 +195,7 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
         u32 bits = 0;
         if (sel) {
           const bool cr = crowd[g] != 0;
-          const double area = areas[g];
+          const double area = areas ? areas[g] : (double)ga[g];
 #pragma unroll
           for (int a = 0; a < 4; ++a) {
             double lo, hi;
@@ -223,7 +225,7 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
   const int nd = s_nd, ng = s_ng;
   if (nd == 0) return;
   for (int i = threadIdx.x; i < nd; i += blockDim.x) {
-    const double dpa = pa[recs[i].det];
+    const double dpa = (double)pa[recs[i].det];
     u32 bits = 0;
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
@@ -238,7 +240,7 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
   const long long lowest = __double_as_longlong(0.5);
   auto iou_between = [&](int d, int j) -> long long {
     const int g = gts[j];
-    const double inter = (double)P[(int64_t)d * G + g], pa_d = pa[d], ga_g = ga[g];
+    const double inter = (double)P[(int64_t)d * G + g], pa_d = (double)pa[d], ga_g = (double)ga[g];
     if (!(inter > 0.0)) return -1;
     const double uni = fmax((target_bits[j] & 16) ? pa_d : (pa_d + ga_g) - inter, 1.0);
     if (inter * 2.001 < uni) return -1;  // clearly under the lowest threshold: no division
@@ -1051,9 +1053,10 @@ int alignment_of(const void* p, int64_t pixels) {
 
 }  // namespace
 
-int launch_match(const void* pairs, bool pairs_u32, const int64_t* pair_off, const int64_t* d_off,
-                 const int64_t* g_off, int single_d, int single_g, int64_t B, const int* pc, const double* pa,
-                 const int* gc, const double* ga, const uint8_t* crowd, const double* areas, int C, int g_max,
+template <typename Count, typename Area>
+int launch_match(const Count* pairs, const int64_t* pair_off, const int64_t* d_off,
+                 const int64_t* g_off, int single_d, int single_g, int64_t B, const int* pc, const Area* pa,
+                 const int* gc, const Area* ga, const uint8_t* crowd, const double* areas, int C, int g_max,
                  int8_t* flags, int64_t chain_stride, int64_t det_stride, int* ranks, int64_t* counts,
                  cudaStream_t stream, const int* gate = nullptr, const uint32_t* class_bits = nullptr) {
   if (B == 0) return kOk;
@@ -1069,30 +1072,29 @@ int launch_match(const void* pairs, bool pairs_u32, const int64_t* pair_off, con
   // Many CTAs are bounded by how many an SM holds at a time (64 images of 133 classes: 30 us with 256 threads, 18.7
   // with 128), few by the longest class (32 images of 80: 17.7 us, 21.8 with 128 threads).
   const unsigned threads = B * C > 4096 ? kMatchThreads / 2 : kMatchThreads;
-  if (pairs_u32) {
-    auto kernel = match_kernel<u32>;
-    if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_kernel(kernel, grid, threads, smem, stream, static_cast<const u32*>(pairs), pair_off, d_off, g_off,
-        single_d, single_g, pc, pa, gc, ga, crowd, areas, C, g_max, layout, ranks, counts, gate, class_bits);
-  } else {
-    auto kernel = match_kernel<int64_t>;
-    if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_kernel(kernel, grid, threads, smem, stream, static_cast<const int64_t*>(pairs), pair_off, d_off, g_off,
-        single_d, single_g, pc, pa, gc, ga, crowd, areas, C, g_max, layout, ranks, counts, gate, class_bits);
-  }
+  auto kernel = match_kernel<Count, Area>;
+  if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  launch_kernel(kernel, grid, threads, smem, stream, pairs, pair_off, d_off, g_off, single_d, single_g, pc, pa, gc, ga,
+      crowd, areas, C, g_max, layout, ranks, counts, gate, class_bits);
   PE_LAUNCHED("match");
   count_launch();
   return kOk;
 }
 
-int launch_match_gated(const void* pairs, bool pairs_u32, const int64_t* pair_off, const int64_t* d_off,
-                       const int64_t* g_off, int64_t B, const int* pc, const double* pa, const int* gc,
-                       const double* ga, const uint8_t* crowd, const double* areas, int C, int g_max, int8_t* flags,
-                       int64_t chain_stride, int64_t det_stride, int* ranks, int64_t* counts, const int* gate,
-                       const uint32_t* class_bits, cudaStream_t stream) {
-  return launch_match(pairs, pairs_u32, pair_off, d_off, g_off, 0, 0, B, pc, pa, gc, ga, crowd, areas, C, g_max,
-                      flags, chain_stride, det_stride, ranks, counts, stream, gate, class_bits);
+template <typename Area>
+int launch_match_gated(const u32* pairs, const int64_t* pair_off, const int64_t* d_off, const int64_t* g_off,
+                       int64_t B, const int* pc, const Area* pa, const int* gc, const Area* ga, const uint8_t* crowd,
+                       const double* areas, int C, int g_max, int8_t* flags, int64_t chain_stride, int64_t det_stride,
+                       int* ranks, int64_t* counts, const int* gate, const uint32_t* class_bits, cudaStream_t stream) {
+  return launch_match(pairs, pair_off, d_off, g_off, 0, 0, B, pc, pa, gc, ga, crowd, areas, C, g_max, flags,
+                      chain_stride, det_stride, ranks, counts, stream, gate, class_bits);
 }
+template int launch_match_gated(const u32*, const int64_t*, const int64_t*, const int64_t*, int64_t, const int*,
+                                const double*, const int*, const double*, const uint8_t*, const double*, int, int,
+                                int8_t*, int64_t, int64_t, int*, int64_t*, const int*, const uint32_t*, cudaStream_t);
+template int launch_match_gated(const u32*, const int64_t*, const int64_t*, const int64_t*, int64_t, const int*,
+                                const u64*, const int*, const u64*, const uint8_t*, const double*, int, int, int8_t*,
+                                int64_t, int64_t, int*, int64_t*, const int*, const uint32_t*, cudaStream_t);
 
 int64_t accumulate_workspace_bytes(int64_t n, int64_t C) {
   // Per-class overflow regions (each class's padded to a power of two, at most twice its records: 2n
@@ -1222,7 +1224,7 @@ PE_API int pe_instance_match(const int64_t* pairs, int64_t D, int64_t G, const i
   const int zeroed = zero_spans({{counts, 32 * C}}, stream);
   if (zeroed != kOk) return zeroed;
   if (D == 0 && G == 0) return kOk;
-  return launch_match(pairs, false, nullptr, nullptr, nullptr, (int)D, (int)G, 1, pc, pa, gc, ga, crowd, areas,
+  return launch_match(pairs, nullptr, nullptr, nullptr, (int)D, (int)G, 1, pc, pa, gc, ga, crowd, areas,
                       (int)C, (int)std::max<int64_t>(G, 1), flags, D, 1, ranks, counts, stream);
 }
 

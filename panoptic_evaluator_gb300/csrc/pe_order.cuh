@@ -40,6 +40,24 @@ __device__ __forceinline__ void gather_image(const int64_t* d, int64_t image, co
   }
 }
 
+// The image's classes for the matching, after gather_image and a block barrier: those of its targets, and of its
+// detections, of which one outside [0, C) marks class 0. class_bits: ceil(C / 32) words per image.
+__device__ __forceinline__ void mark_classes(const int64_t* d, int64_t image, const FieldGather& a, int C,
+                                             u32* class_bits) {
+  const int D = (int)d[kD], G = (int)d[kG], words = (C + 31) / 32;
+  u32* bits = class_bits + image * words;
+  for (int w = threadIdx.x; w < words; w += blockDim.x) bits[w] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < D; i += blockDim.x) {
+    const int c = a.pc[d[kDetBegin] + i], k = c >= 0 && c < C ? c : 0;
+    atomicOr(bits + (k >> 5), 1u << (k & 31));
+  }
+  for (int g = threadIdx.x; g < G; g += blockDim.x) {
+    const int c = a.gc[d[kSlotBegin] + g];
+    if (c >= 0 && c < C) atomicOr(bits + (c >> 5), 1u << (c & 31));
+  }
+}
+
 // Per-image stable descending score order (NaN scores last). Latency bounds it: 32 images of 100
 // detections took 10.6 us, 8 of 256 15.8, with a bitonic network over FP64 keys; 4.5 and 8.5 now.
 constexpr int kSortThreads = 256;

@@ -141,7 +141,7 @@ inst_sample_kernel(const int64_t* __restrict__ descs, int64_t samples, PairSampl
 static_assert(kSampleThreads == kSortThreads, "one block size for both kinds of work");
 __global__ void __launch_bounds__(kSampleThreads)
 inst_begin_kernel(const int64_t* __restrict__ descs, int64_t B, FieldGather fields, ScoreOrder order, int64_t samples,
-                  PairSample sample) {
+                  PairSample sample, int C, u32* class_bits) {
   wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (blockIdx.x >= B) {
@@ -151,6 +151,7 @@ inst_begin_kernel(const int64_t* __restrict__ descs, int64_t B, FieldGather fiel
   const int64_t* d = desc_of(descs, blockIdx.x);
   gather_image(d, blockIdx.x, fields);
   __syncthreads();
+  if (class_bits) mark_classes(d, blockIdx.x, fields, C, class_bits);
   sort_image(d, order, smem_raw);
 }
 
@@ -448,13 +449,15 @@ int launch_counts(const int64_t* descs, int64_t B, int64_t pair_chunks, const in
 }  // namespace
 
 // pe_inst_gather and pe_seg_sort in one launch, which also clears the outputs of pe_inst_counts and, with a limit
-// above 0, samples the masks for it (work: 8 B + 1 u64 of device scratch).
+// above 0, samples the masks for it (work: 8 B + 1 u64 of device scratch). class_bits (optional): the images' classes
+// among C, for pe_inst_match.
 PE_API int pe_inst_begin(const int64_t* descs, const int64_t* fields, int64_t B, int32_t* pc, double* scores,
                          int32_t* gc, uint8_t* crowd, double* areas, int64_t total_detections, int64_t* order,
                          double* sorted_scores, int32_t* sorted_classes, void* workspace, int64_t workspace_bytes,
                          uint32_t* inter, int64_t inter_len, uint64_t* pa, int64_t pa_len, uint64_t* ga,
-                         int64_t ga_len, int64_t limit, uint64_t* work, cudaStream_t stream) {
-  PE_REQUIRE(valid_sample(B, inter_len, pa_len, ga_len) && total_detections >= 0, "invalid batch");
+                         int64_t ga_len, int64_t limit, uint64_t* work, int64_t C, uint32_t* class_bits,
+                         cudaStream_t stream) {
+  PE_REQUIRE(valid_sample(B, inter_len, pa_len, ga_len) && C >= 0 && C < INT_MAX && total_detections >= 0, "invalid batch");
   PE_REQUIRE(workspace_bytes >= pe_seg_sort_workspace(total_detections), "sort workspace too small");
   PE_REQUIRE(limit <= 0 || work, "a sample needs its scratch");
   const int64_t samples = limit > 0 ? B * kSampleParts : 0;
@@ -466,7 +469,7 @@ PE_API int pe_inst_begin(const int64_t* descs, const int64_t* fields, int64_t B,
                                (int)sort_bytes(kOrderCap)));
   launch_kernel(inst_begin_kernel, (unsigned)(B + samples + clearing), kSampleThreads, sort_bytes(out.cap), stream,
       descs, B, FieldGather{fields, pc, scores, gc, crowd, areas}, out, samples,
-      pair_sample(samples ? work : nullptr, B, inter, inter_len, pa, pa_len, ga, ga_len));
+      pair_sample(samples ? work : nullptr, B, inter, inter_len, pa, pa_len, ga, ga_len), (int)C, class_bits);
   PE_LAUNCHED("inst_begin");
   count_launch();
   return kOk;

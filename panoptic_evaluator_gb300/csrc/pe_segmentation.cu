@@ -30,11 +30,11 @@
 
 namespace pe {
 
-int launch_match_gated(const void* pairs, bool pairs_u32, const int64_t* pair_off, const int64_t* d_off,
-                       const int64_t* g_off, int64_t B, const int* pc, const double* pa, const int* gc,
-                       const double* ga, const uint8_t* crowd, const double* areas, int C, int g_max, int8_t* flags,
-                       int64_t chain_stride, int64_t det_stride, int* ranks, int64_t* counts, const int* gate,
-                       const uint32_t* class_bits, cudaStream_t stream);
+template <typename Area>
+int launch_match_gated(const u32* pairs, const int64_t* pair_off, const int64_t* d_off, const int64_t* g_off,
+                       int64_t B, const int* pc, const Area* pa, const int* gc, const Area* ga, const uint8_t* crowd,
+                       const double* areas, int C, int g_max, int8_t* flags, int64_t chain_stride, int64_t det_stride,
+                       int* ranks, int64_t* counts, const int* gate, const uint32_t* class_bits, cudaStream_t stream);
 
 namespace {
 
@@ -866,7 +866,21 @@ PE_API int pe_seg_match(const uint32_t* pairs, const int64_t* pair_off, const in
                         int64_t chain_stride, int64_t det_stride, int32_t* ranks, int64_t* counts,
                         const int32_t* gate, const uint32_t* class_bits, cudaStream_t stream) {
   PE_REQUIRE(B >= 0 && C > 0 && C <= INT_MAX / 120 && g_max >= 0 && g_max < INT_MAX, "invalid batch");
-  return launch_match_gated(pairs, true, pair_off, d_off, g_off, B, pc, pa, gc, ga, crowd, areas, (int)C,
+  return launch_match_gated(pairs, pair_off, d_off, g_off, B, pc, pa, gc, ga, crowd, areas, (int)C,
+                            (int)std::max<int64_t>(g_max, 1), flags, chain_stride, det_stride, ranks, counts, gate,
+                            class_bits, stream);
+}
+
+// pe_seg_match from the pixel counts of pe_inst_counts, for a batch that pe_inst_prepare need not check: 5 us less of
+// the stream. areas (optional): annotation areas, else the targets' pixels.
+PE_API int pe_inst_match(const uint32_t* pairs, const int64_t* pair_off, const int64_t* d_off, const int64_t* g_off,
+                         int64_t B, const int32_t* pc, const uint64_t* pa, const int32_t* gc, const uint64_t* ga,
+                         const uint8_t* crowd, const double* areas, int64_t C, int64_t g_max, int8_t* flags,
+                         int64_t chain_stride, int64_t det_stride, int32_t* ranks, int64_t* counts,
+                         const int32_t* gate, const uint32_t* class_bits, cudaStream_t stream) {
+  PE_REQUIRE(B >= 0 && C > 0 && C <= INT_MAX / 120 && g_max >= 0 && g_max < INT_MAX, "invalid batch");
+  return launch_match_gated(pairs, pair_off, d_off, g_off, B, pc, reinterpret_cast<const u64*>(pa), gc,
+                            reinterpret_cast<const u64*>(ga), crowd, areas, (int)C,
                             (int)std::max<int64_t>(g_max, 1), flags, chain_stride, det_stride, ranks, counts, gate,
                             class_bits, stream);
 }

@@ -112,3 +112,27 @@ def test_records_are_stored_in_stable_score_order(sizes):
                                   np.concatenate([s[o] for s, o in zip(scores, order)]))
     np.testing.assert_array_equal(state["records.classes"].cpu().numpy(),
                                   np.concatenate([c[o] for c, o in zip(classes, order)]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("areas", (False, True))
+@pytest.mark.parametrize("images, dets, gts, classes", [(1, 1, 1, 1), (3, 40, 9, 2), (2, 130, 70, 33), (2, 0, 5, 3)])
+def test_unchecked_updates_match_from_the_pixel_counts(images, dets, gts, classes, areas):
+    """Without validation areas and classes come from other kernels: the results equal the checked update's."""
+    import panoptic_evaluator_gb300 as pe
+    generator = torch.Generator("cuda").manual_seed(dets + gts)
+    draw = lambda n: torch.rand((n, 61, 67), device="cuda", generator=generator) < 0.3  # noqa: E731
+    label = lambda n: torch.randint(0, classes, (n,), device="cuda", generator=generator)  # noqa: E731
+    gm = [draw(gts) for _ in range(images)]
+    pm = [torch.cat((m, draw(dets)))[:dets] for m in gm]  # copies of the targets first
+    args = (pe.InstanceBatch(pm, [label(dets) for _ in pm], [torch.rand(dets, device="cuda", generator=generator) for _ in pm]),
+            pe.InstanceBatch(gm, [label(gts) for _ in gm],
+                             crowd=[torch.rand(gts, device="cuda", generator=generator) < 0.2 for _ in gm],
+                             areas=[m.flatten(1).sum(1).float() * 2 + 0.5 for m in gm] if areas else None))
+    results = []
+    for validate in (True, False):
+        evaluator = pe.InstanceEvaluator(classes, validate=validate)
+        evaluator.update(*args)
+        results.append(evaluator.compute())
+    for key, value in results[0].items():
+        assert torch.equal(value, results[1][key]), key
