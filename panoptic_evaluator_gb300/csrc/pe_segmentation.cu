@@ -364,8 +364,8 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
     __syncwarp();  // the entry is in registers
     if (lane == 0) mbar_arrive(&sm.half_empty[half.at]);
     half.next();
-    const int64_t len = min((int64_t)kHalf, pixels - x0);
     const int64_t x = x0 + (int64_t)ctid * kPassPixels;
+    const bool in_image = x - lane * kPassPixels < pixels;  // any of the warp's pixels
     int t[16];
     {
       int p[16];
@@ -375,7 +375,6 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
         add_pairs(t, p, x, pixels, G, P, image_pairs, bad);
       }
     }
-    const bool in_range = x < x0 + len;
     const LaneSlots ls = lane_slots(t, x, pixels, G, bad);
     for (int r0 = first_row; r0 < end_row; r0 += kStageMasks) {
       const bool got = mbar_wait(&sm.full[stage.at], stage.phase, kWaitLimit);
@@ -383,9 +382,10 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
         ok = false;
         break;
       }
-      // One warp-wide OR tells which masks of the stage have a pixel here (a superset for rows at any
-      // offset: the staged words as they lie); only those are re-aligned and counted, by one copy of the
-      // counting code.
+      // One warp-wide OR tells which masks of the stage have a pixel here (a superset: the staged words of all
+      // lanes as they lie, since a lane's pixels end in the next lane's word, past the image with what the slot held
+      // before); only those are re-aligned and counted, by one copy of the counting code, and `ls` holds no pixel
+      // past the image.
       const unsigned char* staged = &sm.ring[stage.at][0][ctid * kPassPixels];
       constexpr int kRowBytes = kHalf + 16;
       u32 hit = 0;
@@ -399,7 +399,7 @@ seg_pass_bulk_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t total
         }
         hit |= (u32)(any != 0) << k;
       }
-      hit = __reduce_or_sync(0xffffffffu, in_range ? hit : 0u) & ((1u << min(kStageMasks, end_row - r0)) - 1u);
+      hit = __reduce_or_sync(0xffffffffu, in_image ? hit : 0u) & ((1u << min(kStageMasks, end_row - r0)) - 1u);
 #pragma unroll 1
       for (; hit; hit &= hit - 1) {
         const int k = __ffs(hit) - 1;
