@@ -10,10 +10,15 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import os
+import sysconfig
 import threading
+import warnings
 from pathlib import Path
 
 import torch
+
+HOST_MODULE = Path(__file__).resolve().parent / "_host.so"
+HOST_TAG = HOST_MODULE.with_suffix(".tag")  # host_tag() of the build that made the module
 
 # PE_GB300_LIBRARY may name another build of the same ABI (for example a tuning variant).
 LIBRARY = Path(os.environ.get("PE_GB300_LIBRARY", Path(__file__).resolve().parent / "libpe_gb300.so"))
@@ -144,11 +149,16 @@ def check(name, status):
 
 
 _call = call
-_host = None
+_host = None  # the module, or False when there is none for this Python and torch
+
+
+def host_tag() -> str:
+    """What a build of ``_host.so`` is good for: it reads the tensors of one torch through one Python's C API."""
+    return f"{torch.__version__} {sysconfig.get_config_var('SOABI')} {int(torch._C._GLIBCXX_USE_CXX11_ABI)}"
 
 
 def host():
-    """The C++ host path (``_host.so``), or None while ``call`` is replaced.
+    """The C++ host path (``_host.so``), or None while ``call`` is replaced or there is none for this torch.
 
     Each of its functions takes a whole step (checks, tables, launches, result
     views) for plain arguments and returns None for anything else, which then
@@ -157,7 +167,7 @@ def host():
     """
     if call is not _call:
         return None
-    return _host if _host is not None else _load_host()
+    return (_host if _host is not None else _load_host()) or None
 
 
 def _load_host():
@@ -165,14 +175,27 @@ def _load_host():
     lib = library()
     with _lock:
         if _host is None:
-            try:
-                from . import _host as module
-            except ImportError as error:
-                raise RuntimeError("_host.so is not built for this Python and torch; run "
-                                   "`python -m panoptic_evaluator_gb300.build`") from error
-            module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in SIGNATURES})
+            module = _import_host()
+            if module:
+                module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in SIGNATURES})
             _host = module
     return _host
+
+
+def _import_host():
+    """The extension module, or False with a warning. One built for another torch or Python is not opened."""
+    built = HOST_TAG.read_text() if HOST_TAG.exists() and HOST_MODULE.exists() else None
+    if built == host_tag():
+        try:
+            from . import _host as module
+            return module
+        except ImportError as error:
+            reason = str(error)
+    else:
+        reason = f"built for {built!r}, this is {host_tag()!r}" if built else "not built"
+    warnings.warn(f"{HOST_MODULE.name}: {reason}; evaluators take the slower Python host path. Run "
+                  "`python -m panoptic_evaluator_gb300.build --force`", RuntimeWarning, stacklevel=3)
+    return False
 
 
 def size(name, *args) -> int:
