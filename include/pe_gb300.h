@@ -235,7 +235,8 @@ int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, const int
 /* max_p: largest P of the batch; max_pairs: largest G x P (each image's histogram is staged in shared
  * memory when the largest fits 100 KB, else read in place; the results are the same). class_bits
  * (optional, B x ceil(C / 32) u32): each image's classes with detections or thing targets, for
- * pe_seg_match (a detection class outside [0, C) marks class 0). */
+ * pe_seg_match (a detection class outside [0, C) marks class 0). Where a kernel before it gave up (*error
+ * has a bit from 2^20 on: a wait ran out), validate = 0 counts nothing and makes the dataset IoU sums NaN. */
 int pe_seg_score(const int64_t* descs, int64_t B, int64_t max_p, int64_t max_pairs, const uint32_t* pairs,
                  const uint32_t* dpairs,
                  const int32_t* gc, const int32_t* pc, const uint8_t* crowd, int64_t* areas, int32_t* matched,
@@ -243,7 +244,10 @@ int pe_seg_score(const int64_t* descs, int64_t B, int64_t max_p, int64_t max_pai
                  const uint8_t* isthing, const int32_t* det_classes, const double* det_scores, double* det_pa,
                  double* slot_ga, int32_t* slot_class, const double* ann_in, double* ann_out, int validate,
                  int reward, uint32_t* class_bits, int32_t* error, cudaStream_t stream);
-/* class_bits (optional): pe_seg_score's per-image class bits; classes absent from an image are skipped. */
+/* class_bits (optional): pe_seg_score's per-image class bits; classes absent from an image are skipped.
+ * With a nonzero *gate every record gets rank 0 and flags -1 (left out of every curve) and counts stay as
+ * they are, except after an update that checks nothing whose kernels gave up: then counts become -2^40,
+ * for which pe_instance_accumulate gives NaN. */
 int pe_seg_match(const uint32_t* pairs, const int64_t* pair_off, const int64_t* d_off, const int64_t* g_off,
                  int64_t B, const int32_t* pc, const double* pa, const int32_t* gc, const double* ga,
                  const uint8_t* crowd, const double* areas, int64_t C, int64_t g_max, int8_t* flags,

@@ -57,7 +57,9 @@ def raise_combined_error(code: int):
 class SegmentationEvaluator:
     """PQ/mIoU and mask AP/AR with separate predictions and one shared target (combined.py:18-167).
 
-    AP ground truth is exactly the thing segments of the panoptic target.
+    AP ground truth is exactly the thing segments of the panoptic target. With ``validate=False`` an update does not
+    wait for the GPU, so a kernel that gave up (a bounded wait that ran out) raises nothing: PQ, SQ, mIoU, AP and AR
+    are NaN from then on, until ``reset``.
     """
 
     def __init__(self, num_classes: int, *, isthing: Sequence[bool] | None = None,

@@ -29,6 +29,14 @@ enum Status : int {
   kUnsupported = -4,
 };
 
+// Bits of a batched update's error word from 2^20 up: a kernel gave up (a wait ran out, blocks came out of order),
+// whatever the input was. A checked update reads the word and raises. One that checks nothing never reads it, so the
+// kernels after it mark the evaluator's state instead: IoU sums NaN, positives kUnknownCount (any sum with counts is
+// negative). PQ, SQ, mIoU, AP and AR of such a state are NaN until it is reset.
+constexpr int kStoppedBits = ~((1 << 20) - 1);
+constexpr int kUncheckedBit = 1 << 27;  // beside them: the update checks nothing
+constexpr long long kUnknownCount = -(1ll << 40);
+
 void set_error(const char* fmt, ...);
 
 #define PE_REQUIRE(cond, ...)                  \

@@ -109,10 +109,21 @@ match_kernel(const Count* __restrict__ pairs, const int64_t* __restrict__ pair_o
              const int* __restrict__ gc, const Area* __restrict__ ga, const uint8_t* __restrict__ crowd,
              const double* __restrict__ areas, int C, int g_max, FlagLayout flags, int* __restrict__ ranks,
              int64_t* __restrict__ counts, const int* __restrict__ gate,
-             const u32* __restrict__ class_bits) {
+             const u32* __restrict__ class_bits, int unchecked) {
   wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (gate && *reinterpret_cast<const volatile int*>(gate)) return;  // validation failed upstream
+  const int stopped = gate ? *reinterpret_cast<const volatile int*>(gate) : 0;
+  if (stopped) {  // validation failed upstream, or a kernel gave up: an unchecked caller counts these records all the same
+    if (blockIdx.y || blockIdx.z) return;
+    const int64_t d_begin = d_off ? d_off[blockIdx.x] : 0, d_end = d_off ? d_off[blockIdx.x + 1] : single_d;
+    for (int64_t i = d_begin + threadIdx.x; i < d_end; i += blockDim.x) {
+      ranks[i] = 0;
+      for (int k = 0; k < kChains; ++k) flags.base[k * flags.chain_stride + i * flags.det_stride] = -1;
+    }
+    if (blockIdx.x == 0 && (stopped & kStoppedBits) && (unchecked || (stopped & kUncheckedBit)))
+      for (int k = threadIdx.x; k < 4 * C; k += blockDim.x) counts[k] = kUnknownCount;
+    return;
+  }
   // Image b covers detections [d_off[b], d_off[b+1]) and targets [g_off[b], g_off[b+1]);
   // its D x G intersections start at pair_off[b]. Without offsets: one image. CTA (b, k) takes the k-th
   // class of image b: of all classes, or with per-image class bits of those present in it (about a third
@@ -489,6 +500,11 @@ __device__ __forceinline__ int64_t recall_reached_at(int64_t np, int r) {
   return t + (t * 100 == scaled && !exact_ok ? 1 : 0);
 }
 
+// Precision and recall of a class without positives: -1, or NaN where their number is unknown (kUnknownCount).
+__device__ __forceinline__ double without_curve(int64_t positives) {
+  return positives < 0 ? __longlong_as_double(0x7ff8000000000000ll) : -1.0;
+}
+
 // 10 / kT CTAs per class. `scores` == nullptr means the records are already in
 // global descending-score order. Records: classes[n], ranks[n] and flags at
 // flags[chain * chain_stride + record * det_stride]; list / cursor / hist: the
@@ -644,7 +660,7 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
       const int m = ch % 3, a = (ch / 3) % 4, t = ch / 12;
       int nseg = 0, hi = 0;
       unsigned tp = 0;
-      if (sm.npos[a]) {
+      if (sm.npos[a] > 0) {
         const int limit = m == 0 ? 1 : (m == 1 ? 10 : 100);
         const int64_t chain = (int64_t)(a * 10 + t_base + t) * chain_stride;
         // Prefix counts over the records within maxDets: the j-th true positive's cumulative false
@@ -754,10 +770,10 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
       if (lane < kChainsHere) {
         const int a = (lane / 3) % 4, t = t_base + lane / 12;
         const int64_t np = sm.npos[a];
-        const double rc = np ? (double)sm.tp[lane] / (double)np : -1.0;
+        const double rc = np > 0 ? (double)sm.tp[lane] / (double)np : without_curve(np);
         recall[((int64_t)t * C + c) * 12 + lane % 12] = rc;
         if (chain_stats) {
-          double sum = np ? 0.0 : -1.0;
+          double sum = np > 0 ? 0.0 : without_curve(np);
           const int nseg = sm.nseg[lane], hi = sm.hi[lane];
           for (int k = 0; k < nseg; ++k) {
             const int end = k + 1 < nseg ? sm.seg_lo[lane][k + 1] : hi;
@@ -771,7 +787,7 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
     } else {
       for (int e = threadIdx.x; e < kChainsHere * 101; e += kAccThreads - 32) {
         const int k = e % 12, r = (e / 12) % 101, t = e / (12 * 101), ch = t * 12 + k;
-        double v = sm.npos[k / 3] ? 0.0 : -1.0;
+        double v = sm.npos[k / 3] > 0 ? 0.0 : without_curve(sm.npos[k / 3]);
         if (r < sm.hi[ch]) {
           int lo = 0, hi = sm.nseg[ch] - 1;  // the last segment starting at or before r
           while (lo < hi) {
@@ -825,7 +841,7 @@ summarize_chains_kernel(const double* __restrict__ chain_stats, int C, double* _
     }
 #pragma unroll
     for (int j = 0; j < kSummarizeLoads; ++j) {
-      if (v[j] >= 0.0) {
+      if (!(v[j] < 0.0)) {  // NaN: an unknown count
         sum += v[j];
         cnt += weight;
       }
@@ -854,7 +870,7 @@ summarize_chains_kernel(const double* __restrict__ chain_stats, int C, double* _
   }
 }
 
-// The 12 COCO summaries (instance.py:230-248): means of the entries >= 0.
+// The 12 COCO summaries (instance.py:230-248): means of the entries >= 0 (NaN as soon as one is).
 __global__ void __launch_bounds__(256)
 summarize_kernel(const double* __restrict__ precision, const double* __restrict__ recall, int C,
                  double* __restrict__ out) {
@@ -876,7 +892,7 @@ summarize_kernel(const double* __restrict__ precision, const double* __restrict_
       for (int64_t e = threadIdx.x; e < total; e += blockDim.x) {
         const int64_t t = t0 + e / per_t, rc = e % per_t;  // rc = r * C + c
         const double v = precision[((t * 101 * C + rc) * 4 + area) * 3 + 2];
-        if (v >= 0) { sum += v; ++cnt; }
+        if (!(v < 0)) { sum += v; ++cnt; }
       }
     } else {
       int area = 0, mi = 2;
@@ -887,7 +903,7 @@ summarize_kernel(const double* __restrict__ precision, const double* __restrict_
       const int64_t total = (int64_t)10 * C;
       for (int64_t e = threadIdx.x; e < total; e += blockDim.x) {
         const double v = recall[(e * 4 + area) * 3 + mi];
-        if (v >= 0) { sum += v; ++cnt; }
+        if (!(v < 0)) { sum += v; ++cnt; }
       }
     }
     s_sum[threadIdx.x] = sum;
@@ -1061,7 +1077,8 @@ int launch_match(const Count* pairs, const int64_t* pair_off, const int64_t* d_o
                  const int64_t* g_off, int single_d, int single_g, int64_t B, const int* pc, const Area* pa,
                  const int* gc, const Area* ga, const uint8_t* crowd, const double* areas, int C, int g_max,
                  int8_t* flags, int64_t chain_stride, int64_t det_stride, int* ranks, int64_t* counts,
-                 cudaStream_t stream, const int* gate = nullptr, const uint32_t* class_bits = nullptr) {
+                 cudaStream_t stream, const int* gate = nullptr, const uint32_t* class_bits = nullptr,
+                 int unchecked = 0) {
   if (B == 0) return kOk;
   const size_t smem = match_bytes(g_max);
   if (smem > 200 * 1024 || g_max > 65536) {
@@ -1078,7 +1095,7 @@ int launch_match(const Count* pairs, const int64_t* pair_off, const int64_t* d_o
   auto kernel = match_kernel<Count, Area>;
   if (smem > 48 * 1024) PE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   launch_kernel(kernel, grid, threads, smem, stream, pairs, pair_off, d_off, g_off, single_d, single_g, pc, pa, gc, ga,
-      crowd, areas, C, g_max, layout, ranks, counts, gate, class_bits);
+      crowd, areas, C, g_max, layout, ranks, counts, gate, class_bits, unchecked);
   PE_LAUNCHED("match");
   count_launch();
   return kOk;
@@ -1088,16 +1105,18 @@ template <typename Area>
 int launch_match_gated(const u32* pairs, const int64_t* pair_off, const int64_t* d_off, const int64_t* g_off,
                        int64_t B, const int* pc, const Area* pa, const int* gc, const Area* ga, const uint8_t* crowd,
                        const double* areas, int C, int g_max, int8_t* flags, int64_t chain_stride, int64_t det_stride,
-                       int* ranks, int64_t* counts, const int* gate, const uint32_t* class_bits, cudaStream_t stream) {
+                       int* ranks, int64_t* counts, const int* gate, const uint32_t* class_bits, int unchecked,
+                       cudaStream_t stream) {
   return launch_match(pairs, pair_off, d_off, g_off, 0, 0, B, pc, pa, gc, ga, crowd, areas, C, g_max, flags,
-                      chain_stride, det_stride, ranks, counts, stream, gate, class_bits);
+                      chain_stride, det_stride, ranks, counts, stream, gate, class_bits, unchecked);
 }
 template int launch_match_gated(const u32*, const int64_t*, const int64_t*, const int64_t*, int64_t, const int*,
                                 const double*, const int*, const double*, const uint8_t*, const double*, int, int,
-                                int8_t*, int64_t, int64_t, int*, int64_t*, const int*, const uint32_t*, cudaStream_t);
+                                int8_t*, int64_t, int64_t, int*, int64_t*, const int*, const uint32_t*, int,
+                                cudaStream_t);
 template int launch_match_gated(const u32*, const int64_t*, const int64_t*, const int64_t*, int64_t, const int*,
                                 const u64*, const int*, const u64*, const uint8_t*, const double*, int, int, int8_t*,
-                                int64_t, int64_t, int*, int64_t*, const int*, const uint32_t*, cudaStream_t);
+                                int64_t, int64_t, int*, int64_t*, const int*, const uint32_t*, int, cudaStream_t);
 
 int64_t accumulate_workspace_bytes(int64_t n, int64_t C) {
   // Per-class overflow regions (each class's padded to a power of two, at most twice its records: 2n

@@ -562,11 +562,12 @@ compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, c
 #pragma unroll
     for (int q = 0; q < CL; ++q) column += CL > 1 ? cluster.map_shared_rank(col_sum, q)[c] : col_sum[c];
     const double denom = (double)a + 0.5 * ((double)f + (double)n);
-    const double pq = denom > 0 ? s / denom : 0.0;
-    const double sq = a ? s / (double)a : 0.0;
+    const double none = s == s ? 0.0 : s;  // NaN: an update that checks nothing lost its counts
+    const double pq = denom > 0 ? s / denom : none;
+    const double sq = a ? s / (double)a : none;
     const double rq = denom > 0 ? (double)a / denom : 0.0;
     const int64_t uni = row_sum[c] + column - diag;
-    const double iou = uni ? (double)diag / (double)uni : __longlong_as_double(0x7ff8000000000000ll);
+    const double iou = uni && s == s ? (double)diag / (double)uni : __longlong_as_double(0x7ff8000000000000ll);
     per_class[c] = pq;
     per_class[C + c] = sq;
     per_class[2 * C + c] = rq;
@@ -575,7 +576,7 @@ compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, c
     value0[C + c] = sq;
     value0[2 * C + c] = rq;
     value0[3 * C + c] = iou;
-    group0[c] = denom > 0 ? (things[c] ? 1 : 2) : 0;
+    group0[c] = denom > 0 || s != s ? (things[c] ? 1 : 2) : 0;
   }
   if (CL > 1) cluster.sync();
   else __syncthreads();
@@ -586,7 +587,9 @@ compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, c
     double part = 0.0;
     int members = 0;
     for (int c = lane; c < C; c += 32) {
-      const bool in = q < 9 ? (group[c] != 0 && (scope == 0 || group[c] == scope)) : !isnan(value[3 * C + c]);
+      // A class without pixels (NaN IoU) is not in the mean; one whose PQ is NaN too lost its counts.
+      const bool in = q < 9 ? (group[c] != 0 && (scope == 0 || group[c] == scope))
+                            : !isnan(value[3 * C + c]) || isnan(value[c]);
       if (in) part += value[metric * C + c];
       members += in;
     }

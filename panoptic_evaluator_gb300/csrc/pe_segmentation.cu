@@ -34,7 +34,8 @@ template <typename Area>
 int launch_match_gated(const u32* pairs, const int64_t* pair_off, const int64_t* d_off, const int64_t* g_off,
                        int64_t B, const int* pc, const Area* pa, const int* gc, const Area* ga, const uint8_t* crowd,
                        const double* areas, int C, int g_max, int8_t* flags, int64_t chain_stride, int64_t det_stride,
-                       int* ranks, int64_t* counts, const int* gate, const uint32_t* class_bits, cudaStream_t stream);
+                       int* ranks, int64_t* counts, const int* gate, const uint32_t* class_bits, int unchecked,
+                       cudaStream_t stream);
 
 namespace {
 
@@ -437,6 +438,7 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
   wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if ((mode & 4) && *reinterpret_cast<volatile int*>(error)) return;
+  const int stopped = !validate && error ? *reinterpret_cast<volatile int*>(error) & kStoppedBits : 0;
   const int64_t* d = desc_of(descs, blockIdx.x);
   const int G = (int)d[kG], P = (int)d[kP], D = (int)d[kD];
   const int64_t sb = d[kSlotBegin], pb = d[kPSlotBegin], db = d[kDetBegin];
@@ -515,6 +517,12 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
     __syncthreads();
   }
   if (!(mode & 2)) return;
+  if (stopped) {  // the counts are not all there, and nobody reads the word
+    if (blockIdx.x || reward) return;
+    for (int c = threadIdx.x; c < C; c += blockDim.x) out.iou_sum[c] = __longlong_as_double(0x7ff8000000000000ll);
+    if (threadIdx.x == 0) atomicOr(error, kUncheckedBit);
+    return;
+  }
   if (reward) {  // per-image rows [B][C], no confusion (evaluator.py:497-538)
     const int64_t o = (int64_t)blockIdx.x * C;
     ScoreOut row{out.tp + o, out.fp + o, out.fn + o, out.iou_sum + o, nullptr};
@@ -673,6 +681,9 @@ __global__ void inst_prepare_kernel(const int64_t* __restrict__ descs, const u64
     }
   }
   if (err) atomicOr(error, err);
+  if (!validate && error && blockIdx.x == 0 && threadIdx.x == 0 &&
+      (*reinterpret_cast<volatile int*>(error) & kStoppedBits))
+    atomicOr(error, kUncheckedBit);
 }
 
 }  // namespace
@@ -807,7 +818,8 @@ PE_API int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, co
 // (G+P) u64 at slot_begin + pslot_begin; matched: sum of G ints. state: dataset
 // tp/fp/fn/iou_sum [C], confusion [C, C+1]. Validation bits: 1/2/4 panoptic,
 // 8 detection class not a thing, 16 empty detection, 32 non-finite score,
-// 64 invalid annotation area. Accumulation is skipped when any bit is set.
+// 64 invalid annotation area. Accumulation is skipped when any bit is set; without validation, where a kernel before
+// this one gave up (bits from 2^20), the dataset IoU sums become NaN.
 PE_API int pe_seg_score(const int64_t* descs, int64_t B, int64_t max_p, int64_t max_pairs, const uint32_t* pairs,
                         const uint32_t* dpairs,
                         const int32_t* gc, const int32_t* pc, const uint8_t* crowd, int64_t* areas, int32_t* matched,
@@ -857,8 +869,8 @@ PE_API int pe_seg_score(const int64_t* descs, int64_t B, int64_t max_p, int64_t 
   return kOk;
 }
 
-// Batched greedy matching over the descriptor table, gated on *gate (skipped
-// when nonzero). pairs_u32: D x G intersections per image at dpair_begin.
+// Batched greedy matching over the descriptor table, gated on *gate (when
+// nonzero, every record is left out: rank 0, flags -1). pairs_u32: D x G intersections per image at dpair_begin.
 // Offsets are read from device arrays d_off [B+1], g_off [B+1], pair_off [B].
 PE_API int pe_seg_match(const uint32_t* pairs, const int64_t* pair_off, const int64_t* d_off, const int64_t* g_off,
                         int64_t B, const int32_t* pc, const double* pa, const int32_t* gc, const double* ga,
@@ -868,7 +880,7 @@ PE_API int pe_seg_match(const uint32_t* pairs, const int64_t* pair_off, const in
   PE_REQUIRE(B >= 0 && C > 0 && C <= INT_MAX / 120 && g_max >= 0 && g_max < INT_MAX, "invalid batch");
   return launch_match_gated(pairs, pair_off, d_off, g_off, B, pc, pa, gc, ga, crowd, areas, (int)C,
                             (int)std::max<int64_t>(g_max, 1), flags, chain_stride, det_stride, ranks, counts, gate,
-                            class_bits, stream);
+                            class_bits, 0, stream);
 }
 
 // pe_seg_match from the pixel counts of pe_inst_counts, for a batch that pe_inst_prepare need not check: 5 us less of
@@ -882,7 +894,7 @@ PE_API int pe_inst_match(const uint32_t* pairs, const int64_t* pair_off, const i
   return launch_match_gated(pairs, pair_off, d_off, g_off, B, pc, reinterpret_cast<const u64*>(pa), gc,
                             reinterpret_cast<const u64*>(ga), crowd, areas, (int)C,
                             (int)std::max<int64_t>(g_max, 1), flags, chain_stride, det_stride, ranks, counts, gate,
-                            class_bits, stream);
+                            class_bits, 1, stream);
 }
 
 // Mask-vs-mask overlaps and pixel areas for InstanceEvaluator over the

@@ -228,7 +228,11 @@ def summarize(precision, recall, summary):
 
 
 class InstanceEvaluator:
-    """COCO mask AP/AR with GPU intersections, matching and accumulation (instance.py:46-227)."""
+    """COCO mask AP/AR with GPU intersections, matching and accumulation (instance.py:46-227).
+
+    With ``validate=False`` an update does not wait for the GPU, so a kernel that gave up (a bounded wait that ran
+    out) raises nothing: every AP and AR is NaN from then on, until ``reset``.
+    """
 
     def __init__(self, num_classes: int, *, device: str | torch.device = "cuda", validate: bool = True):
         if not isinstance(num_classes, int) or isinstance(num_classes, bool) or num_classes <= 0:
