@@ -864,12 +864,29 @@ prefix_rows_kernel(PrefixMatch match, int splits, int match_blocks, int64_t B, c
                    double* __restrict__ sums, int64_t* __restrict__ confusion, int smem) {
   wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int block = blockIdx.x;
-  if (block < match_blocks)
+  const int block = blockIdx.x, C = match.C;
+  // Unchecked calls never read the word: where the pass gave up, their FP64 results are NaN.
+  const int stopped = match.validate ? 0 : *reinterpret_cast<const volatile int*>(match.error) & kStoppedBits;
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  if (block < match_blocks) {
     match_classes(match, block / splits, block % splits, splits, smem_raw, smem);
-  else
-    score_row(match.descs, B, block - match_blocks, pairs, match.classes, match.gc, match.crowd, match.C, tp, fp, fn,
-              sums, confusion, smem_raw, smem);
+    if (!stopped) return;
+    __syncthreads();
+    const int64_t* d = pdesc(match.descs, block / splits);
+    const int per = (C + splits - 1) / splits, c0 = min(C, block % splits * per), nc = min(C, c0 + per) - c0;
+    const int64_t first = d[kPrefixQBegin] * match.T, n = d[kPrefixQ] * match.T * nc;
+    for (int64_t k = threadIdx.x; k < n; k += blockDim.x) {
+      const int64_t o = (first + k / nc) * C + c0 + k % nc;
+      match.precision[o] = match.recall[o] = nan;
+    }
+    return;
+  }
+  const int64_t row = block - match_blocks;
+  score_row(match.descs, B, row, pairs, match.classes, match.gc, match.crowd, C, tp, fp, fn, sums, confusion, smem_raw,
+            smem);
+  if (!stopped) return;
+  __syncthreads();
+  for (int c = threadIdx.x; c < C; c += blockDim.x) sums[row * C + c] = nan;
 }
 
 }  // namespace
@@ -890,7 +907,8 @@ PE_API int pe_prefix_desc_fields(void) { return kPrefixFields; }
 // [R,C,C+1], itp/ifp/ifn int64 [R,T,C], precision/recall f64 [R,T,C]; then
 // per_class [R,4,C], summaries [R,3,3], counts [R,3], miou [R] (pe_compute).
 // Validation bits in *error: 1 unknown target slot, 2 empty prediction mask,
-// 4 bad target class, 8 target areas vs metadata, 16 bad prediction class.
+// 4 bad target class, 8 target areas vs metadata, 16 bad prediction class. Without validation, where the pass gave
+// up (bits from 2^20), sums, precision and recall are NaN, and with them pq, sq and miou.
 PE_API int pe_prefix(const int64_t* descs, int64_t B, int64_t total_chunks, int64_t total_rows, int64_t max_g,
                      int64_t max_p, int64_t max_cells, const int32_t* step_q, const int32_t* classes,
                      const int32_t* gc, const uint8_t* crowd, const uint8_t* isthing, const double* thresholds,

@@ -311,7 +311,10 @@ def segmentation_prefixes(prediction: InstanceBatch, target: PanopticBatch, num_
 
     Returns one list per image of snapshot dicts with ``prefix``, the
     panoptic/semantic results of the canvas and ``instance`` counts /
-    precision / recall of shape [threshold, class].
+    precision / recall of shape [threshold, class]. With ``validate=False``
+    the call does not wait for the GPU, so a kernel that gave up (a bounded
+    wait that ran out) raises nothing: pq, sq, miou, iou_sum, precision and
+    recall are NaN.
     """
     if not isinstance(num_classes, int) or isinstance(num_classes, bool) or num_classes <= 0:
         raise ValueError("num_classes must be a positive integer")

@@ -132,3 +132,26 @@ def test_gated_matching_defines_its_records(entry, gate, unknown):
     assert ranks.tolist() == [0] * total + [7]
     assert bool((flags[:-1] == -1).all()) and bool((flags[-1] == 7).all())
     assert bool((counts == (UNKNOWN if unknown else 5)).all())
+
+
+def test_prefixes(monkeypatch):
+    """The void slot's pixel count (above 2^20) stands in for the error word of an owner pass that gave up."""
+    import panoptic_evaluator_gb300 as pe
+    maps = torch.zeros((1, 1025, 1100), dtype=torch.int32, device="cuda")
+    maps[:, :30], maps[:, 30:60] = 1, 2
+    classes = torch.tensor([[-1, 0, 70]], dtype=torch.int32, device="cuda")
+    target = pe.PanopticBatch(maps, classes, torch.zeros((1, 3), dtype=torch.bool, device="cuda"))
+    masks = pe.InstanceBatch([torch.stack((maps[0] == 1, maps[0] == 2))], [torch.tensor([0, 70], device="cuda")])
+    expected, = pe.segmentation_prefixes(masks, target, 71, validate=False)
+    call = N.call
+
+    def with_timeout(name, *args):
+        return call(name, *args[:-2], args[15], args[-1]) if name == "pe_prefix" else call(name, *args)
+    monkeypatch.setattr(N, "call", with_timeout)
+    stopped, = pe.segmentation_prefixes(masks, target, 71, validate=False)
+    for now, then in zip(stopped, expected):
+        assert not bool(torch.isnan(then["iou_sum"]).any()) and torch.equal(now["tp"], then["tp"])
+        assert bool(torch.isnan(now["All"]["pq"])) and bool(torch.isnan(now["miou"]))
+        assert bool(torch.isnan(now["iou_sum"]).all())
+        assert bool(torch.isnan(now["instance"]["precision"]).all())
+        assert bool(torch.isnan(now["instance"]["recall"]).all())
