@@ -1417,6 +1417,41 @@ PyObject* prefixes(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+// One part of a packed output (flat tensor, the field's element offset, its shape, is it double, index of the leading
+// dimensions ...): a view like those of the other results, or None.
+PyObject* part(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  constexpr Py_ssize_t kIndex = 4;
+  if (nargs < kIndex || !ordinary() || !PyTuple_CheckExact(args[2]) || !THPVariable_CheckExact(args[0])) return none();
+  const Tensor& base = THPVariable_Unpack(args[0]);
+  if (!plain(args[0], base.is_cuda() ? base.get_device() : kHostOnly) || base.scalar_type() != at::kLong ||
+      base.storage_offset())
+    return none();
+  const Py_ssize_t dims = PyTuple_GET_SIZE(args[2]), leading = nargs - kIndex;
+  int64_t offset = PyLong_AsLongLong(args[1]), numel = 1, count = 1;
+  bool inside = offset >= 0 && leading <= dims;
+  std::vector<int64_t> sizes(dims);
+  for (Py_ssize_t k = dims - 1; k >= 0; --k) {
+    sizes[k] = PyLong_AsLongLong(PyTuple_GET_ITEM(args[2], k));
+    if (k < leading) {
+      const int64_t i = PyLong_AsLongLong(args[kIndex + k]);
+      inside = inside && i >= 0 && i < sizes[k];
+      offset += i * numel;
+    } else {
+      count *= sizes[k];
+    }
+    numel *= sizes[k];
+  }
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return none();
+  }
+  if (!inside || count < 0 || offset + count > base.numel()) return none();
+  return view(base, 8 * offset, args[3] == Py_True ? at::kDouble : at::kLong,
+              at::IntArrayRef(sizes.data() + leading, dims - leading));
+  END_HANDLE_TH_ERRORS
+}
+
 // ---- module -------------------------------------------------------------------------------------------
 
 // bind({name: address}): entry points of the loaded library.
@@ -1457,6 +1492,7 @@ PyMethodDef methods[] = {
     FAST("images_update", images_update),
     FAST("prefixes", prefixes),
     FAST("prefix_tables", prefix_tables),
+    FAST("part", part),
     {nullptr, nullptr, 0, nullptr},
 };
 

@@ -97,10 +97,12 @@ def _output_layout(R, T, C):
 class PackedOutputs(Mapping):
     """pe_prefix's outputs: named views of one int64 allocation, each made on first access and kept."""
 
-    __slots__ = ("flat", "_layout", "_views", "_rows")
+    __slots__ = ("flat", "_layout", "_views", "_part")
 
     def __init__(self, flat, layout):
-        self.flat, self._layout, self._views, self._rows = flat, layout, {}, {}
+        self.flat, self._layout, self._views = flat, layout, {}
+        host = N.host()
+        self._part = host.part if host is not None else None
 
     def __getitem__(self, key):
         view = self._views.get(key)
@@ -110,12 +112,11 @@ class PackedOutputs(Mapping):
             view = self._views[key] = (part if dtype is torch.int64 else part.view(dtype)).view(shape)
         return view
 
-    def rows(self, key):
-        """The rows of a field as a tuple of views, all made when the first one is read."""
-        rows = self._rows.get(key)
-        if rows is None:
-            rows = self._rows[key] = self[key].unbind(0)
-        return rows
+    def at(self, row, key, *index):
+        """A view of field[row, index] alone: reading one checkpoint costs the same however many there are."""
+        offset, shape, dtype = self._layout[key]
+        view = self._part and self._part(self.flat, offset, shape, dtype is torch.float64, row, *index)
+        return self[key][(row, *index)] if view is None else view
 
     def __iter__(self):
         return iter(self._layout)
@@ -220,9 +221,8 @@ _METRICS = ("pq", "sq", "rq", "iou")
 _ROW_FIELDS = {"tp": "tp", "fp": "fp", "fn": "fn", "iou_sum": "sums", "confusion": "confusion", "miou": "miou"}
 
 
-def _row_of(out, r, key):
-    """Row r of a field (packed outputs keep the rows they have made)."""
-    return out.rows(key)[r] if type(out) is PackedOutputs else out[key][r]
+def _part_of(out, row, key, *index):
+    return out[key][(row, *index)]
 
 
 class Snapshot(Mapping):
@@ -249,18 +249,18 @@ class Snapshot(Mapping):
         cache = self._cache
         if key in cache:
             return cache[key]
-        r = self._row
-        row = partial(_row_of, self._out, r)
+        out = self._out
+        row = partial(out.at, self._row) if type(out) is PackedOutputs else partial(_part_of, out, self._row)
         if key == "prefix":
             value = self._prefix
         elif key in _ROW_FIELDS:
             value = row(_ROW_FIELDS[key])
         elif key in _GROUPS:
             i = _GROUPS.index(key)
-            pq, sq, rq = row("summaries")[i].unbind(0)
-            value = dict(pq=pq, sq=sq, rq=rq, n=row("counts")[i])
+            value = dict(pq=row("summaries", i, 0), sq=row("summaries", i, 1), rq=row("summaries", i, 2),
+                         n=row("counts", i))
         elif key == "per_class":
-            value = dict(zip(_METRICS, row("values").unbind(0)))
+            value = {metric: row("values", m) for m, metric in enumerate(_METRICS)}
         elif key == "instance":
             value = dict(iou_thresholds=self._thr, tp=row("itp"), fp=row("ifp"), fn=row("ifn"),
                          precision=row("precision"), recall=row("recall"))
