@@ -478,7 +478,7 @@ constexpr int kComputeCluster = 8;
 constexpr int kComputeClusterClasses = 64;
 
 template <int CL>
-__global__ void __launch_bounds__(kComputeThreads)
+__global__ void __launch_bounds__(kComputeThreads, 2)
 compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, const int64_t* __restrict__ fn,
                const double* __restrict__ sums, const int64_t* __restrict__ confusion,
                const bool* __restrict__ things, double* per_class, double* summaries, int64_t* counts,
@@ -501,7 +501,7 @@ compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, c
   int64_t* col_sum = row_sum + C;                            // C column sums over this CTA's rows
   int64_t* partial = col_sum + C;                            // [warps][kComputeTile], before `value` is written
   double* value = reinterpret_cast<double*>(col_sum + C);    // [4][C]: pq, sq, rq, iou (NaN: no pixels)
-  int* group = reinterpret_cast<int*>(value + 4 * C);        // C: 0 inactive, 1 thing, 2 stuff (active)
+  int* group = reinterpret_cast<int*>(value + 4 * C);        // C: 0 inactive, 1 thing, 2 stuff (active); 4: its counts are lost
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, warps = blockDim.x >> 5;
   const int r_begin = (int)((int64_t)C * rank / CL), r_end = (int)((int64_t)C * (rank + 1) / CL);
   // This thread's (first) class: its counts are in flight while the matrix is read.
@@ -562,12 +562,17 @@ compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, c
 #pragma unroll
     for (int q = 0; q < CL; ++q) column += CL > 1 ? cluster.map_shared_rank(col_sum, q)[c] : col_sum[c];
     const double denom = (double)a + 0.5 * ((double)f + (double)n);
-    const double none = s == s ? 0.0 : s;  // NaN: an update that checks nothing lost its counts
-    const double pq = denom > 0 ? s / denom : none;
-    const double sq = a ? s / (double)a : none;
+    double pq = denom > 0 ? s / denom : 0.0;
+    double sq = a ? s / (double)a : 0.0;
     const double rq = denom > 0 ? (double)a / denom : 0.0;
     const int64_t uni = row_sum[c] + column - diag;
-    const double iou = uni && s == s ? (double)diag / (double)uni : __longlong_as_double(0x7ff8000000000000ll);
+    double iou = uni ? (double)diag / (double)uni : __longlong_as_double(0x7ff8000000000000ll);
+    int kind = denom > 0 ? (things[c] ? 1 : 2) : 0;
+    // A NaN sum (tested as an integer: FP64 runs at 1/64): an update that checks nothing lost its counts.
+    if ((__double2hiint(s) & INT_MAX) > 0x7ff00000) {
+      pq = sq = iou = __longlong_as_double(0x7ff8000000000000ll);
+      kind = 4 | (things[c] ? 1 : 2);
+    }
     per_class[c] = pq;
     per_class[C + c] = sq;
     per_class[2 * C + c] = rq;
@@ -576,7 +581,7 @@ compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, c
     value0[C + c] = sq;
     value0[2 * C + c] = rq;
     value0[3 * C + c] = iou;
-    group0[c] = denom > 0 || s != s ? (things[c] ? 1 : 2) : 0;
+    group0[c] = kind;
   }
   if (CL > 1) cluster.sync();
   else __syncthreads();
@@ -587,9 +592,9 @@ compute_kernel(const int64_t* __restrict__ tp, const int64_t* __restrict__ fp, c
     double part = 0.0;
     int members = 0;
     for (int c = lane; c < C; c += 32) {
-      // A class without pixels (NaN IoU) is not in the mean; one whose PQ is NaN too lost its counts.
-      const bool in = q < 9 ? (group[c] != 0 && (scope == 0 || group[c] == scope))
-                            : !isnan(value[3 * C + c]) || isnan(value[c]);
+      // A class without pixels (NaN IoU) is not in the mean; one that lost its counts makes it NaN.
+      const bool in = q < 9 ? (group[c] != 0 && (scope == 0 || (group[c] & 3) == scope))
+                            : !isnan(value[3 * C + c]) || (group[c] & 4);
       if (in) part += value[metric * C + c];
       members += in;
     }

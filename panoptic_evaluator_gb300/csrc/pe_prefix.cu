@@ -866,7 +866,7 @@ prefix_rows_kernel(PrefixMatch match, int splits, int match_blocks, int64_t B, c
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int block = blockIdx.x, C = match.C;
   // Unchecked calls never read the word: where the pass gave up, their FP64 results are NaN.
-  const int stopped = match.validate ? 0 : *reinterpret_cast<const volatile int*>(match.error) & kStoppedBits;
+  const int stopped = match.validate ? 0 : __ldcg(match.error) & kStoppedBits;
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
   if (block < match_blocks) {
     match_classes(match, block / splits, block % splits, splits, smem_raw, smem);

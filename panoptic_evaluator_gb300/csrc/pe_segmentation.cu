@@ -438,7 +438,7 @@ seg_score_kernel(const int64_t* __restrict__ descs, const u32* __restrict__ pair
   wait_for_earlier_kernels();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if ((mode & 4) && *reinterpret_cast<volatile int*>(error)) return;
-  const int stopped = !validate && error ? *reinterpret_cast<volatile int*>(error) & kStoppedBits : 0;
+  const int stopped = !validate && error ? __ldcg(error) & kStoppedBits : 0;
   const int64_t* d = desc_of(descs, blockIdx.x);
   const int G = (int)d[kG], P = (int)d[kP], D = (int)d[kD];
   const int64_t sb = d[kSlotBegin], pb = d[kPSlotBegin], db = d[kDetBegin];
