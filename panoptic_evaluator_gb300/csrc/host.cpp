@@ -16,6 +16,7 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -72,7 +73,7 @@ struct ReleaseGil {
   X(isthing) X(num_classes) X(validate) X(_scratch) X(_default_crowd) X(_validation_error) X(_state) X(masks)   \
   X(scores) X(areas) X(_store) X(_counts) X(_arena) X(n) X(capacity) X(ranks) X(flags) X(reserve) X(instance)   \
   X(panoptic) X(_isthing_u8) X(_side) X(cuda_stream) X(desc) X(descs) X(d_off) X(g_off) X(pair_off)             \
-  X(total_chunks) X(id) X(category_id) X(iscrowd)
+  X(total_chunks) X(id) X(category_id) X(iscrowd) X(flat) X(_layout)
 
 struct Names {
 #define X(name) PyObject* name = nullptr;
@@ -1417,38 +1418,50 @@ PyObject* prefixes(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// One part of a packed output (flat tensor, the field's element offset, its shape, is it double, index of the leading
-// dimensions ...): a view like those of the other results, or None.
+// prefix._part of PackedOutputs (outputs, row, field, further indices ...): a view like those of the other results.
 PyObject* part(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  constexpr Py_ssize_t kIndex = 4;
-  if (nargs < kIndex || !ordinary() || !PyTuple_CheckExact(args[2]) || !THPVariable_CheckExact(args[0])) return none();
-  const Tensor& base = THPVariable_Unpack(args[0]);
-  if (!plain(args[0], base.is_cuda() ? base.get_device() : kHostOnly) || base.scalar_type() != at::kLong ||
-      base.storage_offset())
-    return none();
-  const Py_ssize_t dims = PyTuple_GET_SIZE(args[2]), leading = nargs - kIndex;
-  int64_t offset = PyLong_AsLongLong(args[1]), numel = 1, count = 1;
-  bool inside = offset >= 0 && leading <= dims;
-  std::vector<int64_t> sizes(dims);
-  for (Py_ssize_t k = dims - 1; k >= 0; --k) {
-    sizes[k] = PyLong_AsLongLong(PyTuple_GET_ITEM(args[2], k));
-    if (k < leading) {
-      const int64_t i = PyLong_AsLongLong(args[kIndex + k]);
-      inside = inside && i >= 0 && i < sizes[k];
-      offset += i * numel;
-    } else {
-      count *= sizes[k];
+  if (nargs < 3) {
+    PyErr_SetString(PyExc_TypeError, "part(outputs, row, field, *index)");
+    return nullptr;
+  }
+  Ref flat = attr(args[0], names.flat), layout = attr(args[0], names._layout);
+  PyObject* entry = layout && PyDict_CheckExact(layout.p) ? PyDict_GetItemWithError(layout.p, args[2]) : nullptr;
+  PyObject* shape = entry && PyTuple_CheckExact(entry) && PyTuple_GET_SIZE(entry) == 3 ? PyTuple_GET_ITEM(entry, 1) : nullptr;
+  const Py_ssize_t leading = nargs - 2, dims = shape && PyTuple_CheckExact(shape) ? PyTuple_GET_SIZE(shape) : 0;
+  constexpr Py_ssize_t kMost = 4;
+  if (flat && THPVariable_CheckExact(flat.p) && leading <= dims && dims <= kMost && ordinary() &&
+      THPDtype_Check(PyTuple_GET_ITEM(entry, 2))) {
+    const Tensor& base = THPVariable_Unpack(flat.p);
+    int64_t offset = PyLong_AsLongLong(PyTuple_GET_ITEM(entry, 0)), numel = 1, count = 1, sizes[kMost];
+    bool inside = offset >= 0;
+    for (Py_ssize_t k = dims - 1; k >= 0; --k) {
+      sizes[k] = PyLong_AsLongLong(PyTuple_GET_ITEM(shape, k));
+      if (k < leading) {
+        const int64_t i = PyLong_AsLongLong(k ? args[k + 2] : args[1]);
+        inside = inside && i >= 0 && i < sizes[k];
+        offset += i * numel;
+      } else {
+        count *= sizes[k];
+      }
+      numel *= sizes[k];
     }
-    numel *= sizes[k];
+    const at::ScalarType type = reinterpret_cast<THPDtype*>(PyTuple_GET_ITEM(entry, 2))->scalar_type;
+    if (!PyErr_Occurred() && inside && count >= 0 && plain(flat.p, base.is_cuda() ? base.get_device() : kHostOnly) &&
+        base.scalar_type() == at::kLong && base.storage_offset() == 0 && offset + count <= base.numel() &&
+        (type == at::kLong || type == at::kDouble))
+      return view(base, 8 * offset, type, at::IntArrayRef(sizes + leading, dims - leading));
   }
-  if (PyErr_Occurred()) {
-    PyErr_Clear();
-    return none();
+  PyErr_Clear();
+  // Anything else: outputs[field][row, index ...].
+  Ref field(PyObject_GetItem(args[0], args[2])), index(PyTuple_New(leading));
+  if (!field || !index) return nullptr;
+  for (Py_ssize_t k = 0; k < leading; ++k) {
+    PyObject* i = k ? args[k + 2] : args[1];
+    Py_INCREF(i);
+    PyTuple_SET_ITEM(index.p, k, i);
   }
-  if (!inside || count < 0 || offset + count > base.numel()) return none();
-  return view(base, 8 * offset, args[3] == Py_True ? at::kDouble : at::kLong,
-              at::IntArrayRef(sizes.data() + leading, dims - leading));
+  return PyObject_GetItem(field.p, index.p);
   END_HANDLE_TH_ERRORS
 }
 

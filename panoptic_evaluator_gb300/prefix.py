@@ -94,15 +94,20 @@ def _output_layout(R, T, C):
     return cached
 
 
+def _part(out, row, key, *index):
+    """A view of out[key][row, index] alone: reading one checkpoint costs the same however many there are."""
+    return out[key][(row, *index)]
+
+
 class PackedOutputs(Mapping):
     """pe_prefix's outputs: named views of one int64 allocation, each made on first access and kept."""
 
-    __slots__ = ("flat", "_layout", "_views", "_part")
+    __slots__ = ("flat", "_layout", "_views", "part")
 
     def __init__(self, flat, layout):
         self.flat, self._layout, self._views = flat, layout, {}
         host = N.host()
-        self._part = host.part if host is not None else None
+        self.part = host.part if host is not None else _part  # called with these outputs first
 
     def __getitem__(self, key):
         view = self._views.get(key)
@@ -111,12 +116,6 @@ class PackedOutputs(Mapping):
             part = self.flat[offset: offset + math.prod(shape)]
             view = self._views[key] = (part if dtype is torch.int64 else part.view(dtype)).view(shape)
         return view
-
-    def at(self, row, key, *index):
-        """A view of field[row, index] alone: reading one checkpoint costs the same however many there are."""
-        offset, shape, dtype = self._layout[key]
-        view = self._part and self._part(self.flat, offset, shape, dtype is torch.float64, row, *index)
-        return self[key][(row, *index)] if view is None else view
 
     def __iter__(self):
         return iter(self._layout)
@@ -221,10 +220,6 @@ _METRICS = ("pq", "sq", "rq", "iou")
 _ROW_FIELDS = {"tp": "tp", "fp": "fp", "fn": "fn", "iou_sum": "sums", "confusion": "confusion", "miou": "miou"}
 
 
-def _part_of(out, row, key, *index):
-    return out[key][(row, *index)]
-
-
 class Snapshot(Mapping):
     """One checkpoint's result dict (prefix.py:125-142), built lazily from the call's packed outputs.
 
@@ -250,7 +245,7 @@ class Snapshot(Mapping):
         if key in cache:
             return cache[key]
         out = self._out
-        row = partial(out.at, self._row) if type(out) is PackedOutputs else partial(_part_of, out, self._row)
+        row = partial(out.part if type(out) is PackedOutputs else _part, out, self._row)
         if key == "prefix":
             value = self._prefix
         elif key in _ROW_FIELDS:

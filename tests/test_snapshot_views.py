@@ -85,4 +85,4 @@ def test_every_view_can_be_changed_in_place(outputs):
 def test_an_index_outside_the_field_is_refused(outputs):
     for row, *index in ((ROWS,), (0, C), (0, 0, 0)):
         with pytest.raises(IndexError):
-            outputs.at(row, "tp", *index)
+            outputs.part(outputs, row, "tp", *index)
