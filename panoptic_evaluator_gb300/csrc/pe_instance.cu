@@ -500,11 +500,6 @@ __device__ __forceinline__ int64_t recall_reached_at(int64_t np, int r) {
   return t + (t * 100 == scaled && !exact_ok ? 1 : 0);
 }
 
-// Precision and recall of a class without positives: -1, or NaN where their number is unknown (kUnknownCount).
-__device__ __forceinline__ double without_curve(int64_t positives) {
-  return positives < 0 ? __longlong_as_double(0x7ff8000000000000ll) : -1.0;
-}
-
 // 10 / kT CTAs per class. `scores` == nullptr means the records are already in
 // global descending-score order. Records: classes[n], ranks[n] and flags at
 // flags[chain * chain_stride + record * det_stride]; list / cursor / hist: the
@@ -542,6 +537,7 @@ struct AccShared {
   int tp_min[4][101];
   int nseg[kChainsHere], hi[kChainsHere], tp[kChainsHere], off[kChainsHere + 1];
   int64_t npos[4];
+  double none[4];  // precision where the curve has none: 0, or -1 without positives, NaN with kUnknownCount
   int count, before;
 };
 
@@ -565,7 +561,11 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
   const unsigned below = (1u << lane) - 1u;
   // The second launch reads the count that the first one found: usually it has nothing to do (5.3 -> 3.0 us).
   if (above >= 0 && hist[c] <= above) return;
-  if (threadIdx.x < 4) sm.npos[threadIdx.x] = positives[c * 4 + threadIdx.x];
+  if (threadIdx.x < 4) {
+    const int64_t np = positives[c * 4 + threadIdx.x];
+    sm.npos[threadIdx.x] = np;
+    sm.none[threadIdx.x] = np > 0 ? 0.0 : (np < 0 ? __longlong_as_double(0x7ff8000000000000ll) : -1.0);
+  }
   // Records of this class, and of the classes before it (where its workspace regions start).
   int count, before;
   if (list) {
@@ -770,10 +770,10 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
       if (lane < kChainsHere) {
         const int a = (lane / 3) % 4, t = t_base + lane / 12;
         const int64_t np = sm.npos[a];
-        const double rc = np > 0 ? (double)sm.tp[lane] / (double)np : without_curve(np);
+        const double rc = np > 0 ? (double)sm.tp[lane] / (double)np : sm.none[a];
         recall[((int64_t)t * C + c) * 12 + lane % 12] = rc;
         if (chain_stats) {
-          double sum = np > 0 ? 0.0 : without_curve(np);
+          double sum = sm.none[a];
           const int nseg = sm.nseg[lane], hi = sm.hi[lane];
           for (int k = 0; k < nseg; ++k) {
             const int end = k + 1 < nseg ? sm.seg_lo[lane][k + 1] : hi;
@@ -787,7 +787,7 @@ accumulate_kernel(const int* __restrict__ classes, int64_t n, const int* __restr
     } else {
       for (int e = threadIdx.x; e < kChainsHere * 101; e += kAccThreads - 32) {
         const int k = e % 12, r = (e / 12) % 101, t = e / (12 * 101), ch = t * 12 + k;
-        double v = sm.npos[k / 3] > 0 ? 0.0 : without_curve(sm.npos[k / 3]);
+        double v = sm.none[k / 3];
         if (r < sm.hi[ch]) {
           int lo = 0, hi = sm.nseg[ch] - 1;  // the last segment starting at or before r
           while (lo < hi) {
