@@ -232,8 +232,8 @@ int pe_seg_pass(const int64_t* descs, int64_t B, int64_t total_chunks, const int
                 int64_t pairs_len, uint32_t* dpairs, int64_t dpairs_len, int64_t pan_cap, int64_t det_cap,
                 int bulk, const int64_t* cta_bounds, int64_t ctas, uint64_t* schedule, int32_t* error,
                 cudaStream_t stream);
-/* max_p: largest P of the batch; max_pairs: largest G x P (each image's histogram is staged in shared
- * memory when the largest fits 100 KB, else read in place; the results are the same). class_bits
+/* max_p: largest P of the batch; max_pairs: largest G x P (they size the shared tables and entry list of an
+ * image; one that does not fit them is scored in place; the results are the same). class_bits
  * (optional, B x ceil(C / 32) u32): each image's classes with detections or thing targets, for
  * pe_seg_match (a detection class outside [0, C) marks class 0). Where a kernel before it gave up (*error
  * has a bit from 2^20 on: a wait ran out), validate = 0 counts nothing and makes the dataset IoU sums NaN. */

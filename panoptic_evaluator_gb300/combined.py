@@ -1,9 +1,10 @@
 """Joint PQ/mIoU and mask AP/AR with one shared panoptic target (API of the reference's combined.py).
 
-One ``update`` over a batch is five launches, independent of the number of
-images: per-image score sort, one fused pass over the pixels (panoptic pair
-histogram + detection x target-slot histogram), per-image scoring (areas and
-validation, then PQ/confusion accumulation), and batched COCO matching. With
+One ``update`` over a batch is a fixed number of launches, independent of the
+number of images: per-image score sort, clearing the counts, one fused pass over
+the pixels (panoptic pair histogram + detection x target-slot histogram),
+per-image scoring (once, or with validation once for areas and checks and once
+for PQ/confusion) and batched COCO matching. With
 ``validate=False`` nothing synchronises with the host, so an update can be
 captured in a CUDA graph.
 """
@@ -134,7 +135,7 @@ class SegmentationEvaluator:
         """Accumulate a batch of uneven images packed in a ``ragged.SegmentationImages`` arena.
 
         The arena's descriptor table is reused, so with ``validate=False`` this
-        call launches the same five kernels with the same pointers every time
+        call launches the same kernels with the same pointers every time
         and can be captured in a CUDA graph.
         """
         if images.device.device != self.device:

@@ -5,8 +5,10 @@
 // 40-400 us. Each function here takes the whole step for plain arguments: lists or tuples of ordinary
 // contiguous tensors of the usual types on the current device, with no dispatch mode or transform active.
 // For anything else it returns None before it has changed or launched anything, and the caller takes the
-// general Python path, which converts what can be converted and raises what has to be raised. Both paths
-// fill the same tables and make the same C ABI calls.
+// general Python path, which converts what can be converted and raises what has to be raised. Both fill the
+// same tables. Instance and joint updates differ in their launches: here gathering, sorting, sampling and
+// clearing are one (pe_inst_begin), masks may be streamed and an unchecked update matches from the pixel
+// counts; the Python path gathers, sorts, contracts and prepares by a launch each. The results are the same.
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
@@ -775,7 +777,7 @@ PyObject* instance_update(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int64_t crowd_at = l.add(G), ann_in_at = l.add(8 * G), order_at = l.add(8 * D), sort_at = l.add(sort_bytes);
   const int64_t pa_d_at = l.add(8 * D), ga_d_at = l.add(8 * G), ann_at = l.add(8 * G);
   const int64_t bits_at = l.add(4 * B * ((*C + 31) / 32)), stream_at = l.add(8 * (8 * B + 1));
-  // Intersections, the error word, then both area counters, without gaps: the contraction clears them at once.
+  // Intersections, the error word, then both area counters, without gaps: pe_inst_begin clears them at once.
   const int64_t inter_len = round_up(p.pairs, 2) + 2, counts_at = l.add(4 * inter_len + 8 * (D + G));
   Tensor work = arena(self, index, l.size);
   work.narrow(0, table_at, 8 * p.words).copy_(p.host.narrow(0, 0, 8 * p.words), /*non_blocking=*/true);
@@ -960,7 +962,7 @@ bool read_segmentation(PyObject* self, int index, int64_t detections, SegEvaluat
 }
 
 // Scratch of the fused pass and what follows it; the counts, the error word and the chunk counter have no
-// gaps between them, so the pass clears them with one memset.
+// gaps between them, so the pass clears them as one span.
 struct SegScratch {
   Layout layout;
   int64_t order, sort, sort_bytes, areas, matched, det_pa, slot_ga, slot_class, ann, bits, counted, dpairs_len;
@@ -1392,7 +1394,7 @@ PyObject* prefixes(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   out[0] = data<int64_t>(flat);
   for (int k = 0; k < 14; ++k) out[k + 1] = out[k] + sizes[k];
   auto f64 = [&](int k) { return reinterpret_cast<double*>(out[k]); };
-  // int32 workspaces back to back: ga, raw, pairs, counters, error (zeroed by the call).
+  // int32 workspaces back to back: ga, raw, pairs, counters (reserved), error (zeroed by the call).
   const int64_t raw_len = S * p.total_masks, counters_len = B * T * C * 2;
   Tensor work = at::empty({B * S + raw_len + p.cells + counters_len + 1}, on(index, at::kInt));
   uint32_t* ga = data<uint32_t>(work);

@@ -6,8 +6,8 @@ namespace pe {
 
 constexpr int kSampleParts = 8;  // CTAs that sample one image
 
-// inst_sample_kernel's estimate of the time that streaming would take (picoseconds, a few entries per image) and
-// the limit up to which it is the faster way. Both kernels read it, so exactly one of them does the work.
+// The sample's estimate of the time that streaming would take (sample_image in pe_pairs.cu: picoseconds, a few entries
+// per image) and the limit up to which it is the faster way. Both kernels read it, so exactly one of them does the work.
 struct Choice {
   const u64* costs;  // null: the contraction runs whatever the masks hold
   int64_t entries, limit;

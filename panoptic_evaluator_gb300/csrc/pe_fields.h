@@ -42,7 +42,7 @@ enum PrefixField : int {
   kPrefixRawBegin,     // offset of this image's [N][G] raw intersections
   kPrefixFlags,        // bit 0: target map 16-byte vectorisable, bit 1: mask rows 16-byte vectorisable
   kPrefixStepBegin,    // offset of this image's step table (N+1 entries: checkpoint index or -1)
-  kPrefixCountBegin,   // offset of this image's [T][C][2] matching counters
+  kPrefixCountBegin,   // reserved: offset of this image's [T][C][2] counters
   kPrefixFields
 };
 

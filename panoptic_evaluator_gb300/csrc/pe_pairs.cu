@@ -81,7 +81,7 @@ struct PairSample {
 
 // Estimates what streaming the image would take where the masks' content decides: costs[kSampleParts * image + part],
 // from the rows with pixels in a part's windows. The blocks behind those of the images clear the outputs and the
-// chunk counter (a memset before).
+// chunk counter.
 __device__ __forceinline__ void sample_image(const int64_t* descs, int64_t samples, int64_t block, const PairSample& a) {
   if (block >= samples) {
     const int64_t first = (block - samples) * kSampleThreads + threadIdx.x;
@@ -377,10 +377,10 @@ inst_pairs_kernel(const int64_t* __restrict__ descs, int64_t B, int64_t whole, i
 
 using namespace pe;
 
-// How long streaming a batch may take, in picoseconds by inst_sample_kernel's estimate, to be faster than its
+// How long streaming a batch may take, in picoseconds by the sample's estimate (sample_image), to be faster than its
 // contraction; 0: contract whatever the masks hold. Image b has dets[b] detection masks, gts[b] target masks and
-// pixels[b] pixels; tma (optional) marks the images that the contraction loads by TMA (as fast as the others);
-// sms: the device's SMs. Host side, no GPU work.
+// pixels[b] pixels; the fourth argument, the images that the contraction loads by TMA, is not read (they take as long
+// as the others); sms: the device's SMs. Host side, no GPU work.
 //
 // Times, from 640 x 640 and 637 x 640 images with 100 x 8 and 100 x 50 masks of 0.8 % of the image: the contraction
 // reads the rows of its tiles, with sixteen rows' worth of fixed work, at 5.6 TB/s, by TMA and staged; streaming reads
@@ -404,7 +404,8 @@ PE_API int64_t pe_stream_limit(const int64_t* dets, const int64_t* gts, const in
     streamed += (D * n + G) * P / kStreamed;
     chunks += std::ceil(P / kPairChunk);
   }
-  // Fewer chunks than CTAs leave SMs without one.
+  // Fewer chunks than CTAs: measured while a chunk was the smallest share of the work, before the last ones went out
+  // in parts (launch_counts), so batches of a few images stay with the contraction longer than they may have to.
   if (chunks > 0.0) streamed *= std::max(1.0, 2.0 * (double)sms / chunks);
   const double limit = contraction - kFixed;
   return streamed < limit ? (int64_t)std::min(limit, 9e18) : 0;
@@ -491,6 +492,7 @@ PE_API int pe_inst_counts(const int64_t* descs, int64_t B, int64_t pair_chunks, 
                        maps, limit, work, error, stream);
 }
 
+// For callers that gather and sort by themselves (updates launch pe_inst_begin and pe_inst_counts):
 // pe_inst_contract for a batch whose masks may be sparse: the same inputs, outputs and counts, streamed where
 // pe_stream_limit's `limit` and a sample of the masks say that this is faster. pair_chunks: 4096-pixel chunks of
 // the descriptor table (kChunkBegin); work: 8 B + 1 u64 of device scratch. Drop-in for the reference's

@@ -1,18 +1,20 @@
 // Panoptic quality, semantic confusion and per-image reward statistics.
 //
-// One update is three stream-ordered kernels with no host round trip:
-//   1. pair_histogram: one pass over the gt/pred segment maps. Each CTA owns a
+// One update is stream-ordered kernels with no host round trip (with
+// validation one, for the error word):
+//   1. slot_histogram (compact int32 maps) or pair_histogram (original IDs and
+//      int64 maps): one pass over the gt/pred segment maps. Each CTA owns a
 //      contiguous run of 4096-pixel tiles, keeps a privatised G x P uint32
 //      histogram in shared memory (global atomics when it does not fit), reads
-//      the int32 maps with 16-byte vector loads, combines equal keys of a
-//      thread's 8 pixels in registers and aggregates the last run across the
-//      warp (__match_any_sync + __reduce_add_sync) before the shared atomic.
-//   2. score (areas + validation): row/column sums of the histogram and the
-//      reference's value checks, written to the caller's `areas` scratch.
-//   3. score (accumulate): per prediction column the confusion contribution,
-//      the integer `inter > union / 2` match test, the FP64 IoU, the
-//      last-same-class-crowd ignore rule and FP/FN. Gated on the device by the
-//      error word, so a failed validation never changes the totals.
+//      the maps with 16-byte vector loads, counts equal keys of a thread's 8
+//      pixels in registers and those of the warp (__match_any_sync +
+//      __reduce_add_sync) before the shared atomic.
+//   2. score_blocks, or score where its tables do not fit: row/column sums of
+//      the histogram and, with validation, the reference's value checks; then
+//      the confusion contributions, the integer `inter > union / 2` match test,
+//      the FP64 IoU, the last-same-class-crowd ignore rule and FP/FN. With
+//      validation two launches: checks first, then accumulation gated on the
+//      device by the error word, so a failed validation never changes the totals.
 // The confusion matrix is derived from the same histogram (no second pixel
 // pass). Per-image class sums are reduced in a fixed order.
 #include "pe_common.cuh"

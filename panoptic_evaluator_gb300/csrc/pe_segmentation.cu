@@ -6,12 +6,12 @@
 //                     sorted scores/classes are written straight into the
 //                     caller's record store.
 //   2. seg_pass       ONE pass over the pixels: target+prediction slot maps
-//                     (16-byte loads) feed the privatised G x P pair histogram
-//                     and the same target slots bin every detection mask
-//                     (16-byte loads of 0/1 bytes, popcount per 16 pixels,
-//                     warp-uniform skip of empty rows). Persistent CTAs walk
-//                     contiguous runs of 8192-pixel chunks and flush their
-//                     shared-memory bins only when the image changes.
+//                     (16-byte loads) feed the G x P pair histogram and the
+//                     same target slots bin every detection mask (staged rows
+//                     of 0/1 bytes, popcount per 16 pixels, warp-uniform skip
+//                     of rows without a pixel). Persistent CTAs take halves of
+//                     8192-pixel chunks from a counter; counts are summed over
+//                     the warp and go to memory as reductions.
 //   3. seg_score      per image: areas and validation, then (gated on the
 //                     device error word) PQ/confusion accumulation and the
 //                     detection areas / thing-class targets for matching.

@@ -1,9 +1,9 @@
 """Generation-order prefix evaluation on the GPU (API of the reference's ``prefix.py``).
 
 ``segmentation_prefixes`` evaluates every image of the batch with one
-``pe_prefix`` call (five launches in total): a single pass over each image's
-target map and mask bytes, a scan, per-checkpoint canvas scoring, per-image
-greedy matching and the per-checkpoint summaries. Results are views of
+``pe_prefix`` call (five launches in total): clearing, a single pass over each
+image's target map and mask bytes, a scan, per-checkpoint canvas scoring beside
+greedy matching, and the per-checkpoint summaries. Results are views of
 device tensors, one list of snapshots per image; a snapshot makes the views of
 its fields when they are read.
 """
@@ -191,7 +191,8 @@ def run_prefixes(maps, gc, crowd, masks, classes, num_classes, isthing, threshol
     classes_flat = (torch.cat(classes).to(torch.int32) if total_masks
                     else torch.empty(0, dtype=torch.int32, device=dev))
     raw_len, pairs_len = S * total_masks, int(cells.sum())
-    # int32 workspaces, one allocation: ga [B x S], raw, pairs, counters [B x T x C x 2], error (zeroed by the call).
+    # int32 workspaces, one allocation: ga [B x S], raw, pairs, counters [B x T x C x 2] (reserved), error (zeroed by
+    # the call).
     work = (B * S, max(raw_len, 1), max(pairs_len, 1), B * T * C * 2, 1)
     workspace = torch.empty(sum(work), dtype=torch.int32, device=dev)  # referenced until the call is queued
     ints = workspace.data_ptr()
