@@ -102,12 +102,10 @@ def _part(out, row, key, *index):
 class PackedOutputs(Mapping):
     """pe_prefix's outputs: named views of one int64 allocation, each made on first access and kept."""
 
-    __slots__ = ("flat", "_layout", "_views", "part")
+    __slots__ = ("flat", "_layout", "_views")
 
     def __init__(self, flat, layout):
         self.flat, self._layout, self._views = flat, layout, {}
-        host = N.host()
-        self.part = host.part if host is not None else _part  # called with these outputs first
 
     def __getitem__(self, key):
         view = self._views.get(key)
@@ -246,7 +244,8 @@ class Snapshot(Mapping):
         if key in cache:
             return cache[key]
         out = self._out
-        row = partial(out.part if type(out) is PackedOutputs else _part, out, self._row)
+        host = N.host() if type(out) is PackedOutputs else None
+        row = partial(_part if host is None else host.part, out, self._row)
         if key == "prefix":
             value = self._prefix
         elif key in _ROW_FIELDS:

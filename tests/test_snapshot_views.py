@@ -1,5 +1,8 @@
 """A checkpoint's result views: independent of one another, as many as are read."""
 
+import copy
+import pickle
+
 import pytest
 import torch
 from torch.utils._python_dispatch import TorchDispatchMode
@@ -83,6 +86,13 @@ def test_every_view_can_be_changed_in_place(outputs):
 
 
 def test_an_index_outside_the_field_is_refused(outputs):
+    part = N.host().part if N.host() is not None else P._part
     for row, *index in ((ROWS,), (0, C), (0, 0, 0)):
         with pytest.raises(IndexError):
-            outputs.part(outputs, row, "tp", *index)
+            part(outputs, row, "tp", *index)
+
+
+def test_a_snapshot_can_be_copied_and_pickled(outputs):
+    snapshot = _snapshots(outputs)[3]
+    for again in (pickle.loads(pickle.dumps(snapshot)), copy.deepcopy(snapshot)):
+        assert torch.equal(again["confusion"], snapshot["confusion"])
