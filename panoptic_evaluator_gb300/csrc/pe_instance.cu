@@ -870,7 +870,7 @@ summarize_chains_kernel(const double* __restrict__ chain_stats, int C, double* _
   }
 }
 
-// The 12 COCO summaries (instance.py:230-248): means of the entries >= 0 (NaN as soon as one is).
+// The 12 COCO summaries (instance.py:230-248): means of the entries >= 0.
 __global__ void __launch_bounds__(256)
 summarize_kernel(const double* __restrict__ precision, const double* __restrict__ recall, int C,
                  double* __restrict__ out) {
@@ -892,7 +892,7 @@ summarize_kernel(const double* __restrict__ precision, const double* __restrict_
       for (int64_t e = threadIdx.x; e < total; e += blockDim.x) {
         const int64_t t = t0 + e / per_t, rc = e % per_t;  // rc = r * C + c
         const double v = precision[((t * 101 * C + rc) * 4 + area) * 3 + 2];
-        if (!(v < 0)) { sum += v; ++cnt; }
+        if (v >= 0) { sum += v; ++cnt; }
       }
     } else {
       int area = 0, mi = 2;
@@ -903,7 +903,7 @@ summarize_kernel(const double* __restrict__ precision, const double* __restrict_
       const int64_t total = (int64_t)10 * C;
       for (int64_t e = threadIdx.x; e < total; e += blockDim.x) {
         const double v = recall[(e * 4 + area) * 3 + mi];
-        if (!(v < 0)) { sum += v; ++cnt; }
+        if (v >= 0) { sum += v; ++cnt; }
       }
     }
     s_sum[threadIdx.x] = sum;
